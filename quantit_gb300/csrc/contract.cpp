@@ -391,6 +391,188 @@ void split_operand(const BT &t, const std::vector<int64_t> &perm, int nrow, std:
 }
 }  // namespace
 
+namespace {
+// Legs of one block with their strides in that block, folded: legs of size 1 dropped and
+// neighbours merged wherever the outer stride is the inner extent times the inner stride
+// (of both operands, for the contracted legs).  At most two groups (outer, inner) remain,
+// or the block does not fold.
+struct Fold {
+    int64_t d1 = 1, d2 = 1;          // extents, outer and inner
+    int64_t x1 = 0, x2 = 0;          // strides of the first operand
+    int64_t y1 = 0, y2 = 0;          // strides of the second (contracted legs)
+};
+struct FoldLeg {
+    int64_t d, x, y;
+};
+bool fold_legs(const FoldLeg *legs, int n, Fold &f) {
+    FoldLeg g[MAXRANK];
+    int k = 0;
+    for (int i = 0; i < n; ++i) {
+        const FoldLeg &l = legs[i];
+        if (l.d == 1) continue;
+        if (k && g[k - 1].x == l.d * l.x && g[k - 1].y == l.d * l.y)
+            g[k - 1] = FoldLeg{g[k - 1].d * l.d, l.x, l.y};
+        else
+            g[k++] = l;
+    }
+    if (k > 2) return false;
+    f = Fold();
+    if (k == 2) {
+        f.d1 = g[0].d;
+        f.x1 = g[0].x;
+        f.y1 = g[0].y;
+    }
+    if (k) {
+        f.d2 = g[k - 1].d;
+        f.x2 = g[k - 1].x;
+        f.y2 = g[k - 1].y;
+    }
+    return true;
+}
+
+struct Strided {
+    int64_t d[MAXRANK], s[MAXRANK];
+};
+Strided block_strides(const BT &t, int64_t b) {
+    Strided r;
+    t.block_shape(b, r.d);
+    int64_t s = 1;
+    for (int i = t.rank - 1; i >= 0; --i) {
+        r.s[i] = s;
+        s *= r.d[i];
+    }
+    return r;
+}
+
+// Pair descriptors that read both operands where they lie; false when a block's legs do
+// not fold to two strides or a stride exceeds 32 bits (the caller packs the operands).
+bool f64_pairs_in_place(const ContractPlan &P, const BT &A, const BT &B, std::vector<F64Pair> &out) {
+    auto fits = [](int64_t v) { return v <= INT32_MAX; };
+    std::vector<Strided> sa(A.nblocks()), sb(B.nblocks());
+    std::vector<Fold> fa(A.nblocks()), fb(B.nblocks());
+    auto free_legs = [&](const BT &t, const std::vector<int64_t> &legs, std::vector<Strided> &st, std::vector<Fold> &fo) {
+        for (int64_t b = 0; b < t.nblocks(); ++b) {
+            st[b] = block_strides(t, b);
+            FoldLeg l[MAXRANK];
+            int n = 0;
+            for (auto d : legs) l[n++] = FoldLeg{st[b].d[d], st[b].s[d], 0};
+            if (!fold_legs(l, n, fo[b])) return false;
+            if (!fits(fo[b].d2) || !fits(fo[b].x1) || !fits(fo[b].x2)) return false;
+        }
+        return true;
+    };
+    if (!free_legs(A, P.freeA, sa, fa) || !free_legs(B, P.freeB, sb, fb)) return false;
+    out.resize(P.pair_a.size());
+    for (size_t k = 0; k < out.size(); ++k) {
+        const int64_t ia = P.pair_a[k], ib = P.pair_b[k];
+        FoldLeg l[MAXRANK];
+        int n = 0;
+        for (size_t i = 0; i < P.dA.size(); ++i)
+            l[n++] = FoldLeg{sa[ia].d[P.dA[i]], sa[ia].s[P.dA[i]], sb[ib].s[P.dB[i]]};
+        Fold c;
+        if (!fold_legs(l, n, c)) return false;
+        if (!fits(c.d1) || !fits(c.d2) || !fits(c.x1) || !fits(c.x2) || !fits(c.y1) || !fits(c.y2)) return false;
+        F64Pair &p = out[k];
+        p.a_off = A.boff[ia];
+        p.b_off = B.boff[ib];
+        p.k1 = int32_t(c.d1);
+        p.k2 = int32_t(c.d2);
+        p.ak1 = int32_t(c.x1);
+        p.ak2 = int32_t(c.x2);
+        p.bk1 = int32_t(c.y1);
+        p.bk2 = int32_t(c.y2);
+        p.am2 = int32_t(std::max<int64_t>(fa[ia].d2, 1));
+        p.as1 = int32_t(fa[ia].x1);
+        p.as2 = int32_t(fa[ia].x2);
+        p.bn2 = int32_t(std::max<int64_t>(fb[ib].d2, 1));
+        p.bs1 = int32_t(fb[ib].x1);
+        p.bs2 = int32_t(fb[ib].x2);
+    }
+    return true;
+}
+
+void contract_f64(const ContractPlan &P, const BT &A, const BT &B, BT &out, const BT *add, double beta, double alpha,
+                  const std::vector<GemmOut> &outs, double flops) {
+    std::vector<F64Pair> pairs;
+    BufPtr pa, pb;
+    const double *Ap = static_cast<const double *>(A.data());
+    const double *Bp = static_cast<const double *>(B.data());
+    if (!f64_pairs_in_place(P, A, B, pairs)) {
+        // matrix form: an operand that is neither (free x contracted) nor its transpose is packed
+        std::vector<int64_t> offa, offb;
+        const std::vector<int64_t> *oa = &A.boff, *ob = &B.boff;
+        if (P.a_mode == 2) {
+            pa = pack_operand(A, P.p1, offa);
+            Ap = static_cast<const double *>(pa->p);
+            oa = &offa;
+        }
+        if (P.b_mode == 2) {
+            pb = pack_operand(B, P.p2, offb);
+            Bp = static_cast<const double *>(pb->p);
+            ob = &offb;
+        }
+        pairs.resize(P.pair_a.size());
+        for (size_t k = 0; k < pairs.size(); ++k) {
+            const int64_t ia = P.pair_a[k], ib = P.pair_b[k];
+            const int64_t M = prod_sizes(A, ia, P.freeA), N = prod_sizes(B, ib, P.freeB), K = prod_sizes(A, ia, P.dA);
+            if (M > INT32_MAX || N > INT32_MAX || K > INT32_MAX) fail(ERR_INVALID_ARGUMENT, "block too large");
+            F64Pair &p = pairs[k];
+            std::memset(&p, 0, sizeof(p));
+            p.a_off = (*oa)[ia];
+            p.b_off = (*ob)[ib];
+            p.k1 = 1;
+            p.k2 = int32_t(K);
+            p.am2 = int32_t(std::max<int64_t>(M, 1));
+            p.bn2 = int32_t(std::max<int64_t>(N, 1));
+            p.as2 = int32_t(P.a_mode == 1 ? 1 : K);
+            p.ak2 = int32_t(P.a_mode == 1 ? M : 1);
+            p.bs2 = int32_t(P.b_mode == 1 ? K : 1);
+            p.bk2 = int32_t(P.b_mode == 1 ? 1 : N);
+        }
+    }
+    // 32 x 32 tiles unless they would leave most SMs without one
+    auto square_tiles = [&]() {
+        int64_t n = 0;
+        for (const GemmOut &o : outs) n += ((int64_t(o.M) + 31) / 32) * ((int64_t(o.N) + 31) / 32);
+        return n;
+    };
+    const bool fine = square_tiles() < 4 * device_sm_count();
+    std::vector<std::pair<double, GemmTile>> wt;
+    for (size_t o = 0; o < outs.size(); ++o) {
+        double ksum = 0;
+        int64_t kmax = 0;
+        for (int32_t p = outs[o].p0; p < outs[o].p1; ++p) {
+            const int64_t K = int64_t(pairs[p].k1) * pairs[p].k2;
+            ksum += double(K);
+            kmax = std::max(kmax, K);
+        }
+        int tm, tn;
+        const int cls = gemm_f64_class(outs[o].M, outs[o].N, kmax, &tm, &tn, fine);
+        for (int64_t m0 = 0; m0 < outs[o].M; m0 += tm)
+            for (int64_t n0 = 0; n0 < outs[o].N; n0 += tn)
+                wt.push_back({ksum, GemmTile{int32_t(o), int32_t(m0), int32_t(n0), cls}});
+    }
+    // longest tiles first: the tail of the grid is made of the cheap ones
+    std::stable_sort(wt.begin(), wt.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
+    std::vector<GemmTile> tiles;
+    tiles.reserve(wt.size());
+    for (auto &w : wt) tiles.push_back(w.second);
+    F64Args g;
+    g.A = Ap;
+    g.B = Bp;
+    g.C = static_cast<double *>(out.data());
+    g.Cadd = add ? static_cast<const double *>(add->data()) : nullptr;
+    g.pairs = upload_vec(pairs);
+    g.outs = upload_vec(outs);
+    g.tiles = upload_vec(tiles);
+    g.ntiles = int32_t(tiles.size());
+    g.alpha = alpha;
+    g.beta = beta;
+    StatScope sc(ST_GEMM, flops);
+    launch_gemm_f64(g);
+}
+}  // namespace
+
 void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, const BT *add, double beta,
                      double alpha, const std::vector<int64_t> *add_block) {
     require_f64(A);
@@ -398,51 +580,10 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
     const int64_t nout = int64_t(P.out_p0.size());
     if (nout == 0) return;
     const int mode = gemm_mode();
-    const bool tc = mode != GEMM_F64;
-    // operand buffers
-    BufPtr pa, pb, ahi, amid, alo, bhi, bmid, blo, amax;
-    std::vector<int64_t> offa, offb;
-    const double *Ap = static_cast<const double *>(A.data());
-    const double *Bp = static_cast<const double *>(B.data());
-    const std::vector<int64_t> *oa = &A.boff, *ob = &B.boff;
-    int a_t = 0, b_t = 0;
-    if (tc) {
-        amax = dev_alloc(2 * sizeof(unsigned long long));
-        cuda_check(cudaMemsetAsync(amax->p, 0, 2 * sizeof(unsigned long long), ctx().stream), "cudaMemsetAsync(amax)");
-        auto *am = static_cast<unsigned long long *>(amax->p);
-        split_operand(A, P.p1, int(P.freeA.size()), offa, ahi, amid, alo, am, mode);
-        split_operand(B, P.p2p, int(P.freeB.size()), offb, bhi, bmid, blo, am + 1, mode);
-        oa = &offa;
-        ob = &offb;
-    } else {
-        if (P.a_mode == 1) a_t = 1;
-        if (P.a_mode == 2) {
-            pa = pack_operand(A, P.p1, offa);
-            Ap = static_cast<const double *>(pa->p);
-            oa = &offa;
-        }
-        if (P.b_mode == 1) b_t = 1;
-        if (P.b_mode == 2) {
-            pb = pack_operand(B, P.p2, offb);
-            Bp = static_cast<const double *>(pb->p);
-            ob = &offb;
-        }
-    }
-    const int TM = tc ? gemm_tile_m(mode) : 64;
-    const int TN = tc ? gemm_tile_n(mode) : 64;
-    std::vector<GemmPair> pairs(P.pair_a.size());
+    std::vector<int64_t> Ks(P.pair_a.size());
+    for (size_t k = 0; k < Ks.size(); ++k) Ks[k] = prod_sizes(A, P.pair_a[k], P.dA);
     std::vector<GemmOut> outs(nout);
-    std::vector<GemmTile> tiles;
     double flops = 0;
-    for (int64_t k = 0; k < int64_t(P.pair_a.size()); ++k) {
-        int64_t ia = P.pair_a[k], ib = P.pair_b[k];
-        pairs[k].a_off = (*oa)[ia];
-        pairs[k].b_off = (*ob)[ib];
-        pairs[k].K = int32_t(prod_sizes(A, ia, P.dA));
-        pairs[k].pad = 0;
-    }
-    std::vector<std::pair<double, GemmTile>> wt;
-    int64_t max_chunks = 0;
     for (int64_t o = 0; o < nout; ++o) {
         int64_t ia = P.pair_a[P.out_p0[o]], ib = P.pair_b[P.out_p0[o]];
         int64_t M = prod_sizes(A, ia, P.freeA), N = prod_sizes(B, ib, P.freeB);
@@ -454,62 +595,68 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
         outs[o].p0 = int32_t(P.out_p0[o]);
         outs[o].p1 = int32_t(P.out_p1[o]);
         double ksum = 0;
+        for (int64_t p = P.out_p0[o]; p < P.out_p1[o]; ++p) ksum += double(Ks[p]);
+        flops += 2.0 * double(M) * double(N) * ksum;
+    }
+    if (mode == GEMM_F64) {
+        contract_f64(P, A, B, out, add, beta, alpha, outs, flops);
+        return;
+    }
+    BufPtr ahi, amid, alo, bhi, bmid, blo, amax;
+    std::vector<int64_t> offa, offb;
+    amax = dev_alloc(2 * sizeof(unsigned long long));
+    cuda_check(cudaMemsetAsync(amax->p, 0, 2 * sizeof(unsigned long long), ctx().stream), "cudaMemsetAsync(amax)");
+    auto *am = static_cast<unsigned long long *>(amax->p);
+    split_operand(A, P.p1, int(P.freeA.size()), offa, ahi, amid, alo, am, mode);
+    split_operand(B, P.p2p, int(P.freeB.size()), offb, bhi, bmid, blo, am + 1, mode);
+    const int TM = gemm_tile_m(mode), TN = gemm_tile_n(mode);
+    std::vector<GemmPair> pairs(P.pair_a.size());
+    for (size_t k = 0; k < pairs.size(); ++k) {
+        pairs[k].a_off = offa[P.pair_a[k]];
+        pairs[k].b_off = offb[P.pair_b[k]];
+        pairs[k].K = int32_t(Ks[k]);
+        pairs[k].pad = 0;
+    }
+    std::vector<std::pair<double, GemmTile>> wt;
+    int64_t max_chunks = 0;
+    for (int64_t o = 0; o < nout; ++o) {
+        double ksum = 0;
         int64_t chunks = 0;
-        for (int64_t p = P.out_p0[o]; p < P.out_p1[o]; ++p) {
+        for (int32_t p = outs[o].p0; p < outs[o].p1; ++p) {
             ksum += pairs[p].K;
             // K chunks of the tensor-core kernels: 32 TF32 (K padded to 8) / 64 BF16 (to 16)
             chunks += mode == GEMM_BF16X3 ? (((pairs[p].K + 15) & ~15) + 63) / 64 : (((pairs[p].K + 7) & ~7) + 31) / 32;
         }
         max_chunks = std::max(max_chunks, chunks);
-        flops += 2.0 * double(M) * double(N) * ksum;
-        for (int64_t m0 = 0; m0 < M; m0 += TM)
-            for (int64_t n0 = 0; n0 < N; n0 += TN)
+        for (int64_t m0 = 0; m0 < outs[o].M; m0 += TM)
+            for (int64_t n0 = 0; n0 < outs[o].N; n0 += TN)
                 wt.push_back({ksum, GemmTile{int32_t(o), int32_t(m0), int32_t(n0), 0}});
     }
     // longest tiles first: the tail of the grid is made of the cheap ones
     std::stable_sort(wt.begin(), wt.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
+    std::vector<GemmTile> tiles;
     tiles.reserve(wt.size());
     for (auto &w : wt) tiles.push_back(w.second);
-    const GemmPair *dpairs = upload_vec(pairs);
-    const GemmOut *douts = upload_vec(outs);
-    const GemmTile *dtiles = upload_vec(tiles);
+    TcArgs g;
+    g.Ahi = ahi->p;
+    g.Amid = amid ? amid->p : nullptr;
+    g.Alo = alo->p;
+    g.Bhi = bhi->p;
+    g.Bmid = bmid ? bmid->p : nullptr;
+    g.Blo = blo->p;
+    g.amax_a = static_cast<const unsigned long long *>(amax->p);
+    g.amax_b = g.amax_a + 1;
+    g.C = static_cast<double *>(out.data());
+    g.Cadd = add ? static_cast<const double *>(add->data()) : nullptr;
+    g.pairs = upload_vec(pairs);
+    g.outs = upload_vec(outs);
+    g.tiles = upload_vec(tiles);
+    g.ntiles = int32_t(tiles.size());
+    g.max_chunks = int32_t(std::min<int64_t>(max_chunks, INT32_MAX));
+    g.alpha = alpha;
+    g.beta = beta;
     StatScope sc(ST_GEMM, flops);
-    if (!tc) {
-        GemmArgs g;
-        g.A = Ap;
-        g.B = Bp;
-        g.C = static_cast<double *>(out.data());
-        g.Cadd = add ? static_cast<const double *>(add->data()) : nullptr;
-        g.pairs = dpairs;
-        g.outs = douts;
-        g.tiles = dtiles;
-        g.ntiles = int32_t(tiles.size());
-        g.a_t = a_t;
-        g.b_t = b_t;
-        g.alpha = alpha;
-        g.beta = beta;
-        launch_gemm_f64(g);
-    } else {
-        TcArgs g;
-        g.Ahi = ahi->p;
-        g.Amid = amid ? amid->p : nullptr;
-        g.Alo = alo->p;
-        g.Bhi = bhi->p;
-        g.Bmid = bmid ? bmid->p : nullptr;
-        g.Blo = blo->p;
-        g.amax_a = static_cast<const unsigned long long *>(amax->p);
-        g.amax_b = g.amax_a + 1;
-        g.C = static_cast<double *>(out.data());
-        g.Cadd = add ? static_cast<const double *>(add->data()) : nullptr;
-        g.pairs = dpairs;
-        g.outs = douts;
-        g.tiles = dtiles;
-        g.ntiles = int32_t(tiles.size());
-        g.max_chunks = int32_t(std::min<int64_t>(max_chunks, INT32_MAX));
-        g.alpha = alpha;
-        g.beta = beta;
-        launch_gemm_tc(g, mode);
-    }
+    launch_gemm_tc(g, mode);
 }
 
 BT tensordot(const BT &a, const BT &b, const std::vector<int64_t> &da, const std::vector<int64_t> &db) {

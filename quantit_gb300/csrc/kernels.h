@@ -34,8 +34,6 @@ void launch_permute(const void *src, void *dst, const PermEntry *entries, const 
 // ------------------------------------------------------------ grouped GEMM
 // Output block o: C[o] (M x N row-major at c_off) = alpha * sum_{p in [p0,p1)} A_p B_p
 //                                                   + beta * Cadd (at add_off, when add_off >= 0).
-// A_p is M x K: row-major at a_off when a_t == 0, stored K x M row-major when a_t == 1.
-// B_p is K x N: row-major at b_off when b_t == 0, stored N x K row-major when b_t == 1.
 struct GemmPair {
     int64_t a_off, b_off;
     int32_t K;
@@ -47,21 +45,35 @@ struct GemmOut {
     int32_t p0, p1;
 };
 struct GemmTile {
-    int32_t out, m0, n0, pad;
+    int32_t out, m0, n0, cls;  // cls: tile class of the FP64 kernel (F64_*)
 };
-struct GemmArgs {
+// FP64 pair: the operands in place, rows, columns and K each folded to two strides:
+//   A(m, k) = A[a_off + (m / am2) as1 + (m % am2) as2 + (k / k2) ak1 + (k % k2) ak2],
+//   B(k, n) = B[b_off + (n / bn2) bs1 + (n % bn2) bs2 + (k / k2) bk1 + (k % k2) bk2],  K = k1 k2.
+struct __align__(16) F64Pair {
+    int64_t a_off, b_off;
+    int32_t k1, k2, ak1, ak2, bk1, bk2;
+    int32_t am2, as1, as2, bn2, bs1, bs2;
+};
+static_assert(sizeof(F64Pair) == 64, "the FP64 GEMM copies pair descriptors in 16-byte pieces");
+struct F64Args {
     const double *A;
     const double *B;
     double *C;
     const double *Cadd;
-    const GemmPair *pairs;
+    const F64Pair *pairs;
     const GemmOut *outs;
     const GemmTile *tiles;
     int32_t ntiles;
-    int32_t a_t, b_t;
     double alpha, beta;
 };
-void launch_gemm_f64(const GemmArgs &a);
+enum : int32_t { F64_SQUARE = 0, F64_SMALL = 1, F64_TALL = 2, F64_WIDE = 3 };
+constexpr int F64_STRIP = 8;  // rows or columns of the short side of a strip
+// The tile class of an M x N output block (K: the longest contracted length of its pairs)
+// and its tile extents; fine: 16 x 16 instead of 32 x 32 tiles (too few of the latter to
+// occupy the SMs).
+int gemm_f64_class(int64_t M, int64_t N, int64_t K, int *tm, int *tn, bool fine);
+void launch_gemm_f64(const F64Args &a);
 
 // Split-precision tensor-core variant (tcgen05).  Operands are first converted,
 // block by block, into "matrix form" split arrays: hi = tf32(x), lo = tf32(x - hi)
