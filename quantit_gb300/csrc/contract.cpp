@@ -321,77 +321,6 @@ int64_t prod_sizes(const BT &t, int64_t b, const std::vector<int64_t> &dims) {
 }  // namespace
 
 namespace {
-// Split every block of t (legs permuted by perm; the first nrow legs form the
-// rows, the rest the contracted K) into hi / lo TF32 arrays (TF32X3) or hi / mid / lo
-// BF16 arrays (BF16X3), tiled in the tensor cores' core matrices (8 rows x 16 bytes),
-// rows zero padded to 8 and K to the MMA's K step (8 TF32 / 16 BF16).
-void split_operand(const BT &t, const std::vector<int64_t> &perm, int nrow, std::vector<int64_t> &offs, BufPtr &hi,
-                   BufPtr &mid, BufPtr &lo, unsigned long long *amax, int mode) {
-    const bool bf16 = mode == GEMM_BF16X3;
-    const int64_t gran = bf16 ? 16 : 8;
-    const int r = t.rank;
-    const int64_t nb = t.nblocks();
-    offs.assign(nb, 0);
-    std::vector<SplitEntry> ents(nb);
-    std::vector<int64_t> lens(nb);
-    int64_t o = 0;
-    for (int64_t b = 0; b < nb; ++b) {
-        int64_t shp[MAXRANK], str[MAXRANK];
-        t.block_shape(b, shp);
-        int64_t s = 1;
-        for (int d = r - 1; d >= 0; --d) {
-            str[d] = s;
-            s *= shp[d];
-        }
-        SplitEntry &e = ents[b];
-        std::memset(&e, 0, sizeof(e));
-        int64_t rows = 1, K = 1;
-        for (int i = 0; i < r; ++i) {
-            e.dims[i] = shp[perm[i]];
-            e.stride[i] = str[perm[i]];
-            (i < nrow ? rows : K) *= shp[perm[i]];
-        }
-        if (K > INT32_MAX) fail(ERR_INVALID_ARGUMENT, "contracted dimension too large");
-        const int64_t K4 = (K + gran - 1) & ~(gran - 1);
-        e.src_off = t.boff[b];
-        e.dst_off = o;
-        e.rank = r;
-        e.K = int32_t(K);
-        e.K4 = int32_t(K4);
-        // index-math fast paths of the split kernels
-        bool contig = true;
-        int64_t sfx = 1;
-        for (int i = r - 1; i >= 0; --i) {
-            if (e.stride[i] != sfx && e.dims[i] != 1) contig = false;
-            sfx *= e.dims[i];
-        }
-        e.flags = (rows * K < int64_t(INT32_MAX) ? SPLIT_SMALL : 0) | (contig ? SPLIT_CONTIG : 0);
-        offs[b] = o;
-        lens[b] = rows * K;
-        o += ((rows + 7) & ~int64_t(7)) * K4;
-    }
-    const size_t bytes = size_t(std::max<int64_t>(o, 8)) * (bf16 ? sizeof(uint16_t) : sizeof(float));
-    std::vector<BufPtr *> parts = {&hi, &lo};
-    if (bf16) parts.push_back(&mid);
-    for (BufPtr *b : parts) {
-        *b = dev_alloc(bytes);
-        cuda_check(cudaMemsetAsync((*b)->p, 0, bytes, ctx().stream), "cudaMemsetAsync(split)");
-    }
-    auto chunks = make_chunks(lens);
-    const double nel = double(std::accumulate(lens.begin(), lens.end(), int64_t(0)));
-    StatScope sc(ST_PACK, (bf16 ? 14.0 : 16.0) * nel);
-    launch_amax(static_cast<const double *>(t.data()), t.nnz, amax);
-    if (bf16)
-        launch_split_bf16x3(static_cast<const double *>(t.data()), hi->p, mid->p, lo->p, upload_vec(ents),
-                            upload_vec(chunks), int64_t(chunks.size()), amax);
-    else
-        launch_split_tf32(static_cast<const double *>(t.data()), static_cast<float *>(hi->p),
-                          static_cast<float *>(lo->p), upload_vec(ents), upload_vec(chunks), int64_t(chunks.size()),
-                          amax);
-}
-}  // namespace
-
-namespace {
 // Legs of one block with their strides in that block, folded: legs of size 1 dropped and
 // neighbours merged wherever the outer stride is the inner extent times the inner stride
 // (of both operands, for the contracted legs).  At most two groups (outer, inner) remain,
@@ -491,8 +420,73 @@ bool f64_pairs_in_place(const ContractPlan &P, const BT &A, const BT &B, std::ve
     return true;
 }
 
+// The blocks of one operand (legs permuted by perm; the first nrow legs form the rows, the
+// rest K) as entries and tiles of the split kernel: offs receives the blocks' byte offsets
+// in the operand's split form, the return value is its size (a multiple of 128 bytes).
+int64_t split_tables(const BT &t, const std::vector<int64_t> &perm, int nrow, int operand, int mode,
+                     std::vector<SplitEntry> &ents, std::vector<SplitTile> &tiles, std::vector<int64_t> &offs) {
+    const int64_t nb = t.nblocks(), ck = split_chunk_bytes(), es = split_elem_bytes(mode);
+    offs.assign(nb, 0);
+    int64_t o = 0;
+    for (int64_t b = 0; b < nb; ++b) {
+        const Strided st = block_strides(t, b);
+        SplitEntry e{};
+        FoldLeg rl[MAXRANK], kl[MAXRANK];
+        int64_t rows = 1, K = 1;
+        for (int i = 0; i < t.rank; ++i) {
+            e.dims[i] = st.d[perm[i]];
+            e.stride[i] = st.s[perm[i]];
+            (i < nrow ? rl[i] : kl[i - nrow]) = FoldLeg{e.dims[i], e.stride[i], 0};
+            (i < nrow ? rows : K) *= e.dims[i];
+        }
+        if (K * es > INT32_MAX - 64) fail(ERR_INVALID_ARGUMENT, "contracted dimension too large");
+        if (rows > INT32_MAX - 64) fail(ERR_INVALID_ARGUMENT, "block too large");
+        Fold fr, fk;
+        e.folded = fold_legs(rl, nrow, fr) && fold_legs(kl, t.rank - nrow, fk) ? 1 : 0;
+        if (e.folded) {
+            e.rd2 = int32_t(std::max<int64_t>(fr.d2, 1));
+            e.rs1 = fr.x1;
+            e.rs2 = fr.x2;
+            e.kd2 = int32_t(std::max<int64_t>(fk.d2, 1));
+            e.ks1 = fk.x1;
+            e.ks2 = fk.x2;
+        }
+        e.src_off = t.boff[b];
+        e.dst_off = o;
+        e.operand = operand;
+        e.rank = t.rank;
+        e.rows = int32_t(rows);
+        e.K = int32_t(K);
+        e.kpb = int32_t((K * es + 31) & ~int64_t(31));
+        offs[b] = o;
+        o += ((rows + 7) / 8) * 8 * int64_t(e.kpb) * split_copies(mode);
+        // 8192 elements a tile or so: few tiles to list, enough of them to spread
+        for (int64_t k0 = 0; k0 < e.kpb; k0 += ck) {
+            const int64_t kv = std::min<int64_t>(ck, e.kpb - k0);
+            const int64_t step = 64 * std::max<int64_t>(1, 128 * es / kv / 2);
+            for (int64_t r0 = 0; r0 < rows; r0 += step)
+                tiles.push_back(SplitTile{int32_t(ents.size()), int32_t(r0), int32_t(std::min(step, rows - r0)), int32_t(k0)});
+        }
+        ents.push_back(e);
+    }
+    return std::max<int64_t>(o, 128);
+}
+
+// Output blocks by falling total K (ties in block order): their tiles in this order leave the
+// cheap ones for the tail of the grid.
+std::vector<int32_t> longest_first(const std::vector<GemmOut> &outs, const std::vector<int64_t> &Ks) {
+    std::vector<int64_t> total(outs.size(), 0);
+    std::vector<int32_t> order(outs.size());
+    for (size_t o = 0; o < outs.size(); ++o) {
+        order[o] = int32_t(o);
+        for (int32_t p = outs[o].p0; p < outs[o].p1; ++p) total[o] += Ks[p];
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return total[x] > total[y]; });
+    return order;
+}
+
 void contract_f64(const ContractPlan &P, const BT &A, const BT &B, BT &out, const BT *add, double beta, double alpha,
-                  const std::vector<GemmOut> &outs, double flops) {
+                  const std::vector<GemmOut> &outs, const std::vector<int64_t> &Ks, double flops) {
     std::vector<F64Pair> pairs;
     BufPtr pa, pb;
     const double *Ap = static_cast<const double *>(A.data());
@@ -537,26 +531,16 @@ void contract_f64(const ContractPlan &P, const BT &A, const BT &B, BT &out, cons
         return n;
     };
     const bool fine = square_tiles() < 4 * device_sm_count();
-    std::vector<std::pair<double, GemmTile>> wt;
-    for (size_t o = 0; o < outs.size(); ++o) {
-        double ksum = 0;
+    std::vector<GemmTile> tiles;
+    for (int32_t o : longest_first(outs, Ks)) {
         int64_t kmax = 0;
-        for (int32_t p = outs[o].p0; p < outs[o].p1; ++p) {
-            const int64_t K = int64_t(pairs[p].k1) * pairs[p].k2;
-            ksum += double(K);
-            kmax = std::max(kmax, K);
-        }
+        for (int32_t p = outs[o].p0; p < outs[o].p1; ++p) kmax = std::max(kmax, Ks[p]);
         int tm, tn;
         const int cls = gemm_f64_class(outs[o].M, outs[o].N, kmax, &tm, &tn, fine);
         for (int64_t m0 = 0; m0 < outs[o].M; m0 += tm)
             for (int64_t n0 = 0; n0 < outs[o].N; n0 += tn)
-                wt.push_back({ksum, GemmTile{int32_t(o), int32_t(m0), int32_t(n0), cls}});
+                tiles.push_back(GemmTile{o, int32_t(m0), int32_t(n0), cls});
     }
-    // longest tiles first: the tail of the grid is made of the cheap ones
-    std::stable_sort(wt.begin(), wt.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
-    std::vector<GemmTile> tiles;
-    tiles.reserve(wt.size());
-    for (auto &w : wt) tiles.push_back(w.second);
     F64Args g;
     g.A = Ap;
     g.B = Bp;
@@ -599,17 +583,48 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
         flops += 2.0 * double(M) * double(N) * ksum;
     }
     if (mode == GEMM_F64) {
-        contract_f64(P, A, B, out, add, beta, alpha, outs, flops);
+        contract_f64(P, A, B, out, add, beta, alpha, outs, Ks, flops);
         return;
     }
-    BufPtr ahi, amid, alo, bhi, bmid, blo, amax;
+    std::vector<SplitEntry> ents;
+    std::vector<SplitTile> stiles;
     std::vector<int64_t> offa, offb;
-    amax = dev_alloc(2 * sizeof(unsigned long long));
-    cuda_check(cudaMemsetAsync(amax->p, 0, 2 * sizeof(unsigned long long), ctx().stream), "cudaMemsetAsync(amax)");
-    auto *am = static_cast<unsigned long long *>(amax->p);
-    split_operand(A, P.p1, int(P.freeA.size()), offa, ahi, amid, alo, am, mode);
-    split_operand(B, P.p2p, int(P.freeB.size()), offb, bhi, bmid, blo, am + 1, mode);
-    const int TM = gemm_tile_m(mode), TN = gemm_tile_n(mode);
+    const int64_t asz = split_tables(A, P.p1, int(P.freeA.size()), 0, mode, ents, stiles, offa);
+    const int64_t bsz = split_tables(B, P.p2p, int(P.freeB.size()), 1, mode, ents, stiles, offb);
+    // one buffer: the two maxima, their per-CTA parts, then the split arrays
+    AmaxArgs am;
+    am.x[0] = static_cast<const double *>(A.data());
+    am.x[1] = static_cast<const double *>(B.data());
+    am.n[0] = A.nnz;
+    am.n[1] = B.nnz;
+    for (int i = 0; i < 2; ++i)
+        am.parts[i] = int32_t(std::min<int64_t>((am.n[i] + 4095) / 4096, 8 * device_sm_count()));
+    const int64_t head = (int64_t(2 + am.parts[0] + am.parts[1]) * 8 + 255) & ~int64_t(255);
+    BufPtr split = dev_alloc(size_t(head + asz + bsz));
+    auto *amax = static_cast<unsigned long long *>(split->p);
+    am.out = amax + 2;
+    SplitArgs sa;
+    for (int i = 0; i < 2; ++i) {
+        sa.src[i] = am.x[i];
+        sa.parts[i] = am.parts[i];
+    }
+    sa.dst[0] = static_cast<char *>(split->p) + head;
+    sa.dst[1] = sa.dst[0] + asz;
+    sa.amax_parts = am.out;
+    sa.amax = amax;
+    {
+        StatScope sc(ST_PACK, (mode == GEMM_BF16X3 ? 14.0 : 16.0) * double(A.nnz + B.nnz));
+        launch_amax(am);
+        sa.ents = upload_vec(ents);
+        sa.tiles = upload_vec(stiles);
+        bool flat = true;
+        for (const SplitEntry &e : ents) flat = flat && e.folded && e.rd2 >= e.rows && e.kd2 >= e.K;
+        launch_split(sa, int64_t(stiles.size()), mode, flat);
+    }
+    const int TM = gemm_tile_m();
+    int64_t wide = 0;
+    for (const GemmOut &o : outs) wide += ((int64_t(o.M) + TM - 1) / TM) * ((int64_t(o.N) + 127) / 128);
+    const int TN = gemm_tile_n(wide);
     std::vector<GemmPair> pairs(P.pair_a.size());
     for (size_t k = 0; k < pairs.size(); ++k) {
         pairs[k].a_off = offa[P.pair_a[k]];
@@ -617,42 +632,25 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
         pairs[k].K = int32_t(Ks[k]);
         pairs[k].pad = 0;
     }
-    std::vector<std::pair<double, GemmTile>> wt;
-    int64_t max_chunks = 0;
-    for (int64_t o = 0; o < nout; ++o) {
-        double ksum = 0;
-        int64_t chunks = 0;
-        for (int32_t p = outs[o].p0; p < outs[o].p1; ++p) {
-            ksum += pairs[p].K;
-            // K chunks of the tensor-core kernels: 32 TF32 (K padded to 8) / 64 BF16 (to 16)
-            chunks += mode == GEMM_BF16X3 ? (((pairs[p].K + 15) & ~15) + 63) / 64 : (((pairs[p].K + 7) & ~7) + 31) / 32;
-        }
-        max_chunks = std::max(max_chunks, chunks);
+    std::vector<GemmTile> tiles;
+    for (int32_t o : longest_first(outs, Ks)) {
+        bool empty = true;
+        for (int32_t p = outs[o].p0; p < outs[o].p1; ++p) empty = empty && Ks[p] == 0;
         for (int64_t m0 = 0; m0 < outs[o].M; m0 += TM)
             for (int64_t n0 = 0; n0 < outs[o].N; n0 += TN)
-                wt.push_back({ksum, GemmTile{int32_t(o), int32_t(m0), int32_t(n0), 0}});
+                tiles.push_back(GemmTile{o, int32_t(m0), int32_t(n0), empty ? 1 : 0});
     }
-    // longest tiles first: the tail of the grid is made of the cheap ones
-    std::stable_sort(wt.begin(), wt.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
-    std::vector<GemmTile> tiles;
-    tiles.reserve(wt.size());
-    for (auto &w : wt) tiles.push_back(w.second);
     TcArgs g;
-    g.Ahi = ahi->p;
-    g.Amid = amid ? amid->p : nullptr;
-    g.Alo = alo->p;
-    g.Bhi = bhi->p;
-    g.Bmid = bmid ? bmid->p : nullptr;
-    g.Blo = blo->p;
-    g.amax_a = static_cast<const unsigned long long *>(amax->p);
-    g.amax_b = g.amax_a + 1;
+    g.A = sa.dst[0];
+    g.B = sa.dst[1];
+    g.amax = amax;
+    g.tn = TN;
     g.C = static_cast<double *>(out.data());
     g.Cadd = add ? static_cast<const double *>(add->data()) : nullptr;
     g.pairs = upload_vec(pairs);
     g.outs = upload_vec(outs);
     g.tiles = upload_vec(tiles);
     g.ntiles = int32_t(tiles.size());
-    g.max_chunks = int32_t(std::min<int64_t>(max_chunks, INT32_MAX));
     g.alpha = alpha;
     g.beta = beta;
     StatScope sc(ST_GEMM, flops);

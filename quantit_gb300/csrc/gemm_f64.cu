@@ -89,10 +89,10 @@ __device__ __forceinline__ void f64_square(const F64Args &g, const GemmTile &t, 
                     for (int u = 0; u < U; ++u) {
 #pragma unroll
                         for (int i = 0; i < RM; ++i)
-                            if (i < rm) a[u][i] = __ldg(pa[i] + oa + (k + u) * ak);
+                            if (i < rm) a[u][i] = *(pa[i] + oa + (k + u) * ak);
 #pragma unroll
                         for (int j = 0; j < RN; ++j)
-                            if (j < rn) b[u][j] = __ldg(pB[j] + ob + (k + u) * bk);
+                            if (j < rn) b[u][j] = *(pB[j] + ob + (k + u) * bk);
                     }
 #pragma unroll
                     for (int u = 0; u < U; ++u)
@@ -107,10 +107,10 @@ __device__ __forceinline__ void f64_square(const F64Args &g, const GemmTile &t, 
                     double a[RM], b[RN];
 #pragma unroll
                     for (int i = 0; i < RM; ++i)
-                        if (i < rm) a[i] = __ldg(pa[i] + oa + k * ak);
+                        if (i < rm) a[i] = *(pa[i] + oa + k * ak);
 #pragma unroll
                     for (int j = 0; j < RN; ++j)
-                        if (j < rn) b[j] = __ldg(pB[j] + ob + k * bk);
+                        if (j < rn) b[j] = *(pB[j] + ob + k * bk);
 #pragma unroll
                     for (int i = 0; i < RM; ++i)
                         if (i < rm)
@@ -171,22 +171,22 @@ __device__ __forceinline__ void f64_strip(const F64Args &g, const GemmTile &t, c
                 for (; k + U <= K2; k += U) {
                     double v[U];
 #pragma unroll
-                    for (int u = 0; u < U; ++u) v[u] = __ldg(xl + (k + u) * lk);
+                    for (int u = 0; u < U; ++u) v[u] = *(xl + (k + u) * lk);
 #pragma unroll
                     for (int u = 0; u < U; ++u)
 #pragma unroll
                         for (int j = 0; j < S; ++j)
                             if (j < ns) {
-                                const double w = __ldg(xs + (k + u) * sk + off[j]);
+                                const double w = *(xs + (k + u) * sk + off[j]);
                                 acc[j] = TALL ? fma(v[u], w, acc[j]) : fma(w, v[u], acc[j]);
                             }
                 }
                 for (; k < K2; ++k) {
-                    const double v = __ldg(xl + k * lk);
+                    const double v = *(xl + k * lk);
 #pragma unroll
                     for (int j = 0; j < S; ++j)
                         if (j < ns) {
-                            const double w = __ldg(xs + k * sk + off[j]);
+                            const double w = *(xs + k * sk + off[j]);
                             acc[j] = TALL ? fma(v, w, acc[j]) : fma(w, v, acc[j]);
                         }
                 }

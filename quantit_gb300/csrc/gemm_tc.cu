@@ -1,31 +1,49 @@
-// Grouped block GEMM on the 5th-generation tensor cores (tcgen05) with
-// split-precision TF32 operands: every FP64 operand element x is split into
-// hi = tf32(x) and lo = tf32(x - hi), and each output tile accumulates
-//     A_hi B_lo + A_lo B_hi + A_hi B_hi
-// in FP32 in tensor memory (TMEM).  The dropped A_lo B_lo term and the FP32
-// accumulation leave about FP32 accuracy (~1e-7 relative) at a third of the TF32
-// tensor throughput -- the "compensated (split-precision) products" of the mixed
-// path; everything outside the block GEMMs stays FP64.
+// Grouped block GEMM on the 5th-generation tensor cores (tcgen05) with split operands:
+// every FP64 operand element x, scaled by a power of two, is split into a few terms of
+// a tensor-core type, and each output tile accumulates the products of the leading
+// orders in FP32 in tensor memory (TMEM); everything outside the block GEMMs stays FP64.
 //
-// Two kernels:
-//  * k_split_tf32: one pass over the operand blocks writes hi / lo as FP32 bit
-//    patterns in the tensor cores' core-matrix tiling: rows padded to 8 and K to 8,
-//    each 8-row x 4-element core matrix (128 bytes) contiguous, the core matrices of
-//    a row group in K order.  A row group's slice of a K chunk is then one contiguous
-//    block of memory.  The FP64 -> FP32 conversion uses integer operations only:
-//    GB300's FP64 pipe is a small fraction of its FP32 / integer rate.
-//  * k_gemm_tf32x3: CTA = one 128 x 128 tile of one output block (same tile and
-//    pair tables as the FP64 kernel), warp-specialised:
-//      - warp 0 (producer) fills a 3-stage shared-memory ring with bulk asynchronous
-//        copies (cp.async.bulk, one per row group and operand copy), counted in bytes
-//        on the stage's "full" mbarrier; the shared layout is the canonical
-//        no-swizzle K-major UMMA layout (LBO 128 B, SBO 1024 B);
-//      - one thread of warp 1 waits on "full", issues the stage's tcgen05.mma
-//        (3 products x up to 4 k-steps of 8) and commits them to the stage's "empty"
-//        mbarrier, which the producer waits on before refilling the stage;
-//      - after the last stage it commits to "done", and all warps run the epilogue:
-//        tcgen05.ld of the accumulator, alpha*acc + beta*add in FP64 (a plain integer
-//        widening when alpha = 1 and there is no add term).
+//  * TF32X3: hi = tf32(x), lo = tf32(x - hi); A_hi B_lo + A_lo B_hi + A_hi B_hi.  The
+//    dropped A_lo B_lo term and the FP32 accumulation leave about FP32 accuracy.
+//  * BF16X3: hi = bf16(x), mid = bf16(x - hi), lo = bf16(x - hi - mid), 24 significant
+//    bits together; the six products of order <= 2, smallest first.  Six BF16 products
+//    cost the tensor time of three TF32 products.
+//
+// Three kernels, two of them templates over the schemes:
+//  * k_amax: per CTA maxima of |x| of both operands (their scales), in one launch.
+//  * k_split: both operands in one launch, straight into the layout the GEMM copies:
+//    a block's K is cut into chunks of CKB bytes per row and term; a chunk holds its rows in
+//    groups of 8, a group its terms one after the other, a term its 16-byte columns as core
+//    matrices (8 rows x 16 bytes).  The rows of an output tile are then ONE contiguous
+//    piece of a chunk, terms included: two bulk copies a stage.  Rows are padded to 8 and
+//    K to a k-step of 32 bytes by the kernel itself.  A thread writes whole 16-byte rows of
+//    core matrices, a warp 512 contiguous bytes.  Bound by memory (4.5 TB/s with the maxima)
+//    since the FP64 -> FP32 conversion takes eight integer instructions and flat layouts no
+//    division; at 40 instructions an element it was bound by the ALUs.
+//  * k_gemm_tc: persistent, CTAS_PER_SM CTAs per SM over the longest-first tile list in
+//    boustrophedon order, warp-specialised:
+//      - warp 0 (producer) fills a ring of stages with bulk asynchronous copies counted on
+//        the stage's "full" mbarrier.  A stage takes CKB bytes of K per row from one or
+//        several pairs: the thin contractions with an MPO tensor have many pairs of K = 1
+//        to 8 per tile.  Tile and pair descriptors are fetched 32 at a time, one per lane.
+//      - one thread of warp 1 issues the stage's tcgen05.mma (32 bytes of K each, N
+//        rounded up to 16) and commits them to the stage's "empty" mbarrier; the
+//        stage's word in shared memory says which units it holds, so this thread reads no
+//        table.  A tile accumulates in TMEM buffer i % 2.
+//      - warps 2-5 run tile i's epilogue from that buffer (tcgen05.ld, transposed through
+//        shared memory so that a warp stores contiguous rows of C) during tile i + 1's MMAs.
+//    What bounds it is the one thread's issue (about 900 clocks a stage of six TF32 MMAs that
+//    take 450) and, for thin tiles, the epilogue; hence two CTAs per SM, each with half the
+//    ring: 88 against 121 us at the D = 4096 theta pair with one CTA and twice the stages,
+//    921 against 1518 us for the three contractions of the cylinder matvec at D = 2048.
+//
+// Against row groups outermost (64 or 96 copies of 1 KB a stage), one pair per stage, one CTA
+// per SM, five launches and as many memsets: theta pair D = 4096, TF32X3 436 -> 172 us (gemm
+// 252 -> 88); D = 1531, BF16X3 127 -> 63 us; cylinder matvec D = 2048, TF32X3 5971 -> 1623 us
+// (its MPO contraction alone 2606 -> 357), all to the same last bit.
+//
+// The order of the MMAs of a tile is that of its pairs and k-steps whatever the stages
+// hold, so results do not depend on the grid or the ring.
 //
 // Every mbarrier wait is bounded; on timeout the kernel records an error code in
 // a device word that the host checks, drains (bounded) the copies and MMAs it
@@ -39,276 +57,297 @@
 
 namespace qtt {
 namespace {
+using namespace tc;
 
-constexpr int TBM = 128, TBN = 128, TBK = 32;  // tile and K chunk (elements)
-constexpr int TTHREADS = 256;
-constexpr int TMEM_COLS = 128;  // FP32 accumulator columns (N)
-constexpr int A_BYTES = TBM * TBK * 4;  // one operand copy: 16 KB
-constexpr int B_BYTES = TBN * TBK * 4;  // 16 KB
-constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;  // hi/lo of A and B: 64 KB
-// up to 3 stages; a launch whose tiles need fewer K chunks uses a smaller ring, so that
-// 2 or 3 CTAs share an SM and hide each other's fixed per-tile latency
-constexpr int smem_bytes(int nstage) { return nstage * STAGE_BYTES + 1024; }
-using tc::LBO;
-using tc::SBO;
-using tc::smem_u32;
-using tc::make_desc;
-using tc::mbar_init;
-using tc::mbar_wait;
-using tc::amax_shift;
-using tc::f64_to_f32_int;
-using tc::f32_to_f64_int;
-using tc::mbar_expect_tx;
-using tc::bulk_g2s;
-using tc::umma_commit;
-using tc::mbar_arrive;
-static_assert(SBO == (TBK * 4 / 16) * 128, "the shared layout assumes 128-byte rows per K chunk");
-
-// kind::tf32, D=F32, A=B=TF32, both K-major, N=128, M=128
-__host__ __device__ constexpr uint32_t idesc_tf32() {
-    return (1u << 4) | (2u << 7) | (2u << 10) | (uint32_t(TBN >> 3) << 17) | (uint32_t(TBM >> 4) << 24);
-}
+constexpr int TBM = 128, TBN = 128;
+constexpr int CKB = 64;                   // bytes of K per row and stage
+constexpr int COPY_BYTES = 128 * CKB;     // one operand copy of a stage
+constexpr int TTHREADS = 192;             // producer, MMA and four epilogue warps
+constexpr int CTAS_PER_SM = 2;
+constexpr int TMEM_COLS = 128;            // FP32 accumulator columns of one tile
+constexpr int EPI_COLS = 16, EPI_PITCH = EPI_COLS + 1;  // an epilogue warp's 32 x 16 patch (floats)
+constexpr int EPI_BYTES = 4 * 32 * EPI_PITCH * 4;
 
 __device__ __forceinline__ uint32_t to_tf32(float x) {
     uint32_t r;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
     return r;
 }
+__device__ __forceinline__ uint32_t to_bf16(float x) {
+    uint16_t r;
+    asm("cvt.rn.bf16.f32 %0, %1;" : "=h"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float from_bf16(uint32_t h) { return __uint_as_float(h << 16); }
 
-__global__ void k_amax(const double *__restrict__ x, int64_t n, unsigned long long *amax) {
+struct Tf32x3 {
+    static constexpr int NC = 2, ELEM = 4, NSTAGE = 3, ERR = 1;
+    // D = F32, A = B = TF32, both K-major, M = 128
+    static __device__ __forceinline__ uint32_t idesc(int n16) {
+        return (1u << 4) | (2u << 7) | (2u << 10) | (uint32_t(n16 * 2) << 17) | (uint32_t(TBM >> 4) << 24);
+    }
+    static __device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+        asm volatile(
+            "{\n .reg .pred q;\n setp.ne.b32 q, %4, 0;\n"
+            " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, q;\n}\n" ::"r"(d),
+            "l"(a), "l"(b), "r"(idesc), "r"(acc));
+    }
+    // one k-step: small terms first, then the leading product
+    static __device__ __forceinline__ void step(uint32_t d, const uint64_t (&a)[NC], const uint64_t (&b)[NC],
+                                                uint32_t idesc, uint32_t acc) {
+        mma(d, a[0], b[1], idesc, acc);
+        mma(d, a[1], b[0], idesc, 1u);
+        mma(d, a[0], b[0], idesc, 1u);
+    }
+    static __device__ __forceinline__ void split(const float (&x)[16 / ELEM], uint4 (&out)[NC]) {
+        uint32_t h[4], l[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            h[i] = to_tf32(x[i]);
+            l[i] = to_tf32(x[i] - __uint_as_float(h[i]));
+        }
+        out[0] = make_uint4(h[0], h[1], h[2], h[3]);
+        out[1] = make_uint4(l[0], l[1], l[2], l[3]);
+    }
+};
+
+struct Bf16x3 {
+    static constexpr int NC = 3, ELEM = 2, NSTAGE = 2, ERR = 3;
+    // D = F32, A = B = BF16, both K-major, M = 128
+    static __device__ __forceinline__ uint32_t idesc(int n16) {
+        return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n16 * 2) << 17) | (uint32_t(TBM >> 4) << 24);
+    }
+    static __device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+        asm volatile(
+            "{\n .reg .pred q;\n setp.ne.b32 q, %4, 0;\n"
+            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, q;\n}\n" ::"r"(d),
+            "l"(a), "l"(b), "r"(idesc), "r"(acc));
+    }
+    // one k-step: second-order terms first, then first order, then the leading product
+    static __device__ __forceinline__ void step(uint32_t d, const uint64_t (&a)[NC], const uint64_t (&b)[NC],
+                                                uint32_t idesc, uint32_t acc) {
+        mma(d, a[0], b[2], idesc, acc);
+        mma(d, a[1], b[1], idesc, 1u);
+        mma(d, a[2], b[0], idesc, 1u);
+        mma(d, a[0], b[1], idesc, 1u);
+        mma(d, a[1], b[0], idesc, 1u);
+        mma(d, a[0], b[0], idesc, 1u);
+    }
+    static __device__ __forceinline__ void split(const float (&x)[16 / ELEM], uint4 (&out)[NC]) {
+        uint32_t w[NC][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t t[2][NC];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float v = x[2 * i + j];
+                t[j][0] = to_bf16(v);
+                const float r = v - from_bf16(t[j][0]);
+                t[j][1] = to_bf16(r);
+                t[j][2] = to_bf16(r - from_bf16(t[j][1]));
+            }
+#pragma unroll
+            for (int c = 0; c < NC; ++c) w[c][i] = t[0][c] | (t[1][c] << 16);
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) out[c] = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
+    }
+};
+
+constexpr int stage_bytes(int nc) { return 2 * nc * COPY_BYTES; }
+constexpr int smem_bytes(int nc, int nstage) { return nstage * stage_bytes(nc) + EPI_BYTES; }
+
+// Maxima of |x| as bit patterns (bit order = value order for non-negative doubles), one
+// per CTA; operand b's CTAs follow operand a's.
+__global__ void __launch_bounds__(256) k_amax(AmaxArgs g) {
+    const int which = int(blockIdx.x) >= g.parts[0];
+    const double *__restrict__ x = g.x[which];
+    const int64_t n = g.n[which];
+    const int64_t first = int64_t(blockIdx.x) - (which ? g.parts[0] : 0), step = int64_t(g.parts[which]) * 1024;
     unsigned long long m = 0;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        const unsigned long long v = static_cast<unsigned long long>(__double_as_longlong(x[i])) & 0x7FFFFFFFFFFFFFFFull;
-        m = v > m ? v : m;
+    auto take = [&](double v) {
+        const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7FFFFFFFFFFFFFFFull;
+        m = u > m ? u : m;
+    };
+    // plain loads: the same loop over __ldg / __ldcg reaches 3.7 TB/s instead of 6.4
+    for (int64_t b = first * 1024 + threadIdx.x; b < n; b += step) {
+        double v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = b + j * 256 < n ? x[b + j * 256] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) take(v[j]);
+    }
+    __shared__ unsigned long long red[8];
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long u = __shfl_xor_sync(0xffffffffu, m, o);
+        m = u > m ? u : m;
+    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) m = red[w] > m ? red[w] : m;
+        g.out[blockIdx.x] = m;
+    }
+}
+
+// The largest of the per-CTA maxima of one operand (every thread of the CTA gets it).
+__device__ __forceinline__ unsigned long long amax_of(const unsigned long long *parts, int n, unsigned long long *red) {
+    unsigned long long m = 0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const unsigned long long u = parts[i];
+        m = u > m ? u : m;
     }
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long u = __shfl_xor_sync(0xffffffffu, m, o);
         m = u > m ? u : m;
     }
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(amax, m);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    m = red[0];
+    for (int w = 1; w < int(blockDim.x >> 5); ++w) m = red[w] > m ? red[w] : m;
+    return m;
 }
 
-__global__ void k_split_tf32(const double *__restrict__ src, float *__restrict__ hi, float *__restrict__ lo,
-                             const SplitEntry *__restrict__ ents, const Chunk *__restrict__ chunks,
-                             const unsigned long long *__restrict__ amax) {
-    const Chunk ch = chunks[blockIdx.x];
-    const SplitEntry &e = ents[ch.seg];
-    const int shift = amax_shift(*amax);
-    for (int i = threadIdx.x; i < ch.len; i += blockDim.x) {
-        const int64_t lin = ch.start + i;
-        const float xf = f64_to_f32_int(src[split_src(e, lin)], shift);
-        const uint32_t h = to_tf32(xf);
-        const uint32_t l = to_tf32(xf - __uint_as_float(h));
-        int64_t row, k;
-        split_rowk(e, lin, row, k);
-        const int64_t dst = e.dst_off + ((row >> 3) * (e.K4 >> 2) + (k >> 2)) * 32 + (row & 7) * 4 + (k & 3);
-        hi[dst] = __uint_as_float(h);
-        lo[dst] = __uint_as_float(l);
-    }
-}
-
-__device__ __forceinline__ void mma_tf32(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n .reg .pred q;\n setp.ne.b32 q, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, q;\n}\n" ::"r"(tmem),
-        "l"(da), "l"(db), "r"(idesc), "r"(acc));
-}
-
-template <int NSTAGE>
-__global__ void __launch_bounds__(TTHREADS, 1) k_gemm_tf32x3(TcArgs g, int *err) {
-    extern __shared__ __align__(1024) char smem_raw[];
-    char *smem = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    __shared__ uint64_t full[NSTAGE], empty[NSTAGE], done;
-    __shared__ uint32_t tmem_base_sh;
-    __shared__ int abort_flag, n_issued, n_consumed;
-
-    const GemmTile t = g.tiles[blockIdx.x];
-    const GemmOut o = g.outs[t.out];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)),
-                     "r"(TMEM_COLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    if (tid == 0) {
-        for (int s = 0; s < NSTAGE; ++s) {
-            mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
+// FLAT: every entry's rows have one stride and its K one (no index arithmetic but two
+// products); otherwise rows and K of two strides each, or any legs.
+template <class S, bool FLAT>
+__global__ void __launch_bounds__(256) k_split(SplitArgs g) {
+    constexpr int EV = 16 / S::ELEM;  // elements of a core matrix row
+    __shared__ unsigned long long red[8];
+    const SplitTile t = g.tiles[blockIdx.x];
+    const SplitEntry &e = g.ents[t.ent];
+    const int op = e.operand;
+    const unsigned long long am = amax_of(g.amax_parts + (op ? g.parts[0] : 0), g.parts[op], red);
+    if (blockIdx.x == 0) {
+        // the GEMM's epilogue reads both maxima
+        const unsigned long long other = amax_of(g.amax_parts + (op ? 0 : g.parts[0]), g.parts[1 - op], red);
+        if (threadIdx.x == 0) {
+            g.amax[op] = am;
+            g.amax[1 - op] = other;
         }
-        mbar_init(&done, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;");
-        abort_flag = 0;
-        n_issued = 0;
-        n_consumed = 0;
     }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = tmem_base_sh;
-
-    int nchunk = 0;
-    for (int p = o.p0; p < o.p1; ++p) nchunk += (((g.pairs[p].K + 7) & ~7) + TBK - 1) / TBK;
-
-    if (warp == 0) {
-        // producer: one bulk copy per (operand copy, row group) of each K chunk
-        const float *srcs[4] = {static_cast<const float *>(g.Ahi), static_cast<const float *>(g.Alo),
-                                static_cast<const float *>(g.Bhi), static_cast<const float *>(g.Blo)};
-        const int rga = min(TBM / 8, (o.M - t.m0 + 7) / 8), rgb = min(TBN / 8, (o.N - t.n0 + 7) / 8);
-        int p = o.p0, k0 = 0, c = 0;
-        for (; c < nchunk; ++c) {
-            const int s = c % NSTAGE;
-            int ok = 1;
-            if (lane == 0 && c >= NSTAGE) ok = mbar_wait(&empty[s], ((c / NSTAGE) - 1) & 1) ? 1 : 0;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) {
-                if (lane == 0) {
-                    atomicExch(err, 1);
-                    atomicExch(&abort_flag, 1);
-                }
-                break;
-            }
-            while (k0 >= ((g.pairs[p].K + 7) & ~7)) {
-                ++p;
-                k0 = 0;
-            }
-            const GemmPair pr = g.pairs[p];
-            const int KP = (pr.K + 7) & ~7, kv = min(TBK, KP - k0);
-            const uint32_t rg_bytes = uint32_t(kv) * 32u;  // kv / 4 core matrices of 128 bytes
-            if (lane == 0) mbar_expect_tx(&full[s], 2u * rg_bytes * uint32_t(rga + rgb));
-            __syncwarp();
-            char *st = smem + s * STAGE_BYTES;
-            const int nA = 2 * rga, ncopy = 2 * (rga + rgb);
-            for (int i = lane; i < ncopy; i += 32) {
-                const bool isA = i < nA;
-                const int j = isA ? i : i - nA, which = j & 1, rg = j >> 1;
-                const int64_t grg = (isA ? t.m0 : t.n0) / 8 + rg;
-                const float *src = srcs[(isA ? 0 : 2) + which] + (isA ? pr.a_off : pr.b_off) +
-                                   (grg * (KP / 4) + k0 / 4) * 32;
-                char *dst = st + (isA ? 0 : 2 * A_BYTES) + which * (isA ? A_BYTES : B_BYTES) + rg * int(SBO);
-                bulk_g2s(dst, src, rg_bytes, &full[s]);
-            }
-            k0 += TBK;
-        }
-        if (lane == 0) n_issued = c;
-    } else if (warp == 1 && lane == 0) {
-        // MMA issuer
-        const uint32_t idesc = idesc_tf32();
-        int p = o.p0, k0 = 0, c = 0;
-        for (; c < nchunk; ++c) {
-            const int s = c % NSTAGE;
-            if (!mbar_wait(&full[s], (c / NSTAGE) & 1)) {
-                atomicExch(err, 2);
-                atomicExch(&abort_flag, 1);
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;");
-            while (k0 >= ((g.pairs[p].K + 7) & ~7)) {
-                ++p;
-                k0 = 0;
-            }
-            const int kv = min(TBK, ((g.pairs[p].K + 7) & ~7) - k0);
-            char *st = smem + s * STAGE_BYTES;
-            const uint32_t a_hi = smem_u32(st), a_lo = a_hi + A_BYTES, b_hi = a_hi + 2 * A_BYTES, b_lo = b_hi + B_BYTES;
-            for (int ks = 0; ks < kv / 8; ++ks) {
-                const uint32_t koff = uint32_t(ks) * 2u * LBO;  // 8 tf32 = 2 core matrices along K
-                const uint32_t acc0 = (c > 0 || ks > 0) ? 1u : 0u;
-                // small terms first, then the leading product
-                mma_tf32(tmem, make_desc(a_hi + koff), make_desc(b_lo + koff), idesc, acc0);
-                mma_tf32(tmem, make_desc(a_lo + koff), make_desc(b_hi + koff), idesc, 1u);
-                mma_tf32(tmem, make_desc(a_hi + koff), make_desc(b_hi + koff), idesc, 1u);
-            }
-            umma_commit(&empty[s]);
-            k0 += TBK;
-        }
-        n_consumed = c;
-        umma_commit(&done);
-    }
-    // everyone: the accumulator is final once "done" fires
-    if (lane == 0 && !mbar_wait(&done, 0)) atomicExch(err, 2);
-    __syncwarp();
-    __syncthreads();
-    if (tid == 0) {
-        // copies issued but never consumed (only after a timeout) must land before exit
-        for (int c = n_consumed; c < n_issued; ++c)
-            if (!mbar_wait(&full[c % NSTAGE], (c / NSTAGE) & 1)) atomicExch(err, 2);
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    __syncthreads();
-
-    // epilogue: warp w reads TMEM lanes 32*(w%4).., columns 64*(w/4) .. +63
-    const int quarter = warp & 3, half = warp >> 2;
-    const int shift = amax_shift(*g.amax_a) + amax_shift(*g.amax_b);
-    const int row = quarter * 32 + lane;
-    const int gm = t.m0 + row;
-    const bool have_acc = nchunk > 0 && !abort_flag;
+    const int shift = amax_shift(am);
+    const bool fast = f64_fast(am, shift);
+    const uint32_t rebase = f64_rebase(shift);
+    const double *__restrict__ src = g.src[op] + e.src_off;
+    const int kvb = min(CKB, e.kpb - t.k0b), nq = kvb / 16;
+    const int rows = e.rows, K = e.K, nrg = (rows + 7) >> 3, k00 = t.k0b / S::ELEM;
+    const int total = ((t.rows + 7) >> 3) * nq * 8, inv = (65536 + nq - 1) / nq;
+    const int64_t rs2 = e.rs2, ks2 = e.ks2;
+    char *dst0 = g.dst[op] + e.dst_off + int64_t(t.k0b / CKB) * nrg * (8 * S::NC * CKB);
+#pragma unroll 2
+    for (int i = threadIdx.x; i < total; i += 256) {
+        const int u = i >> 3, rg = (u * inv) >> 16, core = u - rg * nq;  // u / nq, u < 2^14
+        const int row = t.row0 + rg * 8 + (i & 7), k = k00 + core * EV;
+        const int nk = row < rows ? K - k : 0;  // elements of this core matrix row within the block
+        double d[EV];
+        if (FLAT) {
+            const double *__restrict__ p = src + int64_t(row) * rs2 + int64_t(k) * ks2;
 #pragma unroll
-    for (int cb = 0; cb < 2; ++cb) {
-        const int col0 = half * 64 + cb * 32;
-        uint32_t v[32];
-        if (have_acc) {
-            const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(col0);
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                  "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
-                  "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
-                  "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                : "r"(taddr));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int v = 0; v < EV; ++v) d[v] = v < nk ? p[v * ks2] : 0.0;
+        } else if (e.folded) {
+            const int rq = row / e.rd2, kq = k / e.kd2;
+            const double *__restrict__ p = src + int64_t(rq) * e.rs1 + int64_t(row - rq * e.rd2) * rs2;
+            int k2 = k - kq * e.kd2;
+            int64_t off = int64_t(kq) * e.ks1 + int64_t(k2) * ks2;
+#pragma unroll
+            for (int v = 0; v < EV; ++v) {
+                d[v] = v < nk ? p[off] : 0.0;
+                off += ks2;
+                if (++k2 == e.kd2) {
+                    k2 = 0;
+                    off += e.ks1 - int64_t(e.kd2) * ks2;
+                }
+            }
+        } else {
+            // legs that do not fold: the row-major index over all of them
+#pragma unroll
+            for (int v = 0; v < EV; ++v) {
+                d[v] = 0.0;
+                if (v >= nk) continue;
+                int64_t rem = int64_t(row) * K + (k + v), so = 0;
+#pragma unroll 1
+                for (int l = e.rank - 1; l >= 0; --l) {
+                    const int64_t q = rem / e.dims[l];
+                    so += (rem - q * e.dims[l]) * e.stride[l];
+                    rem = q;
+                }
+                d[v] = src[so];
+            }
+        }
+        float x[EV];
+        if (fast) {
+#pragma unroll
+            for (int v = 0; v < EV; ++v) x[v] = f64_to_f32_fast(d[v], rebase);
         } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = 0u;
+            for (int v = 0; v < EV; ++v) x[v] = f64_to_f32_int(d[v], shift);
         }
-        if (gm < o.M) {
-            // GB300's FP64 pipe is narrow: the plain case (alpha = 1, no add term) converts
-            // with integer operations only; FP64 arithmetic only for tensorgdot's epilogue
-            const bool plain = g.alpha == 1.0 && o.add_off < 0;
+        uint4 out[S::NC];
+        S::split(x, out);
+        char *dst = dst0 + int64_t(row >> 3) * (8 * S::NC * kvb) + core * 128 + (row & 7) * 16;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const int gn = t.n0 + col0 + j;
-                if (gn < o.N) {
-                    const int64_t idx = int64_t(gm) * o.N + gn;
-                    double val = f32_to_f64_int(__uint_as_float(v[j]), shift);
-                    if (!plain) {
-                        val *= g.alpha;
-                        if (o.add_off >= 0) val += g.beta * g.Cadd[o.add_off + idx];
-                    }
-                    g.C[o.c_off + idx] = val;
-                }
-            }
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    if (warp == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+        for (int c = 0; c < S::NC; ++c) *reinterpret_cast<uint4 *>(dst + c * 8 * kvb) = out[c];
     }
 }
 
-// Persistent variant for launches of many tiles: one CTA per SM walks the sorted tile
-// list (tiles blockIdx.x, + gridDim.x, ...).  The producer warp streams the K chunks of
-// its tiles through the ring without draining it between tiles; the MMA thread
-// accumulates tile i in TMEM buffer i % 2 (2 x 128 columns) and commits it to
-// acc_full[i % 2]; warps 4-7 (one TMEM lane quarter each) run tile i's epilogue from
-// that buffer and release it on acc_empty[i % 2] while the MMAs of tile i + 1 proceed.
-template <int NSTAGE>
-__global__ void __launch_bounds__(TTHREADS, 1) k_gemm_tf32x3_persistent(TcArgs g, int *err) {
-    extern __shared__ __align__(1024) char smem_raw[];
-    char *smem = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    __shared__ uint64_t full[NSTAGE], empty[NSTAGE], acc_full[2], acc_empty[2];
+// What a stage holds, for the MMA thread: up to CKB / 32 units of k-steps (3 bits each from
+// bit 0), flags, and the tile's N in units of 16.
+constexpr uint32_t ST_FIRST = 1u << 12, ST_LAST = 1u << 13, ST_END = 1u << 14;
+constexpr int ST_N16 = 16;
+
+// Descriptors of up to 32 tiles of a CTA's list, one per lane.
+struct TileRegs {
+    int m0, n0, cls, M, N, p0, p1;
+    int64_t c_off, add_off;
+    __device__ __forceinline__ void fetch(const TcArgs &g, int tile) {
+        cls = -1;
+        if (tile >= g.ntiles) return;
+        const GemmTile t = g.tiles[tile];
+        const GemmOut o = g.outs[t.out];
+        m0 = t.m0;
+        n0 = t.n0;
+        cls = t.cls;
+        M = o.M;
+        N = o.N;
+        p0 = o.p0;
+        p1 = o.p1;
+        c_off = o.c_off;
+        add_off = o.add_off;
+    }
+    __device__ __forceinline__ TileRegs of_lane(int l) const {
+        TileRegs r;
+        r.m0 = __shfl_sync(0xffffffffu, m0, l);
+        r.n0 = __shfl_sync(0xffffffffu, n0, l);
+        r.cls = __shfl_sync(0xffffffffu, cls, l);
+        r.M = __shfl_sync(0xffffffffu, M, l);
+        r.N = __shfl_sync(0xffffffffu, N, l);
+        r.p0 = __shfl_sync(0xffffffffu, p0, l);
+        r.p1 = __shfl_sync(0xffffffffu, p1, l);
+        r.c_off = __shfl_sync(0xffffffffu, c_off, l);
+        r.add_off = __shfl_sync(0xffffffffu, add_off, l);
+        return r;
+    }
+};
+
+template <class S, int NSTAGE>
+__global__ void __launch_bounds__(TTHREADS, CTAS_PER_SM) k_gemm_tc(TcArgs g, int *err) {
+    constexpr int NC = S::NC, STAGE = stage_bytes(NC);
+    extern __shared__ __align__(128) char smem[];
+    __shared__ uint64_t full[NSTAGE], empty[NSTAGE], acc_full[2], acc_empty[2], drained;
+    __shared__ uint32_t stage_word[NSTAGE];
     __shared__ uint32_t tmem_base_sh;
-    __shared__ int n_issued, n_consumed;
+    __shared__ int n_issued, n_consumed;  // stages sent out by the producer, taken by the MMA thread
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // round r of the longest-first tile list, in boustrophedon order across the CTAs, so
     // that every CTA's tiles add up to about the same work
     auto snake_tile = [&](int r) {
-        const int G = int(gridDim.x), b = int(blockIdx.x);
-        return r * G + ((r & 1) ? (G - 1 - b) : b);
+        const int64_t G = gridDim.x, b = blockIdx.x;
+        const int64_t t = int64_t(r) * G + ((r & 1) ? (G - 1 - b) : b);
+        return int(min(t, int64_t(INT32_MAX)));
     };
+    const int rounds = (g.ntiles + int(gridDim.x) - 1) / int(gridDim.x);
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)),
@@ -324,6 +363,7 @@ __global__ void __launch_bounds__(TTHREADS, 1) k_gemm_tf32x3_persistent(TcArgs g
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 4);  // one arrival per epilogue warp
         }
+        mbar_init(&drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
         n_issued = 0;
         n_consumed = 0;
@@ -332,173 +372,262 @@ __global__ void __launch_bounds__(TTHREADS, 1) k_gemm_tf32x3_persistent(TcArgs g
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = tmem_base_sh;
-    auto tile_chunks = [&](const GemmOut &o) {
-        int n = 0;
-        for (int p = o.p0; p < o.p1; ++p) n += (((g.pairs[p].K + 7) & ~7) + TBK - 1) / TBK;
-        return n;
-    };
 
     if (warp == 0) {
-        const float *srcs[4] = {static_cast<const float *>(g.Ahi), static_cast<const float *>(g.Alo),
-                                static_cast<const float *>(g.Bhi), static_cast<const float *>(g.Blo)};
-        int gc = 0;
+        int slot = 0, issued = 0;
+        uint32_t phase = 0;  // parity of the ring's current lap
         bool stop = false;
-        for (int r = 0; r * int(gridDim.x) < g.ntiles && !stop; ++r) {
-            const int tile = snake_tile(r);
-            if (tile >= g.ntiles) continue;
-            const GemmTile t = g.tiles[tile];
-            const GemmOut o = g.outs[t.out];
-            const int rga = min(TBM / 8, (o.M - t.m0 + 7) / 8), rgb = min(TBN / 8, (o.N - t.n0 + 7) / 8);
-            const int nch = tile_chunks(o);
-            int p = o.p0, k0 = 0;
-            for (int c = 0; c < nch; ++c) {
-                const int s = gc % NSTAGE;
-                int ok = 1;
-                if (lane == 0 && gc >= NSTAGE) ok = mbar_wait(&empty[s], ((gc / NSTAGE) - 1) & 1) ? 1 : 0;
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) {
-                    if (lane == 0) atomicExch(err, 1);
-                    stop = true;
-                    break;
-                }
-                while (k0 >= ((g.pairs[p].K + 7) & ~7)) {
-                    ++p;
-                    k0 = 0;
-                }
-                const GemmPair pr = g.pairs[p];
-                const int KP = (pr.K + 7) & ~7, kv = min(TBK, KP - k0);
-                const uint32_t rg_bytes = uint32_t(kv) * 32u;
-                if (lane == 0) mbar_expect_tx(&full[s], 2u * rg_bytes * uint32_t(rga + rgb));
-                __syncwarp();
-                char *st = smem + s * STAGE_BYTES;
-                const int nA = 2 * rga, ncopy = 2 * (rga + rgb);
-                for (int i = lane; i < ncopy; i += 32) {
-                    const bool isA = i < nA;
-                    const int j = isA ? i : i - nA, which = j & 1, rg = j >> 1;
-                    const int64_t grg = (isA ? t.m0 : t.n0) / 8 + rg;
-                    const float *src = srcs[(isA ? 0 : 2) + which] + (isA ? pr.a_off : pr.b_off) +
-                                       (grg * (KP / 4) + k0 / 4) * 32;
-                    char *dst = st + (isA ? 0 : 2 * A_BYTES) + which * (isA ? A_BYTES : B_BYTES) + rg * int(SBO);
-                    bulk_g2s(dst, src, rg_bytes, &full[s]);
-                }
-                k0 += TBK;
-                ++gc;
+        // lane 0 copies A, lane 1 B
+        const bool copies = lane < 2, is_a = lane == 0;
+        const char *const base = is_a ? g.A : g.B;
+        char *const stage0 = smem + (is_a ? 0 : NC * COPY_BYTES);
+        auto wait_slot = [&]() {
+            const bool ok = issued < NSTAGE || mbar_wait(&empty[slot], phase ^ 1);
+            if (__all_sync(0xffffffffu, ok)) return true;
+            if (lane == 0) atomicExch(err, S::ERR);
+            stop = true;
+            return false;
+        };
+        auto next_slot = [&]() {
+            ++issued;
+            if (++slot == NSTAGE) {
+                slot = 0;
+                phase ^= 1;
             }
-        }
-        if (lane == 0) n_issued = gc;
-    } else if (warp == 1 && lane == 0) {
-        const uint32_t idesc = idesc_tf32();
-        int gc = 0, i = 0;
-        bool stop = false;
-        for (int r = 0; r * int(gridDim.x) < g.ntiles && !stop; ++r) {
-            const int tile = snake_tile(r);
-            if (tile >= g.ntiles) continue;
-            const GemmOut o = g.outs[g.tiles[tile].out];
-            const int b = i & 1;
-            if (i >= 2 && !mbar_wait(&acc_empty[b], ((i / 2) - 1) & 1)) {
-                atomicExch(err, 2);
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;");
-            const uint32_t acc_t = tmem + uint32_t(b * TMEM_COLS);
-            const int nch = tile_chunks(o);
-            int p = o.p0, k0 = 0;
-            for (int c = 0; c < nch; ++c) {
-                const int s = gc % NSTAGE;
-                if (!mbar_wait(&full[s], (gc / NSTAGE) & 1)) {
-                    atomicExch(err, 2);
-                    stop = true;
-                    break;
+        };
+        TileRegs mine;
+        mine.cls = -1;
+        for (int r = 0; r < rounds && !stop; ++r) {
+            if ((r & 31) == 0) mine.fetch(g, r + lane < rounds ? snake_tile(r + lane) : INT32_MAX);
+            const TileRegs t = mine.of_lane(r & 31);
+            if (t.cls != 0) continue;  // past the list, or a tile whose pairs all have K = 0
+            const int rga = min(TBM / 8, (t.M - t.m0 + 7) / 8), rgb = min(g.tn / 8, (t.N - t.n0 + 7) / 8);
+            const uint32_t row_bytes = uint32_t(NC * 8) * uint32_t(rga + rgb);  // per byte of K
+            const uint32_t my_rows = uint32_t(is_a ? rga : rgb) * uint32_t(8 * NC);
+            const int64_t my_chunk = int64_t(((is_a ? t.M : t.N) + 7) / 8) * (8 * NC * CKB);
+            const int64_t my_first = int64_t(is_a ? t.m0 : t.n0) * NC;
+            uint32_t word = (uint32_t(rgb + 1) / 2 << ST_N16) | ST_FIRST;
+            int width = 0, nu = 0;  // of the open stage: narrow units wait in it for company
+            bool ended = false;     // the tile's last stage has gone out
+            const int np = t.p1 - t.p0;
+            auto close_stage = [&](uint32_t last) {
+                if (lane == 0) {
+                    stage_word[slot] = word | last;
+                    mbar_arrive(&full[slot]);
                 }
-                asm volatile("tcgen05.fence::after_thread_sync;");
-                while (k0 >= ((g.pairs[p].K + 7) & ~7)) {
-                    ++p;
-                    k0 = 0;
+                next_slot();
+                word &= 0xFu << ST_N16;
+                width = nu = 0;
+            };
+            // the pair of each lane (a batch of 32): offset for this lane's operand and padded K
+            for (int pb = 0; pb < np && !stop; pb += 32) {
+                int64_t a_off = 0, b_off = 0;
+                int kpb = 0;
+                if (pb + lane < np) {
+                    const GemmPair pr = g.pairs[t.p0 + pb + lane];
+                    a_off = pr.a_off;
+                    b_off = pr.b_off;
+                    kpb = (pr.K * S::ELEM + 31) & ~31;
                 }
-                const int kv = min(TBK, ((g.pairs[p].K + 7) & ~7) - k0);
-                char *st = smem + s * STAGE_BYTES;
-                const uint32_t a_hi = smem_u32(st), a_lo = a_hi + A_BYTES, b_hi = a_hi + 2 * A_BYTES,
-                               b_lo = b_hi + B_BYTES;
-                for (int ks = 0; ks < kv / 8; ++ks) {
-                    const uint32_t koff = uint32_t(ks) * 2u * LBO;
-                    const uint32_t acc0 = (c > 0 || ks > 0) ? 1u : 0u;
-                    mma_tf32(acc_t, make_desc(a_hi + koff), make_desc(b_lo + koff), idesc, acc0);
-                    mma_tf32(acc_t, make_desc(a_lo + koff), make_desc(b_hi + koff), idesc, 1u);
-                    mma_tf32(acc_t, make_desc(a_hi + koff), make_desc(b_hi + koff), idesc, 1u);
-                }
-                umma_commit(&empty[s]);
-                k0 += TBK;
-                ++gc;
-            }
-            umma_commit(&acc_full[b]);  // this tile's accumulator is final once its MMAs complete
-            ++i;
-        }
-        n_consumed = gc;
-    } else if (warp >= 4) {
-        // epilogue: warp 4 + q reads TMEM lanes 32 q .. 32 q + 31 (rows), all 128 columns
-        const int quarter = warp - 4;
-        const int shift = amax_shift(*g.amax_a) + amax_shift(*g.amax_b);
-        const int row = quarter * 32 + lane;
-        int i = 0;
-        for (int r = 0; r * int(gridDim.x) < g.ntiles; ++r) {
-            const int tile = snake_tile(r);
-            if (tile >= g.ntiles) continue;
-            const GemmTile t = g.tiles[tile];
-            const GemmOut o = g.outs[t.out];
-            const int b = i & 1;
-            int ok = 1;
-            if (lane == 0) ok = mbar_wait(&acc_full[b], (i / 2) & 1) ? 1 : 0;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) {
-                if (lane == 0) atomicExch(err, 2);
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;");
-            const bool have_acc = tile_chunks(o) > 0;
-            const int gm = t.m0 + row;
-            const bool plain = g.alpha == 1.0 && o.add_off < 0;
-#pragma unroll 1
-            for (int cb = 0; cb < 4; ++cb) {
-                const int col0 = cb * 32;
-                uint32_t v[32];
-                const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(b * TMEM_COLS + col0);
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                    "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                      "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
-                      "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
-                      "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(taddr));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (gm < o.M) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const int gn = t.n0 + col0 + j;
-                        if (gn < o.N) {
-                            const int64_t idx = int64_t(gm) * o.N + gn;
-                            double val = have_acc ? f32_to_f64_int(__uint_as_float(v[j]), shift) : 0.0;
-                            if (!plain) {
-                                val *= g.alpha;
-                                if (o.add_off >= 0) val += g.beta * g.Cadd[o.add_off + idx];
+                for (uint32_t live = __ballot_sync(0xffffffffu, kpb > 0); live && !stop; live &= live - 1) {
+                    const int p = __ffs(int(live)) - 1;
+                    const int kp = __shfl_sync(0xffffffffu, kpb, p);
+                    const int64_t ao = __shfl_sync(0xffffffffu, a_off, p), bo = __shfl_sync(0xffffffffu, b_off, p);
+                    const char *src = base + (is_a ? ao : bo);
+                    int k = 0;
+                    if (kp >= CKB) {
+                        if (width && !stop) close_stage(0);
+                        const bool ends = (live & (live - 1)) == 0 && pb + 32 >= np && kp % CKB == 0;
+                        for (; k + CKB <= kp; k += CKB) {
+                            if (!wait_slot()) break;
+                            if (lane == 0) {
+                                stage_word[slot] = word | uint32_t(CKB / 32) | (ends && k + CKB == kp ? ST_LAST : 0u);
+                                mbar_arrive_expect_tx(&full[slot], row_bytes * CKB);
                             }
-                            g.C[o.c_off + idx] = val;
+                            __syncwarp();
+                            if (copies) bulk_g2s(stage0 + slot * STAGE, src + my_first * CKB, my_rows * CKB, &full[slot]);
+                            src += my_chunk;
+                            next_slot();
+                            word &= 0xFu << ST_N16;
                         }
+                        if (stop) break;
+                        ended = ends;
+                    }
+                    const int kv = kp - k;
+                    if (kv > 0) {
+                        if (width + kv > CKB) close_stage(0);
+                        if (width == 0 && !wait_slot()) break;
+                        if (lane == 0) mbar_expect_tx_only(&full[slot], row_bytes * uint32_t(kv));
+                        __syncwarp();
+                        if (copies)
+                            bulk_g2s(stage0 + slot * STAGE + width * (128 * NC), src + my_first * kv, my_rows * uint32_t(kv),
+                                     &full[slot]);
+                        word |= uint32_t(kv / 32) << (3 * nu++);
+                        width += kv;
                     }
                 }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[b]);
-            ++i;
+            if (!stop && !ended && (width || wait_slot())) close_stage(ST_LAST);
+        }
+        if (!stop && wait_slot()) {
+            if (lane == 0) {
+                stage_word[slot] = ST_END;
+                mbar_arrive(&full[slot]);
+            }
+            next_slot();
+        }
+        if (lane == 0) n_issued = issued;
+    } else if (warp == 1 && lane == 0) {
+        int slot = 0, taken = 0, i = 0;
+        uint32_t phase = 0, acc = 0, d = tmem;
+        // the descriptors' fixed part; a stage and a k-step only move their start address
+        const uint64_t first = make_desc(smem_u32(smem), 0);
+        for (;;) {
+            if (!mbar_wait(&full[slot], phase)) {
+                atomicExch(err, S::ERR + 1);
+                break;
+            }
+            const uint32_t word = *reinterpret_cast<volatile uint32_t *>(&stage_word[slot]);
+            if (word & ST_END) {
+                ++taken;
+                break;
+            }
+            if (word & ST_FIRST) {
+                if (i >= 2 && !mbar_wait(&acc_empty[i & 1], ((i / 2) - 1) & 1)) {
+                    atomicExch(err, S::ERR + 1);
+                    break;
+                }
+                d = tmem + uint32_t((i & 1) * TMEM_COLS);
+                acc = 0;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            const uint32_t idesc = S::idesc(int((word >> ST_N16) & 15u));
+            uint64_t at = first + uint64_t(slot * (STAGE / 16));
+            // n k-steps of 32 bytes: a copy of 8 rows takes n * 256 bytes
+            auto k_steps = [&](uint64_t from, int n) {
+                const uint64_t rows8 = uint64_t(n * (256 / 16));
+                from += (rows8 * NC) << 32;
+                uint64_t a[NC], b[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    a[c] = from + c * rows8;
+                    b[c] = from + uint64_t(NC * (COPY_BYTES / 16)) + c * rows8;
+                }
+#pragma unroll
+                for (int j = 0; j < CKB / 32; ++j) {
+                    if (j >= n) break;
+                    S::step(d, a, b, idesc, acc);
+                    acc = 1;
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        a[c] += 2 * LBO / 16;
+                        b[c] += 2 * LBO / 16;
+                    }
+                }
+            };
+            if ((word & 7u) == CKB / 32) {
+                k_steps(at, CKB / 32);
+            } else {
+                for (uint32_t w = word & 0xFFFu; w; w >>= 3) {
+                    const uint32_t n = w & 7u;
+                    k_steps(at, int(n));
+                    at += uint64_t(n * 32 * 128 * NC / 16);
+                }
+            }
+            umma_commit(&empty[slot]);
+            if (word & ST_LAST) {
+                umma_commit(&acc_full[i & 1]);  // this tile's accumulator is final once its MMAs complete
+                ++i;
+            }
+            ++taken;
+            if (++slot == NSTAGE) {
+                slot = 0;
+                phase ^= 1;
+            }
+        }
+        n_consumed = taken;
+        umma_commit(&drained);
+    } else if (warp >= 2) {
+        // epilogue: the four warps read one TMEM lane quarter (32 rows) each
+        const int quarter = warp & 3;
+        float *patch = reinterpret_cast<float *>(smem + NSTAGE * STAGE) + quarter * 32 * EPI_PITCH;
+        const int shift = amax_shift(g.amax[0]) + amax_shift(g.amax[1]);
+        int i = 0;
+        TileRegs mine;
+        mine.cls = -1;
+        for (int r = 0; r < rounds; ++r) {
+            if ((r & 31) == 0) mine.fetch(g, r + lane < rounds ? snake_tile(r + lane) : INT32_MAX);
+            const TileRegs t = mine.of_lane(r & 31);
+            if (t.cls < 0) continue;
+            const bool have_acc = t.cls == 0;
+            const int b = i & 1;
+            if (have_acc) {
+                int ok = 1;
+                if (lane == 0) ok = mbar_wait(&acc_full[b], (i / 2) & 1) ? 1 : 0;
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (!ok) {
+                    if (lane == 0) atomicExch(err, S::ERR + 1);
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;");
+            }
+            const bool plain = g.alpha == 1.0 && t.add_off < 0;
+            const int row0 = t.m0 + quarter * 32, nr = min(32, t.M - row0), nv = min(g.tn, t.N - t.n0);
+            double *const C = g.C + t.c_off + int64_t(row0) * t.N + t.n0;
+            const double *const Cadd = t.add_off >= 0 ? g.Cadd + t.add_off + int64_t(row0) * t.N + t.n0 : nullptr;
+#pragma unroll 1
+            for (int col0 = 0; col0 < nv; col0 += EPI_COLS) {
+                if (have_acc) {
+                    uint32_t v[EPI_COLS];
+                    tmem_load16(v, tmem + (uint32_t(quarter * 32) << 16) + uint32_t(b * TMEM_COLS + col0));
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < EPI_COLS; ++j) patch[lane * EPI_PITCH + j] = __uint_as_float(v[j]);
+                    __syncwarp();
+                }
+                // The patch's elements in row-major order, 4 x 32 at a time: (x inv) >> 16 is x / w
+                // for x < 512, w <= 16.  GB300's FP64 pipe is narrow: the plain case (alpha = 1, no
+                // add term) converts with integer operations only; FP64 arithmetic only for
+                // tensorgdot's epilogue.
+                const int w = min(EPI_COLS, nv - col0), n = nr * w, inv = (65536 + w - 1) / w;
+#pragma unroll 1
+                for (int x0 = lane; x0 < n; x0 += 128) {
+                    float f[4];
+                    int64_t at[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int x = min(x0 + 32 * u, n - 1), row = (x * inv) >> 16, col = x - row * w;
+                        f[u] = have_acc ? patch[row * EPI_PITCH + col] : 0.0f;
+                        at[u] = int64_t(row) * t.N + (col0 + col);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (x0 + 32 * u >= n) break;
+                        double val = have_acc ? f32_to_f64_int(f[u], shift) : 0.0;
+                        if (!plain) {
+                            val *= g.alpha;
+                            if (Cadd) val += g.beta * Cadd[at[u]];
+                        }
+                        C[at[u]] = val;
+                    }
+                }
+            }
+            if (have_acc) {
+                asm volatile("tcgen05.fence::before_thread_sync;");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[b]);
+                ++i;
+            }
         }
     }
     __syncthreads();
     if (tid == 0) {
-        // copies issued but never consumed (only after a timeout) must land before exit
+        // copies issued but never consumed (only after a timeout) must land before exit, and
+        // every MMA must have completed before TMEM is freed
         for (int c = n_consumed; c < n_issued; ++c)
-            if (!mbar_wait(&full[c % NSTAGE], (c / NSTAGE) & 1)) atomicExch(err, 2);
+            if (!mbar_wait(&full[c % NSTAGE], (c / NSTAGE) & 1)) atomicExch(err, S::ERR + 1);
+        if (!mbar_wait(&drained, 0)) atomicExch(err, S::ERR + 1);
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
@@ -519,67 +648,71 @@ int *err_word() {
     return c.tc_err;
 }
 
-}  // namespace
-
-int gemm_tile_m(int) { return TBM; }
-int gemm_tile_n(int) { return TBN; }
-
-void launch_split_tf32(const double *src, float *hi, float *lo, const SplitEntry *e, const Chunk *chunks,
-                       int64_t nchunks, const unsigned long long *amax) {
-    if (nchunks <= 0) return;
-    k_split_tf32<<<unsigned(nchunks), 256, 0, ctx().stream>>>(src, hi, lo, e, chunks, amax);
-    count_launch();
-    cuda_check(cudaGetLastError(), "split kernel launch");
+template <class S, int NSTAGE>
+void launch_ring(const TcArgs &a, int grid) {
+    static std::atomic<uint64_t> attr{0};
+    once_per_device(attr, [] {
+        cuda_check(cudaFuncSetAttribute(k_gemm_tc<S, NSTAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        smem_bytes(S::NC, NSTAGE)),
+                   "tcgen05 GEMM smem attribute");
+    });
+    k_gemm_tc<S, NSTAGE><<<grid, TTHREADS, smem_bytes(S::NC, NSTAGE), ctx().stream>>>(a, err_word());
 }
 
-void launch_amax(const double *x, int64_t n, unsigned long long *amax) {
+template <class S>
+void launch_gemm(const TcArgs &a) {
+    // CTAS_PER_SM persistent CTAs an SM; one CTA per tile with the persistent grid switched off.
+    // With no more tiles than SMs a CTA has its SM to itself and takes twice the stages.
+    const int sms = device_sm_count();
+    const int grid = persistent_gemm() ? std::min(a.ntiles, CTAS_PER_SM * sms) : a.ntiles;
+    if (a.ntiles <= sms)
+        launch_ring<S, 2 * S::NSTAGE>(a, grid);
+    else
+        launch_ring<S, S::NSTAGE>(a, grid);
+}
+
+}  // namespace
+
+int gemm_tile_m() { return TBM; }
+int gemm_tile_n(int64_t tiles) { return tiles <= device_sm_count() ? TBN / 2 : TBN; }
+int split_copies(int mode) { return mode == GEMM_BF16X3 ? Bf16x3::NC : Tf32x3::NC; }
+int split_elem_bytes(int mode) { return mode == GEMM_BF16X3 ? Bf16x3::ELEM : Tf32x3::ELEM; }
+int split_chunk_bytes() { return CKB; }
+
+void launch_amax(const AmaxArgs &a) {
+    const int n = a.parts[0] + a.parts[1];
     if (n <= 0) return;
-    const int64_t blocks = std::min<int64_t>((n + 2047) / 2048, 4 * 152);
-    k_amax<<<unsigned(blocks), 256, 0, ctx().stream>>>(x, n, amax);
+    k_amax<<<n, 256, 0, ctx().stream>>>(a);
     count_launch();
     cuda_check(cudaGetLastError(), "amax kernel launch");
 }
 
-int tc_sm_count() { return device_sm_count(); }
-
-void launch_tf32x3_persistent(const TcArgs &a) {
-    static std::atomic<uint64_t> attr{0};
-    once_per_device(attr, [] {
-        cuda_check(cudaFuncSetAttribute(k_gemm_tf32x3_persistent<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        smem_bytes(3)),
-                   "tcgen05 persistent GEMM smem attribute");
-    });
-    const int grid = std::min(a.ntiles, tc_sm_count());
-    k_gemm_tf32x3_persistent<3><<<grid, TTHREADS, smem_bytes(3), ctx().stream>>>(a, err_word());
-}
-
-template <int NST>
-void launch_tf32x3(const TcArgs &a) {
-    static std::atomic<uint64_t> attr{0};
-    once_per_device(attr, [] {
-        cuda_check(cudaFuncSetAttribute(k_gemm_tf32x3<NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(NST)),
-                   "tcgen05 GEMM smem attribute");
-    });
-    k_gemm_tf32x3<NST><<<a.ntiles, TTHREADS, smem_bytes(NST), ctx().stream>>>(a, err_word());
+void launch_split(const SplitArgs &a, int64_t ntiles, int mode, bool flat) {
+    if (ntiles <= 0) return;
+    const unsigned grid = unsigned(ntiles);
+    const cudaStream_t st = ctx().stream;
+    if (mode == GEMM_BF16X3) {
+        if (flat)
+            k_split<Bf16x3, true><<<grid, 256, 0, st>>>(a);
+        else
+            k_split<Bf16x3, false><<<grid, 256, 0, st>>>(a);
+    } else {
+        if (flat)
+            k_split<Tf32x3, true><<<grid, 256, 0, st>>>(a);
+        else
+            k_split<Tf32x3, false><<<grid, 256, 0, st>>>(a);
+    }
+    count_launch();
+    cuda_check(cudaGetLastError(), "split kernel launch");
 }
 
 void launch_gemm_tc(const TcArgs &a, int mode) {
     if (mode != GEMM_TF32X3 && mode != GEMM_BF16X3) fail(ERR_INVALID_ARGUMENT, "unknown tensor-core GEMM mode");
     if (a.ntiles <= 0) return;
-    if (mode == GEMM_BF16X3) {
-        launch_gemm_bf16x3(a, err_word(), ctx().stream);
-        ctx().tc_used = true;
-        return;
-    }
-    const int mc = a.max_chunks;
-    if (a.ntiles >= 2 * tc_sm_count() && persistent_gemm())
-        launch_tf32x3_persistent(a);
-    else if (mc == 1)
-        launch_tf32x3<1>(a);
-    else if (mc == 2)
-        launch_tf32x3<2>(a);
+    if (mode == GEMM_BF16X3)
+        launch_gemm<Bf16x3>(a);
     else
-        launch_tf32x3<3>(a);
+        launch_gemm<Tf32x3>(a);
     count_launch();
     ctx().tc_used = true;
     cuda_check(cudaGetLastError(), "tcgen05 GEMM launch");

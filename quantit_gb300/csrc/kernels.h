@@ -75,85 +75,68 @@ constexpr int F64_STRIP = 8;  // rows or columns of the short side of a strip
 int gemm_f64_class(int64_t M, int64_t N, int64_t K, int *tm, int *tn, bool fine);
 void launch_gemm_f64(const F64Args &a);
 
-// Split-precision tensor-core variant (tcgen05).  Operands are first converted,
-// block by block, into "matrix form" split arrays: hi = tf32(x), lo = tf32(x - hi)
-// as FP32 bit patterns, rows x K4 row-major (K contiguous, K4 = K rounded up to 4,
-// zero padded), so the GEMM producers only move 16-byte vectors.
-// Segment = one operand block; element e of the (rows x K) matrix reads
-// src[src_off + sum_d idx_d(e) * stride[d]] with idx(e) the row-major index over dims.
+// Split-precision tensor-core variant (tcgen05).  Both operands are first converted, block
+// by block, into "matrix form" split arrays (gemm_tc.cu): `copies` arrays per operand
+// (hi / lo TF32, or hi / mid / lo BF16), each rows x K in chunks of split_chunk_bytes() of
+// K per row, rows padded to 8 and K to 32 bytes.  Offsets in them are in bytes.
+// Every element is scaled by the exact power of two 2^-ilogb(max |x| of the operand) before
+// the split, so operands of any magnitude use the FP32 range, and the GEMM epilogue undoes
+// the two scales exactly.
+struct AmaxArgs {
+    const double *x[2];
+    int64_t n[2];
+    int32_t parts[2];          // CTAs of each operand
+    unsigned long long *out;   // one maximum per CTA, operand 0's first
+};
+void launch_amax(const AmaxArgs &a);
 struct SplitEntry {
-    int64_t src_off, dst_off;  // dst_off: element offset of the block in the split arrays
-    // K4: the padded K (rounded up to 8 for TF32X3, 16 for BF16X3); blocks are tiled in
-    // core matrices of 8 rows x 16 bytes (rows padded to 8), a row group's core
-    // matrices in K order
-    int32_t rank, K, K4;
-    int32_t flags;  // SPLIT_SMALL: rows * K < 2^31 (32-bit index math); SPLIT_CONTIG: row-major source
+    int64_t src_off, dst_off;  // source elements; bytes within the operand's split form
+    int32_t operand, rows, K;
+    int32_t kpb;               // padded K in bytes
+    // folded: element (row, k) is at (row / rd2) rs1 + (row % rd2) rs2 + (k / kd2) ks1 + (k % kd2) ks2;
+    // otherwise at the row-major index row K + k over dims, with these strides
+    int32_t folded, rd2, kd2, rank;
+    int64_t rs1, rs2, ks1, ks2;
     int64_t dims[8];
     int64_t stride[8];
 };
-enum : int32_t { SPLIT_SMALL = 1, SPLIT_CONTIG = 2 };
-// Source offset of element `lin` (row-major over dims) of a split entry.
-__device__ __forceinline__ int64_t split_src(const SplitEntry &e, int64_t lin) {
-    if (e.flags & SPLIT_CONTIG) return e.src_off + lin;
-    if (e.flags & SPLIT_SMALL) {
-        uint32_t rem = uint32_t(lin), off = 0;
-        for (int d = e.rank - 1; d >= 0; --d) {
-            const uint32_t n = uint32_t(e.dims[d]), q = rem / n;
-            off += (rem - q * n) * uint32_t(e.stride[d]);
-            rem = q;
-        }
-        return e.src_off + off;
-    }
-    int64_t rem = lin, so = e.src_off;
-    for (int d = e.rank - 1; d >= 0; --d) {
-        const int64_t n = e.dims[d], q = rem / n;
-        so += (rem - q * n) * e.stride[d];
-        rem = q;
-    }
-    return so;
-}
-// (row, k) of element `lin` of a split entry's rows x K matrix.
-__device__ __forceinline__ void split_rowk(const SplitEntry &e, int64_t lin, int64_t &row, int64_t &k) {
-    if (e.flags & SPLIT_SMALL) {
-        const uint32_t r = uint32_t(lin) / uint32_t(e.K);
-        row = r;
-        k = int64_t(uint32_t(lin) - r * uint32_t(e.K));
-    } else {
-        row = lin / e.K;
-        k = lin - row * e.K;
-    }
-}
-// amax: the bit pattern of max |x| over the operand (launch_amax); every element is
-// scaled by the exact power of two 2^-ilogb(amax) before the split, so operands of any
-// magnitude use the FP32 range, and the GEMM epilogue undoes the two scales exactly.
-void launch_split_tf32(const double *src, float *hi, float *lo, const SplitEntry *e, const Chunk *chunks,
-                       int64_t nchunks, const unsigned long long *amax);
-// *amax (zeroed by the caller) <- max(*amax, bits of |x|) over n doubles (bit order =
-// value order for non-negative doubles, so the maximum is exact and deterministic).
-void launch_amax(const double *x, int64_t n, unsigned long long *amax);
-// Split-BF16 variant: hi / mid / lo bf16 (uint16) arrays in the same tiling (core
-// matrices of 8 rows x 8 elements, K padded to 16); the same amax scaling.
-void launch_split_bf16x3(const double *src, void *hi, void *mid, void *lo, const SplitEntry *e, const Chunk *chunks,
-                         int64_t nchunks, const unsigned long long *amax);
-// A pair's a_off / b_off index the split arrays (core-matrix tiling); A rows = M,
-// B rows = N (TF32X3: hi / lo, mid unused; BF16X3: hi / mid / lo).
+// One CTA: `rows` rows from row0 (a multiple of 8) of one chunk (k0b: its first byte of K).
+struct SplitTile {
+    int32_t ent, row0, rows, k0b;
+};
+struct SplitArgs {
+    const double *src[2];
+    char *dst[2];
+    const SplitEntry *ents;
+    const SplitTile *tiles;
+    const unsigned long long *amax_parts;
+    int32_t parts[2];
+    unsigned long long *amax;  // receives the two operands' maxima
+};
+// flat: every entry is folded with rd2 >= rows and kd2 >= K (one stride each)
+void launch_split(const SplitArgs &a, int64_t ntiles, int mode, bool flat);
+int split_copies(int mode);
+int split_elem_bytes(int mode);
+int split_chunk_bytes();
+// A pair's a_off / b_off: byte offsets of its blocks in split form; A rows = M,
+// B rows = N.  A tile whose pairs all have K = 0 has cls 1, the others 0.
 struct TcArgs {
-    const void *Ahi, *Amid, *Alo, *Bhi, *Bmid, *Blo;
-    const unsigned long long *amax_a, *amax_b;  // operand scales (see launch_split_tf32)
+    const char *A, *B;
+    const unsigned long long *amax;
     double *C;
     const double *Cadd;
     const GemmPair *pairs;
     const GemmOut *outs;
     const GemmTile *tiles;
     int32_t ntiles;
-    int32_t max_chunks;  // most K chunks of any tile (sizes the shared-memory ring; 0: unknown)
+    int32_t tn;  // columns of a tile: gemm_tile_n
     double alpha, beta;
 };
 void launch_gemm_tc(const TcArgs &a, int mode);
-// the BF16X3 kernel (called by launch_gemm_tc); err: the context's device error word
-void launch_gemm_bf16x3(const TcArgs &a, int *err, cudaStream_t stream);
-int gemm_tile_m(int mode);
-int gemm_tile_n(int mode);
+int gemm_tile_m();
+// Tile columns for a launch of `tiles` tiles of 128 columns: 128, or 64 where those would not
+// fill the SMs.
+int gemm_tile_n(int64_t tiles);
 
 // ------------------------------------------------------------ elementwise
 // A coefficient: mult * (dev ? f(*dev) : 1) with f(x) = x, or f(x) = 1/x when
