@@ -59,12 +59,20 @@ __device__ __forceinline__ float ldcg(const float *p) { return __ldcg(p); }
 // For small angles c rounds to 1 while 1 - c = s tau does not, so the plain form
 // c x - s y would scale both columns by sqrt(1 + t^2) at every such rotation; in
 // FP32 that bias accumulates to ~1e-5 in the singular values over a few sweeps.
+// In FP64 the same rotation as three shears, x -= tau y, y += s x, x -= tau y: three
+// instead of four instructions of GB300's narrow FP64 pipe per element pair.
 template <class T>
 __device__ __forceinline__ void rot_apply(T &x, T &y, T s, T tau) {
-    const T u = fma(tau, x, y);
-    const T v = fma(-tau, y, x);
-    x = fma(-s, u, x);
-    y = fma(s, v, y);
+    if constexpr (sizeof(T) == 8) {
+        x = fma(-tau, y, x);
+        y = fma(s, x, y);
+        x = fma(-tau, y, x);
+    } else {
+        const T u = fma(tau, x, y);
+        const T v = fma(-tau, y, x);
+        x = fma(-s, u, x);
+        y = fma(s, v, y);
+    }
 }
 
 // Hestenes rotation for column norms al, be and inner product ga: s and tau.
@@ -506,6 +514,76 @@ __device__ __forceinline__ void bj_params_fast(float al, float be, float ga, flo
     tau = __fdividef(t, 1.0f + w2 * rh);
 }
 
+// x 2^-sh as FP32 by integer operations (no FP64 conversion): sh within the exponent range,
+// results below FP32's normal range flush to zero, above it are not allowed for.
+__device__ __forceinline__ float scaled_f32(double x, int sh) {
+    const uint32_t hi = uint32_t(__double2hiint(x)), lo = uint32_t(__double2loint(x));
+    const int t = int(hi & 0x7FFFFFFFu) - ((896 + sh) << 20);
+    const uint32_t f = __funnelshift_l(lo, uint32_t(t), 3);
+    return __uint_as_float((hi & 0x80000000u) | (t < (1 << 20) ? 0u : f));
+}
+// FP32 (normal or zero) -> FP64 by integer operations.
+__device__ __forceinline__ double widen_f32(float f) {
+    const uint32_t b = __float_as_uint(f), m = b & 0x7FFFFFFFu;
+    const uint32_t hi = (b & 0x80000000u) | (m < 0x00800000u ? 0u : (m >> 3) + (896u << 20));
+    return __hiloint2double(int(hi), m < 0x00800000u ? 0 : int(b << 29));
+}
+
+// FP64 rotation parameters with few FP64 instructions.  GB300 issues an FP64 warp
+// instruction in 64 clocks per scheduler, so the square roots and divisions of
+// rot_params (over 100 instructions with their FP64 iterations) cost a round more than
+// its columns up to p ~ 1000.  The angle need not be the exact optimum -- any tau gives an
+// orthogonal rotation as long as s = 2 tau / (1 + tau^2) holds to FP64, and an angle off by
+// 1e-7 leaves 1e-7 of the coupling, which the quadratic convergence of the sweeps leaves
+// behind anyway -- so tau comes from FP32 and the multi-function unit, on operands brought
+// into FP32's range by their exponents, and only s (a reciprocal with one cubically convergent
+// step) and the norms' update are FP64: 12 instructions.  The difference of the norms is
+// formed in FP64 first: near-equal norms would lose it in FP32.
+// Returns 0: no rotation (coupling within tol), 1: s, tau, rel set and al, be updated, 2: norms
+// further apart than FP32's exponents allow for (the caller takes the plain formulas).
+__device__ __forceinline__ int bj_params_fast64(double &al, double &be, double ga, float tol, double &sn, double &tau,
+                                                float &rel) {
+    const int ea = int((uint32_t(__double2hiint(al)) >> 20) & 0x7FFu), eb = int((uint32_t(__double2hiint(be)) >> 20) & 0x7FFu);
+    // half the exponents: columns of norm ~ 2^ka, 2^kb
+    const int ka = (ea - 1023) >> 1, kb = (eb - 1023) >> 1, d = kb - ka, sh = ka + kb;
+    if (d > 50 || d < -50 || ea < 64 || eb < 64 || ea > 1982 || eb > 1982) return 2;
+    const float ma = scaled_f32(al, 2 * ka), mb = scaled_f32(be, 2 * kb);  // in [1, 4)
+    const float g = scaled_f32(ga, sh);                                    // |g| <= 4
+    rel = fabsf(g) * rsqrtf(ma) * rsqrtf(mb);
+    if (!(rel > tol)) return 0;
+    const double diff = be - al;
+    const float df = scaled_f32(diff, sh);                                 // up to 2^52
+    const float zeta = __fdividef(df, 2.0f * g), az = fabsf(zeta);         // up to 2^105
+    float t;
+    if (az > 1e9f)
+        t = __fdividef(0.5f, zeta);
+    else {
+        const float w = fmaf(zeta, zeta, 1.0f);
+        t = copysignf(__fdividef(1.0f, az + w * rsqrtf(w)), zeta);
+    }
+    const float w2 = fmaf(t, t, 1.0f);
+    const float tf = __fdividef(t, 1.0f + w2 * rsqrtf(w2));  // tan(theta / 2), |tf| <= 0.4143
+    if (fabsf(tf) < 1.17549435e-38f) return 2;
+    tau = widen_f32(tf);
+    const double r0 = widen_f32(__fdividef(1.0f, fmaf(tf, tf, 1.0f)));  // 1 / (1 + tau^2) to ~1e-7
+    const double u = fma(tau, tau, 1.0);
+    const double e = fma(-u, r0, 1.0);
+    const double r = fma(r0, fma(e, e, e), r0);              // to FP64 precision (e^3)
+    sn = (tau + tau) * r;
+    const double c = fma(-sn, tau, 1.0);
+    const double q = fma(-c, ga + ga, sn * diff);            // al' = c^2 al - 2 c s ga + s^2 be
+    al = fma(sn, q, al);
+    be = fma(-sn, q, be);
+    return 1;
+}
+
+// Whether an updated squared norm kept more than 1/16 of the old one (FP64: by the high words,
+// without an FP64 instruction).
+__device__ __forceinline__ bool norm_kept(float a2, float al) { return a2 > al * 0.0625f; }
+__device__ __forceinline__ bool norm_kept(double a2, double al) {
+    return __double2hiint(a2) > __double2hiint(al) - (4 << 20);
+}
+
 // Hestenes rotation of two register-resident columns with tracked squared norms
 // al, be: only the inner product is formed; after the rotation the norms follow
 // from al' = al - t ga, be' = be + t ga (t = tan theta), and are recomputed from
@@ -521,23 +599,36 @@ __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], T &al, T &be, T 
     if (pair_skipped(al, be, skip)) return false;
     const T ga = bj_dot(x, y);
     if (ga == T(0)) return false;
-    T t;
+    T t, a2, b2;
     if constexpr (sizeof(T) == 4) {
         const float rel = fabsf(ga) * rsqrtf(al) * rsqrtf(be);
         if (rel <= tol) return false;
         rmax = fmaxf(rmax, rel);
         bj_params_fast(al, be, ga, sn, tau, t);
+        a2 = al - t * ga;
+        b2 = be + t * ga;
     } else {
-        const double rel = fabs(ga) / sqrt(al * be);
-        if (rel <= tol) return false;
-        rmax = fmaxf(rmax, float(rel));
-        rot_params(al, be, ga, sn, tau, t);
+        float rel32;
+        a2 = al;
+        b2 = be;
+        const int how = bj_params_fast64(a2, b2, ga, float(tol), sn, tau, rel32);
+        if (how == 0) return false;
+        if (how == 1) {
+            rmax = fmaxf(rmax, rel32);
+        } else {
+            const double rel = fabs(ga) / (sqrt(al) * sqrt(be));
+            if (!(rel > tol)) return false;
+            rmax = fmaxf(rmax, float(rel));
+            rot_params(al, be, ga, sn, tau, t);
+            a2 = al - t * ga;
+            b2 = be + t * ga;
+        }
     }
 #pragma unroll
     for (int i = 0; i < R; ++i) rot_apply(x[i], y[i], sn, tau);
-    const T a2 = al - t * ga, b2 = be + t * ga;
-    al = (a2 > al * T(0.0625)) ? a2 : bj_dot(x, x);
-    be = (b2 > be * T(0.0625)) ? b2 : bj_dot(y, y);
+    // recomputed when the update cancelled (an exponent comparison: 1/16 of the norm)
+    al = norm_kept(a2, al) ? a2 : bj_dot(x, x);
+    be = norm_kept(b2, be) ? b2 : bj_dot(y, y);
     if (thr > T(0)) {
         if (al <= thr) {
 #pragma unroll
@@ -947,10 +1038,12 @@ __global__ void __launch_bounds__(1024) k_finish(const T *__restrict__ work, con
     }
     __syncthreads();
     for (int j = threadIdx.x; j < q; j += blockDim.x) {
-        double v = sig[j];
+        // bit order: that of the (non-negative) values, and total, so that the ranks are a
+        // permutation even with NaN among them
+        const long long v = __double_as_longlong(sig[j]);
         int rk = 0;
         for (int i = 0; i < q; ++i) {
-            double u = sig[i];
+            const long long u = __double_as_longlong(sig[i]);
             bool before = sd.mode == 0 ? (u > v || (u == v && i < j)) : (u < v || (u == v && i < j));
             rk += before;
         }
@@ -1235,10 +1328,15 @@ bool bjacobi_launch(const BJacobiParams<T> &P, int max_block_steps, int64_t sum_
     return true;
 }
 
-// Register slice (elements per lane and column) for columns of at most max_p.
-int r_class(int max_p) {
-    for (int R : {4, 8, 16, 24, 32, 48, 64})
-        if (max_p <= 32 * R) return R;
+// Register slice (elements per lane and column) for columns of at most max_p.  A slice longer
+// than the columns is work on zeros, and in FP64 every element of it costs 64 clocks a warp
+// instruction: fine steps there.
+int r_class(int max_p, bool f32) {
+    static constexpr int f32_r[] = {4, 8, 12, 16, 24, 32, 48, 64};
+    static constexpr int f64_r[] = {2, 4, 6, 8, 10, 12, 16, 20, 24, 28, 32, 40, 48, 64};
+    const int *r = f32 ? f32_r : f64_r;
+    for (int i = 0, n = f32 ? 8 : 14; i < n; ++i)
+        if (max_p <= 32 * r[i]) return r[i];
     return 0;
 }
 
@@ -1264,15 +1362,17 @@ bool bjacobi_dispatch(const BJacobiParams<T> &P, int max_steps_per_sweep, int ma
         const int nb = (max_qp + b - 1) / b;
         return nb + (nb & 1) - 1;
     };
-    const int R = r_class(max_p);
+    const int R = r_class(max_p, sizeof(T) == 4);
 #define QTT_BJ(BB, RR)                                                                                            \
     if (B == BB && R == RR) return bjacobi_launch<T, BB, RR>(P, steps(BB), sum_q, vwork, vwork_bytes, stream);
     if constexpr (sizeof(T) == 4) {
-        QTT_BJ(16, 4) QTT_BJ(16, 8) QTT_BJ(16, 16) QTT_BJ(16, 24) QTT_BJ(16, 32)
-        QTT_BJ(8, 4) QTT_BJ(8, 8) QTT_BJ(8, 16) QTT_BJ(8, 24) QTT_BJ(8, 32) QTT_BJ(8, 48) QTT_BJ(8, 64)
+        QTT_BJ(16, 4) QTT_BJ(16, 8) QTT_BJ(16, 12) QTT_BJ(16, 16) QTT_BJ(16, 24) QTT_BJ(16, 32)
+        QTT_BJ(8, 4) QTT_BJ(8, 8) QTT_BJ(8, 12) QTT_BJ(8, 16) QTT_BJ(8, 24) QTT_BJ(8, 32) QTT_BJ(8, 48) QTT_BJ(8, 64)
     } else {
-        QTT_BJ(8, 4) QTT_BJ(8, 8) QTT_BJ(8, 16) QTT_BJ(8, 24) QTT_BJ(8, 32) QTT_BJ(8, 48)
-        QTT_BJ(4, 4) QTT_BJ(4, 8) QTT_BJ(4, 16) QTT_BJ(4, 24) QTT_BJ(4, 32) QTT_BJ(4, 48)
+        QTT_BJ(8, 2) QTT_BJ(8, 4) QTT_BJ(8, 6) QTT_BJ(8, 8) QTT_BJ(8, 10) QTT_BJ(8, 12) QTT_BJ(8, 16) QTT_BJ(8, 20)
+        QTT_BJ(8, 24) QTT_BJ(8, 28) QTT_BJ(8, 32) QTT_BJ(8, 40) QTT_BJ(8, 48)
+        QTT_BJ(4, 2) QTT_BJ(4, 4) QTT_BJ(4, 6) QTT_BJ(4, 8) QTT_BJ(4, 10) QTT_BJ(4, 12) QTT_BJ(4, 16) QTT_BJ(4, 20)
+        QTT_BJ(4, 24) QTT_BJ(4, 28) QTT_BJ(4, 32) QTT_BJ(4, 40) QTT_BJ(4, 48)
     }
 #undef QTT_BJ
     return false;
@@ -1354,11 +1454,11 @@ void jacobi_impl(T *work, T *rot, const SectorDesc *sec, const int *slot_start, 
         B.skip = skip;
         B.max_q = max_steps_per_sweep + 1;  // the widest sector's even column count bounds q
         const bool f32 = sizeof(T) == 4;
-        const std::vector<int> cands = block_widths(f32, r_class(max_p));
+        const std::vector<int> cands = block_widths(f32, r_class(max_p, f32));
         if (!cands.empty()) {
             int ci = 0;
             bool timing = false;
-            const TuneKey key{f32 ? 1 : 0, r_class(max_p), ceil_log2(max_steps_per_sweep + 1), ceil_log2(nsec)};
+            const TuneKey key{f32 ? 1 : 0, r_class(max_p, f32), ceil_log2(max_steps_per_sweep + 1), ceil_log2(nsec)};
             if (g_autotune.load() && cands.size() > 1) {
                 std::lock_guard<std::mutex> lk(g_tune_mu);
                 tune_load_locked();
