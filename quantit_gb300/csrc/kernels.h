@@ -194,6 +194,16 @@ struct WarmDesc {
     int32_t p, q, tile_start, pad;
 };
 void launch_warm_apply(void *work, void *rot, void *tmp, const WarmDesc *wd, int nwarm, int ntiles, int f32);
+// LQ preconditioning (lq.cu): for each listed sector work (p x q, column-major at w_off) <- W Q and
+// rot (q x q at rot_off) <- Q, or rot Q with from_rot, Q orthogonal, W Q lower trapezoidal on its rows by falling norm.
+// 2 <= q <= lq_max_q(f32, sectors) <= p.  The other offsets are the launcher's.
+struct LqSec {
+    int64_t w_off, rot_off, x_off, v_off, o_off;
+    int32_t p, q, from_rot, pad;
+};
+constexpr size_t LQ_SMEM_MAX = 200 * 1024;
+int lq_max_q(int f32, int nsec);
+void launch_lq(void *work, void *rot, const std::vector<LqSec> &secs, int f32);
 // FP64 refinement of an FP32 sector decomposition (mixed path): from the FP32
 // rotations rot32 (at rot_off), vb <- the FP64-orthogonalised rotation (two
 // Newton-Schulz steps through va, with g as q x q scratch), w1 <- w64 vb (at w_off).

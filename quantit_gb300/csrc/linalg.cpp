@@ -248,7 +248,9 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     // The mixed path (split-precision block GEMMs) runs its SVD sweeps in FP32 first and
     // finishes them in FP64 (svd_refine.cu): the result is an FP64 SVD either way.  eigh
     // always runs in FP64.
-    const int f32 = (mode == 0 && gemm_mode() != GEMM_F64) ? 1 : 0;
+    // A decomposition that is run again because its estimated truncation fell short is FP64 throughout.
+    const bool redo = trunc_hint().active && !trunc_hint().allow_discard;
+    const int f32 = (mode == 0 && gemm_mode() != GEMM_F64 && !redo) ? 1 : 0;
     const size_t es = f32 ? 4 : 8;
     D.work = dev_alloc(size_t(std::max<int64_t>(wtot, 1)) * es);
     D.rot = dev_alloc(size_t(std::max<int64_t>(rtot, 1)) * es);
@@ -282,9 +284,28 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             }
         }
     }
+    // Sectors that are LQ-preconditioned (lq.cu).  Under a truncation, from 12 columns on: svd of a
+    // graded theta at D = 60 1664 -> 907 us, at D = 100 2846 -> 1383, at D = 600 35.0 -> 12.7 ms.
+    // The plain svd also sees matrices that are not graded (bMPS.move_oc of a random state), where
+    // the sweeps saved do not pay for the factorisation of a small sector: D = 120 806 us without
+    // against 925 with.  With the deflation switched off the sweeps run from the identity as well: null
+    // columns that stay in keep a factored start sweeping as long.
+    const int lq_least = !trunc_hint().active ? 48 : (svd_deflation() ? 12 : INT32_MAX);
+    auto lq_fits = [&](const SectorDesc &d, int prec32) { return d.q >= lq_least && d.q <= lq_max_q(prec32, nsec); };
+    auto lq_of = [](const SectorDesc &d, bool from_rot) {
+        LqSec s{};
+        s.w_off = d.w_off;
+        s.rot_off = d.rot_off;
+        s.p = d.p;
+        s.q = d.q;
+        s.from_rot = from_rot ? 1 : 0;
+        return s;
+    };
     // warm starts: a sector whose key (orientation, batch element, q-side sections) matches
     // an entry of the previous decomposition at this bond starts from that rotation; the
-    // long side may differ (W V0 is defined for any number of rows)
+    // long side may differ (W V0 is defined for any number of rows).  The LQ factorisation beats
+    // it also on a converged state (sweeps of the L = 32 chain at D = 128 / 256, FP64: 132 / 250 ms
+    // warm, 111 / 206 ms factored), so only sectors below its range start warm.
     WarmStart *ws = mode == 0 ? trunc_hint().ws : nullptr;
     std::vector<std::vector<int64_t>> keys;
     std::vector<WarmDesc> wdesc;
@@ -301,7 +322,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                     key.push_back(sr.size);
                 }
                 for (const WarmStart::Entry &en : ws->entries) {
-                    if (en.f32 != f32 || en.key != key || d.q < 2) continue;
+                    if (en.f32 != f32 || en.key != key || d.q < 2 || lq_fits(d, f32)) continue;
                     d.warm = 1;
                     WarmDesc w{};
                     w.w_off = d.w_off;
@@ -318,6 +339,14 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             }
         }
     }
+    // the other sectors start from the Q of an LQ factorisation
+    std::vector<LqSec> lq;
+    if (mode == 0)
+        for (SectorDesc &d : D.desc)
+            if (lq_fits(d, f32)) {
+                lq.push_back(lq_of(d, false));
+                d.warm = 1;
+            }
     SectorDesc *dsec = static_cast<SectorDesc *>(upload(D.desc.data(), D.desc.size() * sizeof(SectorDesc)));
     const int64_t packed = std::accumulate(lens.begin(), lens.end(), int64_t(0));
     const PackEntry *dpe = upload_vec(pe);
@@ -366,6 +395,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             BufPtr tmp = dev_alloc(size_t(std::max<int64_t>(wtot, 1)) * es);
             launch_warm_apply(W, D.rot->p, tmp->p, upload_vec(wdesc), int(wdesc.size()), ntiles, f32);
         }
+        launch_lq(W, D.rot->p, lq, f32);
         const int *dslots = upload_vec(slots);
         launch_jacobi(W, D.rot->p, dsec, dslots, nsec, max_steps, max_sweeps, sweeps, flags, f32, max_p, stot,
                       vwork->p, vb, deflate ? thr->p : nullptr, deflate ? dnorm->p : nullptr);
@@ -379,6 +409,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
         // >= 4 eps32 ||W_s|| carries FP32 rounding noise of at most a quarter of itself.  The
         // truncation is checked against tau all the same (svd_truncated).
         std::vector<double> discard, null2;
+        bool resolve_anew = false;  // the truncation was estimated to reach below FP32's resolution
         std::vector<int> kept_cols;  // discard path: columns of each sector's compact restricted sweeps
         TruncHint &th = trunc_hint();
         if (f32 && deflate && th.allow_discard && th.max_size > 0) {
@@ -394,22 +425,24 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             const double t_est = kept_threshold(vals, th.tol, th.pw, th.min_size, th.max_size);
             discard.assign(nsec, 0.0);
             null2.assign(nsec, 0.0);
-            double tau_max = 0.0;
+            // The level has to clear FP32's resolution in every sector: the noise of one that it does
+            // not clear is among the values the threshold was estimated from (estimates from such
+            // noise had the decomposition run twice: D = 600, 14 decades 31.8 ms, FP64 alone 12.8).
+            const double tau = 0.5 * t_est;
+            bool clears = t_est > 0.0;
             for (int i = 0; i < nsec; ++i) {
                 const SectorDesc &d = D.desc[i];
                 double f2 = 0.0;
                 for (int j = 0; j < d.q; ++j) f2 += n2[d.s_off + j];
                 null2[i] = kDeflateF64 * kDeflateF64 * f2;
-                const double tau = 0.5 * t_est;
-                if (t_est > 0.0 && tau > 4.0 * kDeflateF32 * std::sqrt(f2)) {
-                    discard[i] = tau;
-                    tau_max = std::max(tau_max, tau);
-                }
+                discard[i] = tau;
+                clears = clears && tau > 4.0 * kDeflateF32 * std::sqrt(f2);
             }
-            if (tau_max > 0.0)
-                th.discard_tau = std::max(th.discard_tau, tau_max);
+            if (clears)
+                th.discard_tau = std::max(th.discard_tau, tau);
             else
                 discard.clear();
+            resolve_anew = discard.empty();
         }
         if (f32) {
             StatScope sc64(ST_SVD64, 0.0);
@@ -422,11 +455,27 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             gbuf = dev_alloc(size_t(std::max<int64_t>(rtot, 1)) * 8);
             cuda_check(cudaMemsetAsync(w64->p, 0, size_t(wtot) * 8, ctx().stream), "cudaMemsetAsync(work64)");
             launch_pack(static_cast<const double *>(t.data()), w64->p, dpe, dch, int64_t(chunks.size()), dsec, 0);
-            launch_svd_refine(static_cast<const float *>(D.rot->p), static_cast<const double *>(w64->p),
-                              static_cast<double *>(w1->p), static_cast<double *>(va->p),
-                              static_cast<double *>(vbuf->p), static_cast<double *>(gbuf->p), D.desc);
+            std::vector<LqSec> lq64;
+            if (resolve_anew) {
+                // The truncation reaches below FP32's resolution: the values there have to be resolved
+                // in FP64 from scratch, and the factored FP64 sweeps do that from the matrix itself as
+                // quickly as from the FP32 rotation (D = 600: 35.8 ms with the refinement, 12.8 ms the
+                // FP64 sweeps alone).
+                cuda_check(cudaMemcpyAsync(w1->p, w64->p, size_t(wtot) * 8, cudaMemcpyDeviceToDevice, ctx().stream),
+                           "cudaMemcpyAsync(work64)");
+            } else {
+                launch_svd_refine(static_cast<const float *>(D.rot->p), static_cast<const double *>(w64->p),
+                                  static_cast<double *>(w1->p), static_cast<double *>(va->p),
+                                  static_cast<double *>(vbuf->p), static_cast<double *>(gbuf->p), D.desc);
+            }
             std::vector<SectorDesc> d64 = D.desc;
-            for (SectorDesc &d : d64) d.warm = 1;
+            for (SectorDesc &d : d64) {
+                d.warm = resolve_anew ? 0 : 1;
+                if (discard.empty() && lq_fits(d, 0)) {
+                    lq64.push_back(lq_of(d, !resolve_anew));
+                    d.warm = 1;
+                }
+            }
             const SectorDesc *dsec64 = upload_vec(d64);
             ibuf64 = dev_alloc(size_t(nsec) * (max_sweeps + 1) * sizeof(int));
             int *sw64 = static_cast<int *>(ibuf64->p);
@@ -442,6 +491,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                               skip);
             };
             if (discard.empty()) {
+                launch_lq(w1->p, vbuf->p, lq64, 0);
                 fp64_sweeps(max_sweeps, thr64 ? thr64->p : nullptr, nullptr);
             } else {
                 // one sweep decouples the columns (pairs of two discarded columns stay as they
@@ -531,7 +581,11 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             fw = w1->p;
             fr = vbuf->p;
         }
-        last_sweeps() = {f32 ? ibuf64 : ibuf, ibuf, nsec, f32 != 0};
+        // (a decomposition run again keeps the record of the FP32 sweeps before its first run)
+        if (redo && last_sweeps().mixed && last_sweeps().n == nsec)
+            last_sweeps().buf = ibuf;
+        else
+            last_sweeps() = {f32 ? ibuf64 : ibuf, ibuf, nsec, f32 != 0};
         if (mode == 0 && stats_enabled() && !ctx().capturing) {
             // the sweeps' FLOPs, read from the sweep counters once the statistics are read
             cudaEvent_t raw = nullptr;
