@@ -80,6 +80,7 @@ bool is_identity(const std::vector<int64_t> &p) {
 
 namespace {
 void host_join(ContractPlan &P, const BT &A, const BT &B, int dl);
+bool host_join_packed(ContractPlan &P, const BT &A, const BT &B, int dl);
 void set_operand_modes(ContractPlan &P);
 
 bool device_present() {
@@ -180,7 +181,7 @@ ContractPlan plan_contraction(const BT &A, const BT &B, const std::vector<int64_
             host_check();
         }
     }
-    if (!on_device) host_join(P, A, B, dl);
+    if (!on_device && !host_join_packed(P, A, B, dl)) host_join(P, A, B, dl);
     o.boff.assign(P.out_p0.size(), 0);
     o.compact_offsets();
     set_operand_modes(P);
@@ -190,6 +191,100 @@ ContractPlan plan_contraction(const BT &A, const BT &B, const std::vector<int64_
 }
 
 namespace {
+// A block's legs in the order `perm` packed into one integer, the first leg most significant: integer
+// order is the lexicographic order of the permuted indices.
+struct KeyBlock {
+    uint64_t key;
+    int32_t id;
+};
+int leg_bits(const BT &t, int64_t d) {
+    int b = 0;
+    while ((int64_t(1) << b) < t.sbd[d]) ++b;
+    return b;
+}
+std::vector<KeyBlock> packed_sorted(const BT &t, const std::vector<int64_t> &perm) {
+    const int64_t nb = t.nblocks();
+    int bits[MAXRANK];
+    for (int i = 0; i < t.rank; ++i) bits[i] = leg_bits(t, perm[i]);
+    std::vector<KeyBlock> out(nb);
+    bool sorted = true;
+    for (int64_t b = 0; b < nb; ++b) {
+        const int64_t *ix = t.idx(b);
+        uint64_t k = 0;
+        for (int i = 0; i < t.rank; ++i) k = k << bits[i] | uint64_t(ix[perm[i]]);
+        out[b] = KeyBlock{k, int32_t(b)};
+        sorted = sorted && (b == 0 || out[b - 1].key < k);
+    }
+    if (!sorted) std::sort(out.begin(), out.end(), [](const KeyBlock &x, const KeyBlock &y) { return x.key < y.key; });
+    return out;
+}
+
+// host_join on packed keys: the same output block list and pair order.  False when the keys do not
+// fit 63 bits, or the contracted part 32 (nothing done).
+bool host_join_packed(ContractPlan &P, const BT &A, const BT &B, int dl) {
+    int abits = 0, bbits = 0, sbits = 0;
+    for (int i = 0; i < A.rank; ++i) abits += leg_bits(A, i);
+    for (int i = 0; i < B.rank; ++i) bbits += leg_bits(B, i);
+    for (int i = 0; i < dl; ++i) sbits += leg_bits(A, P.dA[i]);
+    if (abits > 63 || bbits > 63 || sbits > 31 || A.nblocks() > INT32_MAX || B.nblocks() > INT32_MAX) return false;
+    BT &o = P.out;
+    const std::vector<KeyBlock> ka = packed_sorted(A, P.p1), kb = packed_sorted(B, P.p2p);
+    const int64_t na = int64_t(ka.size()), nb = int64_t(kb.size());
+    const uint64_t smask = (uint64_t(1) << sbits) - 1;
+    // runs of B (equal free prefix) and its entries by (contracted suffix, position): positions follow
+    // the runs, so the entries of one suffix are in run order
+    std::vector<int32_t> run(nb);
+    std::vector<uint64_t> by_suffix(nb);
+    for (int64_t i = 0; i < nb; ++i) {
+        run[i] = i == 0 ? 0 : run[i - 1] + (kb[i].key >> sbits != kb[i - 1].key >> sbits ? 1 : 0);
+        by_suffix[i] = (kb[i].key & smask) << 32 | uint64_t(i);
+    }
+    std::sort(by_suffix.begin(), by_suffix.end());
+    // where each suffix starts, for all of them if they are few
+    std::vector<int32_t> first;
+    if (sbits <= 14) {
+        first.assign((size_t(1) << sbits) + 1, 0);
+        for (uint64_t e : by_suffix) ++first[(e >> 32) + 1];
+        for (size_t k = 1; k < first.size(); ++k) first[k] += first[k - 1];
+    }
+    struct Match {
+        uint64_t order;  // run of B, then position within the run of A (the suffix order)
+        int32_t pos;
+    };
+    std::vector<Match> m;
+    for (int64_t i0 = 0; i0 < na;) {
+        int64_t i1 = i0 + 1;
+        while (i1 < na && ka[i1].key >> sbits == ka[i0].key >> sbits) ++i1;
+        m.clear();
+        for (int64_t i = i0; i < i1; ++i) {
+            const uint64_t s = ka[i].key & smask;
+            int64_t at = first.empty() ? std::lower_bound(by_suffix.begin(), by_suffix.end(), s << 32) - by_suffix.begin()
+                                       : first[s];
+            for (; at < nb && by_suffix[at] >> 32 == s; ++at) {
+                const int32_t pos = int32_t(by_suffix[at] & 0xFFFFFFFFu);
+                m.push_back(Match{uint64_t(run[pos]) << 32 | uint64_t(i - i0), pos});
+            }
+        }
+        if (i1 - i0 > 1) std::sort(m.begin(), m.end(), [](const Match &x, const Match &y) { return x.order < y.order; });
+        const int64_t *ia = A.idx(ka[i0].id);
+        for (size_t k = 0; k < m.size();) {
+            size_t e = k;
+            P.out_p0.push_back(int64_t(P.pair_a.size()));
+            for (; e < m.size() && m[e].order >> 32 == m[k].order >> 32; ++e) {
+                P.pair_a.push_back(ka[i0 + int64_t(m[e].order & 0xFFFFFFFFu)].id);
+                P.pair_b.push_back(kb[m[e].pos].id);
+            }
+            P.out_p1.push_back(int64_t(P.pair_a.size()));
+            const int64_t *ib = B.idx(kb[m[k].pos].id);
+            for (auto d : P.freeA) o.bidx.push_back(ia[d]);
+            for (auto d : P.freeB) o.bidx.push_back(ib[d]);
+            k = e;
+        }
+        i0 = i1;
+    }
+    return true;
+}
+
 void host_join(ContractPlan &P, const BT &A, const BT &B, int dl) {
     BT &o = P.out;
     // merge-join (btensor.cpp:1998-2114): for every run of A (equal free prefix) and
@@ -318,6 +413,18 @@ int64_t prod_sizes(const BT &t, int64_t b, const std::vector<int64_t> &dims) {
     for (auto d : dims) p *= shp[d];
     return p;
 }
+// the product of the sizes of legs `dims`, for every block
+std::vector<int64_t> sizes_of(const BT &t, const std::vector<int64_t> &dims) {
+    const auto ad = t.addrs();
+    std::vector<int64_t> out(t.nblocks());
+    for (int64_t b = 0; b < t.nblocks(); ++b) {
+        const int64_t *ix = t.idx(b);
+        int64_t p = 1;
+        for (auto d : dims) p *= t.ssz[ad[d] + ix[d]];
+        out[b] = p;
+    }
+    return out;
+}
 }  // namespace
 
 namespace {
@@ -377,45 +484,67 @@ Strided block_strides(const BT &t, int64_t b) {
 // not fold to two strides or a stride exceeds 32 bits (the caller packs the operands).
 bool f64_pairs_in_place(const ContractPlan &P, const BT &A, const BT &B, std::vector<F64Pair> &out) {
     auto fits = [](int64_t v) { return v <= INT32_MAX; };
-    std::vector<Strided> sa(A.nblocks()), sb(B.nblocks());
-    std::vector<Fold> fa(A.nblocks()), fb(B.nblocks());
-    auto free_legs = [&](const BT &t, const std::vector<int64_t> &legs, std::vector<Strided> &st, std::vector<Fold> &fo) {
+    // per block: the folded free legs, and the contracted legs of more than one element (the same
+    // ones in both blocks of a pair)
+    struct Side {
+        int32_t d2, s1, s2, n;
+        int64_t d[2], s[2];
+    };
+    bool narrow = true;  // no block has more than two such legs
+    auto side = [&](const BT &t, const std::vector<int64_t> &free, const std::vector<int64_t> &legs, std::vector<Side> &v) {
+        v.resize(t.nblocks());
         for (int64_t b = 0; b < t.nblocks(); ++b) {
-            st[b] = block_strides(t, b);
+            const Strided st = block_strides(t, b);
             FoldLeg l[MAXRANK];
             int n = 0;
-            for (auto d : legs) l[n++] = FoldLeg{st[b].d[d], st[b].s[d], 0};
-            if (!fold_legs(l, n, fo[b])) return false;
-            if (!fits(fo[b].d2) || !fits(fo[b].x1) || !fits(fo[b].x2)) return false;
+            for (auto d : free)
+                if (st.d[d] != 1) l[n++] = FoldLeg{st.d[d], st.s[d], 0};
+            Fold f;
+            if (!fold_legs(l, n, f) || !fits(f.d2) || !fits(f.x1) || !fits(f.x2)) return false;
+            Side &x = v[b];
+            x.d2 = int32_t(std::max<int64_t>(f.d2, 1));
+            x.s1 = int32_t(f.x1);
+            x.s2 = int32_t(f.x2);
+            x.n = 0;
+            for (auto d : legs)
+                if (st.d[d] != 1) {
+                    if (x.n < 2) {
+                        x.d[x.n] = st.d[d];
+                        x.s[x.n] = st.s[d];
+                    }
+                    ++x.n;
+                }
+            narrow = narrow && x.n <= 2;
         }
         return true;
     };
-    if (!free_legs(A, P.freeA, sa, fa) || !free_legs(B, P.freeB, sb, fb)) return false;
+    std::vector<Side> va, vb;
+    if (!side(A, P.freeA, P.dA, va) || !side(B, P.freeB, P.dB, vb)) return false;
     out.resize(P.pair_a.size());
     for (size_t k = 0; k < out.size(); ++k) {
         const int64_t ia = P.pair_a[k], ib = P.pair_b[k];
-        FoldLeg l[MAXRANK];
-        int n = 0;
-        for (size_t i = 0; i < P.dA.size(); ++i)
-            l[n++] = FoldLeg{sa[ia].d[P.dA[i]], sa[ia].s[P.dA[i]], sb[ib].s[P.dB[i]]};
+        const Side &x = va[ia], &y = vb[ib];
         Fold c;
-        if (!fold_legs(l, n, c)) return false;
+        if (x.n == 1) {
+            c.d2 = x.d[0];
+            c.x2 = x.s[0];
+            c.y2 = y.s[0];
+        } else if (x.n > 1) {
+            FoldLeg l[MAXRANK];
+            int n = 0;
+            if (narrow) {
+                for (; n < 2; ++n) l[n] = FoldLeg{x.d[n], x.s[n], y.s[n]};
+            } else {
+                const Strided sa = block_strides(A, ia), sb = block_strides(B, ib);
+                for (size_t i = 0; i < P.dA.size(); ++i)
+                    l[n++] = FoldLeg{sa.d[P.dA[i]], sa.s[P.dA[i]], sb.s[P.dB[i]]};
+            }
+            if (!fold_legs(l, n, c)) return false;
+        }
         if (!fits(c.d1) || !fits(c.d2) || !fits(c.x1) || !fits(c.x2) || !fits(c.y1) || !fits(c.y2)) return false;
-        F64Pair &p = out[k];
-        p.a_off = A.boff[ia];
-        p.b_off = B.boff[ib];
-        p.k1 = int32_t(c.d1);
-        p.k2 = int32_t(c.d2);
-        p.ak1 = int32_t(c.x1);
-        p.ak2 = int32_t(c.x2);
-        p.bk1 = int32_t(c.y1);
-        p.bk2 = int32_t(c.y2);
-        p.am2 = int32_t(std::max<int64_t>(fa[ia].d2, 1));
-        p.as1 = int32_t(fa[ia].x1);
-        p.as2 = int32_t(fa[ia].x2);
-        p.bn2 = int32_t(std::max<int64_t>(fb[ib].d2, 1));
-        p.bs1 = int32_t(fb[ib].x1);
-        p.bs2 = int32_t(fb[ib].x2);
+        out[k] = F64Pair{A.boff[ia],     B.boff[ib],     int32_t(c.d1),  int32_t(c.d2),  int32_t(c.x1), int32_t(c.x2),
+                         int32_t(c.y1),  int32_t(c.y2),  x.d2,           x.s1,           x.s2,          y.d2,
+                         y.s1,           y.s2};
     }
     return true;
 }
@@ -475,13 +604,16 @@ int64_t split_tables(const BT &t, const std::vector<int64_t> &perm, int nrow, in
 // Output blocks by falling total K (ties in block order): their tiles in this order leave the
 // cheap ones for the tail of the grid.
 std::vector<int32_t> longest_first(const std::vector<GemmOut> &outs, const std::vector<int64_t> &Ks) {
-    std::vector<int64_t> total(outs.size(), 0);
-    std::vector<int32_t> order(outs.size());
+    constexpr uint64_t top = UINT32_MAX;
+    std::vector<uint64_t> keys(outs.size());
     for (size_t o = 0; o < outs.size(); ++o) {
-        order[o] = int32_t(o);
-        for (int32_t p = outs[o].p0; p < outs[o].p1; ++p) total[o] += Ks[p];
+        uint64_t total = 0;
+        for (int32_t p = outs[o].p0; p < outs[o].p1; ++p) total += uint64_t(Ks[p]);
+        keys[o] = (top - std::min(total, top)) << 32 | uint64_t(o);
     }
-    std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return total[x] > total[y]; });
+    std::sort(keys.begin(), keys.end());
+    std::vector<int32_t> order(outs.size());
+    for (size_t o = 0; o < outs.size(); ++o) order[o] = int32_t(keys[o] & top);
     return order;
 }
 
@@ -546,9 +678,7 @@ void contract_f64(const ContractPlan &P, const BT &A, const BT &B, BT &out, cons
     g.B = Bp;
     g.C = static_cast<double *>(out.data());
     g.Cadd = add ? static_cast<const double *>(add->data()) : nullptr;
-    g.pairs = upload_vec(pairs);
-    g.outs = upload_vec(outs);
-    g.tiles = upload_vec(tiles);
+    upload_many({table(pairs, g.pairs), table(outs, g.outs), table(tiles, g.tiles)});
     g.ntiles = int32_t(tiles.size());
     g.alpha = alpha;
     g.beta = beta;
@@ -564,13 +694,14 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
     const int64_t nout = int64_t(P.out_p0.size());
     if (nout == 0) return;
     const int mode = gemm_mode();
+    const std::vector<int64_t> rows = sizes_of(A, P.freeA), cols = sizes_of(B, P.freeB), depth = sizes_of(A, P.dA);
     std::vector<int64_t> Ks(P.pair_a.size());
-    for (size_t k = 0; k < Ks.size(); ++k) Ks[k] = prod_sizes(A, P.pair_a[k], P.dA);
+    for (size_t k = 0; k < Ks.size(); ++k) Ks[k] = depth[P.pair_a[k]];
     std::vector<GemmOut> outs(nout);
     double flops = 0;
     for (int64_t o = 0; o < nout; ++o) {
         int64_t ia = P.pair_a[P.out_p0[o]], ib = P.pair_b[P.out_p0[o]];
-        int64_t M = prod_sizes(A, ia, P.freeA), N = prod_sizes(B, ib, P.freeB);
+        const int64_t M = rows[ia], N = cols[ib];
         if (M > INT32_MAX || N > INT32_MAX) fail(ERR_INVALID_ARGUMENT, "block too large");
         outs[o].c_off = out.boff[o];
         outs[o].add_off = (add && add_block && (*add_block)[o] >= 0) ? add->boff[(*add_block)[o]] : -1;
@@ -612,15 +743,6 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
     sa.dst[1] = sa.dst[0] + asz;
     sa.amax_parts = am.out;
     sa.amax = amax;
-    {
-        StatScope sc(ST_PACK, (mode == GEMM_BF16X3 ? 14.0 : 16.0) * double(A.nnz + B.nnz));
-        launch_amax(am);
-        sa.ents = upload_vec(ents);
-        sa.tiles = upload_vec(stiles);
-        bool flat = true;
-        for (const SplitEntry &e : ents) flat = flat && e.folded && e.rd2 >= e.rows && e.kd2 >= e.K;
-        launch_split(sa, int64_t(stiles.size()), mode, flat);
-    }
     const int TM = gemm_tile_m();
     int64_t wide = 0;
     for (const GemmOut &o : outs) wide += ((int64_t(o.M) + TM - 1) / TM) * ((int64_t(o.N) + 127) / 128);
@@ -647,12 +769,18 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
     g.tn = TN;
     g.C = static_cast<double *>(out.data());
     g.Cadd = add ? static_cast<const double *>(add->data()) : nullptr;
-    g.pairs = upload_vec(pairs);
-    g.outs = upload_vec(outs);
-    g.tiles = upload_vec(tiles);
     g.ntiles = int32_t(tiles.size());
     g.alpha = alpha;
     g.beta = beta;
+    {
+        StatScope sc(ST_PACK, (mode == GEMM_BF16X3 ? 14.0 : 16.0) * double(A.nnz + B.nnz));
+        launch_amax(am);
+        upload_many({table(ents, sa.ents), table(stiles, sa.tiles), table(pairs, g.pairs), table(outs, g.outs),
+                     table(tiles, g.tiles)});
+        bool flat = true;
+        for (const SplitEntry &e : ents) flat = flat && e.folded && e.rd2 >= e.rows && e.kd2 >= e.K;
+        launch_split(sa, int64_t(stiles.size()), mode, flat);
+    }
     StatScope sc(ST_GEMM, flops);
     launch_gemm_tc(g, mode);
 }

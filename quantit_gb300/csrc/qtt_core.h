@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <atomic>
 #include <functional>
+#include <initializer_list>
 #include <cstdint>
 #include <cstring>
 #include <memory>
@@ -194,6 +195,17 @@ BufPtr dev_alloc(size_t bytes);
 // Copy a host table to device memory valid for work issued afterwards on the
 // current stream (ring-buffered; the region is reused after the stream passes it).
 void *upload(const void *host, size_t bytes);
+// Several tables in one copy; each device pointer lands in *dev (null for an empty table).
+struct HostTable {
+    const void *host;
+    size_t bytes;
+    const void **dev;
+};
+void upload_many(std::initializer_list<HostTable> tables);
+template <class T>
+HostTable table(const std::vector<T> &v, const T *&dev) {
+    return HostTable{v.data(), v.size() * sizeof(T), reinterpret_cast<const void **>(&dev)};
+}
 template <class T>
 T *upload_vec(const std::vector<T> &v) {
     return v.empty() ? nullptr : static_cast<T *>(upload(v.data(), v.size() * sizeof(T)));

@@ -77,35 +77,59 @@ BufPtr dev_alloc(size_t bytes) {
     return b;
 }
 
-void *upload(const void *host, size_t bytes) {
+void upload_many(std::initializer_list<HostTable> tables) {
     Ctx &c = ctx();
-    size_t need = (bytes + 255) & ~size_t(255);
-    if (c.capturing) {
+    auto padded = [](size_t n) { return (n + 255) & ~size_t(255); };
+    size_t need = 0;
+    for (const HostTable &t : tables) need += padded(t.bytes);
+    char *d = nullptr, *h = nullptr;
+    std::vector<char> staged;
+    if (need == 0) {
+    } else if (c.capturing) {
         // a captured graph replays its kernels long after this call: its tables live in
         // their own buffers, filled now (relaxed capture mode allows the synchronous copy)
-        void *d = nullptr;
-        cuda_check(cudaMalloc(&d, std::max<size_t>(need, 256)), "cudaMalloc(graph table)");
-        c.capture_tables->push_back(d);
-        cuda_check(cudaMemcpy(d, host, bytes, cudaMemcpyHostToDevice), "cudaMemcpy(graph table)");
-        return d;
+        void *p = nullptr;
+        cuda_check(cudaMalloc(&p, need), "cudaMalloc(graph table)");
+        c.capture_tables->push_back(p);
+        d = static_cast<char *>(p);
+        staged.resize(need);
+        h = staged.data();
+    } else {
+        if (need > c.ring_bytes / 2) {
+            if (tables.size() == 1) fail(ERR_RUNTIME, "planning table larger than the staging ring");
+            for (const HostTable &t : tables) upload_many({t});
+            return;
+        }
+        const size_t half = c.ring_bytes / 2;
+        if (c.ring_pos + need > (c.cur_half + 1) * half) {
+            // leave the current half: mark where the stream is, then enter the other half
+            cuda_check(cudaEventRecord(c.half_done[c.cur_half], c.stream), "cudaEventRecord");
+            c.half_used[c.cur_half] = true;
+            c.cur_half ^= 1;
+            if (c.half_used[c.cur_half]) cuda_check(cudaEventSynchronize(c.half_done[c.cur_half]), "cudaEventSync");
+            c.ring_pos = c.cur_half * half;
+        }
+        d = c.dev_ring + c.ring_pos;
+        h = c.host_ring + c.ring_pos;
+        c.ring_pos += need;
     }
-    if (need > c.ring_bytes / 2) fail(ERR_RUNTIME, "planning table larger than the staging ring");
-    size_t half = c.ring_bytes / 2;
-    size_t half_end = (c.cur_half + 1) * half;
-    if (c.ring_pos + need > half_end) {
-        // leave the current half: mark where the stream is, then enter the other half
-        cuda_check(cudaEventRecord(c.half_done[c.cur_half], c.stream), "cudaEventRecord");
-        c.half_used[c.cur_half] = true;
-        c.cur_half ^= 1;
-        if (c.half_used[c.cur_half]) cuda_check(cudaEventSynchronize(c.half_done[c.cur_half]), "cudaEventSync");
-        c.ring_pos = c.cur_half * half;
+    size_t at = 0;
+    for (const HostTable &t : tables) {
+        *t.dev = t.bytes ? d + at : nullptr;
+        if (t.bytes) std::memcpy(h + at, t.host, t.bytes);
+        at += padded(t.bytes);
     }
-    std::memcpy(c.host_ring + c.ring_pos, host, bytes);
-    void *d = c.dev_ring + c.ring_pos;
-    cuda_check(cudaMemcpyAsync(d, c.host_ring + c.ring_pos, bytes, cudaMemcpyHostToDevice, c.stream),
-               "cudaMemcpyAsync(plan)");
-    c.ring_pos += need;
-    return d;
+    if (need == 0) return;
+    if (c.capturing)
+        cuda_check(cudaMemcpy(d, h, need, cudaMemcpyHostToDevice), "cudaMemcpy(graph table)");
+    else
+        cuda_check(cudaMemcpyAsync(d, h, need, cudaMemcpyHostToDevice, c.stream), "cudaMemcpyAsync(plan)");
+}
+
+void *upload(const void *host, size_t bytes) {
+    const void *d = nullptr;
+    upload_many({HostTable{host, bytes, &d}});
+    return const_cast<void *>(d);
 }
 
 // ---------------------------------------------------------------- statistics
