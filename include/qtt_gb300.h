@@ -179,6 +179,12 @@ int qtt_svd_split(qtt_bt t, int64_t split, qtt_bt *U, qtt_bt *d, qtt_bt *V);
 /* svd(A, split, tol, min_size, max_size, pow) (LinearAlgebra.h:115; btensor_linalg.cpp:805) */
 int qtt_svd_truncate(qtt_bt t, int64_t split, double tol, int64_t min_size, int64_t max_size, double pow,
                      qtt_bt *U, qtt_bt *d, qtt_bt *V);
+/* The same decomposition with plain sweeps: from the identity, with exactly computed
+ * rotation angles.  For tensors with equal singular values (an MPO's, bMPO::coalesce):
+ * the basis of their subspaces, which the decomposition leaves open, then does not
+ * depend on the preconditioning of the sweeps. */
+int qtt_svd_truncate_plain(qtt_bt t, int64_t split, double tol, int64_t min_size, int64_t max_size, double pow,
+                           qtt_bt *U, qtt_bt *d, qtt_bt *V);
 /* truncate(U, d, V, max, min, tol, pow) (LinearAlgebra.h:246; btensor_linalg.cpp:658-755) */
 int qtt_truncate(qtt_bt U, qtt_bt d, qtt_bt V, int64_t max_size, int64_t min_size, double tol, double pow,
                  qtt_bt *Uo, qtt_bt *do_, qtt_bt *Vo);

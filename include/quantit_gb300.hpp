@@ -389,7 +389,11 @@ class bMPO : public std::vector<btensor> {
     // bMPO::coalesce (sources/MPT.cpp:154-168)
     bMPO &coalesce(btensor::Scalar cutoff = 0) {
         for (size_t i = 0; i + 1 < size(); ++i) {
-            auto [U, d, V] = svd((*this)[i].permute({0, 1, 3, 2}), size_t(3), cutoff);
+            // plain sweeps: an MPO tensor's singular values are often equal
+            const btensor w = (*this)[i].permute({0, 1, 3, 2});
+            qtt_bt u, s, v;
+            auto [U, d, V] = detail::svd_out(qtt_svd_truncate_plain(w.get(), 3, double(cutoff), 1, INT64_MAX, 2.0, &u, &s, &v),
+                                             u, s, v);
             (*this)[i + 1] = tensordot(V.conj(), (*this)[i + 1], {0}, {0});
             (*this)[i] = U.mul(d).permute({0, 1, 3, 2});
         }

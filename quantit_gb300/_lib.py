@@ -70,6 +70,7 @@ SIGNATURES = {
     "qtt_svd": (C.c_int, [bt, P(bt), P(bt), P(bt)]),
     "qtt_svd_split": (C.c_int, [bt, i64, P(bt), P(bt), P(bt)]),
     "qtt_svd_truncate": (C.c_int, [bt, i64, f64, i64, i64, f64, P(bt), P(bt), P(bt)]),
+    "qtt_svd_truncate_plain": (C.c_int, [bt, i64, f64, i64, i64, f64, P(bt), P(bt), P(bt)]),
     "qtt_truncate": (C.c_int, [bt, bt, bt, i64, i64, f64, f64, P(bt), P(bt), P(bt)]),
     "qtt_eigh": (C.c_int, [bt, i32, P(bt), P(bt)]),
     "qtt_eigh_split": (C.c_int, [bt, i64, P(bt), P(bt)]),

@@ -349,6 +349,18 @@ int qtt_svd_truncate(qtt_bt t, int64_t split, double tol, int64_t min_size, int6
         *V = wrap(std::move(r.V));
     });
 }
+int qtt_svd_truncate_plain(qtt_bt t, int64_t split, double tol, int64_t min_size, int64_t max_size, double pw,
+                           qtt_bt *U, qtt_bt *d, qtt_bt *V) {
+    return guarded([&] {
+        out_check(U);
+        out_check(d);
+        out_check(V);
+        auto r = qtt::svd_truncated(T(t), split, tol, min_size, max_size, pw, nullptr, true);
+        *U = wrap(std::move(r.U));
+        *d = wrap(std::move(r.d));
+        *V = wrap(std::move(r.V));
+    });
+}
 int qtt_truncate(qtt_bt U, qtt_bt d, qtt_bt V, int64_t max_size, int64_t min_size, double tol, double pw,
                  qtt_bt *Uo, qtt_bt *do_, qtt_bt *Vo) {
     return guarded([&] {

@@ -61,9 +61,9 @@ __device__ __forceinline__ float ldcg(const float *p) { return __ldcg(p); }
 // FP32 that bias accumulates to ~1e-5 in the singular values over a few sweeps.
 // In FP64 the same rotation as three shears, x -= tau y, y += s x, x -= tau y: three
 // instead of four instructions of GB300's narrow FP64 pipe per element pair.
-template <class T>
+template <class T, bool EXACT = false>
 __device__ __forceinline__ void rot_apply(T &x, T &y, T s, T tau) {
-    if constexpr (sizeof(T) == 8) {
+    if constexpr (sizeof(T) == 8 && !EXACT) {
         x = fma(-tau, y, x);
         y = fma(s, x, y);
         x = fma(-tau, y, x);
@@ -579,8 +579,11 @@ __device__ __forceinline__ int bj_params_fast64(double &al, double &be, double g
 
 // Whether an updated squared norm kept more than 1/16 of the old one (FP64: by the high words,
 // without an FP64 instruction).
+template <bool EXACT>
 __device__ __forceinline__ bool norm_kept(float a2, float al) { return a2 > al * 0.0625f; }
+template <bool EXACT>
 __device__ __forceinline__ bool norm_kept(double a2, double al) {
+    if constexpr (EXACT) return a2 > al * 0.0625;
     return __double2hiint(a2) > __double2hiint(al) - (4 << 20);
 }
 
@@ -592,7 +595,8 @@ __device__ __forceinline__ bool norm_kept(double a2, double al) {
 // A zero column (norm 0) is skipped without forming the product; with thr > 0 a
 // column whose squared norm falls to thr or below after the rotation is deflated
 // (set to zero, norm 0; dx / dy receive its squared norm before, else stay 0).
-template <class T, int R>
+// EXACT: the plain formulas in FP64 too (launch_jacobi's `exact`).
+template <class T, int R, bool EXACT>
 __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], T &al, T &be, T tol, T thr, T &sn, T &tau, T &dx,
                                           T &dy, T skip, float &rmax) {
     if (al == T(0) || be == T(0)) return false;
@@ -605,6 +609,13 @@ __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], T &al, T &be, T 
         if (rel <= tol) return false;
         rmax = fmaxf(rmax, rel);
         bj_params_fast(al, be, ga, sn, tau, t);
+        a2 = al - t * ga;
+        b2 = be + t * ga;
+    } else if constexpr (EXACT) {
+        const double rel = fabs(ga) / sqrt(al * be);
+        if (rel <= tol) return false;
+        rmax = fmaxf(rmax, float(rel));
+        rot_params(al, be, ga, sn, tau, t);
         a2 = al - t * ga;
         b2 = be + t * ga;
     } else {
@@ -625,10 +636,10 @@ __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], T &al, T &be, T 
         }
     }
 #pragma unroll
-    for (int i = 0; i < R; ++i) rot_apply(x[i], y[i], sn, tau);
-    // recomputed when the update cancelled (an exponent comparison: 1/16 of the norm)
-    al = norm_kept(a2, al) ? a2 : bj_dot(x, x);
-    be = norm_kept(b2, be) ? b2 : bj_dot(y, y);
+    for (int i = 0; i < R; ++i) rot_apply<T, EXACT>(x[i], y[i], sn, tau);
+    // recomputed when the update cancelled (below about 1/16 of the norm)
+    al = norm_kept<EXACT>(a2, al) ? a2 : bj_dot(x, x);
+    be = norm_kept<EXACT>(b2, be) ? b2 : bj_dot(y, y);
     if (thr > T(0)) {
         if (al <= thr) {
 #pragma unroll
@@ -717,7 +728,7 @@ __device__ void bj_vwork(const BJacobiParams<T> &P, int64_t st, T *Qs, int *s_un
     }
 }
 
-template <class T, int B, int R>
+template <class T, int B, int R, bool EXACT>
 __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
     constexpr int NP = 2 * B;   // columns (players) of a block pair
     constexpr int PP = 32 * R;  // shared-memory slot per column (zero-padded)
@@ -859,14 +870,14 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                         bj_load(x, cols + u * PP, lane);
                         bj_load(y, cols + v * PP, lane);
                         T al = nrm[u], be = nrm[v], dx = T(0), dy = T(0);
-                        if (bj_rotate(x, y, al, be, tol, thr, sn, tau, dx, dy, skp, rmax)) {
+                        if (bj_rotate<T, R, EXACT>(x, y, al, be, tol, thr, sn, tau, dx, dy, skp, rmax)) {
                             if (lane == 0 && dx > T(0)) P.dnorm[sd.s_off + column(u)] = dx;
                             if (lane == 0 && dy > T(0)) P.dnorm[sd.s_off + column(v)] = dy;
                             bj_store(x, cols + u * PP, lane);
                             bj_store(y, cols + v * PP, lane);
                             if (lane < NP) {
                                 T qu = Qs[u * NP + lane], qv = Qs[v * NP + lane];
-                                rot_apply(qu, qv, sn, tau);
+                                rot_apply<T, EXACT>(qu, qv, sn, tau);
                                 Qs[u * NP + lane] = qu;
                                 Qs[v * NP + lane] = qv;
                             }
@@ -895,13 +906,13 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                     if (mine && valid(j)) {
                         bj_load(y, cols + j * PP, lane);
                         T be = nrm[j], dx = T(0), dy = T(0);
-                        if (bj_rotate(x, y, al, be, tol, thr, sn, tau, dx, dy, skp, rmax)) {
+                        if (bj_rotate<T, R, EXACT>(x, y, al, be, tol, thr, sn, tau, dx, dy, skp, rmax)) {
                             if (lane == 0 && dx > T(0)) P.dnorm[sd.s_off + column(warp)] = dx;
                             if (lane == 0 && dy > T(0)) P.dnorm[sd.s_off + column(j)] = dy;
                             bj_store(y, cols + j * PP, lane);
                             if (lane < NP) {
                                 T qy = Qs[j * NP + lane];
-                                rot_apply(qx, qy, sn, tau);
+                                rot_apply<T, EXACT>(qx, qy, sn, tau);
                                 Qs[j * NP + lane] = qy;
                             }
                             if (lane == 0) nrm[j] = be;
@@ -1281,20 +1292,20 @@ size_t bj_vwork_bytes(int B, size_t es, int nsec, int64_t sum_q, int64_t max_ste
            256;
 }
 
-template <class T, int B, int R>
+template <class T, int B, int R, bool EXACT = false>
 bool bjacobi_launch(const BJacobiParams<T> &P, int max_block_steps, int64_t sum_q, void *vwork, size_t vwork_bytes,
                     cudaStream_t stream) {
     const size_t smem = size_t(2 * B) * (32 * R + 2 * B + 1) * sizeof(T) + size_t(3 * P.nsec + 1) * sizeof(int);
     if (smem > BJ_SMEM_MAX) return false;
     static std::atomic<uint64_t> attr{0};
     once_per_device(attr, [] {
-        cuda_check(cudaFuncSetAttribute(k_bjacobi<T, B, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cuda_check(cudaFuncSetAttribute(k_bjacobi<T, B, R, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         int(BJ_SMEM_MAX)),
                    "block Jacobi smem attribute");
     });
     const int nsm = sm_count();
     int occ = 0;
-    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bjacobi<T, B, R>, 32 * B, smem), "occupancy");
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bjacobi<T, B, R, EXACT>, 32 * B, smem), "occupancy");
     if (occ < 1) fail(ERR_RUNTIME, "the block Jacobi kernel cannot be resident on an SM");
     BJacobiParams<T> Pc = P;
     Pc.max_steps = int64_t(P.max_sweeps) * std::max(1, max_block_steps) + 1;
@@ -1322,7 +1333,7 @@ bool bjacobi_launch(const BJacobiParams<T> &P, int max_block_steps, int64_t sum_
     const int64_t items = sum_q / (2 * B) + P.nsec;
     dim3 grid(unsigned(std::min<int64_t>(int64_t(nsm) * std::min(occ, 2), std::max<int64_t>(1, items)))),
         block(32 * B);
-    cuda_check(cudaLaunchCooperativeKernel((void *)k_bjacobi<T, B, R>, grid, block, args, smem, stream),
+    cuda_check(cudaLaunchCooperativeKernel((void *)k_bjacobi<T, B, R, EXACT>, grid, block, args, smem, stream),
                "cooperative block Jacobi launch");
     count_launch();
     return true;
@@ -1332,13 +1343,17 @@ bool bjacobi_launch(const BJacobiParams<T> &P, int max_block_steps, int64_t sum_
 // than the columns is work on zeros, and in FP64 every element of it costs 64 clocks a warp
 // instruction: fine steps there.
 int r_class(int max_p, bool f32) {
-    static constexpr int f32_r[] = {4, 8, 12, 16, 24, 32, 48, 64};
+    static constexpr int f32_r[] = {4, 8, 16, 24, 32, 48, 64};
     static constexpr int f64_r[] = {2, 4, 6, 8, 10, 12, 16, 20, 24, 28, 32, 40, 48, 64};
     const int *r = f32 ? f32_r : f64_r;
-    for (int i = 0, n = f32 ? 8 : 14; i < n; ++i)
+    for (int i = 0, n = f32 ? 7 : 14; i < n; ++i)
         if (max_p <= 32 * r[i]) return r[i];
     return 0;
 }
+
+// Register slice of the FP64 kernels with exactly computed angles (launch_jacobi's `exact`); 0: longer
+// columns than they are built for.
+int exact_r_class(int max_p) { return max_p <= 128 ? 4 : max_p <= 256 ? 8 : max_p <= 512 ? 16 : 0; }
 
 // Block widths the block kernel is built with for (element type, R): FP32 16 (R <= 32)
 // and 8 (R <= 64); FP64 8 and 4 (R <= 48).  The first entry is the default.
@@ -1356,18 +1371,25 @@ std::vector<int> block_widths(bool f32, int R) {
 // returns false when the scalar kernel has to run instead.
 template <class T>
 bool bjacobi_dispatch(const BJacobiParams<T> &P, int max_steps_per_sweep, int max_p, int64_t sum_q, void *vwork,
-                      size_t vwork_bytes, int B, cudaStream_t stream) {
+                      size_t vwork_bytes, int B, bool exact, cudaStream_t stream) {
     const int max_qp = max_steps_per_sweep + 1;  // the widest sector's even column count
     auto steps = [&](int b) {
         const int nb = (max_qp + b - 1) / b;
         return nb + (nb & 1) - 1;
     };
     const int R = r_class(max_p, sizeof(T) == 4);
+    if constexpr (sizeof(T) == 8) {
+        const int E = exact ? exact_r_class(max_p) : 0;
+#define QTT_BJX(BB, RR) \
+    if (B == BB && E == RR) return bjacobi_launch<T, BB, RR, true>(P, steps(BB), sum_q, vwork, vwork_bytes, stream);
+        QTT_BJX(8, 4) QTT_BJX(8, 8) QTT_BJX(8, 16) QTT_BJX(4, 4) QTT_BJX(4, 8) QTT_BJX(4, 16)
+#undef QTT_BJX
+    }
 #define QTT_BJ(BB, RR)                                                                                            \
     if (B == BB && R == RR) return bjacobi_launch<T, BB, RR>(P, steps(BB), sum_q, vwork, vwork_bytes, stream);
     if constexpr (sizeof(T) == 4) {
-        QTT_BJ(16, 4) QTT_BJ(16, 8) QTT_BJ(16, 12) QTT_BJ(16, 16) QTT_BJ(16, 24) QTT_BJ(16, 32)
-        QTT_BJ(8, 4) QTT_BJ(8, 8) QTT_BJ(8, 12) QTT_BJ(8, 16) QTT_BJ(8, 24) QTT_BJ(8, 32) QTT_BJ(8, 48) QTT_BJ(8, 64)
+        QTT_BJ(16, 4) QTT_BJ(16, 8) QTT_BJ(16, 16) QTT_BJ(16, 24) QTT_BJ(16, 32)
+        QTT_BJ(8, 4) QTT_BJ(8, 8) QTT_BJ(8, 16) QTT_BJ(8, 24) QTT_BJ(8, 32) QTT_BJ(8, 48) QTT_BJ(8, 64)
     } else {
         QTT_BJ(8, 2) QTT_BJ(8, 4) QTT_BJ(8, 6) QTT_BJ(8, 8) QTT_BJ(8, 10) QTT_BJ(8, 12) QTT_BJ(8, 16) QTT_BJ(8, 20)
         QTT_BJ(8, 24) QTT_BJ(8, 28) QTT_BJ(8, 32) QTT_BJ(8, 40) QTT_BJ(8, 48)
@@ -1435,7 +1457,7 @@ void tune_save(const TuneKey &k, int w) {
 template <class T>
 void jacobi_impl(T *work, T *rot, const SectorDesc *sec, const int *slot_start, int nsec, int max_steps_per_sweep,
                  int max_sweeps, int *sweeps_out, int *flags, int max_p, int64_t sum_q, void *vwork, size_t vwork_bytes,
-                 const T *defl, T *dnorm, cudaStream_t stream, bool tune, const T *skip) {
+                 const T *defl, T *dnorm, cudaStream_t stream, bool tune, const T *skip, bool exact) {
     if (nsec > 12 * 1024) fail(ERR_INVALID_ARGUMENT, "too many sectors for one decomposition launch");
     const size_t smem = size_t(2 * nsec) * sizeof(int);
     cuda_check(cudaMemsetAsync(flags, 0, size_t(nsec) * max_sweeps * sizeof(int), stream), "memset flags");
@@ -1454,11 +1476,12 @@ void jacobi_impl(T *work, T *rot, const SectorDesc *sec, const int *slot_start, 
         B.skip = skip;
         B.max_q = max_steps_per_sweep + 1;  // the widest sector's even column count bounds q
         const bool f32 = sizeof(T) == 4;
-        const std::vector<int> cands = block_widths(f32, r_class(max_p, f32));
+        const int ex = exact && !f32 ? exact_r_class(max_p) : 0, R = ex ? ex : r_class(max_p, f32);
+        const std::vector<int> cands = block_widths(f32, R);
         if (!cands.empty()) {
             int ci = 0;
             bool timing = false;
-            const TuneKey key{f32 ? 1 : 0, r_class(max_p, f32), ceil_log2(max_steps_per_sweep + 1), ceil_log2(nsec)};
+            const TuneKey key{f32 ? 1 : 0, R, ceil_log2(max_steps_per_sweep + 1), ceil_log2(nsec)};
             if (g_autotune.load() && cands.size() > 1) {
                 std::lock_guard<std::mutex> lk(g_tune_mu);
                 tune_load_locked();
@@ -1476,7 +1499,7 @@ void jacobi_impl(T *work, T *rot, const SectorDesc *sec, const int *slot_start, 
                 cuda_check(cudaEventCreate(&e1), "cudaEventCreate");
                 cuda_check(cudaEventRecord(e0, stream), "cudaEventRecord");
             }
-            const bool ok = bjacobi_dispatch(B, max_steps_per_sweep, max_p, sum_q, vwork, vwork_bytes, cands[ci], stream);
+            const bool ok = bjacobi_dispatch(B, max_steps_per_sweep, max_p, sum_q, vwork, vwork_bytes, cands[ci], exact, stream);
             if (timing) {
                 float ms = 0.f;
                 cuda_check(cudaEventRecord(e1, stream), "cudaEventRecord");
@@ -1579,26 +1602,27 @@ void launch_eigh_prepare(void *work, SectorDesc *sec, int nsec, int upper, int f
 void launch_jacobi_on(cudaStream_t stream, void *work, void *rot, const SectorDesc *sec, const int *slot_start,
                       int nsec, int max_steps_per_sweep, int max_sweeps, int *sweeps_out, int *flags, int f32,
                       int max_p, int64_t sum_q, void *vwork, size_t vwork_bytes, const void *defl, void *dnorm,
-                      bool tune, const void *skip) {
+                      bool tune, const void *skip, bool exact) {
     if (nsec <= 0) return;
     if ((defl == nullptr) != (dnorm == nullptr)) fail(ERR_INVALID_ARGUMENT, "deflation needs thresholds and norms");
     if (f32)
         jacobi_impl(static_cast<float *>(work), static_cast<float *>(rot), sec, slot_start, nsec, max_steps_per_sweep,
                     max_sweeps, sweeps_out, flags, max_p, sum_q, vwork, vwork_bytes,
                     static_cast<const float *>(defl), static_cast<float *>(dnorm), stream, tune,
-                    static_cast<const float *>(skip));
+                    static_cast<const float *>(skip), false);
     else
         jacobi_impl(static_cast<double *>(work), static_cast<double *>(rot), sec, slot_start, nsec,
                     max_steps_per_sweep, max_sweeps, sweeps_out, flags, max_p, sum_q, vwork, vwork_bytes,
                     static_cast<const double *>(defl), static_cast<double *>(dnorm), stream, tune,
-                    static_cast<const double *>(skip));
+                    static_cast<const double *>(skip), exact);
 }
 
 void launch_jacobi(void *work, void *rot, const SectorDesc *sec, const int *slot_start, int nsec,
                    int max_steps_per_sweep, int max_sweeps, int *sweeps_out, int *flags, int f32, int max_p,
-                   int64_t sum_q, void *vwork, size_t vwork_bytes, const void *defl, void *dnorm, const void *skip) {
+                   int64_t sum_q, void *vwork, size_t vwork_bytes, const void *defl, void *dnorm, const void *skip,
+                   bool exact) {
     launch_jacobi_on(ctx().stream, work, rot, sec, slot_start, nsec, max_steps_per_sweep, max_sweeps, sweeps_out, flags,
-                     f32, max_p, sum_q, vwork, vwork_bytes, defl, dnorm, true, skip);
+                     f32, max_p, sum_q, vwork, vwork_bytes, defl, dnorm, true, skip, exact);
 }
 
 void launch_warm_apply(void *work, void *rot, void *tmp, const WarmDesc *wd, int nwarm, int ntiles, int f32) {

@@ -252,12 +252,14 @@ void launch_eigh_prepare(void *work, SectorDesc *sec, int nsec, int upper, int f
 // defl (optional, launch_deflation_thresholds, the work type): per sector, a column
 // whose squared norm falls to the threshold or below is set to zero and leaves the
 // sweeps (a numerically zero column); null: no deflation.
+// exact: FP64 rotation angles from FP64 square roots and divisions (columns up to 512), so that
+// the basis of equal singular values is that of the plain formulas; otherwise from FP32.
 // skip (optional, the work type): per sector, a pair whose squared column norms are both
 // below it is not rotated (columns the caller will discard).
 void launch_jacobi(void *work, void *rot, const SectorDesc *sec, const int *slot_start, int nsec,
                    int max_steps_per_sweep, int max_sweeps, int *sweeps_out, int *flags, int f32, int max_p,
                    int64_t sum_q, void *vwork = nullptr, size_t vwork_bytes = 0, const void *defl = nullptr,
-                   void *dnorm = nullptr, const void *skip = nullptr);
+                   void *dnorm = nullptr, const void *skip = nullptr, bool exact = false);
 // thr[s] <- delta^2 ||W_s||_F^2 for every svd sector (0 for eigh), in the work type.
 void launch_deflation_thresholds(const void *work, const SectorDesc *sec, int nsec, double delta, void *thr, int f32);
 // dnorm (with defl; the work type, sum of q entries at s_off, zero on entry) receives
@@ -281,7 +283,7 @@ void launch_jacobi_on(cudaStream_t stream, void *work, void *rot, const SectorDe
                       int nsec, int max_steps_per_sweep, int max_sweeps, int *sweeps_out, int *flags, int f32,
                       int max_p, int64_t sum_q, void *vwork = nullptr, size_t vwork_bytes = 0,
                       const void *defl = nullptr, void *dnorm = nullptr, bool tune = true,
-                      const void *skip = nullptr);
+                      const void *skip = nullptr, bool exact = false);
 void launch_finish_on(cudaStream_t stream, const void *work, const void *rot, double *U, double *V, double *s,
                       const SectorDesc *sec, int nsec, int max_q, double *scratch, int f32, int complete_cap = -1,
                       const void *dnorm = nullptr, int *dpos = nullptr, int *perm_out = nullptr,

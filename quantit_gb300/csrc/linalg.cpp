@@ -165,6 +165,7 @@ struct TruncHint {
     int64_t max_size = 0;
     bool allow_discard = true;
     double discard_tau = 0.0;
+    bool plain = false;  // sweeps from the identity with exactly computed angles (svd_truncated)
 };
 TruncHint &trunc_hint() {
     thread_local TruncHint h;
@@ -248,8 +249,17 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     // The mixed path (split-precision block GEMMs) runs its SVD sweeps in FP32 first and
     // finishes them in FP64 (svd_refine.cu): the result is an FP64 SVD either way.  eigh
     // always runs in FP64.
-    // A decomposition that is run again because its estimated truncation fell short is FP64 throughout.
-    const bool redo = trunc_hint().active && !trunc_hint().allow_discard;
+    // Sectors that are LQ-preconditioned (lq.cu).  Under a truncation, from 16 columns on: svd of a
+    // graded theta at D = 60 1664 -> 907 us, at D = 100 2846 -> 1383, at D = 600 35.0 -> 12.7 ms.
+    // The plain svd also sees matrices that are not graded (bMPS.move_oc of a random state), where
+    // the sweeps saved do not pay for the factorisation of a small sector: D = 120 806 us without
+    // against 925 with.  With the deflation switched off the sweeps run from the identity as well: null
+    // columns that stay in keep a factored start sweeping as long.
+    const int lq_least = mode != 0 || trunc_hint().plain ? INT32_MAX : !trunc_hint().active ? 48 : svd_deflation() ? 16 : INT32_MAX;
+    auto lq_fits = [&](const SectorDesc &d, int prec32) { return d.q >= lq_least && d.q <= lq_max_q(prec32, nsec); };
+    // A decomposition that is run again because its estimated truncation fell short is FP64
+    // throughout, if the factorisation speeds its FP64 sweeps up.
+    const bool redo = trunc_hint().active && !trunc_hint().allow_discard && max_q >= lq_least;
     const int f32 = (mode == 0 && gemm_mode() != GEMM_F64 && !redo) ? 1 : 0;
     const size_t es = f32 ? 4 : 8;
     D.work = dev_alloc(size_t(std::max<int64_t>(wtot, 1)) * es);
@@ -284,14 +294,6 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             }
         }
     }
-    // Sectors that are LQ-preconditioned (lq.cu).  Under a truncation, from 12 columns on: svd of a
-    // graded theta at D = 60 1664 -> 907 us, at D = 100 2846 -> 1383, at D = 600 35.0 -> 12.7 ms.
-    // The plain svd also sees matrices that are not graded (bMPS.move_oc of a random state), where
-    // the sweeps saved do not pay for the factorisation of a small sector: D = 120 806 us without
-    // against 925 with.  With the deflation switched off the sweeps run from the identity as well: null
-    // columns that stay in keep a factored start sweeping as long.
-    const int lq_least = !trunc_hint().active ? 48 : (svd_deflation() ? 12 : INT32_MAX);
-    auto lq_fits = [&](const SectorDesc &d, int prec32) { return d.q >= lq_least && d.q <= lq_max_q(prec32, nsec); };
     auto lq_of = [](const SectorDesc &d, bool from_rot) {
         LqSec s{};
         s.w_off = d.w_off;
@@ -398,7 +400,8 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
         launch_lq(W, D.rot->p, lq, f32);
         const int *dslots = upload_vec(slots);
         launch_jacobi(W, D.rot->p, dsec, dslots, nsec, max_steps, max_sweeps, sweeps, flags, f32, max_p, stot,
-                      vwork->p, vb, deflate ? thr->p : nullptr, deflate ? dnorm->p : nullptr);
+                      vwork->p, vb, deflate ? thr->p : nullptr, deflate ? dnorm->p : nullptr, nullptr,
+                      trunc_hint().plain);
         const void *fw = W, *fr = D.rot->p;
         BufPtr w64, w1, va, vbuf, gbuf, ibuf64;
         // The FP32 sweeps resolved every value above FP32 resolution.  When the truncation
@@ -425,24 +428,27 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             const double t_est = kept_threshold(vals, th.tol, th.pw, th.min_size, th.max_size);
             discard.assign(nsec, 0.0);
             null2.assign(nsec, 0.0);
-            // The level has to clear FP32's resolution in every sector: the noise of one that it does
-            // not clear is among the values the threshold was estimated from (estimates from such
-            // noise had the decomposition run twice: D = 600, 14 decades 31.8 ms, FP64 alone 12.8).
+            // Where factored FP64 sweeps stand ready, the level has to clear FP32's resolution in every
+            // sector: the noise of one that it does not clear is among the values the threshold was
+            // estimated from (estimates from such noise had the decomposition run twice: D = 600, 14
+            // decades 31.8 ms, FP64 alone 12.8).  Otherwise each sector that it clears discards.
             const double tau = 0.5 * t_est;
-            bool clears = t_est > 0.0;
+            bool clears = t_est > 0.0, any = false;
             for (int i = 0; i < nsec; ++i) {
                 const SectorDesc &d = D.desc[i];
                 double f2 = 0.0;
                 for (int j = 0; j < d.q; ++j) f2 += n2[d.s_off + j];
                 null2[i] = kDeflateF64 * kDeflateF64 * f2;
-                discard[i] = tau;
-                clears = clears && tau > 4.0 * kDeflateF32 * std::sqrt(f2);
+                const bool here = t_est > 0.0 && tau > 4.0 * kDeflateF32 * std::sqrt(f2);
+                discard[i] = here ? tau : 0.0;
+                any = any || here;
+                clears = clears && here;
             }
-            if (clears)
+            if (lq.empty() ? any : clears)
                 th.discard_tau = std::max(th.discard_tau, tau);
             else
                 discard.clear();
-            resolve_anew = discard.empty();
+            resolve_anew = discard.empty() && !lq.empty();
         }
         if (f32) {
             StatScope sc64(ST_SVD64, 0.0);
@@ -488,7 +494,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             auto fp64_sweeps = [&](int cap_sweeps, const void *thr, const void *skip) {
                 launch_jacobi(w1->p, vbuf->p, dsec64, dslots, nsec, max_steps, cap_sweeps, sw64, sw64 + nsec, 0,
                               max_p, stot, vwork64->p, vb64, deflate ? thr : nullptr, deflate ? dnorm->p : nullptr,
-                              skip);
+                              skip, th.plain);
             };
             if (discard.empty()) {
                 launch_lq(w1->p, vbuf->p, lq64, 0);
@@ -570,7 +576,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                                "cudaMemsetAsync(compact dnorm)");
                 }
                 launch_jacobi(wk->p, rk->p, ddk, dkslots, nsec, kmax_steps, max_sweeps, sw64, sw64 + nsec, 0, max_p, ks,
-                              vworkk->p, vbk, deflate ? thr64->p : nullptr, deflate ? dnk->p : nullptr, nullptr);
+                              vworkk->p, vbk, deflate ? thr64->p : nullptr, deflate ? dnk->p : nullptr, nullptr, th.plain);
                 launch_rot_product(static_cast<const double *>(vg->p), static_cast<const double *>(rk->p),
                                    static_cast<double *>(vn->p), rp);
                 launch_col_copy(static_cast<const double *>(wk->p), static_cast<double *>(w1->p), wscatter);
@@ -955,8 +961,9 @@ SVDOut truncate(SVDOut &&in, int64_t max_size, int64_t min_size, double tol, dou
 }
 
 SVDOut svd_truncated(const BT &t, int64_t split, double tol, int64_t min_size, int64_t max_size, double pw,
-                     WarmStart *ws) {
+                     WarmStart *ws, bool plain) {
     TruncHint h;
+    h.plain = plain;
     h.active = tol > 0.0;
     h.min_size = min_size;
     h.ws = ws;

@@ -354,8 +354,11 @@ struct WarmStart {
     std::vector<Entry> entries;
 };
 // ws (optional): warm starts read from and written back to ws.
+// plain: Jacobi sweeps from the identity with exactly computed angles, for tensors with equal singular
+// values (an MPO's): the basis of their subspaces then does not depend on how the sweeps are
+// preconditioned or on an angle's rounding.
 SVDOut svd_truncated(const BT &t, int64_t split, double tol, int64_t min_size, int64_t max_size, double pw,
-                     WarmStart *ws = nullptr);
+                     WarmStart *ws = nullptr, bool plain = false);
 struct EighOut {
     BT d, U;
 };

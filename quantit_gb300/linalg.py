@@ -25,6 +25,15 @@ def svd(tensor, split=None, tol=None, *, min_size=1, max_size=SIZE_MAX, pow=2):
                  float(pow))
 
 
+def svd_plain(tensor, split, tol, *, min_size=1, max_size=SIZE_MAX, pow=2):
+    """svd(tensor, split, tol, ...) with plain sweeps: from the identity, with exactly
+    computed rotation angles.  For tensors with equal singular values, such as an MPO's
+    (``bMPO.coalesce``): the basis of their subspaces, which the decomposition leaves open,
+    then does not depend on how the sweeps are preconditioned.  No reference counterpart."""
+    return _out3("qtt_svd_truncate_plain", tensor._h, int(split), float(tol), int(min_size),
+                 int(min(max_size, SIZE_MAX)), float(pow))
+
+
 def truncate(U, d, V, max_size, min_size, tol, pow=2):
     """truncate(U, d, V, max, min, tol, pow) (blockTensor/LinearAlgebra.h:246)."""
     Uo, do, Vo = C.c_void_p(), C.c_void_p(), C.c_void_p()

@@ -29,7 +29,7 @@ class bMPO(list):
         site absorbs V^H.  Linearly dependent MPO channels vanish, so the bond
         dimension drops to the operator's rank seen from the left.  On the GPU."""
         for i in range(len(self) - 1):
-            U, d, V = linalg.svd(self[i].permute([0, 1, 3, 2]), 3, float(cutoff))
+            U, d, V = linalg.svd_plain(self[i].permute([0, 1, 3, 2]), 3, float(cutoff))
             self[i + 1] = V.conj().tensordot(self[i + 1], ([0], [0]))
             self[i] = U.mul(d).permute([0, 1, 3, 2])
         return self
