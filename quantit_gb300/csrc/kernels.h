@@ -205,11 +205,11 @@ constexpr size_t LQ_SMEM_MAX = 200 * 1024;
 int lq_max_q(int f32, int nsec);
 void launch_lq(void *work, void *rot, const std::vector<LqSec> &secs, int f32);
 // FP64 refinement of an FP32 sector decomposition (mixed path): from the FP32
-// rotations rot32 (at rot_off), vb <- the FP64-orthogonalised rotation (two
-// Newton-Schulz steps through va, with g as q x q scratch), w1 <- w64 vb (at w_off).
+// rotations rot32 (at rot_off; rot_size elements in all), vb <- the FP64-orthogonalised rotation
+// (two Newton-Schulz steps through va, with g as q x q scratch), w1 <- w64 vb (at w_off).
 // The FP64 Jacobi then runs warm on (w1, vb).
-void launch_svd_refine(const float *rot32, const double *w64, double *w1, double *va, double *vb, double *g,
-                       const std::vector<SectorDesc> &secs);
+void launch_svd_refine(const float *rot32, int64_t rot_size, const double *w64, double *w1, double *va, double *vb,
+                       double *g, const std::vector<SectorDesc> &secs);
 // out[s_off + j] = squared norm (FP64) of column j of every sector's work matrix (f32:
 // FP32 work matrices)
 void launch_col_norms(const void *W, const SectorDesc *secs, int nsec, int max_q, double *out, int f32);
@@ -260,8 +260,9 @@ void launch_jacobi(void *work, void *rot, const SectorDesc *sec, const int *slot
                    int max_steps_per_sweep, int max_sweeps, int *sweeps_out, int *flags, int f32, int max_p,
                    int64_t sum_q, void *vwork = nullptr, size_t vwork_bytes = 0, const void *defl = nullptr,
                    void *dnorm = nullptr, const void *skip = nullptr, bool exact = false);
-// thr[s] <- delta^2 ||W_s||_F^2 for every svd sector (0 for eigh), in the work type.
-void launch_deflation_thresholds(const void *work, const SectorDesc *sec, int nsec, double delta, void *thr, int f32);
+// thr[s] <- delta^2 ||W_s||_F^2 for every svd sector (0 for eigh), in the work type; norms: the
+// squared column norms (launch_col_norms).
+void launch_deflation_thresholds(const double *norms, const SectorDesc *sec, int nsec, double delta, void *thr, int f32);
 // dnorm (with defl; the work type, sum of q entries at s_off, zero on entry) receives
 // the squared norm of every deflated column.
 size_t jacobi_vwork_bytes(int nsec, int64_t sum_q, int max_steps_per_sweep, int max_sweeps, int f32);
@@ -272,10 +273,12 @@ size_t jacobi_vwork_bytes(int nsec, int64_t sum_q, int max_steps_per_sweep, int 
 // completes only the first complete_cap null columns of each sector (in value
 // order): the caller truncates the others away.  perm_out (sum of q ints at s_off) with
 // complete_cap == 0: the factor writes run on many CTAs per sector (max_elems: the
-// largest q * (p + q) over the sectors).
+// largest q * (p + q) over the sectors).  norms (optional): work's squared column norms, which one
+// CTA per sector otherwise forms.
 void launch_finish(const void *work, const void *rot, double *U, double *V, double *s, const SectorDesc *sec,
                    int nsec, int max_q, double *scratch, int f32, int complete_cap = -1, const void *dnorm = nullptr,
-                   int *dpos = nullptr, int *perm_out = nullptr, int64_t max_elems = 0);
+                   int *dpos = nullptr, int *perm_out = nullptr, int64_t max_elems = 0,
+                   const double *norms = nullptr);
 // The same two launches on an explicit stream (no library context involved).
 // tune == false never times block widths (no host synchronisation): the width the
 // autotuner settled on for the class is used if there is one, else the default.
@@ -287,7 +290,7 @@ void launch_jacobi_on(cudaStream_t stream, void *work, void *rot, const SectorDe
 void launch_finish_on(cudaStream_t stream, const void *work, const void *rot, double *U, double *V, double *s,
                       const SectorDesc *sec, int nsec, int max_q, double *scratch, int f32, int complete_cap = -1,
                       const void *dnorm = nullptr, int *dpos = nullptr, int *perm_out = nullptr,
-                      int64_t max_elems = 0);
+                      int64_t max_elems = 0, const double *norms = nullptr);
 // Segment = one output block (rows x k row-major at dst_off) from a column-major
 // (ld x *) sector matrix at src_off: dst[i*k + j] = src[src_off + (r0 + i) + j*ld].
 struct ScatterEntry {

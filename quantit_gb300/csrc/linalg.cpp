@@ -383,13 +383,16 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
         // otherwise be rotated against each other for many sweeps to no effect.  Its
         // last norm is kept as its value (below any threshold a truncation keeps).
         const bool deflate = cap == 0 && svd_deflation();
+        BufPtr norm_buf = dev_alloc(size_t(std::max<int64_t>(stot, 1)) * 8);
+        double *norms = static_cast<double *>(norm_buf->p);
         auto deflation = [&](const void *w, int prec32, BufPtr &thr, BufPtr &dn) {
             const size_t e = prec32 ? 4 : 8;
             thr = dev_alloc(size_t(nsec) * e);
             dn = dev_alloc(size_t(std::max<int64_t>(stot, 1)) * e);
             cuda_check(cudaMemsetAsync(dn->p, 0, size_t(std::max<int64_t>(stot, 1)) * e, ctx().stream),
                        "cudaMemsetAsync(dnorm)");
-            launch_deflation_thresholds(w, dsec, nsec, prec32 ? kDeflateF32 : kDeflateF64, thr->p, prec32);
+            launch_col_norms(w, dsec, nsec, max_q, norms, prec32);
+            launch_deflation_thresholds(norms, dsec, nsec, prec32 ? kDeflateF32 : kDeflateF64, thr->p, prec32);
         };
         BufPtr thr, dnorm;
         if (deflate) deflation(W, f32, thr, dnorm);
@@ -470,7 +473,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                 cuda_check(cudaMemcpyAsync(w1->p, w64->p, size_t(wtot) * 8, cudaMemcpyDeviceToDevice, ctx().stream),
                            "cudaMemcpyAsync(work64)");
             } else {
-                launch_svd_refine(static_cast<const float *>(D.rot->p), static_cast<const double *>(w64->p),
+                launch_svd_refine(static_cast<const float *>(D.rot->p), rtot, static_cast<const double *>(w64->p),
                                   static_cast<double *>(w1->p), static_cast<double *>(va->p),
                                   static_cast<double *>(vbuf->p), static_cast<double *>(gbuf->p), D.desc);
             }
@@ -637,10 +640,11 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             permbuf = dev_alloc(size_t(std::max<int64_t>(stot, 1)) * sizeof(int));
             for (const SectorDesc &d : D.desc) max_elems = std::max(max_elems, int64_t(d.q) * (d.p + d.q));
         }
+        launch_col_norms(fw, dsec, nsec, max_q, norms, 0);
         launch_finish(fw, fr, static_cast<double *>(D.U->p), static_cast<double *>(D.V->p),
                       static_cast<double *>(D.S->p), dsec, nsec, max_q, static_cast<double *>(scratch->p), 0, cap,
                       dnorm ? dnorm->p : nullptr, nullptr, permbuf ? static_cast<int *>(permbuf->p) : nullptr,
-                      max_elems);
+                      max_elems, norms);
         if (ws) {
             // this decomposition's rotations (of the first stage) start the next one at the same bond
             std::vector<WarmStart::Entry> next;

@@ -7,129 +7,172 @@
 // the FP64 sector matrix:
 //
 //   1. V0 is orthogonal only to ~1e-6 (FP32 accumulation).  Two Newton-Schulz steps
-//      V <- V (3 I - V^T V) / 2 in FP64 make it orthogonal to FP64 precision (each step
-//      squares the departure from orthogonality: 1e-6 -> 1e-12 -> 1e-16).
+//      V <- V + V E, E = (I - V^T V) / 2, in FP64 make it orthogonal to FP64 precision (each
+//      step squares the departure from orthogonality: 1e-6 -> 1e-12 -> 1e-16).
 //   2. W1 = W V in FP64 from the FP64 sector matrix W.
 //   3. The FP64 Jacobi sweeps run on (W1, V).  Any orthogonal V gives an exact SVD of
 //      W (W V = U S Vt^T => W = U S (V Vt)^T), so the factors are an FP64 SVD; from the
 //      near-diagonal W1 the columns FP32 resolved converge in a sweep or two.
 //
-// All three steps are batched FP64 GEMMs over the sectors of one decomposition
-// (k_secgemm): 64 x 64 output tiles, 256 threads with 4 x 4 outputs each, K slabs
-// of 16 through shared memory.  GB300's FP64 pipe (about 2 FMA per clock per SM)
-// bounds them; shared-memory traffic is 8 loads per 16 FMA.
+// The Gram matrices and W V are FP64 products of the grouped block GEMM (gemm_f64.cu), all sectors
+// of a decomposition in one launch.  The correction V E is formed in FP32: E is at most 1e-6 (then
+// 1e-12), so its relative error of 1e-7 leaves 1e-13 behind in the first step, which the second
+// removes with the rest, and 1e-19 in the second.  That leaves 2 q^3 of 6 q^3 FP64 FLOP to the
+// orthogonalisation; with it and the finer tiles of the Grams' upper halves (64 x 64 tiles of a q ~
+// 900 sector left the SMs a last wave of a few) the five products of the cylinder theta at D = 2048
+// went from 19.3 to 7.7 ms (its whole decomposition from 70 to 58 ms).
 #include "kernels.h"
 #include "qtt_core.h"
 
 namespace qtt {
 namespace {
 
-// C[M x N] (column-major, ldc) = op(A) B', A = M x K (a_trans: stored K x M), and
-// B' = B (K x N) or, with b_ns, 1.5 I - 0.5 B (the Newton-Schulz factor).  sym bit 0: C is
-// symmetric (A^T A), only tiles on or above the diagonal are computed; bit 1: B is such a
-// matrix, its elements below the diagonal are read from above it.
-struct SecGemm {
-    int64_t a_off, b_off, c_off;
-    int32_t M, N, K, lda, ldb, ldc;
-    int32_t a_trans, b_ns, tile_start, sym;
+constexpr int CT = 64, CK = 16;  // FP32 correction: tile and K slab
+
+// out = V + 0.5 V (I - G) per sector (q x q, column-major); G's elements below the diagonal are
+// read from above it (G[min + max q]).
+struct Correction {
+    int64_t off;
+    int32_t q, tile_start;
 };
 
-template <class TA, class TB>
-__global__ void __launch_bounds__(256) k_secgemm(const TA *__restrict__ A, const TB *__restrict__ B,
-                                                 double *__restrict__ C, const SecGemm *__restrict__ g, int ng) {
-    __shared__ double As[16][64 + 1];
-    __shared__ double Bs[16][64 + 1];
-    int lo = 0, hi = ng - 1;
+template <class TV>
+__global__ void __launch_bounds__(256) k_ns_correct(const TV *__restrict__ V, const double *__restrict__ G,
+                                                    double *__restrict__ out, const Correction *__restrict__ cs, int n) {
+    __shared__ float As[CK][CT + 1];
+    __shared__ float Bs[CK][CT + 1];
+    int lo = 0, hi = n - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (g[mid].tile_start <= int(blockIdx.x))
+        if (cs[mid].tile_start <= int(blockIdx.x))
             lo = mid;
         else
             hi = mid - 1;
     }
-    const SecGemm d = g[lo];
-    const int tm = (d.M + 63) / 64;
-    const int t = int(blockIdx.x) - d.tile_start;
-    const int r0 = (t % tm) * 64, c0 = (t / tm) * 64;
-    if ((d.sym & 1) && c0 + 63 < r0) return;  // strictly below the diagonal of a symmetric C
-    const TA *a = A + d.a_off;
-    const TB *b = B + d.b_off;
+    const Correction c = cs[lo];
+    const int q = c.q, tm = (q + CT - 1) / CT, t = int(blockIdx.x) - c.tile_start;
+    const int r0 = (t % tm) * CT, c0 = (t / tm) * CT;
+    const TV *v = V + c.off;
+    const double *g = G + c.off;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[4][4];
+    float acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-    for (int k0 = 0; k0 < d.K; k0 += 16) {
-        for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            // A tile: the stored layout's contiguous index runs fastest across threads
-            int i, kk;
-            if (d.a_trans) {
-                kk = e % 16;
-                i = e / 16;
-            } else {
-                i = e % 64;
-                kk = e / 64;
-            }
-            const int r = r0 + i, k = k0 + kk;
-            double av = 0.0;
-            if (r < d.M && k < d.K)
-                av = double(d.a_trans ? a[int64_t(r) * d.lda + k] : a[int64_t(k) * d.lda + r]);
-            As[kk][i] = av;
-            // B tile: k contiguous within a column
-            const int kb = e % 16, jj = e / 16;
-            const int c = c0 + jj, kq = k0 + kb;
-            double bv = 0.0;
-            if (c < d.N && kq < d.K) {
-                const int lo = (d.sym & 2) ? min(kq, c) : kq, hi = (d.sym & 2) ? max(kq, c) : c;
-                bv = double(b[int64_t(hi) * d.ldb + lo]);
-                if (d.b_ns) bv = (kq == c ? 1.5 : 0.0) - 0.5 * bv;
-            }
-            Bs[kb][jj] = bv;
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    for (int k0 = 0; k0 < q; k0 += CK) {
+        for (int e = threadIdx.x; e < CK * CT; e += 256) {
+            const int i = e % CT, kk = e / CT, r = r0 + i, k = k0 + kk;
+            As[kk][i] = r < q && k < q ? float(v[int64_t(k) * q + r]) : 0.0f;
+            const int kb = e % CK, jj = e / CK, col = c0 + jj, kq = k0 + kb;
+            float x = 0.0f;
+            if (col < q && kq < q) x = float((kq == col ? 1.0 : 0.0) - g[int64_t(max(kq, col)) * q + min(kq, col)]);
+            Bs[kb][jj] = x;
         }
         __syncthreads();
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            double av[4], bv[4];
+        for (int kk = 0; kk < CK; ++kk) {
+            float a[4], b[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) av[i] = As[kk][tx + 16 * i];
+            for (int i = 0; i < 4; ++i) a[i] = As[kk][tx + 16 * i];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][ty + 16 * j];
+            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][ty + 16 * j];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
         __syncthreads();
     }
-    double *c = C + d.c_off;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int col = c0 + ty + 16 * j;
-        if (col >= d.N) continue;
+        if (col >= q) continue;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int row = r0 + tx + 16 * i;
-            if (row < d.M) c[int64_t(col) * d.ldc + row] = acc[i][j];
+            if (row < q) out[c.off + int64_t(col) * q + row] = double(v[int64_t(col) * q + row]) + 0.5 * double(acc[i][j]);
         }
     }
 }
 
-template <class TA, class TB>
-void secgemm(const TA *A, const TB *B, double *C, std::vector<SecGemm> &tasks, cudaStream_t st) {
+template <class TV>
+void ns_correct(const TV *V, const double *G, double *out, const std::vector<SectorDesc> &secs) {
+    std::vector<Correction> cs;
     int tiles = 0;
-    std::vector<SecGemm> live;
-    for (SecGemm &t : tasks) {
-        if (t.M <= 0 || t.N <= 0 || t.K <= 0) continue;
-        t.tile_start = tiles;
-        tiles += ((t.M + 63) / 64) * ((t.N + 63) / 64);
-        live.push_back(t);
+    for (const SectorDesc &s : secs) {
+        if (s.q <= 0) continue;
+        cs.push_back(Correction{s.rot_off, s.q, tiles});
+        const int t = (s.q + CT - 1) / CT;
+        tiles += t * t;
     }
-    if (live.empty()) return;
-    const SecGemm *dg = upload_vec(live);
-    k_secgemm<TA, TB><<<tiles, 256, 0, st>>>(A, B, C, dg, int(live.size()));
+    if (cs.empty()) return;
+    k_ns_correct<TV><<<tiles, 256, 0, ctx().stream>>>(V, G, out, upload_vec(cs), int(cs.size()));
     count_launch();
-    cuda_check(cudaGetLastError(), "sector GEMM launch");
+    cuda_check(cudaGetLastError(), "Newton-Schulz correction launch");
+}
+
+// One FP64 product per task in one launch of the grouped block GEMM, column-major:
+// C (M x N, ldc = M) = op(A) B, A M x K (a_trans: stored K x M), B K x N.  upper: C is symmetric, tiles
+// strictly below the diagonal are left out.
+struct Product {
+    int64_t a_off, b_off, c_off;
+    int32_t M, N, K;
+    bool a_trans, upper;
+};
+void products(const double *A, const double *B, double *C, const std::vector<Product> &tasks) {
+    // the GEMM writes row-major: C^T = B^T op(A)^T, so its rows are our columns
+    std::vector<F64Pair> pairs;
+    std::vector<GemmOut> outs;
+    std::vector<GemmTile> tiles;
+    int64_t square = 0;
+    for (const Product &t : tasks) square += ((int64_t(t.M) + 31) / 32) * ((int64_t(t.N) + 31) / 32);
+    const bool fine = square < 4 * device_sm_count();
+    for (const Product &t : tasks) {
+        if (t.M <= 0 || t.N <= 0 || t.K <= 0) continue;
+        F64Pair p{};
+        p.a_off = t.b_off;
+        p.b_off = t.a_off;
+        p.k1 = 1;
+        p.k2 = t.K;
+        p.ak2 = 1;
+        p.bk2 = t.a_trans ? 1 : t.M;
+        p.am2 = t.N;
+        p.as2 = t.K;
+        p.bn2 = t.M;
+        p.bs2 = t.a_trans ? t.K : 1;
+        GemmOut o{};
+        o.c_off = t.c_off;
+        o.add_off = -1;
+        o.M = t.N;
+        o.N = t.M;
+        o.p0 = int32_t(pairs.size());
+        o.p1 = o.p0 + 1;
+        int tm, tn;
+        const int cls = gemm_f64_class(o.M, o.N, t.K, &tm, &tn, fine);
+        for (int m0 = 0; m0 < o.M; m0 += tm)
+            for (int n0 = 0; n0 < o.N; n0 += tn) {
+                // (row of C^T = column of C) a tile is needed if it reaches the diagonal or above
+                if (t.upper && n0 > m0 + tm - 1) continue;
+                tiles.push_back(GemmTile{int32_t(outs.size()), m0, n0, cls});
+            }
+        pairs.push_back(p);
+        outs.push_back(o);
+    }
+    if (tiles.empty()) return;
+    std::stable_sort(tiles.begin(), tiles.end(), [&](const GemmTile &x, const GemmTile &y) {
+        return pairs[x.out].k2 > pairs[y.out].k2;
+    });
+    F64Args g;
+    g.A = B;
+    g.B = A;
+    g.C = C;
+    g.Cadd = nullptr;
+    upload_many({table(pairs, g.pairs), table(outs, g.outs), table(tiles, g.tiles)});
+    g.ntiles = int32_t(tiles.size());
+    g.alpha = 1.0;
+    g.beta = 0.0;
+    launch_gemm_f64(g);
 }
 
 // Squared column norms of every sector matrix (one warp per column).
@@ -167,10 +210,9 @@ void launch_col_copy(const double *src, double *dst, const std::vector<ColCopy> 
 }
 
 void launch_rot_product(const double *vg, const double *r, double *vn, const std::vector<RotProduct> &t) {
-    std::vector<SecGemm> g;
-    for (const RotProduct &e : t)
-        g.push_back({e.vg_off, e.r_off, e.vn_off, e.vrows, e.k, e.k, e.vrows, e.k, e.vrows, 0, 0, 0, 0});
-    secgemm(vg, r, vn, g, ctx().stream);
+    std::vector<Product> g;
+    for (const RotProduct &e : t) g.push_back({e.vg_off, e.r_off, e.vn_off, e.vrows, e.k, e.k, false, false});
+    products(vg, r, vn, g);
 }
 
 void launch_col_norms(const void *W, const SectorDesc *secs, int nsec, int max_q, double *out, int f32) {
@@ -184,40 +226,21 @@ void launch_col_norms(const void *W, const SectorDesc *secs, int nsec, int max_q
     cuda_check(cudaGetLastError(), "column norm launch");
 }
 
-void launch_svd_refine(const float *rot32, const double *w64, double *w1, double *va, double *vb, double *g,
-                       const std::vector<SectorDesc> &secs) {
-    cudaStream_t st = ctx().stream;
-    auto gram = [&]() {
-        std::vector<SecGemm> t;
-        for (const SectorDesc &s : secs)
-            t.push_back({s.rot_off, s.rot_off, s.rot_off, s.q, s.q, s.q, s.q, s.q, s.q, 1, 0, 0, 1});
-        return t;
-    };
-    auto ns = [&]() {
-        std::vector<SecGemm> t;
-        for (const SectorDesc &s : secs)
-            t.push_back({s.rot_off, s.rot_off, s.rot_off, s.q, s.q, s.q, s.q, s.q, s.q, 0, 1, 0, 2});
-        return t;
-    };
-    // Newton-Schulz step 1 from the FP32 rotation: G = V0^T V0, va = V0 (1.5 I - 0.5 G)
-    {
-        auto t = gram();
-        secgemm(rot32, rot32, g, t, st);
-        auto u = ns();
-        secgemm(rot32, static_cast<const double *>(g), va, u, st);
+void launch_svd_refine(const float *rot32, int64_t rot_size, const double *w64, double *w1, double *va, double *vb,
+                       double *g, const std::vector<SectorDesc> &secs) {
+    std::vector<Product> gram, wv;
+    for (const SectorDesc &s : secs) {
+        gram.push_back({s.rot_off, s.rot_off, s.rot_off, s.q, s.q, s.q, true, true});
+        wv.push_back({s.w_off, s.rot_off, s.w_off, s.p, s.q, s.q, false, false});
     }
-    // step 2 in FP64: G = va^T va, vb = va (1.5 I - 0.5 G)
-    {
-        auto t = gram();
-        secgemm(static_cast<const double *>(va), static_cast<const double *>(va), g, t, st);
-        auto u = ns();
-        secgemm(static_cast<const double *>(va), static_cast<const double *>(g), vb, u, st);
-    }
-    // W1 = W vb
-    std::vector<SecGemm> t;
-    for (const SectorDesc &s : secs)
-        t.push_back({s.w_off, s.rot_off, s.w_off, s.p, s.q, s.q, s.p, s.q, s.p, 0, 0, 0, 0});
-    secgemm(w64, static_cast<const double *>(vb), w1, t, st);
+    // step 1 from the FP32 rotation (widened into vb): va = V0 + V0 (I - V0^T V0) / 2
+    launch_convert(rot32, vb, rot_size, 0, 1);
+    products(vb, vb, g, gram);
+    ns_correct(rot32, g, va, secs);
+    // step 2: vb = va + va (I - va^T va) / 2
+    products(va, va, g, gram);
+    ns_correct(static_cast<const double *>(va), g, vb, secs);
+    products(w64, vb, w1, wv);
 }
 
 }  // namespace qtt
