@@ -479,7 +479,7 @@ __device__ __forceinline__ void bj_store(const T (&x)[R], T *slot, int lane) {
 // Per-lane partial sums in NA independent chains (the dot product is on the
 // critical path of every round: R dependent FMAs would cost R FMA latencies).
 template <class T, int R>
-__device__ __forceinline__ T bj_dot(const T (&x)[R], const T (&y)[R]) {
+__device__ __forceinline__ T bj_lane_dot(const T (&x)[R], const T (&y)[R]) {
     constexpr int NA = R >= 16 ? 4 : (R >= 4 ? 2 : 1);
     T a[NA];
 #pragma unroll
@@ -490,7 +490,53 @@ __device__ __forceinline__ T bj_dot(const T (&x)[R], const T (&y)[R]) {
     for (int w = NA / 2; w > 0; w >>= 1)
 #pragma unroll
         for (int k = 0; k < w; ++k) a[k] += a[k + w];
-    return wsum(a[0]);
+    return a[0];
+}
+template <class T, int R>
+__device__ __forceinline__ T bj_dot(const T (&x)[R], const T (&y)[R]) {
+    return wsum(bj_lane_dot(x, y));
+}
+
+// x 2^-sh as FP32 by integer operations (no FP64 conversion): sh within the exponent range,
+// results below FP32's normal range flush to zero, above it are not allowed for.
+__device__ __forceinline__ float scaled_f32(double x, int sh) {
+    const uint32_t hi = uint32_t(__double2hiint(x)), lo = uint32_t(__double2loint(x));
+    const int t = int(hi & 0x7FFFFFFFu) - ((896 + sh) << 20);
+    const uint32_t f = __funnelshift_l(lo, uint32_t(t), 3);
+    return __uint_as_float((hi & 0x80000000u) | (t < (1 << 20) ? 0u : f));
+}
+// FP32 (normal or zero) -> FP64, times 2^sh, by integer operations.
+__device__ __forceinline__ double widen_f32(float f, int sh = 0) {
+    const uint32_t b = __float_as_uint(f), m = b & 0x7FFFFFFFu;
+    const uint32_t hi = (b & 0x80000000u) | (m < 0x00800000u ? 0u : (m >> 3) + (uint32_t(896 + sh) << 20));
+    return __hiloint2double(int(hi), m < 0x00800000u ? 0 : int(b << 29));
+}
+
+// Warp sum of doubles with sum |v| < 2^(sh + 2), in fixed point with 2^(sh - 60) as the unit: three
+// integer reductions of the multi-function unit instead of five FP64 additions (64 clocks each).  A lane is
+// cut at the unit, the sum of the lanes is exact.
+__device__ __forceinline__ double fixed_wsum(double v, int sh) {
+    const uint32_t hi = uint32_t(__double2hiint(v)), lo = uint32_t(__double2loint(v));
+    const int e = int((hi >> 20) & 0x7FFu);
+    // mantissa 2^52 .. 2^53, worth 2^(e - 1075); in units: shifted by e - 1075 + 60 - sh
+    const int s = e - 1015 - sh;
+    long long f = (long long)(((unsigned long long)((hi & 0xFFFFFu) | (e ? 0x100000u : 0u)) << 32) | lo);
+    f = s >= 0 ? f << min(s, 10) : (s > -54 ? f >> -s : 0);
+    if (hi & 0x80000000u) f = -f;
+    const int s0 = __reduce_add_sync(0xffffffffu, int(f & 0x1FFFFF));
+    const int s1 = __reduce_add_sync(0xffffffffu, int((f >> 21) & 0x1FFFFF));
+    const int s2 = __reduce_add_sync(0xffffffffu, int(f >> 42));
+    const long long t = ((long long)s2 << 42) + ((long long)s1 << 21) + s0;
+    // back to a double, rounded to nearest
+    const unsigned long long a = t < 0 ? (unsigned long long)(-t) : (unsigned long long)t;
+    if (a == 0) return 0.0;
+    const int z = __clzll((long long)a);
+    const unsigned long long n = a << z;  // leading one at bit 63, worth 2^(63 - z + sh - 60)
+    unsigned long long m = (n >> 11) + ((n >> 10) & 1ull);
+    // m's leading one adds to the exponent field
+    const unsigned long long ex = (unsigned long long)(63 - z + sh - 60 + 1023 - 1);
+    m += ex << 52;
+    return __longlong_as_double((long long)(m | (t < 0 ? 1ull << 63 : 0ull)));
 }
 
 // Rotation parameters from the multi-function unit (FP32 only).  t need not be
@@ -514,21 +560,6 @@ __device__ __forceinline__ void bj_params_fast(float al, float be, float ga, flo
     tau = __fdividef(t, 1.0f + w2 * rh);
 }
 
-// x 2^-sh as FP32 by integer operations (no FP64 conversion): sh within the exponent range,
-// results below FP32's normal range flush to zero, above it are not allowed for.
-__device__ __forceinline__ float scaled_f32(double x, int sh) {
-    const uint32_t hi = uint32_t(__double2hiint(x)), lo = uint32_t(__double2loint(x));
-    const int t = int(hi & 0x7FFFFFFFu) - ((896 + sh) << 20);
-    const uint32_t f = __funnelshift_l(lo, uint32_t(t), 3);
-    return __uint_as_float((hi & 0x80000000u) | (t < (1 << 20) ? 0u : f));
-}
-// FP32 (normal or zero) -> FP64 by integer operations.
-__device__ __forceinline__ double widen_f32(float f) {
-    const uint32_t b = __float_as_uint(f), m = b & 0x7FFFFFFFu;
-    const uint32_t hi = (b & 0x80000000u) | (m < 0x00800000u ? 0u : (m >> 3) + (896u << 20));
-    return __hiloint2double(int(hi), m < 0x00800000u ? 0 : int(b << 29));
-}
-
 // FP64 rotation parameters with few FP64 instructions.  GB300 issues an FP64 warp
 // instruction in 64 clocks per scheduler, so the square roots and divisions of
 // rot_params (over 100 instructions with their FP64 iterations) cost a round more than
@@ -537,22 +568,29 @@ __device__ __forceinline__ double widen_f32(float f) {
 // 1e-7 leaves 1e-7 of the coupling, which the quadratic convergence of the sweeps leaves
 // behind anyway -- so tau comes from FP32 and the multi-function unit, on operands brought
 // into FP32's range by their exponents, and only s (a reciprocal with one cubically convergent
-// step) and the norms' update are FP64: 12 instructions.  The difference of the norms is
-// formed in FP64 first: near-equal norms would lose it in FP32.
-// Returns 0: no rotation (coupling within tol), 1: s, tau, rel set and al, be updated, 2: norms
-// further apart than FP32's exponents allow for (the caller takes the plain formulas).
-__device__ __forceinline__ int bj_params_fast64(double &al, double &be, double ga, float tol, double &sn, double &tau,
-                                                float &rel) {
+// step) is FP64.  The difference of the norms is formed in FP64 first: near-equal norms would lose it
+// in FP32.  The norms' change t ga is FP32 as well: 1e-7 of it matters only while couplings of that
+// size are left, and the norms are formed anew at the next step.  Eight FP64 instructions in all.
+//
+// Columns of norm ~ 2^ka, 2^kb (half the exponents of al, be); false: norms further apart, or closer to
+// the ends of the exponent range, than the conversions allow for (the caller takes the plain formulas).
+__device__ __forceinline__ bool bj_exponents(double al, double be, int &ka, int &kb) {
     const int ea = int((uint32_t(__double2hiint(al)) >> 20) & 0x7FFu), eb = int((uint32_t(__double2hiint(be)) >> 20) & 0x7FFu);
-    // half the exponents: columns of norm ~ 2^ka, 2^kb
-    const int ka = (ea - 1023) >> 1, kb = (eb - 1023) >> 1, d = kb - ka, sh = ka + kb;
-    if (d > 50 || d < -50 || ea < 64 || eb < 64 || ea > 1982 || eb > 1982) return 2;
+    ka = (ea - 1023) >> 1;
+    kb = (eb - 1023) >> 1;
+    const int d = kb - ka;
+    return d <= 50 && d >= -50 && ea >= 64 && eb >= 64 && ea <= 1982 && eb <= 1982;
+}
+// 0: no rotation (coupling within tol), 1: s, tau, rel set and al, be updated, 2: an angle below
+// FP32's range (the plain formulas).
+__device__ __forceinline__ int bj_params_fast64(double &al, double &be, double ga, int ka, int kb, float tol, double &sn,
+                                                double &tau, float &rel) {
+    const int sh = ka + kb;
     const float ma = scaled_f32(al, 2 * ka), mb = scaled_f32(be, 2 * kb);  // in [1, 4)
     const float g = scaled_f32(ga, sh);                                    // |g| <= 4
     rel = fabsf(g) * rsqrtf(ma) * rsqrtf(mb);
     if (!(rel > tol)) return 0;
-    const double diff = be - al;
-    const float df = scaled_f32(diff, sh);                                 // up to 2^52
+    const float df = scaled_f32(be - al, sh);                              // up to 2^52
     const float zeta = __fdividef(df, 2.0f * g), az = fabsf(zeta);         // up to 2^105
     float t;
     if (az > 1e9f)
@@ -566,14 +604,12 @@ __device__ __forceinline__ int bj_params_fast64(double &al, double &be, double g
     if (fabsf(tf) < 1.17549435e-38f) return 2;
     tau = widen_f32(tf);
     const double r0 = widen_f32(__fdividef(1.0f, fmaf(tf, tf, 1.0f)));  // 1 / (1 + tau^2) to ~1e-7
-    const double u = fma(tau, tau, 1.0);
-    const double e = fma(-u, r0, 1.0);
+    const double e = fma(-fma(tau, tau, 1.0), r0, 1.0);
     const double r = fma(r0, fma(e, e, e), r0);              // to FP64 precision (e^3)
-    sn = (tau + tau) * r;
-    const double c = fma(-sn, tau, 1.0);
-    const double q = fma(-c, ga + ga, sn * diff);            // al' = c^2 al - 2 c s ga + s^2 be
-    al = fma(sn, q, al);
-    be = fma(-sn, q, be);
+    sn = widen_f32(2.0f * tf) * r;
+    const double dn = widen_f32(t * g, sh);                  // al' = al - t ga, be' = be + t ga
+    al -= dn;
+    be += dn;
     return 1;
 }
 
@@ -601,33 +637,32 @@ __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], T &al, T &be, T 
                                           T &dy, T skip, float &rmax) {
     if (al == T(0) || be == T(0)) return false;
     if (pair_skipped(al, be, skip)) return false;
-    const T ga = bj_dot(x, y);
-    if (ga == T(0)) return false;
-    T t, a2, b2;
+    T ga, t, a2, b2;
     if constexpr (sizeof(T) == 4) {
+        ga = bj_dot(x, y);
+        if (ga == T(0)) return false;
         const float rel = fabsf(ga) * rsqrtf(al) * rsqrtf(be);
         if (rel <= tol) return false;
         rmax = fmaxf(rmax, rel);
         bj_params_fast(al, be, ga, sn, tau, t);
         a2 = al - t * ga;
         b2 = be + t * ga;
-    } else if constexpr (EXACT) {
-        const double rel = fabs(ga) / sqrt(al * be);
-        if (rel <= tol) return false;
-        rmax = fmaxf(rmax, float(rel));
-        rot_params(al, be, ga, sn, tau, t);
-        a2 = al - t * ga;
-        b2 = be + t * ga;
     } else {
-        float rel32;
+        int ka = 0, kb = 0, how = 2;
+        const bool fast = !EXACT && bj_exponents(al, be, ka, kb);
+        ga = bj_lane_dot(x, y);
+        ga = fast ? fixed_wsum(ga, ka + kb) : wsum(ga);
+        if (ga == T(0)) return false;
         a2 = al;
         b2 = be;
-        const int how = bj_params_fast64(a2, b2, ga, float(tol), sn, tau, rel32);
-        if (how == 0) return false;
-        if (how == 1) {
-            rmax = fmaxf(rmax, rel32);
-        } else {
-            const double rel = fabs(ga) / (sqrt(al) * sqrt(be));
+        if (fast) {
+            float rel32;
+            how = bj_params_fast64(a2, b2, ga, ka, kb, float(tol), sn, tau, rel32);
+            if (how == 0) return false;
+            if (how == 1) rmax = fmaxf(rmax, rel32);
+        }
+        if (how == 2) {
+            const double rel = EXACT ? fabs(ga) / sqrt(al * be) : fabs(ga) / (sqrt(al) * sqrt(be));
             if (!(rel > tol)) return false;
             rmax = fmaxf(rmax, float(rel));
             rot_params(al, be, ga, sn, tau, t);
