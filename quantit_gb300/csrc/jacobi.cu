@@ -59,11 +59,14 @@ __device__ __forceinline__ float ldcg(const float *p) { return __ldcg(p); }
 // For small angles c rounds to 1 while 1 - c = s tau does not, so the plain form
 // c x - s y would scale both columns by sqrt(1 + t^2) at every such rotation; in
 // FP32 that bias accumulates to ~1e-5 in the singular values over a few sweeps.
-// In FP64 the same rotation as three shears, x -= tau y, y += s x, x -= tau y: three
-// instead of four instructions of GB300's narrow FP64 pipe per element pair.
-template <class T, bool EXACT = false>
+// In FP64 the block kernel rotates columns of more than 128 rows by the same rotation as three shears, x -= tau y, y += s x,
+// x -= tau y: three instead of four instructions of GB300's narrow FP64 pipe per element pair.  A third
+// dependent rounding makes the values' error ~1.2 times that of the form above, which LQ's fewer sweeps more
+// than win back; shorter columns, which mostly run without LQ, keep the form above (eigh D = 300: 2.00 ms with
+// the shears, 2.08 with the four instructions).
+template <class T, bool FOUR = true>
 __device__ __forceinline__ void rot_apply(T &x, T &y, T s, T tau) {
-    if constexpr (sizeof(T) == 8 && !EXACT) {
+    if constexpr (sizeof(T) == 8 && !FOUR) {
         x = fma(-tau, y, x);
         y = fma(s, x, y);
         x = fma(-tau, y, x);
@@ -505,6 +508,12 @@ __device__ __forceinline__ float scaled_f32(double x, int sh) {
     const uint32_t f = __funnelshift_l(lo, uint32_t(t), 3);
     return __uint_as_float((hi & 0x80000000u) | (t < (1 << 20) ? 0u : f));
 }
+// What scaled_f32 cut off: x 2^-sh - f for f = scaled_f32(x, sh), from x's last 29 bits.
+__device__ __forceinline__ float scaled_low(double x, float f) {
+    const uint32_t b = __float_as_uint(f), e = b & 0x7F800000u;
+    const float unit = __uint_as_float(e > (52u << 23) ? (e - (52u << 23)) | (b & 0x80000000u) : 0u);
+    return float(uint32_t(__double2loint(x)) & 0x1FFFFFFFu) * unit;
+}
 // FP32 (normal or zero) -> FP64, times 2^sh, by integer operations.
 __device__ __forceinline__ double widen_f32(float f, int sh = 0) {
     const uint32_t b = __float_as_uint(f), m = b & 0x7FFFFFFFu;
@@ -563,14 +572,16 @@ __device__ __forceinline__ void bj_params_fast(float al, float be, float ga, flo
 // FP64 rotation parameters with few FP64 instructions.  GB300 issues an FP64 warp
 // instruction in 64 clocks per scheduler, so the square roots and divisions of
 // rot_params (over 100 instructions with their FP64 iterations) cost a round more than
-// its columns up to p ~ 1000.  The angle need not be the exact optimum -- any tau gives an
-// orthogonal rotation as long as s = 2 tau / (1 + tau^2) holds to FP64, and an angle off by
-// 1e-7 leaves 1e-7 of the coupling, which the quadratic convergence of the sweeps leaves
-// behind anyway -- so tau comes from FP32 and the multi-function unit, on operands brought
-// into FP32's range by their exponents, and only s (a reciprocal with one cubically convergent
-// step) is FP64.  The difference of the norms is formed in FP64 first: near-equal norms would lose it
-// in FP32.  The norms' change t ga is FP32 as well: 1e-7 of it matters only while couplings of that
-// size are left, and the norms are formed anew at the next step.  Eight FP64 instructions in all.
+// its columns up to p ~ 1000.  tau starts from FP32 and the multi-function unit, on operands
+// brought into FP32's range by their exponents, and takes one Newton step whose residual is
+// formed in pairs of FP32 numbers (rot_residual: 1e-13 of tau over all angles; the FP32 angle alone
+// leaves 4e-7 of the coupling behind, which after a late sweep lies under the acceptance threshold and
+// stays: the columns of small sectors came out up to 2.8 times less orthogonal).  Any tau gives an
+// orthogonal rotation as long as s = 2 tau / (1 + tau^2) holds to FP64: s comes from a
+// reciprocal with one cubically convergent step.  The difference of the norms is formed in FP64 first:
+// near-equal norms would lose it in FP32.  The norms' change t ga is FP32: 1e-7 of it matters only while
+// couplings of that size are left, and the norms are formed anew at the next step.  Nine FP64
+// instructions in all.
 //
 // Columns of norm ~ 2^ka, 2^kb (half the exponents of al, be); false: norms further apart, or closer to
 // the ends of the exponent range, than the conversions allow for (the caller takes the plain formulas).
@@ -581,6 +592,19 @@ __device__ __forceinline__ bool bj_exponents(double al, double be, int &ka, int 
     const int d = kb - ka;
     return d <= 50 && d >= -50 && ea >= 64 && eb >= 64 && ea <= 1982 && eb <= 1982;
 }
+// Newton's change of t = tan(theta / 2) towards the zero of ga (6 t^2 - 1 - t^4) + 2 (be - al) t (1 - t^2)
+// (the coupling after the rotation, times (1 + t^2)^2), ga = g + gl and be - al = d + dl.
+__device__ __forceinline__ float rot_residual(float t, float g, float gl, float d, float dl) {
+    const float p = t * t, pl = fmaf(t, t, -p);
+    const float q = 6.0f - p, ql = ((6.0f - q) - p) - pl;
+    const float m = p * q, ml = fmaf(p, q, -m) + fmaf(p, ql, pl * q);
+    const float c = m - 1.0f, cl = ((-1.0f - c) + m) + ml;
+    const float b = 1.0f - p, bl = ((1.0f - b) - p) - pl;
+    const float u = 2.0f * t * b, ul = fmaf(2.0f * t, b, -u) + 2.0f * t * bl;
+    const float x = g * c, xl = fmaf(g, c, -x) + fmaf(g, cl, gl * c);
+    const float y = d * u, yl = fmaf(d, u, -y) + fmaf(d, ul, dl * u);
+    return __fdividef(-((x + y) + (xl + yl)), fmaf(g * t, 12.0f - 4.0f * p, 2.0f * d * fmaf(-3.0f, p, 1.0f)));
+}
 // 0: no rotation (coupling within tol), 1: s, tau, rel set and al, be updated, 2: an angle below
 // FP32's range (the plain formulas).
 __device__ __forceinline__ int bj_params_fast64(double &al, double &be, double ga, int ka, int kb, float tol, double &sn,
@@ -590,7 +614,8 @@ __device__ __forceinline__ int bj_params_fast64(double &al, double &be, double g
     const float g = scaled_f32(ga, sh);                                    // |g| <= 4
     rel = fabsf(g) * rsqrtf(ma) * rsqrtf(mb);
     if (!(rel > tol)) return 0;
-    const float df = scaled_f32(be - al, sh);                              // up to 2^52
+    const double diff = be - al;
+    const float df = scaled_f32(diff, sh);                                 // up to 2^52
     const float zeta = __fdividef(df, 2.0f * g), az = fabsf(zeta);         // up to 2^105
     float t;
     if (az > 1e9f)
@@ -602,11 +627,11 @@ __device__ __forceinline__ int bj_params_fast64(double &al, double &be, double g
     const float w2 = fmaf(t, t, 1.0f);
     const float tf = __fdividef(t, 1.0f + w2 * rsqrtf(w2));  // tan(theta / 2), |tf| <= 0.4143
     if (fabsf(tf) < 1.17549435e-38f) return 2;
-    tau = widen_f32(tf);
-    const double r0 = widen_f32(__fdividef(1.0f, fmaf(tf, tf, 1.0f)));  // 1 / (1 + tau^2) to ~1e-7
-    const double e = fma(-fma(tau, tau, 1.0), r0, 1.0);
-    const double r = fma(r0, fma(e, e, e), r0);              // to FP64 precision (e^3)
-    sn = widen_f32(2.0f * tf) * r;
+    tau = widen_f32(tf) + widen_f32(rot_residual(tf, g, scaled_low(ga, g), df, scaled_low(diff, df)));
+    const float r1 = __fdividef(1.0f, fmaf(tf, tf, 1.0f));   // 1 / (1 + tau^2) to ~1e-7
+    const double e = fma(-fma(tau, tau, 1.0), widen_f32(r1), 1.0);
+    const double r2 = widen_f32(r1 + r1);
+    sn = tau * fma(r2, fma(e, e, e), r2);                    // to FP64 precision (e^3)
     const double dn = widen_f32(t * g, sh);                  // al' = al - t ga, be' = be + t ga
     al -= dn;
     be += dn;
@@ -671,7 +696,7 @@ __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], T &al, T &be, T 
         }
     }
 #pragma unroll
-    for (int i = 0; i < R; ++i) rot_apply<T, EXACT>(x[i], y[i], sn, tau);
+    for (int i = 0; i < R; ++i) rot_apply<T, EXACT || R <= 4>(x[i], y[i], sn, tau);
     // recomputed when the update cancelled (below about 1/16 of the norm)
     al = norm_kept<EXACT>(a2, al) ? a2 : bj_dot(x, x);
     be = norm_kept<EXACT>(b2, be) ? b2 : bj_dot(y, y);
@@ -912,7 +937,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                             bj_store(y, cols + v * PP, lane);
                             if (lane < NP) {
                                 T qu = Qs[u * NP + lane], qv = Qs[v * NP + lane];
-                                rot_apply<T, EXACT>(qu, qv, sn, tau);
+                                rot_apply<T, EXACT || R <= 4>(qu, qv, sn, tau);
                                 Qs[u * NP + lane] = qu;
                                 Qs[v * NP + lane] = qv;
                             }
@@ -947,7 +972,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                             bj_store(y, cols + j * PP, lane);
                             if (lane < NP) {
                                 T qy = Qs[j * NP + lane];
-                                rot_apply<T, EXACT>(qx, qy, sn, tau);
+                                rot_apply<T, EXACT || R <= 4>(qx, qy, sn, tau);
                                 Qs[j * NP + lane] = qy;
                             }
                             if (lane == 0) nrm[j] = be;
