@@ -425,8 +425,8 @@ struct BJacobiParams {
     int *sweeps;   // per sector (written at the end)
     int *rotated;  // nsec * max_sweeps flags, zero on entry
     // deferred V updates (null qbuf: each CTA updates V at the end of its block pair)
-    T *qbuf;       // 2 x max_jobs rotation matrices (NP x NP), by step parity
-    int *jobs;     // 2 x max_jobs x {sector, block a, block b, valid columns a | b << 16}
+    T *qbuf;       // 2 x max_jobs rotation matrices (NP x NP) or rotation lists in their place, by step parity
+    int *jobs;     // 2 x max_jobs x {sector, block a, block b, valid columns a | b << 8 | k == 0 << 16}
     int *njobs;    // per step: jobs recorded (zero on entry)
     int *vnext;    // per step: V work units claimed (zero on entry)
     int max_jobs;  // >= block pairs per step
@@ -760,9 +760,67 @@ __device__ __forceinline__ void bj_apply_v(T *V, int q, int a, int b, int na, in
     }
 }
 
+// Rotations of a block pair as the FP64 kernels keep them (LIST): (s, tau) of the inter-block pair
+// (w, B + (w + round) % B) at round * B + w, of the intra-block pairs (those of rr_pair(B, round, .)) behind
+// them, (0, 0) where nothing was rotated; 2 B^2 - B pairs of numbers, in the place of the 4 B^2 of Q.
+template <int B>
+__host__ __device__ constexpr int bj_intra(int round, int half, int slot) {
+    return B * B + round * B + half * (B / 2) + slot;
+}
+
+// V[r, cols] <- V[r, cols] Q by the rotations themselves: a row's 2B elements in registers take
+// 3 instructions a pair (FOUR: 4) where Q takes 4 (2 B x 2 B elements over B x B pairs), and none for
+// the pairs of the later sweeps that were not rotated; and nobody forms Q.  FP64 only, where the
+// instructions of the FP64 pipe are what the V updates cost (48 % of a full sweep's with Q); FP32 keeps Q,
+// whose independent products have no chain of rotations in them.
+template <class T, int B, bool FOUR>
+__device__ __forceinline__ void bj_apply_rots(T *V, int q, int a, int b, int na, int nbc, bool intra,
+                                              const double2 *rots, int r0, int r1, int tid) {
+    constexpr int NP = 2 * B, NT = 32 * B;
+    auto valid = [&](int j) { return j < B ? j < na : (j - B) < nbc; };
+    auto column = [&](int j) { return j < B ? a * B + j : b * B + (j - B); };
+    for (int r = r0 + tid; r < r1; r += NT) {
+        T vr[NP];
+#pragma unroll
+        for (int j = 0; j < NP; ++j) vr[j] = valid(j) ? ldcg(V + int64_t(column(j)) * q + r) : T(0);
+        auto rotate = [&](T &x, T &y, const double2 st) {
+            if (__double2hiint(st.y)) rot_apply<T, FOUR>(x, y, T(st.x), T(st.y));
+        };
+        if (intra) {
+#pragma unroll
+            for (int round = 0; round < B - 1; ++round)
+#pragma unroll
+                for (int w = 0; w < B; ++w) {
+                    const int half = w / (B / 2), slot = w % (B / 2);
+                    // rr_pair(B, round, slot) on constants
+                    const int m = B - 1, u = slot == 0 ? 0 : 1 + (round + slot) % m,
+                              v = slot == 0 ? 1 + round : 1 + (round - slot + m) % m;
+                    rotate(vr[u + half * B], vr[v + half * B], rots[bj_intra<B>(round, half, slot)]);
+                }
+        }
+#pragma unroll
+        for (int round = 0; round < B; ++round)
+#pragma unroll
+            for (int w = 0; w < B; ++w) rotate(vr[w], vr[B + (w + round) % B], rots[round * B + w]);
+#pragma unroll
+        for (int j = 0; j < NP; ++j)
+            if (valid(j)) V[int64_t(column(j)) * q + r] = vr[j];
+    }
+}
+
+// The V update of a block pair in whichever form Qs holds it.
+template <class T, int B, bool LIST, bool FOUR>
+__device__ __forceinline__ void bj_update_v(T *V, int q, int a, int b, int na, int nbc, bool intra, const T *Qs, int r0,
+                                            int r1, int tid) {
+    if constexpr (LIST)
+        bj_apply_rots<T, B, FOUR>(V, q, a, b, na, nbc, intra, reinterpret_cast<const double2 *>(Qs), r0, r1, tid);
+    else
+        bj_apply_v<T, B>(V, q, a, b, na, nbc, Qs, r0, r1, tid);
+}
+
 // The deferred V updates of step `st`: CTAs claim (job, row chunk) units from a
 // counter until none are left, so CTAs without a block pair take most of them.
-template <class T, int B>
+template <class T, int B, bool LIST, bool FOUR>
 __device__ void bj_vwork(const BJacobiParams<T> &P, int64_t st, T *Qs, int *s_unit, int tid) {
     constexpr int NP = 2 * B, NT = 32 * B;
     const int nj = __ldcg(P.njobs + st);
@@ -783,7 +841,8 @@ __device__ void bj_vwork(const BJacobiParams<T> &P, int64_t st, T *Qs, int *s_un
         const T *qsrc = P.qbuf + (int64_t(par) * P.max_jobs + jb) * NP * NP;
         for (int e = tid; e < NP * NP; e += NT) Qs[e] = ldcg(qsrc + e);
         __syncthreads();
-        bj_apply_v<T, B>(P.rot + sd.rot_off, sd.q, a, b, nn & 0xFFFF, nn >> 16, Qs, r0, min(sd.q, r0 + NT), tid);
+        bj_update_v<T, B, LIST, FOUR>(P.rot + sd.rot_off, sd.q, a, b, nn & 0xFF, (nn >> 8) & 0xFF, nn >> 16, Qs, r0,
+                                      min(sd.q, r0 + NT), tid);
         __syncthreads();
     }
 }
@@ -793,10 +852,13 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
     constexpr int NP = 2 * B;   // columns (players) of a block pair
     constexpr int PP = 32 * R;  // shared-memory slot per column (zero-padded)
     constexpr int NT = 32 * B;
+    constexpr bool LIST = sizeof(T) == 8 && !EXACT;  // V by the rotations, not by Q (bj_apply_rots)
+    constexpr bool FOUR = EXACT || R <= 4;
     cg::grid_group grid = cg::this_grid();
     extern __shared__ __align__(16) unsigned char bsh[];
     T *cols = reinterpret_cast<T *>(bsh);  // NP slots of PP
-    T *Qs = cols + NP * PP;                // NP x NP, column-major
+    T *Qs = cols + NP * PP;                // NP x NP, column-major, or the list of rotations (LIST)
+    double2 *rots = reinterpret_cast<double2 *>(Qs);
     T *nrm = Qs + NP * NP;                 // NP squared column norms
     const int nsec = P.nsec;
     int *done = reinterpret_cast<int *>(nrm + NP);
@@ -909,7 +971,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                 }
                 if (lane == 0) nrm[j] = acc;
             }
-            for (int e = tid; e < NP * NP; e += NT) Qs[e] = (e % (NP + 1) == 0) ? T(1) : T(0);
+            for (int e = tid; e < NP * NP; e += NT) Qs[e] = (!LIST && e % (NP + 1) == 0) ? T(1) : T(0);
             if (tid == 0) {
                 any_rot = 0;
                 s_rmax = 0;
@@ -935,9 +997,11 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                             if (lane == 0 && dy > T(0)) P.dnorm[sd.s_off + column(v)] = dy;
                             bj_store(x, cols + u * PP, lane);
                             bj_store(y, cols + v * PP, lane);
-                            if (lane < NP) {
+                            if constexpr (LIST) {
+                                if (lane == 0) rots[bj_intra<B>(round, half, slot)] = make_double2(sn, tau);
+                            } else if (lane < NP) {
                                 T qu = Qs[u * NP + lane], qv = Qs[v * NP + lane];
-                                rot_apply<T, EXACT || R <= 4>(qu, qv, sn, tau);
+                                rot_apply<T, FOUR>(qu, qv, sn, tau);
                                 Qs[u * NP + lane] = qu;
                                 Qs[v * NP + lane] = qv;
                             }
@@ -957,7 +1021,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                 T qx = T(0), al = T(0);
                 if (mine) {
                     bj_load(x, cols + warp * PP, lane);
-                    if (lane < NP) qx = Qs[warp * NP + lane];
+                    if (!LIST && lane < NP) qx = Qs[warp * NP + lane];
                     al = nrm[warp];
                 }
                 bool mine_rot = false;
@@ -970,9 +1034,11 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                             if (lane == 0 && dx > T(0)) P.dnorm[sd.s_off + column(warp)] = dx;
                             if (lane == 0 && dy > T(0)) P.dnorm[sd.s_off + column(j)] = dy;
                             bj_store(y, cols + j * PP, lane);
-                            if (lane < NP) {
+                            if constexpr (LIST) {
+                                if (lane == 0) rots[round * B + warp] = make_double2(sn, tau);
+                            } else if (lane < NP) {
                                 T qy = Qs[j * NP + lane];
-                                rot_apply<T, EXACT || R <= 4>(qx, qy, sn, tau);
+                                rot_apply<T, FOUR>(qx, qy, sn, tau);
                                 Qs[j * NP + lane] = qy;
                             }
                             if (lane == 0) nrm[j] = be;
@@ -983,7 +1049,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                 }
                 if (mine_rot) {
                     bj_store(x, cols + warp * PP, lane);
-                    if (lane < NP) Qs[warp * NP + lane] = qx;
+                    if (!LIST && lane < NP) Qs[warp * NP + lane] = qx;
                     rotated_any = true;
                 }
             }
@@ -1003,7 +1069,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                     }
                 }
                 if (defer_v) {
-                    // record Q and the job; the V update runs in the next step (bj_vwork)
+                    // record Q or the rotations, and the job; the V update runs in the next step (bj_vwork)
                     if (tid == 0) s_unit = atomicAdd(P.njobs + step, 1);
                     __syncthreads();
                     const int jb = s_unit;
@@ -1015,10 +1081,10 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                         jr[0] = s;
                         jr[1] = a;
                         jr[2] = b;
-                        jr[3] = na | (nbc << 16);
+                        jr[3] = na | (nbc << 8) | ((k == 0) << 16);
                     }
                 } else {
-                    bj_apply_v<T, B>(V, q, a, b, na, nbc, Qs, 0, q, tid);
+                    bj_update_v<T, B, LIST, FOUR>(V, q, a, b, na, nbc, k == 0, Qs, 0, q, tid);
                 }
                 if (tid == 0) atomicMax(P.rotated + int64_t(s) * P.max_sweeps + sweep[s], s_rmax);
             }
@@ -1026,7 +1092,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
         }
         // the previous step's V updates: their columns are disjoint within that step,
         // and the next step's updates of the same columns come after the next barrier
-        if (defer_v && step > 0) bj_vwork<T, B>(P, step - 1, Qs, &s_unit, tid);
+        if (defer_v && step > 0) bj_vwork<T, B, LIST, FOUR>(P, step - 1, Qs, &s_unit, tid);
         grid.sync();
         for (int s = tid; s < nsec; s += NT) {
             if (done[s]) continue;
@@ -1044,7 +1110,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
         }
         __syncthreads();
     }
-    if (defer_v && steps_run > 0) bj_vwork<T, B>(P, steps_run - 1, Qs, &s_unit, tid);
+    if (defer_v && steps_run > 0) bj_vwork<T, B, LIST, FOUR>(P, steps_run - 1, Qs, &s_unit, tid);
     if (blockIdx.x == 0)
         for (int s = tid; s < nsec; s += NT) P.sweeps[s] = sweep[s];
 }
