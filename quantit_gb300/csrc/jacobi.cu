@@ -78,6 +78,13 @@ __device__ __forceinline__ void rot_apply(T &x, T &y, T s, T tau) {
     }
 }
 
+// Whether a rotation's cosine is 1 in FP64 (|s| < 2^-27, s^2 / 2 under a quarter of eps): x -= s y, y += s x is the
+// whole rotation then.  Two instructions an element pair instead of three or four; graded columns have such
+// angles (coupling times the ratio of the norms) from the first sweep on, all have them in the last.
+__device__ __forceinline__ bool unit_cosine(double s) {
+    return (uint32_t(__double2hiint(s)) & 0x7FFFFFFFu) < (uint32_t(1023 - 27) << 20);
+}
+
 // Hestenes rotation for column norms al, be and inner product ga: s and tau.
 template <class T>
 __device__ __forceinline__ void rot_params(T al, T be, T ga, T &s, T &tau, T &t) {
@@ -628,10 +635,14 @@ __device__ __forceinline__ int bj_params_fast64(double &al, double &be, double g
     const float tf = __fdividef(t, 1.0f + w2 * rsqrtf(w2));  // tan(theta / 2), |tf| <= 0.4143
     if (fabsf(tf) < 1.17549435e-38f) return 2;
     tau = widen_f32(tf) + widen_f32(rot_residual(tf, g, scaled_low(ga, g), df, scaled_low(diff, df)));
-    const float r1 = __fdividef(1.0f, fmaf(tf, tf, 1.0f));   // 1 / (1 + tau^2) to ~1e-7
-    const double e = fma(-fma(tau, tau, 1.0), widen_f32(r1), 1.0);
-    const double r2 = widen_f32(r1 + r1);
-    sn = tau * fma(r2, fma(e, e, e), r2);                    // to FP64 precision (e^3)
+    if (fabsf(tf) < 3.7252903e-9f) {                             // 2^-28: unit_cosine
+        sn = tau + tau;
+    } else {
+        const float r1 = __fdividef(1.0f, fmaf(tf, tf, 1.0f));   // 1 / (1 + tau^2) to ~1e-7
+        const double e = fma(-fma(tau, tau, 1.0), widen_f32(r1), 1.0);
+        const double r2 = widen_f32(r1 + r1);
+        sn = tau * fma(r2, fma(e, e, e), r2);                    // to FP64 precision (e^3)
+    }
     const double dn = widen_f32(t * g, sh);                  // al' = al - t ga, be' = be + t ga
     al -= dn;
     be += dn;
@@ -695,8 +706,18 @@ __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], T &al, T &be, T 
             b2 = be + t * ga;
         }
     }
+    bool whole = true;
+    if constexpr (sizeof(T) == 8 && !EXACT) whole = !unit_cosine(sn);
+    if (whole) {
 #pragma unroll
-    for (int i = 0; i < R; ++i) rot_apply<T, EXACT || R <= 4>(x[i], y[i], sn, tau);
+        for (int i = 0; i < R; ++i) rot_apply<T, EXACT || R <= 4>(x[i], y[i], sn, tau);
+    } else {
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            x[i] = fma(-sn, y[i], x[i]);
+            y[i] = fma(sn, x[i], y[i]);
+        }
+    }
     // recomputed when the update cancelled (below about 1/16 of the norm)
     al = norm_kept<EXACT>(a2, al) ? a2 : bj_dot(x, x);
     be = norm_kept<EXACT>(b2, be) ? b2 : bj_dot(y, y);
@@ -784,7 +805,12 @@ __device__ __forceinline__ void bj_apply_rots(T *V, int q, int a, int b, int na,
 #pragma unroll
         for (int j = 0; j < NP; ++j) vr[j] = valid(j) ? ldcg(V + int64_t(column(j)) * q + r) : T(0);
         auto rotate = [&](T &x, T &y, const double2 st) {
-            if (__double2hiint(st.y)) rot_apply<T, FOUR>(x, y, T(st.x), T(st.y));
+            if (!unit_cosine(st.x)) {
+                rot_apply<T, FOUR>(x, y, T(st.x), T(st.y));
+            } else if (__double2hiint(st.x)) {
+                x = fma(-T(st.x), y, x);
+                y = fma(T(st.x), x, y);
+            }
         };
         if (intra) {
 #pragma unroll
