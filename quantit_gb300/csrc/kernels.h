@@ -206,10 +206,10 @@ int lq_max_q(int f32, int nsec);
 void launch_lq(void *work, void *rot, const std::vector<LqSec> &secs, int f32);
 // FP64 refinement of an FP32 sector decomposition (mixed path): from the FP32
 // rotations rot32 (at rot_off; rot_size elements in all), vb <- the FP64-orthogonalised rotation
-// (two Newton-Schulz steps through va, with g as q x q scratch), w1 <- w64 vb (at w_off).
+// (two Newton-Schulz steps through va, with g as q x q scratch; exact: wholly in FP64 products), w1 <- w64 vb (at w_off).
 // The FP64 Jacobi then runs warm on (w1, vb).
 void launch_svd_refine(const float *rot32, int64_t rot_size, const double *w64, double *w1, double *va, double *vb,
-                       double *g, const std::vector<SectorDesc> &secs);
+                       double *g, const std::vector<SectorDesc> &secs, bool exact);
 // out[s_off + j] = squared norm (FP64) of column j of every sector's work matrix (f32:
 // FP32 work matrices)
 void launch_col_norms(const void *W, const SectorDesc *secs, int nsec, int max_q, double *out, int f32);

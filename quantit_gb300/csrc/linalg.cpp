@@ -475,7 +475,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             } else {
                 launch_svd_refine(static_cast<const float *>(D.rot->p), rtot, static_cast<const double *>(w64->p),
                                   static_cast<double *>(w1->p), static_cast<double *>(va->p),
-                                  static_cast<double *>(vbuf->p), static_cast<double *>(gbuf->p), D.desc);
+                                  static_cast<double *>(vbuf->p), static_cast<double *>(gbuf->p), D.desc, th.plain);
             }
             std::vector<SectorDesc> d64 = D.desc;
             for (SectorDesc &d : d64) {

@@ -112,6 +112,20 @@ void ns_correct(const TV *V, const double *G, double *out, const std::vector<Sec
     cuda_check(cudaGetLastError(), "Newton-Schulz correction launch");
 }
 
+// G <- 1.5 I - G / 2 with G's elements below the diagonal read from above it: the factor of a Newton-Schulz step
+// taken as one FP64 product, V <- V (3 I - V^T V) / 2.
+__global__ void __launch_bounds__(256) k_ns_factor(double *__restrict__ G, const SectorDesc *__restrict__ secs) {
+    const int q = secs[blockIdx.y].q;
+    double *g = G + secs[blockIdx.y].rot_off;
+    for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < int64_t(q) * q; e += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t r = e % q, c = e / q;
+        if (r > c) continue;
+        const double v = (r == c ? 1.5 : 0.0) - 0.5 * g[e];
+        g[e] = v;
+        g[r * q + c] = v;
+    }
+}
+
 // One FP64 product per task in one launch of the grouped block GEMM, column-major:
 // C (M x N, ldc = M) = op(A) B, A M x K (a_trans: stored K x M), B K x N.  upper: C is symmetric, tiles
 // strictly below the diagonal are left out.
@@ -227,19 +241,38 @@ void launch_col_norms(const void *W, const SectorDesc *secs, int nsec, int max_q
 }
 
 void launch_svd_refine(const float *rot32, int64_t rot_size, const double *w64, double *w1, double *va, double *vb,
-                       double *g, const std::vector<SectorDesc> &secs) {
-    std::vector<Product> gram, wv;
+                       double *g, const std::vector<SectorDesc> &secs, bool exact) {
+    std::vector<Product> gram, wv, ns;
+    int max_q = 0;
     for (const SectorDesc &s : secs) {
+        max_q = std::max(max_q, int(s.q));
+        ns.push_back({s.rot_off, s.rot_off, s.rot_off, s.q, s.q, s.q, false, false});
         gram.push_back({s.rot_off, s.rot_off, s.rot_off, s.q, s.q, s.q, true, true});
         wv.push_back({s.w_off, s.rot_off, s.w_off, s.p, s.q, s.q, false, false});
     }
     // step 1 from the FP32 rotation (widened into vb): va = V0 + V0 (I - V0^T V0) / 2
     launch_convert(rot32, vb, rot_size, 0, 1);
     products(vb, vb, g, gram);
-    ns_correct(rot32, g, va, secs);
-    // step 2: vb = va + va (I - va^T va) / 2
-    products(va, va, g, gram);
-    ns_correct(static_cast<const double *>(va), g, vb, secs);
+    if (exact && max_q > 0) {
+        // all FP64, as whole products: the values do not depend on how the correction is cut
+        const dim3 grid(unsigned(std::min<int64_t>((int64_t(max_q) * max_q + 2047) / 2048, 1024)), unsigned(secs.size()));
+        const SectorDesc *dsec = upload_vec(secs);
+        auto factor = [&] {
+            k_ns_factor<<<grid, 256, 0, ctx().stream>>>(g, dsec);
+            count_launch();
+            cuda_check(cudaGetLastError(), "Newton-Schulz factor launch");
+        };
+        factor();
+        products(vb, g, va, ns);
+        products(va, va, g, gram);
+        factor();
+        products(va, g, vb, ns);
+    } else {
+        ns_correct(rot32, g, va, secs);
+        // step 2: vb = va + va (I - va^T va) / 2
+        products(va, va, g, gram);
+        ns_correct(static_cast<const double *>(va), g, vb, secs);
+    }
     products(w64, vb, w1, wv);
 }
 
