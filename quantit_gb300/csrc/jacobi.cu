@@ -452,50 +452,87 @@ __device__ __forceinline__ int bj_items(int q, int B) {
 
 // 16-byte shared-memory chunks: lane l holds elements (32 i + l) * V + c of a
 // column, V = 16 / sizeof(T); slots are zero-padded to PP, so no bounds checks.
+// The kernel is built for the longest column of the decomposition.  Columns of at most bj_half slices of 32 elements
+// leave the upper registers alone (full = false): in FP64 every slice of zeros costs 64 clocks an instruction.
+// One branch, not one per slice: the slices' chains have to overlap (with a test at each of them svd D = 600
+// takes 11.4 instead of 10.8 ms).
 template <class T, int R>
-__device__ __forceinline__ void bj_load(T (&x)[R], const T *slot, int lane) {
-    if constexpr (sizeof(T) == 4) {
+__host__ __device__ constexpr int bj_half() {
+    return sizeof(T) == 4 ? (R >= 8 ? (R / 2 + 3) / 4 * 4 : R) : (R == 2 ? 1 : (R / 2 + 1) / 2 * 2);
+}
+template <class T, int R, class F>
+__device__ __forceinline__ void bj_each(bool full, F f) {
+    constexpr int H = bj_half<T, R>();
 #pragma unroll
-        for (int i = 0; i < R / 4; ++i) {
-            const float4 v = reinterpret_cast<const float4 *>(slot)[32 * i + lane];
-            x[4 * i] = v.x;
-            x[4 * i + 1] = v.y;
-            x[4 * i + 2] = v.z;
-            x[4 * i + 3] = v.w;
-        }
-    } else {
+    for (int i = 0; i < H; ++i) f(i);
+    if (full) {
 #pragma unroll
-        for (int i = 0; i < R / 2; ++i) {
-            const double2 v = reinterpret_cast<const double2 *>(slot)[32 * i + lane];
-            x[2 * i] = v.x;
-            x[2 * i + 1] = v.y;
-        }
+        for (int i = H; i < R; ++i) f(i);
     }
 }
-
 template <class T, int R>
-__device__ __forceinline__ void bj_store(const T (&x)[R], T *slot, int lane) {
-    if constexpr (sizeof(T) == 4) {
+__device__ __forceinline__ void bj_load(T (&x)[R], const T *slot, int lane, bool full) {
+    constexpr int G = 16 / sizeof(T), H = bj_half<T, R>();
+    if constexpr (H % G) {
+        if (!full) {  // R = 2 in FP64: one element a lane
+            x[0] = slot[lane];
+            return;
+        }
+    }
+    auto vec = [&](int i) {
+        if constexpr (sizeof(T) == 4) {
+            const float4 v = reinterpret_cast<const float4 *>(slot)[8 * i + lane];
+            x[i] = v.x;
+            x[i + 1] = v.y;
+            x[i + 2] = v.z;
+            x[i + 3] = v.w;
+        } else {
+            const double2 v = reinterpret_cast<const double2 *>(slot)[16 * i + lane];
+            x[i] = v.x;
+            x[i + 1] = v.y;
+        }
+    };
+    constexpr int L = H % G ? R : H;
 #pragma unroll
-        for (int i = 0; i < R / 4; ++i)
-            reinterpret_cast<float4 *>(slot)[32 * i + lane] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
-    } else {
+    for (int i = 0; i < L; i += G) vec(i);
+    if (full) {
 #pragma unroll
-        for (int i = 0; i < R / 2; ++i)
-            reinterpret_cast<double2 *>(slot)[32 * i + lane] = make_double2(x[2 * i], x[2 * i + 1]);
+        for (int i = L; i < R; i += G) vec(i);
+    }
+}
+template <class T, int R>
+__device__ __forceinline__ void bj_store(const T (&x)[R], T *slot, int lane, bool full) {
+    constexpr int G = 16 / sizeof(T), H = bj_half<T, R>();
+    if constexpr (H % G) {
+        if (!full) {
+            slot[lane] = x[0];
+            return;
+        }
+    }
+    auto vec = [&](int i) {
+        if constexpr (sizeof(T) == 4)
+            reinterpret_cast<float4 *>(slot)[8 * i + lane] = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+        else
+            reinterpret_cast<double2 *>(slot)[16 * i + lane] = make_double2(x[i], x[i + 1]);
+    };
+    constexpr int L = H % G ? R : H;
+#pragma unroll
+    for (int i = 0; i < L; i += G) vec(i);
+    if (full) {
+#pragma unroll
+        for (int i = L; i < R; i += G) vec(i);
     }
 }
 
 // Per-lane partial sums in NA independent chains (the dot product is on the
 // critical path of every round: R dependent FMAs would cost R FMA latencies).
 template <class T, int R>
-__device__ __forceinline__ T bj_lane_dot(const T (&x)[R], const T (&y)[R]) {
+__device__ __forceinline__ T bj_lane_dot(const T (&x)[R], const T (&y)[R], bool full) {
     constexpr int NA = R >= 16 ? 4 : (R >= 4 ? 2 : 1);
     T a[NA];
 #pragma unroll
     for (int k = 0; k < NA; ++k) a[k] = T(0);
-#pragma unroll
-    for (int i = 0; i < R; ++i) a[i % NA] = fma(x[i], y[i], a[i % NA]);
+    bj_each<T, R>(full, [&](int i) { a[i % NA] = fma(x[i], y[i], a[i % NA]); });
 #pragma unroll
     for (int w = NA / 2; w > 0; w >>= 1)
 #pragma unroll
@@ -503,8 +540,8 @@ __device__ __forceinline__ T bj_lane_dot(const T (&x)[R], const T (&y)[R]) {
     return a[0];
 }
 template <class T, int R>
-__device__ __forceinline__ T bj_dot(const T (&x)[R], const T (&y)[R]) {
-    return wsum(bj_lane_dot(x, y));
+__device__ __forceinline__ T bj_dot(const T (&x)[R], const T (&y)[R], bool full) {
+    return wsum(bj_lane_dot(x, y, full));
 }
 
 // x 2^-sh as FP32 by integer operations (no FP64 conversion): sh within the exponent range,
@@ -669,13 +706,13 @@ __device__ __forceinline__ bool norm_kept(double a2, double al) {
 // (set to zero, norm 0; dx / dy receive its squared norm before, else stay 0).
 // EXACT: the plain formulas in FP64 too (launch_jacobi's `exact`).
 template <class T, int R, bool EXACT>
-__device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], T &al, T &be, T tol, T thr, T &sn, T &tau, T &dx,
+__device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], bool full, T &al, T &be, T tol, T thr, T &sn, T &tau, T &dx,
                                           T &dy, T skip, float &rmax) {
     if (al == T(0) || be == T(0)) return false;
     if (pair_skipped(al, be, skip)) return false;
     T ga, t, a2, b2;
     if constexpr (sizeof(T) == 4) {
-        ga = bj_dot(x, y);
+        ga = bj_dot(x, y, full);
         if (ga == T(0)) return false;
         const float rel = fabsf(ga) * rsqrtf(al) * rsqrtf(be);
         if (rel <= tol) return false;
@@ -686,7 +723,7 @@ __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], T &al, T &be, T 
     } else {
         int ka = 0, kb = 0, how = 2;
         const bool fast = !EXACT && bj_exponents(al, be, ka, kb);
-        ga = bj_lane_dot(x, y);
+        ga = bj_lane_dot(x, y, full);
         ga = fast ? fixed_wsum(ga, ka + kb) : wsum(ga);
         if (ga == T(0)) return false;
         a2 = al;
@@ -709,18 +746,16 @@ __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], T &al, T &be, T 
     bool whole = true;
     if constexpr (sizeof(T) == 8 && !EXACT) whole = !unit_cosine(sn);
     if (whole) {
-#pragma unroll
-        for (int i = 0; i < R; ++i) rot_apply<T, EXACT || R <= 4>(x[i], y[i], sn, tau);
+        bj_each<T, R>(full, [&](int i) { rot_apply<T, EXACT || R <= 4>(x[i], y[i], sn, tau); });
     } else {
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
+        bj_each<T, R>(full, [&](int i) {
             x[i] = fma(-sn, y[i], x[i]);
             y[i] = fma(sn, x[i], y[i]);
-        }
+        });
     }
     // recomputed when the update cancelled (below about 1/16 of the norm)
-    al = norm_kept<EXACT>(a2, al) ? a2 : bj_dot(x, x);
-    be = norm_kept<EXACT>(b2, be) ? b2 : bj_dot(y, y);
+    al = norm_kept<EXACT>(a2, al) ? a2 : bj_dot(x, x, full);
+    be = norm_kept<EXACT>(b2, be) ? b2 : bj_dot(y, y, full);
     if (thr > T(0)) {
         if (al <= thr) {
 #pragma unroll
@@ -966,6 +1001,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
             T *W = P.work + sd.w_off;
             T *V = P.rot + sd.rot_off;
             const T tol = Eps<T>::tol(p);
+            const bool full = EXACT || p > 32 * bj_half<T, R>();
             const T thr = P.defl ? P.defl[s] : T(0);
             const T skp = P.skip ? P.skip[s] : T(0);
             bool zeroed = false;
@@ -981,11 +1017,10 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                     v[i] = r < p ? ldcg(src + r) : T(0);
                 }
                 T acc = 0;
-#pragma unroll
-                for (int i = 0; i < R; ++i) {
+                bj_each<T, R>(full, [&](int i) {
                     acc = fma(v[i], v[i], acc);
                     cols[j * PP + lane + 32 * i] = v[i];
-                }
+                });
                 acc = wsum(acc);
                 if (thr > T(0) && acc > T(0) && acc <= thr) {
                     // a numerically zero column: deflated (zero from here on)
@@ -1015,14 +1050,14 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                     u += half * B;
                     v += half * B;
                     if (valid(u) && valid(v)) {
-                        bj_load(x, cols + u * PP, lane);
-                        bj_load(y, cols + v * PP, lane);
+                        bj_load(x, cols + u * PP, lane, full);
+                        bj_load(y, cols + v * PP, lane, full);
                         T al = nrm[u], be = nrm[v], dx = T(0), dy = T(0);
-                        if (bj_rotate<T, R, EXACT>(x, y, al, be, tol, thr, sn, tau, dx, dy, skp, rmax)) {
+                        if (bj_rotate<T, R, EXACT>(x, y, full, al, be, tol, thr, sn, tau, dx, dy, skp, rmax)) {
                             if (lane == 0 && dx > T(0)) P.dnorm[sd.s_off + column(u)] = dx;
                             if (lane == 0 && dy > T(0)) P.dnorm[sd.s_off + column(v)] = dy;
-                            bj_store(x, cols + u * PP, lane);
-                            bj_store(y, cols + v * PP, lane);
+                            bj_store(x, cols + u * PP, lane, full);
+                            bj_store(y, cols + v * PP, lane, full);
                             if constexpr (LIST) {
                                 if (lane == 0) rots[bj_intra<B>(round, half, slot)] = make_double2(sn, tau);
                             } else if (lane < NP) {
@@ -1046,7 +1081,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                 const bool mine = valid(warp);
                 T qx = T(0), al = T(0);
                 if (mine) {
-                    bj_load(x, cols + warp * PP, lane);
+                    bj_load(x, cols + warp * PP, lane, full);
                     if (!LIST && lane < NP) qx = Qs[warp * NP + lane];
                     al = nrm[warp];
                 }
@@ -1054,12 +1089,12 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                 for (int round = 0; round < B; ++round) {
                     const int j = B + (warp + round) % B;
                     if (mine && valid(j)) {
-                        bj_load(y, cols + j * PP, lane);
+                        bj_load(y, cols + j * PP, lane, full);
                         T be = nrm[j], dx = T(0), dy = T(0);
-                        if (bj_rotate<T, R, EXACT>(x, y, al, be, tol, thr, sn, tau, dx, dy, skp, rmax)) {
+                        if (bj_rotate<T, R, EXACT>(x, y, full, al, be, tol, thr, sn, tau, dx, dy, skp, rmax)) {
                             if (lane == 0 && dx > T(0)) P.dnorm[sd.s_off + column(warp)] = dx;
                             if (lane == 0 && dy > T(0)) P.dnorm[sd.s_off + column(j)] = dy;
-                            bj_store(y, cols + j * PP, lane);
+                            bj_store(y, cols + j * PP, lane, full);
                             if constexpr (LIST) {
                                 if (lane == 0) rots[round * B + warp] = make_double2(sn, tau);
                             } else if (lane < NP) {
@@ -1074,7 +1109,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                     __syncthreads();
                 }
                 if (mine_rot) {
-                    bj_store(x, cols + warp * PP, lane);
+                    bj_store(x, cols + warp * PP, lane, full);
                     if (!LIST && lane < NP) Qs[warp * NP + lane] = qx;
                     rotated_any = true;
                 }
