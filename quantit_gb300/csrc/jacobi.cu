@@ -816,25 +816,56 @@ __device__ __forceinline__ void bj_apply_v(T *V, int q, int a, int b, int na, in
     }
 }
 
+// Columns of a sector's blocks: B, or (EVEN, the FP64 kernel for columns of up to 64 elements) equal blocks, as many as a
+// step pairs (an odd count's phantom block included).  Narrow sectors take fewer rounds a step than with blocks of B
+// columns and a rest, and fewer warps on an SM's FP64 pipe: site svd D = 48 (at most 11 columns, 11 rounds a step
+// instead of 15) 252 -> 234 us.  Wider ones have full blocks either way, and the run-time width costs them
+// 2 to 3 % (svd D = 600, eigh D = 300).
+template <int B, bool EVEN>
+__device__ __forceinline__ int bj_width(int q) {
+    if (!EVEN) return B;
+    const int nb = (q + B - 1) / B, nbp = nb + (nb & 1);
+    return nb == 1 ? q : (q + nbp - 1) / nbp;
+}
+
 // Rotations of a block pair as the FP64 kernels keep them (LIST): (s, tau) of the inter-block pair
-// (w, B + (w + round) % B) at round * B + w, of the intra-block pairs (those of rr_pair(B, round, .)) behind
+// (w, B + j) at ((j - w) mod B) * B + w, of the intra-block pairs (those of rr_pair(width, round, .)) behind
 // them, (0, 0) where nothing was rotated; 2 B^2 - B pairs of numbers, in the place of the 4 B^2 of Q.
 template <int B>
 __host__ __device__ constexpr int bj_intra(int round, int half, int slot) {
     return B * B + round * B + half * (B / 2) + slot;
 }
 
+// The intra-block rotations of one row, blocks of BE columns (even, a phantom last one if their number is odd).
+template <class T, int B, int BE, class F>
+__device__ __forceinline__ void bj_intra_rots(T (&vr)[2 * B], const double2 *rots, F rotate) {
+#pragma unroll
+    for (int round = 0; round < BE - 1; ++round)
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+            for (int slot = 0; slot < BE / 2; ++slot) {
+                // rr_pair(BE, round, slot) on constants
+                const int m = BE - 1, u = slot == 0 ? 0 : 1 + (round + slot) % m,
+                          v = slot == 0 ? 1 + round : 1 + (round - slot + m) % m;
+                rotate(vr[u + half * B], vr[v + half * B], rots[bj_intra<B>(round, half, slot)]);
+            }
+}
+
 // V[r, cols] <- V[r, cols] Q by the rotations themselves: a row's 2B elements in registers take
 // 3 instructions a pair (FOUR: 4) where Q takes 4 (2 B x 2 B elements over B x B pairs), and none for
 // the pairs of the later sweeps that were not rotated; and nobody forms Q.  FP64 only, where the
 // instructions of the FP64 pipe are what the V updates cost (48 % of a full sweep's with Q); FP32 keeps Q,
-// whose independent products have no chain of rotations in them.
-template <class T, int B, bool FOUR>
-__device__ __forceinline__ void bj_apply_rots(T *V, int q, int a, int b, int na, int nbc, bool intra,
-                                              const double2 *rots, int r0, int r1, int tid) {
+// whose independent products have no chain of rotations in them.  Blocks of bs columns; roff: the list, in bytes from the start
+// of shared memory.
+template <class T, int B, bool FOUR, bool EVEN>
+__device__ __forceinline__ void bj_apply_rots(T *V, int q, int bs, int a, int b, int na, int nbc, bool intra, int roff, int r0,
+                                           int r1, int tid) {
     constexpr int NP = 2 * B, NT = 32 * B;
+    extern __shared__ __align__(16) unsigned char bsh[];
+    const double2 *rots = reinterpret_cast<const double2 *>(bsh + roff);
     auto valid = [&](int j) { return j < B ? j < na : (j - B) < nbc; };
-    auto column = [&](int j) { return j < B ? a * B + j : b * B + (j - B); };
+    auto column = [&](int j) { return j < B ? a * bs + j : b * bs + (j - B); };
     for (int r = r0 + tid; r < r1; r += NT) {
         T vr[NP];
 #pragma unroll
@@ -848,17 +879,16 @@ __device__ __forceinline__ void bj_apply_rots(T *V, int q, int a, int b, int na,
             }
         };
         if (intra) {
-#pragma unroll
-            for (int round = 0; round < B - 1; ++round)
-#pragma unroll
-                for (int w = 0; w < B; ++w) {
-                    const int half = w / (B / 2), slot = w % (B / 2);
-                    // rr_pair(B, round, slot) on constants
-                    const int m = B - 1, u = slot == 0 ? 0 : 1 + (round + slot) % m,
-                              v = slot == 0 ? 1 + round : 1 + (round - slot + m) % m;
-                    rotate(vr[u + half * B], vr[v + half * B], rots[bj_intra<B>(round, half, slot)]);
-                }
+            const int be = bs + (bs & 1);
+            if (!EVEN || be == B) bj_intra_rots<T, B, B>(vr, rots, rotate);
+            if constexpr (EVEN && B == 8) {
+                if (be == 6) bj_intra_rots<T, B, 6>(vr, rots, rotate);
+                if (be == 4) bj_intra_rots<T, B, 4>(vr, rots, rotate);
+            }
+            if (EVEN && be == 2) bj_intra_rots<T, B, 2>(vr, rots, rotate);
         }
+        // in the order of the rounds for every column: (w + round) mod bs wraps later than mod B does, and
+        // what lies between is empty
 #pragma unroll
         for (int round = 0; round < B; ++round)
 #pragma unroll
@@ -870,19 +900,19 @@ __device__ __forceinline__ void bj_apply_rots(T *V, int q, int a, int b, int na,
 }
 
 // The V update of a block pair in whichever form Qs holds it.
-template <class T, int B, bool LIST, bool FOUR>
-__device__ __forceinline__ void bj_update_v(T *V, int q, int a, int b, int na, int nbc, bool intra, const T *Qs, int r0,
-                                            int r1, int tid) {
+template <class T, int B, bool LIST, bool FOUR, bool EVEN>
+__device__ __forceinline__ void bj_update_v(T *V, int q, int a, int b, int na, int nbc, bool intra, const T *Qs, int roff,
+                                            int r0, int r1, int tid) {
     if constexpr (LIST)
-        bj_apply_rots<T, B, FOUR>(V, q, a, b, na, nbc, intra, reinterpret_cast<const double2 *>(Qs), r0, r1, tid);
+        bj_apply_rots<T, B, FOUR, EVEN>(V, q, bj_width<B, EVEN>(q), a, b, na, nbc, intra, roff, r0, r1, tid);
     else
         bj_apply_v<T, B>(V, q, a, b, na, nbc, Qs, r0, r1, tid);
 }
 
 // The deferred V updates of step `st`: CTAs claim (job, row chunk) units from a
 // counter until none are left, so CTAs without a block pair take most of them.
-template <class T, int B, bool LIST, bool FOUR>
-__device__ void bj_vwork(const BJacobiParams<T> &P, int64_t st, T *Qs, int *s_unit, int tid) {
+template <class T, int B, bool LIST, bool FOUR, bool EVEN>
+__device__ void bj_vwork(const BJacobiParams<T> &P, int64_t st, T *Qs, int roff, int *s_unit, int tid) {
     constexpr int NP = 2 * B, NT = 32 * B;
     const int nj = __ldcg(P.njobs + st);
     const int total = nj * P.upj;
@@ -902,7 +932,7 @@ __device__ void bj_vwork(const BJacobiParams<T> &P, int64_t st, T *Qs, int *s_un
         const T *qsrc = P.qbuf + (int64_t(par) * P.max_jobs + jb) * NP * NP;
         for (int e = tid; e < NP * NP; e += NT) Qs[e] = ldcg(qsrc + e);
         __syncthreads();
-        bj_update_v<T, B, LIST, FOUR>(P.rot + sd.rot_off, sd.q, a, b, nn & 0xFF, (nn >> 8) & 0xFF, nn >> 16, Qs, r0,
+        bj_update_v<T, B, LIST, FOUR, EVEN>(P.rot + sd.rot_off, sd.q, a, b, nn & 0xFF, (nn >> 8) & 0xFF, nn >> 16, Qs, roff, r0,
                                       min(sd.q, r0 + NT), tid);
         __syncthreads();
     }
@@ -915,11 +945,13 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
     constexpr int NT = 32 * B;
     constexpr bool LIST = sizeof(T) == 8 && !EXACT;  // V by the rotations, not by Q (bj_apply_rots)
     constexpr bool FOUR = EXACT || R <= 4;
+    constexpr bool EVEN = LIST && R == 2;            // equal blocks (bj_width)
     cg::grid_group grid = cg::this_grid();
     extern __shared__ __align__(16) unsigned char bsh[];
     T *cols = reinterpret_cast<T *>(bsh);  // NP slots of PP
     T *Qs = cols + NP * PP;                // NP x NP, column-major, or the list of rotations (LIST)
     double2 *rots = reinterpret_cast<double2 *>(Qs);
+    constexpr int roff = NP * PP * int(sizeof(T));
     T *nrm = Qs + NP * NP;                 // NP squared column norms
     const int nsec = P.nsec;
     int *done = reinterpret_cast<int *>(nrm + NP);
@@ -993,11 +1025,12 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                 a = b;
                 b = t;
             }
-            const bool has_b = b < nb;  // otherwise b is the phantom block
+            const int bs = bj_width<B, EVEN>(q), be = bs + (bs & 1);
+            const bool has_b = EVEN ? b * bs < q : b < nb;  // otherwise b is the phantom block (or empty: EVEN)
             if (!has_b && k != 0) continue;
-            const int na = min(B, q - a * B), nbc = has_b ? min(B, q - b * B) : 0;
+            const int na = min(bs, q - a * bs), nbc = has_b ? min(bs, q - b * bs) : 0;
             auto valid = [&](int j) { return j < B ? j < na : (j - B) < nbc; };
-            auto column = [&](int j) { return j < B ? a * B + j : b * B + (j - B); };
+            auto column = [&](int j) { return j < B ? a * bs + j : b * bs + (j - B); };
             T *W = P.work + sd.w_off;
             T *V = P.rot + sd.rot_off;
             const T tol = Eps<T>::tol(p);
@@ -1042,14 +1075,19 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
             float rmax = zeroed ? 1.17549435e-38f : 0.0f;  // a deflation removes couplings and adds none
             T x[R], y[R], sn, tau;
             if (k == 0) {
-                // intra-block pairs: round-robin over the B columns of each block
+                // intra-block pairs: round-robin over the columns of each block
                 const int half = warp / (B / 2), slot = warp % (B / 2);
                 for (int round = 0; round < B - 1; ++round) {
                     int u, v;
-                    rr_pair(B, round, slot, u, v);
+                    if (EVEN && be < B) {
+                        if (round >= be - 1) break;
+                        rr_pair(be, round, slot, u, v);
+                    } else {
+                        rr_pair(B, round, slot, u, v);
+                    }
                     u += half * B;
                     v += half * B;
-                    if (valid(u) && valid(v)) {
+                    if ((!EVEN || slot < be / 2) && valid(u) && valid(v)) {
                         bj_load(x, cols + u * PP, lane, full);
                         bj_load(y, cols + v * PP, lane, full);
                         T al = nrm[u], be = nrm[v], dx = T(0), dy = T(0);
@@ -1087,7 +1125,12 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                 }
                 bool mine_rot = false;
                 for (int round = 0; round < B; ++round) {
-                    const int j = B + (warp + round) % B;
+                    int jj = (warp + round) % B;
+                    if constexpr (EVEN) {
+                        if (round >= bs) break;
+                        if (bs < B) jj = warp + round < bs ? warp + round : warp + round - bs;
+                    }
+                    const int j = B + jj;
                     if (mine && valid(j)) {
                         bj_load(y, cols + j * PP, lane, full);
                         T be = nrm[j], dx = T(0), dy = T(0);
@@ -1096,7 +1139,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                             if (lane == 0 && dy > T(0)) P.dnorm[sd.s_off + column(j)] = dy;
                             bj_store(y, cols + j * PP, lane, full);
                             if constexpr (LIST) {
-                                if (lane == 0) rots[round * B + warp] = make_double2(sn, tau);
+                                if (lane == 0) rots[(jj - warp + B) % B * B + warp] = make_double2(sn, tau);
                             } else if (lane < NP) {
                                 T qy = Qs[j * NP + lane];
                                 rot_apply<T, FOUR>(qx, qy, sn, tau);
@@ -1145,7 +1188,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                         jr[3] = na | (nbc << 8) | ((k == 0) << 16);
                     }
                 } else {
-                    bj_update_v<T, B, LIST, FOUR>(V, q, a, b, na, nbc, k == 0, Qs, 0, q, tid);
+                    bj_update_v<T, B, LIST, FOUR, EVEN>(V, q, a, b, na, nbc, k == 0, Qs, roff, 0, q, tid);
                 }
                 if (tid == 0) atomicMax(P.rotated + int64_t(s) * P.max_sweeps + sweep[s], s_rmax);
             }
@@ -1153,7 +1196,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
         }
         // the previous step's V updates: their columns are disjoint within that step,
         // and the next step's updates of the same columns come after the next barrier
-        if (defer_v && step > 0) bj_vwork<T, B, LIST, FOUR>(P, step - 1, Qs, &s_unit, tid);
+        if (defer_v && step > 0) bj_vwork<T, B, LIST, FOUR, EVEN>(P, step - 1, Qs, roff, &s_unit, tid);
         grid.sync();
         for (int s = tid; s < nsec; s += NT) {
             if (done[s]) continue;
@@ -1171,7 +1214,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
         }
         __syncthreads();
     }
-    if (defer_v && steps_run > 0) bj_vwork<T, B, LIST, FOUR>(P, steps_run - 1, Qs, &s_unit, tid);
+    if (defer_v && steps_run > 0) bj_vwork<T, B, LIST, FOUR, EVEN>(P, steps_run - 1, Qs, roff, &s_unit, tid);
     if (blockIdx.x == 0)
         for (int s = tid; s < nsec; s += NT) P.sweeps[s] = sweep[s];
 }
