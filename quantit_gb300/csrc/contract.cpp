@@ -729,7 +729,7 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
     am.n[0] = A.nnz;
     am.n[1] = B.nnz;
     for (int i = 0; i < 2; ++i)
-        am.parts[i] = int32_t(std::min<int64_t>((am.n[i] + 4095) / 4096, 8 * device_sm_count()));
+        am.parts[i] = int32_t(std::min<int64_t>((am.n[i] + 4095) / 4096, 2 * device_sm_count()));
     const int64_t head = (int64_t(2 + am.parts[0] + am.parts[1]) * 8 + 255) & ~int64_t(255);
     BufPtr split = dev_alloc(size_t(head + asz + bsz));
     auto *amax = static_cast<unsigned long long *>(split->p);

@@ -19,7 +19,9 @@
 //    K to a k-step of 32 bytes by the kernel itself.  A thread writes whole 16-byte rows of
 //    core matrices, a warp 512 contiguous bytes.  Bound by memory (4.5 TB/s with the maxima)
 //    since the FP64 -> FP32 conversion takes eight integer instructions and flat layouts no
-//    division; at 40 instructions an element it was bound by the ALUs.
+//    division; at 40 instructions an element it was bound by the ALUs.  A CTA's first elements
+//    are loaded before it reduces the maxima, of which there are two an SM and operand: 429 -> 392 us for
+//    the three splits of the cylinder matvec at D = 2048.
 //  * k_gemm_tc: persistent, CTAS_PER_SM CTAs per SM over the longest-first tile list in
 //    boustrophedon order, warp-specialised:
 //      - warp 0 (producer) fills a ring of stages with bulk asynchronous copies counted on
@@ -64,6 +66,7 @@ constexpr int CKB = 64;                   // bytes of K per row and stage
 constexpr int COPY_BYTES = 128 * CKB;     // one operand copy of a stage
 constexpr int TTHREADS = 192;             // producer, MMA and four epilogue warps
 constexpr int CTAS_PER_SM = 2;
+constexpr int AMAX_THREADS = 512;
 constexpr int TMEM_COLS = 128;            // FP32 accumulator columns of one tile
 constexpr int EPI_COLS = 16, EPI_PITCH = EPI_COLS + 1;  // an epilogue warp's 32 x 16 patch (floats)
 constexpr int EPI_BYTES = 4 * 32 * EPI_PITCH * 4;
@@ -159,25 +162,26 @@ constexpr int smem_bytes(int nc, int nstage) { return nstage * stage_bytes(nc) +
 
 // Maxima of |x| as bit patterns (bit order = value order for non-negative doubles), one
 // per CTA; operand b's CTAs follow operand a's.
-__global__ void __launch_bounds__(256) k_amax(AmaxArgs g) {
+__global__ void __launch_bounds__(AMAX_THREADS) k_amax(AmaxArgs g) {
+    constexpr int VEC = 8, SPAN = AMAX_THREADS * VEC;
     const int which = int(blockIdx.x) >= g.parts[0];
     const double *__restrict__ x = g.x[which];
     const int64_t n = g.n[which];
-    const int64_t first = int64_t(blockIdx.x) - (which ? g.parts[0] : 0), step = int64_t(g.parts[which]) * 1024;
+    const int64_t first = int64_t(blockIdx.x) - (which ? g.parts[0] : 0), step = int64_t(g.parts[which]) * SPAN;
     unsigned long long m = 0;
     auto take = [&](double v) {
         const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7FFFFFFFFFFFFFFFull;
         m = u > m ? u : m;
     };
     // plain loads: the same loop over __ldg / __ldcg reaches 3.7 TB/s instead of 6.4
-    for (int64_t b = first * 1024 + threadIdx.x; b < n; b += step) {
-        double v[4];
+    for (int64_t b = first * SPAN + threadIdx.x; b < n; b += step) {
+        double v[VEC];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = b + j * 256 < n ? x[b + j * 256] : 0.0;
+        for (int j = 0; j < VEC; ++j) v[j] = b + j * AMAX_THREADS < n ? x[b + j * AMAX_THREADS] : 0.0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) take(v[j]);
+        for (int j = 0; j < VEC; ++j) take(v[j]);
     }
-    __shared__ unsigned long long red[8];
+    __shared__ unsigned long long red[AMAX_THREADS / 32];
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long u = __shfl_xor_sync(0xffffffffu, m, o);
         m = u > m ? u : m;
@@ -185,7 +189,7 @@ __global__ void __launch_bounds__(256) k_amax(AmaxArgs g) {
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) m = red[w] > m ? red[w] : m;
+        for (int w = 1; w < AMAX_THREADS / 32; ++w) m = red[w] > m ? red[w] : m;
         g.out[blockIdx.x] = m;
     }
 }
@@ -218,30 +222,23 @@ __global__ void __launch_bounds__(256) k_split(SplitArgs g) {
     const SplitTile t = g.tiles[blockIdx.x];
     const SplitEntry &e = g.ents[t.ent];
     const int op = e.operand;
-    const unsigned long long am = amax_of(g.amax_parts + (op ? g.parts[0] : 0), g.parts[op], red);
-    if (blockIdx.x == 0) {
-        // the GEMM's epilogue reads both maxima
-        const unsigned long long other = amax_of(g.amax_parts + (op ? 0 : g.parts[0]), g.parts[1 - op], red);
-        if (threadIdx.x == 0) {
-            g.amax[op] = am;
-            g.amax[1 - op] = other;
-        }
-    }
-    const int shift = amax_shift(am);
-    const bool fast = f64_fast(am, shift);
-    const uint32_t rebase = f64_rebase(shift);
     const double *__restrict__ src = g.src[op] + e.src_off;
     const int kvb = min(CKB, e.kpb - t.k0b), nq = kvb / 16;
     const int rows = e.rows, K = e.K, nrg = (rows + 7) >> 3, k00 = t.k0b / S::ELEM;
     const int total = ((t.rows + 7) >> 3) * nq * 8, inv = (65536 + nq - 1) / nq;
     const int64_t rs2 = e.rs2, ks2 = e.ks2;
     char *dst0 = g.dst[op] + e.dst_off + int64_t(t.k0b / CKB) * nrg * (8 * S::NC * CKB);
-#pragma unroll 2
-    for (int i = threadIdx.x; i < total; i += 256) {
-        const int u = i >> 3, rg = (u * inv) >> 16, core = u - rg * nq;  // u / nq, u < 2^14
-        const int row = t.row0 + rg * 8 + (i & 7), k = k00 + core * EV;
-        const int nk = row < rows ? K - k : 0;  // elements of this core matrix row within the block
-        double d[EV];
+    // row and 16-byte column of core matrix row i
+    auto place = [&](int i, int &row, int &core) {
+        const int u = i >> 3, rg = (u * inv) >> 16;  // u / nq, u < 2^14
+        core = u - rg * nq;
+        row = t.row0 + rg * 8 + (i & 7);
+    };
+    auto load = [&](int i, double (&d)[EV]) {
+        int row, core;
+        place(i, row, core);
+        const int k = k00 + core * EV;
+        const int nk = i < total && row < rows ? K - k : 0;  // elements of this core matrix row within the block
         if (FLAT) {
             const double *__restrict__ p = src + int64_t(row) * rs2 + int64_t(k) * ks2;
 #pragma unroll
@@ -276,6 +273,27 @@ __global__ void __launch_bounds__(256) k_split(SplitArgs g) {
                 d[v] = src[so];
             }
         }
+    };
+    // the first elements are on their way while the maximum is formed
+    double d0[EV], d1[EV];
+    load(threadIdx.x, d0);
+    load(threadIdx.x + 256, d1);
+    const unsigned long long am = amax_of(g.amax_parts + (op ? g.parts[0] : 0), g.parts[op], red);
+    if (blockIdx.x == 0) {
+        // the GEMM's epilogue reads both maxima
+        const unsigned long long other = amax_of(g.amax_parts + (op ? 0 : g.parts[0]), g.parts[1 - op], red);
+        if (threadIdx.x == 0) {
+            g.amax[op] = am;
+            g.amax[1 - op] = other;
+        }
+    }
+    const int shift = amax_shift(am);
+    const bool fast = f64_fast(am, shift);
+    const uint32_t rebase = f64_rebase(shift);
+    auto store = [&](int i, const double (&d)[EV]) {
+        if (i >= total) return;
+        int row, core;
+        place(i, row, core);
         float x[EV];
         if (fast) {
 #pragma unroll
@@ -289,6 +307,14 @@ __global__ void __launch_bounds__(256) k_split(SplitArgs g) {
         char *dst = dst0 + int64_t(row >> 3) * (8 * S::NC * kvb) + core * 128 + (row & 7) * 16;
 #pragma unroll
         for (int c = 0; c < S::NC; ++c) *reinterpret_cast<uint4 *>(dst + c * 8 * kvb) = out[c];
+    };
+    store(threadIdx.x, d0);
+    store(threadIdx.x + 256, d1);
+    for (int i = threadIdx.x + 512; i < total; i += 512) {
+        load(i, d0);
+        load(i + 256, d1);
+        store(i, d0);
+        store(i + 256, d1);
     }
 }
 
@@ -682,7 +708,7 @@ int split_chunk_bytes() { return CKB; }
 void launch_amax(const AmaxArgs &a) {
     const int n = a.parts[0] + a.parts[1];
     if (n <= 0) return;
-    k_amax<<<n, 256, 0, ctx().stream>>>(a);
+    k_amax<<<n, AMAX_THREADS, 0, ctx().stream>>>(a);
     count_launch();
     cuda_check(cudaGetLastError(), "amax kernel launch");
 }
