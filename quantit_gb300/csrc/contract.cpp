@@ -688,7 +688,7 @@ void contract_f64(const ContractPlan &P, const BT &A, const BT &B, BT &out, cons
 }  // namespace
 
 void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, const BT *add, double beta,
-                     double alpha, const std::vector<int64_t> *add_block) {
+                     double alpha, const std::vector<int64_t> *add_block, const Maxima *a_max, Maxima *c_max) {
     require_f64(A);
     require_f64(B);
     const int64_t nout = int64_t(P.out_p0.size());
@@ -722,7 +722,9 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
     std::vector<int64_t> offa, offb;
     const int64_t asz = split_tables(A, P.p1, int(P.freeA.size()), 0, mode, ents, stiles, offa);
     const int64_t bsz = split_tables(B, P.p2p, int(P.freeB.size()), 1, mode, ents, stiles, offb);
-    // one buffer: the two maxima, their per-CTA parts, then the split arrays
+    // one buffer: the two maxima, their per-CTA parts, then the split arrays.  The maxima of an operand that a
+    // GEMM has just written come from its epilogue: reading the operand again for them is 8 of the 24 bytes an
+    // element that the split moves otherwise.
     AmaxArgs am;
     am.x[0] = static_cast<const double *>(A.data());
     am.x[1] = static_cast<const double *>(B.data());
@@ -730,6 +732,8 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
     am.n[1] = B.nnz;
     for (int i = 0; i < 2; ++i)
         am.parts[i] = int32_t(std::min<int64_t>((am.n[i] + 4095) / 4096, 2 * device_sm_count()));
+    const bool known = a_max && a_max->parts > 0;
+    if (known) am.parts[0] = 0;
     const int64_t head = (int64_t(2 + am.parts[0] + am.parts[1]) * 8 + 255) & ~int64_t(255);
     BufPtr split = dev_alloc(size_t(head + asz + bsz));
     auto *amax = static_cast<unsigned long long *>(split->p);
@@ -738,10 +742,14 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
     for (int i = 0; i < 2; ++i) {
         sa.src[i] = am.x[i];
         sa.parts[i] = am.parts[i];
+        sa.amax_parts[i] = am.out + (i ? am.parts[0] : 0);
+    }
+    if (known) {
+        sa.parts[0] = a_max->parts;
+        sa.amax_parts[0] = static_cast<const unsigned long long *>(a_max->buf->p);
     }
     sa.dst[0] = static_cast<char *>(split->p) + head;
     sa.dst[1] = sa.dst[0] + asz;
-    sa.amax_parts = am.out;
     sa.amax = amax;
     const int TM = gemm_tile_m();
     int64_t wide = 0;
@@ -772,6 +780,14 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
     g.ntiles = int32_t(tiles.size());
     g.alpha = alpha;
     g.beta = beta;
+    if (c_max && !add && alpha == 1.0) {
+        const int grid = gemm_tc_grid(g.ntiles);
+        if (grid <= 2 * device_sm_count()) {
+            c_max->buf = dev_alloc(size_t(grid) * 8);
+            c_max->parts = grid;
+            g.amax_out = static_cast<unsigned long long *>(c_max->buf->p);
+        }
+    }
     {
         StatScope sc(ST_PACK, (mode == GEMM_BF16X3 ? 14.0 : 16.0) * double(A.nnz + B.nnz));
         launch_amax(am);
@@ -785,7 +801,8 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
     launch_gemm_tc(g, mode);
 }
 
-BT tensordot(const BT &a, const BT &b, const std::vector<int64_t> &da, const std::vector<int64_t> &db) {
+BT tensordot(const BT &a, const BT &b, const std::vector<int64_t> &da, const std::vector<int64_t> &db, const Maxima *a_max,
+             Maxima *c_max) {
     ContractPlan P = plan_contraction(a, b, da, db);
     BT out = P.out;
     if (!a.has_data || !b.has_data) {
@@ -793,7 +810,7 @@ BT tensordot(const BT &a, const BT &b, const std::vector<int64_t> &da, const std
         return out;
     }
     out.alloc_data();
-    run_contraction(P, a, b, out, nullptr, 0.0, 1.0, nullptr);
+    run_contraction(P, a, b, out, nullptr, 0.0, 1.0, nullptr, a_max, c_max);
     return out;
 }
 

@@ -31,6 +31,7 @@ ContractPlan plan_contraction(const BT &A, const BT &B, const std::vector<int64_
 // Run the grouped GEMM of a plan into out (whose offsets index out's buffer).
 // add / add_block: optional beta*add term per output block (-1: none).
 void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, const BT *add, double beta,
-                     double alpha, const std::vector<int64_t> *add_block);
+                     double alpha, const std::vector<int64_t> *add_block,
+                     const Maxima *a_max = nullptr, Maxima *c_max = nullptr);
 
 }  // namespace qtt

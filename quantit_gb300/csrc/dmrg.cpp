@@ -22,21 +22,24 @@ BT compute_2sites_hamil(const BT &wl, const BT &wr) {
 }
 
 BT hamil2site_times_state(const BT &state, const BT &hamil, const BT &L, const BT &R) {
-    BT out = tensordot(L, state, {0}, {0});
-    out = tensordot(out, hamil, {0, 2, 3}, {0, 4, 5});
-    return tensordot(out, R, {1, 4}, {0, 1});
+    Maxima m1, m2;
+    BT out = tensordot(L, state, {0}, {0}, nullptr, &m1);
+    out = tensordot(out, hamil, {0, 2, 3}, {0, 4, 5}, &m1, &m2);
+    return tensordot(out, R, {1, 4}, {0, 1}, &m2);
 }
 
 BT compute_left_env(const BT &W, const BT &A, const BT &L) {
-    BT out = tensordot(L, A, {0}, {0});
-    out = tensordot(out, W, {0, 2}, {0, 3});
-    return tensordot(out, conj(A), {0, 2}, {0, 1});
+    Maxima m1, m2;
+    BT out = tensordot(L, A, {0}, {0}, nullptr, &m1);
+    out = tensordot(out, W, {0, 2}, {0, 3}, &m1, &m2);
+    return tensordot(out, conj(A), {0, 2}, {0, 1}, &m2);
 }
 
 BT compute_right_env(const BT &W, const BT &A, const BT &R) {
-    BT out = tensordot(R, A, {0}, {2});
-    out = tensordot(out, W, {0, 3}, {2, 3});
-    return tensordot(out, conj(A), {3, 0}, {1, 2});
+    Maxima m1, m2;
+    BT out = tensordot(R, A, {0}, {2}, nullptr, &m1);
+    out = tensordot(out, W, {0, 3}, {2, 3}, &m1, &m2);
+    return tensordot(out, conj(A), {3, 0}, {1, 2}, &m2);
 }
 
 void eig2x2(double a0, double a1, double b, double &E, double &o, double &n) {

@@ -40,9 +40,11 @@
 //    921 against 1518 us for the three contractions of the cylinder matvec at D = 2048.
 //
 // Against row groups outermost (64 or 96 copies of 1 KB a stage), one pair per stage, one CTA
-// per SM, five launches and as many memsets: theta pair D = 4096, TF32X3 436 -> 172 us (gemm
-// 252 -> 88); D = 1531, BF16X3 127 -> 63 us; cylinder matvec D = 2048, TF32X3 5971 -> 1623 us
-// (its MPO contraction alone 2606 -> 357), all to the same last bit.
+// per SM, five launches and as many memsets: theta pair D = 4096, TF32X3 436 -> 162 us (gemm
+// 252 -> 82); D = 1531, BF16X3 130 -> 49 us; cylinder matvec D = 2048, TF32X3 5974 -> 1418 us
+// (its MPO contraction alone 2606 -> 357), all to the same last bit.  The epilogue also gives the
+// largest result of each CTA, from which the next contraction of a chain takes its operand's scale: reading the
+// product again for it was 1543 us instead of 1418.
 //
 // The order of the MMAs of a tile is that of its pairs and k-steps whatever the stages
 // hold, so results do not depend on the grid or the ring.
@@ -278,10 +280,10 @@ __global__ void __launch_bounds__(256) k_split(SplitArgs g) {
     double d0[EV], d1[EV];
     load(threadIdx.x, d0);
     load(threadIdx.x + 256, d1);
-    const unsigned long long am = amax_of(g.amax_parts + (op ? g.parts[0] : 0), g.parts[op], red);
+    const unsigned long long am = amax_of(g.amax_parts[op], g.parts[op], red);
     if (blockIdx.x == 0) {
         // the GEMM's epilogue reads both maxima
-        const unsigned long long other = amax_of(g.amax_parts + (op ? 0 : g.parts[0]), g.parts[1 - op], red);
+        const unsigned long long other = amax_of(g.amax_parts[1 - op], g.parts[1 - op], red);
         if (threadIdx.x == 0) {
             g.amax[op] = am;
             g.amax[1 - op] = other;
@@ -364,6 +366,7 @@ __global__ void __launch_bounds__(TTHREADS, CTAS_PER_SM) k_gemm_tc(TcArgs g, int
     __shared__ uint64_t full[NSTAGE], empty[NSTAGE], acc_full[2], acc_empty[2], drained;
     __shared__ uint32_t stage_word[NSTAGE];
     __shared__ uint32_t tmem_base_sh;
+    __shared__ unsigned long long epi_top[4];  // per epilogue warp: largest result
     __shared__ int n_issued, n_consumed;  // stages sent out by the producer, taken by the MMA thread
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // round r of the longest-first tile list, in boustrophedon order across the CTAs, so
@@ -579,6 +582,7 @@ __global__ void __launch_bounds__(TTHREADS, CTAS_PER_SM) k_gemm_tc(TcArgs g, int
         const int quarter = warp & 3;
         float *patch = reinterpret_cast<float *>(smem + NSTAGE * STAGE) + quarter * 32 * EPI_PITCH;
         const int shift = amax_shift(g.amax[0]) + amax_shift(g.amax[1]);
+        uint32_t top = 0;  // largest |accumulator|, as bits
         int i = 0;
         TileRegs mine;
         mine.cls = -1;
@@ -630,6 +634,7 @@ __global__ void __launch_bounds__(TTHREADS, CTAS_PER_SM) k_gemm_tc(TcArgs g, int
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         if (x0 + 32 * u >= n) break;
+                        top = max(top, __float_as_uint(f[u]) & 0x7FFFFFFFu);
                         double val = have_acc ? f32_to_f64_int(f[u], shift) : 0.0;
                         if (!plain) {
                             val *= g.alpha;
@@ -646,8 +651,12 @@ __global__ void __launch_bounds__(TTHREADS, CTAS_PER_SM) k_gemm_tc(TcArgs g, int
                 ++i;
             }
         }
+        // scaling back is monotonic: the largest accumulator is the largest result
+        top = __reduce_max_sync(0xffffffffu, top);
+        if (lane == 0) epi_top[quarter] = static_cast<unsigned long long>(__double_as_longlong(f32_to_f64_int(__uint_as_float(top), shift)));
     }
     __syncthreads();
+    if (tid == 0 && g.amax_out) g.amax_out[blockIdx.x] = max(max(epi_top[0], epi_top[1]), max(epi_top[2], epi_top[3]));
     if (tid == 0) {
         // copies issued but never consumed (only after a timeout) must land before exit, and
         // every MMA must have completed before TMEM is freed
@@ -690,7 +699,7 @@ void launch_gemm(const TcArgs &a) {
     // CTAS_PER_SM persistent CTAs an SM; one CTA per tile with the persistent grid switched off.
     // With no more tiles than SMs a CTA has its SM to itself and takes twice the stages.
     const int sms = device_sm_count();
-    const int grid = persistent_gemm() ? std::min(a.ntiles, CTAS_PER_SM * sms) : a.ntiles;
+    const int grid = gemm_tc_grid(a.ntiles);
     if (a.ntiles <= sms)
         launch_ring<S, 2 * S::NSTAGE>(a, grid);
     else
@@ -699,6 +708,7 @@ void launch_gemm(const TcArgs &a) {
 
 }  // namespace
 
+int gemm_tc_grid(int ntiles) { return persistent_gemm() ? std::min(ntiles, CTAS_PER_SM * device_sm_count()) : ntiles; }
 int gemm_tile_m() { return TBM; }
 int gemm_tile_n(int64_t tiles) { return tiles <= device_sm_count() ? TBN / 2 : TBN; }
 int split_copies(int mode) { return mode == GEMM_BF16X3 ? Bf16x3::NC : Tf32x3::NC; }

@@ -109,7 +109,7 @@ struct SplitArgs {
     char *dst[2];
     const SplitEntry *ents;
     const SplitTile *tiles;
-    const unsigned long long *amax_parts;
+    const unsigned long long *amax_parts[2];  // per operand: maxima of its pieces (k_amax's, or a GEMM's amax_out)
     int32_t parts[2];
     unsigned long long *amax;  // receives the two operands' maxima
 };
@@ -130,9 +130,11 @@ struct TcArgs {
     const GemmTile *tiles;
     int32_t ntiles;
     int32_t tn;  // columns of a tile: gemm_tile_n
+    unsigned long long *amax_out = nullptr;  // not null: one maximum of |C| per CTA (alpha = 1, no add term)
     double alpha, beta;
 };
 void launch_gemm_tc(const TcArgs &a, int mode);
+int gemm_tc_grid(int ntiles);  // its CTAs
 int gemm_tile_m();
 // Tile columns for a launch of `tiles` tiles of 128 columns: 128, or 64 where those would not
 // fill the SMs.

@@ -321,7 +321,15 @@ BT reshape(const BT &t, const std::vector<int64_t> &groups);
 BT reshape_as(const BT &t, const BT &shape);
 BT inverse_cvals(const BT &t);
 BT conj(const BT &t);
-BT tensordot(const BT &a, const BT &b, const std::vector<int64_t> &da, const std::vector<int64_t> &db);
+// Maxima of |x| over the pieces of a tensor's data, on the device (parts = 0: not known).  A contraction on the
+// tensor cores gives those of its result (c_max) and takes those of its first operand (a_max): for a product that goes
+// straight into the next one, with nothing written to it in between.
+struct Maxima {
+    BufPtr buf;
+    int32_t parts = 0;
+};
+BT tensordot(const BT &a, const BT &b, const std::vector<int64_t> &da, const std::vector<int64_t> &db,
+             const Maxima *a_max = nullptr, Maxima *c_max = nullptr);
 BT tensorgdot(const BT &add, const BT &a, const BT &b, const std::vector<int64_t> &da,
               const std::vector<int64_t> &db, double beta, double alpha);
 BT add_scaled(const BT &a, const BT &b, double ca, double cb);
@@ -393,7 +401,7 @@ int jacobi_variant();
 // Block-width autotuner of the block-Jacobi kernel (on by default) and its decisions.
 void set_autotune(int on);
 std::string autotune_report();
-// Persistent tensor-core GEMM for launches of at least two tiles per SM (on by default).
+// Persistent tensor-core GEMM (on by default); off: one CTA per tile.
 void set_persistent_gemm(int on);
 int persistent_gemm();
 // Block-sparsity planner of tensordot: 0 host merge-join (the default), 1 device
