@@ -93,8 +93,8 @@ int qtt_set_planner(int mode, int64_t auto_blocks);
  * calls[2] device attempts beyond its limits (planned on the host); secs[0], secs[1]:
  * host wall seconds spent planning on each path.  reset != 0 clears them. */
 int qtt_planner_stats(int64_t *calls, double *secs, int reset);
-/* Persistent split-TF32 / split-BF16 GEMMs (one CTA per SM walking the tile list, double-buffered TMEM
- * accumulator) for launches of at least two tiles per SM; on by default (no reference
+/* Persistent split-TF32 / split-BF16 GEMMs (two CTAs per SM walking the tile list, double-buffered TMEM
+ * accumulator); on by default.  Off: one CTA per tile, the same sums (no reference
  * counterpart). */
 int qtt_set_persistent_gemm(int on);
 /* Free and total bytes of the calling thread's device (no reference counterpart;

@@ -56,7 +56,7 @@ def planner_stats(reset=False):
 
 
 def set_persistent_gemm(on):
-    """Persistent split-TF32 GEMM for launches of many tiles (on by default)."""
+    """Persistent tensor-core GEMMs (on by default); off: one CTA per tile, the same sums."""
     from ._lib import call
     call("qtt_set_persistent_gemm", 1 if on else 0)
 

@@ -17,10 +17,10 @@
 //    an MPO tensor (N or M of a few, K of a few), which are bound by memory.
 // Against 64 x 64 x 16 tiles staged in shared memory (17 us of FP64 pipe for any tile,
 // however small the block), same sums to the last bit: theta pair contraction at D = 2048
-// 1787 -> 1352 us (0.95 TFLOP/s, 87% of cuBLAS DGEMM); the matvec of a Hubbard chain at
-// D = 512 2584 -> 1277 us, of which its kernels now take less than the host's planning; an
-// environment update of a spin chain at D = 777 1271 -> 336 us; a 24-dimensional site pair
-// 34 -> 19 us.
+// 1787 -> 1303 us (0.98 TFLOP/s, 82% of what independent FMAs reach; mma.sync FP64 runs on the same pipe at
+// 1.05 against their 1.20 TFLOP/s); the matvec of a Hubbard chain at D = 512 2584 -> 771 us, of which its kernels
+// take 124 and the host's planning the rest; an environment update of a spin chain at D = 777
+// 1271 -> 315 us; a 24-dimensional site pair 34 -> 15 us.
 #include "kernels.h"
 #include "qtt_core.h"
 
