@@ -128,14 +128,13 @@ __global__ void k_zero(double *p, int64_t n) {
         p[i] = 0.0;
 }
 
-__global__ void k_scatter(const double *__restrict__ src, double *__restrict__ dst,
-                          const ScatterEntry *__restrict__ ents, const Chunk *__restrict__ chunks) {
+__global__ void k_scatter(const ScatterEntry *__restrict__ ents, const Chunk *__restrict__ chunks) {
     const Chunk ch = chunks[blockIdx.x];
     const ScatterEntry e = ents[ch.seg];
     for (int i = threadIdx.x; i < ch.len; i += blockDim.x) {
         int64_t k = ch.start + i;
         int r = int(k / e.k), c = int(k - int64_t(r) * e.k);
-        dst[e.dst_off + k] = src[e.src_off + int64_t(e.r0 + r) + int64_t(c) * e.ld];
+        e.dst[k] = e.src[int64_t(e.r0 + r) + int64_t(c) * e.ld];
     }
 }
 
@@ -226,9 +225,9 @@ void launch_zero(double *p, int64_t n) {
     cuda_check(cudaGetLastError(), "zero kernel launch");
 }
 
-void launch_scatter(const double *src, double *dst, const ScatterEntry *e, const Chunk *chunks, int64_t nchunks) {
+void launch_scatter(const ScatterEntry *e, const Chunk *chunks, int64_t nchunks) {
     if (nchunks <= 0) return;
-    k_scatter<<<grid_for(nchunks), TPB, 0, ctx().stream>>>(src, dst, e, chunks);
+    k_scatter<<<grid_for(nchunks), TPB, 0, ctx().stream>>>(e, chunks);
     count_launch();
     cuda_check(cudaGetLastError(), "scatter kernel launch");
 }

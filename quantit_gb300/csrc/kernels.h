@@ -296,10 +296,11 @@ void launch_finish_on(cudaStream_t stream, const void *work, const void *rot, do
 // Segment = one output block (rows x k row-major at dst_off) from a column-major
 // (ld x *) sector matrix at src_off: dst[i*k + j] = src[src_off + (r0 + i) + j*ld].
 struct ScatterEntry {
-    int64_t src_off, dst_off;
+    const double *src;
+    double *dst;
     int32_t ld, r0, k, pad;
 };
-void launch_scatter(const double *src, double *dst, const ScatterEntry *e, const Chunk *chunks, int64_t nchunks);
+void launch_scatter(const ScatterEntry *e, const Chunk *chunks, int64_t nchunks);
 
 // ------------------------------------------------------------ 2x2 Ritz step on device
 // s[0]=a0, s[1]=b, s[2]=a1  ->  s[3]=E, s[4]=o, s[5]=n, s[6]=nan flag

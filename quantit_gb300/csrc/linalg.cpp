@@ -349,11 +349,14 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                 lq.push_back(lq_of(d, false));
                 d.warm = 1;
             }
-    SectorDesc *dsec = static_cast<SectorDesc *>(upload(D.desc.data(), D.desc.size() * sizeof(SectorDesc)));
     const int64_t packed = std::accumulate(lens.begin(), lens.end(), int64_t(0));
-    const PackEntry *dpe = upload_vec(pe);
     auto chunks = make_chunks(lens);
-    const Chunk *dch = upload_vec(chunks);
+    const SectorDesc *desc_table = nullptr;
+    const PackEntry *dpe = nullptr;
+    const Chunk *dch = nullptr;
+    const int *dslots = nullptr;
+    upload_many({table(D.desc, desc_table), table(pe, dpe), table(chunks, dch), table(slots, dslots)});
+    SectorDesc *dsec = const_cast<SectorDesc *>(desc_table);  // (eigh writes its shifts there)
     {
         StatScope sc(ST_PACK, 2.0 * 8.0 * double(packed));
         launch_pack(static_cast<const double *>(t.data()), W, dpe, dch, int64_t(chunks.size()), dsec, f32);
@@ -401,7 +404,6 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             launch_warm_apply(W, D.rot->p, tmp->p, upload_vec(wdesc), int(wdesc.size()), ntiles, f32);
         }
         launch_lq(W, D.rot->p, lq, f32);
-        const int *dslots = upload_vec(slots);
         launch_jacobi(W, D.rot->p, dsec, dslots, nsec, max_steps, max_sweeps, sweeps, flags, f32, max_p, stot,
                       vwork->p, vb, deflate ? thr->p : nullptr, deflate ? dnorm->p : nullptr, nullptr,
                       trunc_hint().plain);
@@ -660,13 +662,32 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     }
 }
 
-// Write blocks of `out` (its structure already set, offsets compact) from the
-// sector factor buffer: out block = (lead..., rows of section, k columns).
-void scatter_factor(BT &out, const Decomp &D, const BufPtr &src, bool rows_side_U, const std::vector<int64_t> &blk_sec,
-                    const std::vector<int64_t> &blk_kcols) {
-    const int r = out.rank;
-    std::vector<ScatterEntry> se;
+// The factors' blocks, written in one launch from one copy of tables: a launch and two copies for each of
+// U, V and d were an eighth of a small svd (site svd D = 48 234 -> 204 us).
+struct Scatter {
+    static constexpr size_t kChunks = size_t(1) << 19;
+    std::vector<ScatterEntry> ents;
     std::vector<int64_t> lens;
+    void run() const {
+        const std::vector<Chunk> chunks = make_chunks(lens);
+        // (more than one launch only for factors of several GB together: a table has to fit the staging ring)
+        for (size_t first = 0; first < chunks.size(); first += kChunks) {
+            const std::vector<Chunk> part(chunks.begin() + first, chunks.begin() + std::min(chunks.size(), first + kChunks));
+            const ScatterEntry *e = nullptr;
+            const Chunk *c = nullptr;
+            upload_many({table(ents, e), table(part, c)});
+            launch_scatter(e, c, int64_t(part.size()));
+        }
+    }
+};
+
+// Blocks of `out` (its structure already set, offsets compact) from the
+// sector factor buffer: out block = (lead..., rows of section, k columns).
+void scatter_factor(Scatter &sc, BT &out, const Decomp &D, const BufPtr &src, bool rows_side_U,
+                    const std::vector<int64_t> &blk_sec, const std::vector<int64_t> &blk_kcols) {
+    const int r = out.rank;
+    const double *from = static_cast<const double *>(src->p);
+    double *to = static_cast<double *>(out.data());
     for (int64_t b = 0; b < out.nblocks(); ++b) {
         const int64_t g = blk_sec[b];
         const Sector &s = D.secs[g];
@@ -676,40 +697,35 @@ void scatter_factor(BT &out, const Decomp &D, const BufPtr &src, bool rows_side_
         for (int64_t e = 0; e < s.batch; ++e) {
             const SectorDesc &d = D.desc[D.first_desc[g] + e];
             ScatterEntry x{};
-            x.src_off = rows_side_U ? d.u_off : d.v_off;
-            x.dst_off = out.boff[b] + e * rr.size * k;
+            x.src = from + (rows_side_U ? d.u_off : d.v_off);
+            x.dst = to + out.boff[b] + e * rr.size * k;
             x.ld = rows_side_U ? d.m : d.n;
             x.r0 = int32_t(rr.start);
             x.k = int32_t(k);
-            se.push_back(x);
-            lens.push_back(rr.size * k);
+            sc.ents.push_back(x);
+            sc.lens.push_back(rr.size * k);
         }
     }
-    auto chunks = make_chunks(lens);
-    launch_scatter(static_cast<const double *>(src->p), static_cast<double *>(out.data()), upload_vec(se),
-                   upload_vec(chunks), int64_t(chunks.size()));
 }
 
-void scatter_values(BT &d, const Decomp &D, const std::vector<int64_t> &blk_sec, const std::vector<int64_t> &blk_k) {
-    std::vector<ScatterEntry> se;
-    std::vector<int64_t> lens;
+void scatter_values(Scatter &sc, BT &d, const Decomp &D, const std::vector<int64_t> &blk_sec,
+                    const std::vector<int64_t> &blk_k) {
+    const double *from = static_cast<const double *>(D.S->p);
+    double *to = static_cast<double *>(d.data());
     for (int64_t b = 0; b < d.nblocks(); ++b) {
         const Sector &s = D.secs[blk_sec[b]];
         for (int64_t e = 0; e < s.batch; ++e) {
             const SectorDesc &x = D.desc[D.first_desc[blk_sec[b]] + e];
             ScatterEntry y{};
-            y.src_off = x.s_off;
-            y.dst_off = d.boff[b] + e * blk_k[b];
+            y.src = from + x.s_off;
+            y.dst = to + d.boff[b] + e * blk_k[b];
             y.ld = 1;
             y.r0 = 0;
             y.k = int32_t(blk_k[b]);
-            se.push_back(y);
-            lens.push_back(blk_k[b]);
+            sc.ents.push_back(y);
+            sc.lens.push_back(blk_k[b]);
         }
     }
-    auto chunks = make_chunks(lens);
-    launch_scatter(static_cast<const double *>(D.S->p), static_cast<double *>(d.data()), upload_vec(se),
-                   upload_vec(chunks), int64_t(chunks.size()));
 }
 
 }  // namespace
@@ -784,9 +800,11 @@ SVDOut svd(const BT &t) {
     o.U.alloc_data();
     o.V.alloc_data();
     o.d.alloc_data();
-    scatter_factor(o.U, D, D.U, true, us, uk);
-    scatter_factor(o.V, D, D.V, false, vs, vk);
-    scatter_values(o.d, D, ds, dk);
+    Scatter sc;
+    scatter_factor(sc, o.U, D, D.U, true, us, uk);
+    scatter_factor(sc, o.V, D, D.V, false, vs, vk);
+    scatter_values(sc, o.d, D, ds, dk);
+    sc.run();
     return o;
 }
 
@@ -1049,8 +1067,10 @@ EighOut eigh(const BT &t, bool upper) {
     run_decomp(t, D, 1, upper ? 1 : 0);
     o.U.alloc_data();
     o.d.alloc_data();
-    scatter_factor(o.U, D, D.U, true, us, uk);
-    scatter_values(o.d, D, ds, dk);
+    Scatter sc;
+    scatter_factor(sc, o.U, D, D.U, true, us, uk);
+    scatter_values(sc, o.d, D, ds, dk);
+    sc.run();
     return o;
 }
 
