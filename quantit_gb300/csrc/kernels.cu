@@ -134,7 +134,7 @@ __global__ void k_scatter(const ScatterEntry *__restrict__ ents, const Chunk *__
     for (int i = threadIdx.x; i < ch.len; i += blockDim.x) {
         int64_t k = ch.start + i;
         int r = int(k / e.k), c = int(k - int64_t(r) * e.k);
-        e.dst[k] = e.src[int64_t(e.r0 + r) + int64_t(c) * e.ld];
+        e.dst[k] = e.src[r * e.rs + c * e.cs];
     }
 }
 

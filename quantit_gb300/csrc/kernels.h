@@ -296,9 +296,10 @@ void launch_finish_on(cudaStream_t stream, const void *work, const void *rot, do
 // Segment = one output block (rows x k row-major at dst_off) from a column-major
 // (ld x *) sector matrix at src_off: dst[i*k + j] = src[src_off + (r0 + i) + j*ld].
 struct ScatterEntry {
-    const double *src;
-    double *dst;
-    int32_t ld, r0, k, pad;
+    const double *src;  // element (row, column) of the block: src[row rs + column cs]
+    double *dst;        // row-major, k columns
+    int64_t rs, cs;
+    int32_t k, pad;
 };
 void launch_scatter(const ScatterEntry *e, const Chunk *chunks, int64_t nchunks);
 

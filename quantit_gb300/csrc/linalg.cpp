@@ -662,7 +662,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     }
 }
 
-// The factors' blocks, written in one launch from one copy of tables: a launch and two copies for each of
+// The factors' blocks (whole or truncated), written in one launch from one copy of tables: a launch and two copies for each of
 // U, V and d were an eighth of a small svd (site svd D = 48 234 -> 204 us).
 struct Scatter {
     static constexpr size_t kChunks = size_t(1) << 19;
@@ -697,10 +697,10 @@ void scatter_factor(Scatter &sc, BT &out, const Decomp &D, const BufPtr &src, bo
         for (int64_t e = 0; e < s.batch; ++e) {
             const SectorDesc &d = D.desc[D.first_desc[g] + e];
             ScatterEntry x{};
-            x.src = from + (rows_side_U ? d.u_off : d.v_off);
+            x.src = from + (rows_side_U ? d.u_off : d.v_off) + rr.start;
             x.dst = to + out.boff[b] + e * rr.size * k;
-            x.ld = rows_side_U ? d.m : d.n;
-            x.r0 = int32_t(rr.start);
+            x.rs = 1;
+            x.cs = rows_side_U ? d.m : d.n;
             x.k = int32_t(k);
             sc.ents.push_back(x);
             sc.lens.push_back(rr.size * k);
@@ -719,8 +719,7 @@ void scatter_values(Scatter &sc, BT &d, const Decomp &D, const std::vector<int64
             ScatterEntry y{};
             y.src = from + x.s_off;
             y.dst = to + d.boff[b] + e * blk_k[b];
-            y.ld = 1;
-            y.r0 = 0;
+            y.cs = 1;
             y.k = int32_t(blk_k[b]);
             sc.ents.push_back(y);
             sc.lens.push_back(blk_k[b]);
@@ -853,9 +852,9 @@ void remove_unit_blocks(std::vector<int64_t> &list, const BT &U, int64_t sector)
     list.resize(n - (dest - src));
 }
 
-// Materialise a truncated unitary: blocks `list` of U, the ones on `kcols`
+// A truncated unitary, its copy added to sc: blocks `list` of U, the ones on `kcols`
 // sectors sliced to their first k columns.
-BT materialise(const BT &U, const std::vector<int64_t> &list, const std::vector<int64_t> &new_ssz_last) {
+BT materialise(Scatter &sc, const BT &U, const std::vector<int64_t> &list, const std::vector<int64_t> &new_ssz_last) {
     BT o = U.shape_only();
     const int r = U.rank;
     const int64_t last = U.addr(r - 1);
@@ -865,27 +864,21 @@ BT materialise(const BT &U, const std::vector<int64_t> &list, const std::vector<
     o.compact_offsets();
     if (!U.has_data) return o;
     o.alloc_data();
-    std::vector<PermEntry> ents(list.size());
-    std::vector<int64_t> lens(list.size());
     for (size_t k = 0; k < list.size(); ++k) {
         const int64_t b = list[k];
         const int64_t kf = U.ssz[last + U.idx(b)[r - 1]];
         const int64_t kn = o.block_numel(int64_t(k));
         const int64_t rows = kf ? U.block_numel(b) / kf : 0;
         const int64_t kk = rows ? kn / rows : 0;
-        PermEntry &e = ents[k];
-        std::memset(&e, 0, sizeof(e));
-        e.src_off = U.boff[b];
-        e.dst_off = o.boff[k];
-        e.rank = 2;
-        e.dims[0] = rows;
-        e.dims[1] = kk;
-        e.stride[0] = kf;
-        e.stride[1] = 1;
-        lens[k] = kn;
+        ScatterEntry e{};
+        e.src = static_cast<const double *>(U.data()) + U.boff[b];
+        e.dst = static_cast<double *>(o.data()) + o.boff[k];
+        e.rs = kf;
+        e.cs = 1;
+        e.k = int32_t(kk);
+        sc.ents.push_back(e);
+        sc.lens.push_back(kn);
     }
-    auto chunks = make_chunks(lens);
-    launch_permute(U.data(), o.data(), upload_vec(ents), upload_vec(chunks), int64_t(chunks.size()), 8);
     return o;
 }
 }  // namespace
@@ -951,8 +944,9 @@ SVDOut truncate(SVDOut &&in, int64_t max_size, int64_t min_size, double tol, dou
         }
     }
     SVDOut o;
-    o.U = materialise(U, ulist, ku);
-    if (V) o.V = materialise(*V, vlist, kv);
+    Scatter sc;
+    o.U = materialise(sc, U, ulist, ku);
+    if (V) o.V = materialise(sc, *V, vlist, kv);
     // d: same walk on a rank-1 tensor (its "rows" are a single row)
     BT dd = d.shape_only();
     for (int64_t s = 0; s < nsec; ++s) dd.ssz[s] = kd[s];
@@ -961,20 +955,16 @@ SVDOut truncate(SVDOut &&in, int64_t max_size, int64_t min_size, double tol, dou
     dd.boff.assign(dlist.size(), 0);
     dd.compact_offsets();
     dd.alloc_data();
-    std::vector<PermEntry> ents(dlist.size());
-    std::vector<int64_t> lens(dlist.size());
     for (size_t k = 0; k < dlist.size(); ++k) {
-        PermEntry &e = ents[k];
-        std::memset(&e, 0, sizeof(e));
-        e.src_off = d.boff[dlist[k]];
-        e.dst_off = dd.boff[k];
-        e.rank = 1;
-        e.dims[0] = dd.block_numel(int64_t(k));
-        e.stride[0] = 1;
-        lens[k] = e.dims[0];
+        ScatterEntry e{};
+        e.src = static_cast<const double *>(d.data()) + d.boff[dlist[k]];
+        e.dst = static_cast<double *>(dd.data()) + dd.boff[k];
+        e.cs = 1;
+        e.k = int32_t(dd.block_numel(int64_t(k)));
+        sc.ents.push_back(e);
+        sc.lens.push_back(e.k);
     }
-    auto chunks = make_chunks(lens);
-    launch_permute(d.data(), dd.data(), upload_vec(ents), upload_vec(chunks), int64_t(chunks.size()), 8);
+    sc.run();
     o.d = dd;
     o.discarded = dropped;
     o.total = total;
