@@ -62,8 +62,8 @@ __device__ __forceinline__ float ldcg(const float *p) { return __ldcg(p); }
 // In FP64 the block kernel rotates columns of more than 128 rows by the same rotation as three shears, x -= tau y, y += s x,
 // x -= tau y: three instead of four instructions of GB300's narrow FP64 pipe per element pair.  A third
 // dependent rounding makes the values' error ~1.2 times that of the form above, which LQ's fewer sweeps more
-// than win back; shorter columns, which mostly run without LQ, keep the form above (eigh D = 300: 2.00 ms with
-// the shears, 2.08 with the four instructions).
+// than win back; shorter columns, which mostly run without LQ, keep the form above (eigh D = 300: 4 % more
+// time for the four instructions).
 template <class T, bool FOUR = true>
 __device__ __forceinline__ void rot_apply(T &x, T &y, T s, T tau) {
     if constexpr (sizeof(T) == 8 && !FOUR) {
@@ -418,9 +418,9 @@ __global__ void __launch_bounds__(JJ) k_jacobi(JacobiParams<T> P) {
 //     registers and the J columns move through shared memory.
 // Every column pair of the sector is thus visited exactly once per sweep, as in
 // the scalar ordering, but a sweep costs ~q/B grid barriers instead of ~q.  The
-// rotations of a step are accumulated into a 2B x 2B orthogonal matrix Q (one
-// element per lane and column) and applied to the rotation matrix V once at the
-// end of the step (V[:, I u J] <- V[:, I u J] Q).
+// rotations of a step reach the rotation matrix V once, behind the step: FP32 accumulates them
+// into a 2B x 2B orthogonal matrix Q (one element per lane and column; V[:, I u J] <- V[:, I u J] Q),
+// FP64 keeps the rotations themselves (bj_apply_rots).
 template <class T>
 struct BJacobiParams {
     T *work;
