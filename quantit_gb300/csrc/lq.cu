@@ -6,9 +6,9 @@
 // columns graded over 8 to 14 decades): 15 to 30 sweeps.  On the columns of L -- the rows of R
 // in A^T P = Q R, with the rows of A sorted by norm -- it needs about 7 whatever the grading (Drmac
 // and Veselic's preconditioning, SIAM J. Matrix Anal. Appl. 29 (2008), with one sorted instead of a
-// pivoted factorisation; unsorted it gains nothing).  Q is a product of Householder reflections,
-// orthogonal to working precision whatever the data, and any orthogonal start gives an exact SVD, so
-// the factorisation decides the speed alone.
+// pivoted factorisation; unsorted it gains nothing).  Q is a product of Householder reflections, each
+// formed from its row scaled by a power of two and so orthogonal to working precision at any magnitude
+// (scale_row), and any orthogonal start gives an exact SVD: the factorisation decides the speed alone.
 //
 // All sectors go through one cooperative launch in panels of NB = 8 reflections.  The vectors
 // (the p rows of W and the q rows of the identity, q long, contiguous in X) are independent under
@@ -103,6 +103,29 @@ __device__ __forceinline__ void apply_panel(T *x, const T *V, const T *Tm, int l
     }
 }
 
+// The exact powers of two that bring a row's largest |x| to about 1 and back (scale_row: false where there
+// is nothing to reflect by: zeros, an infinity or a NaN).  Sums of squares of the row as it is leave the work type's
+// range long before its elements do -- FP32 elements of 1e-20 have subnormal squares -- and a reflection from an inexact
+// sum is not orthogonal.
+__device__ __forceinline__ bool scale_row(const float *x, int first, int len, int lane, float &up, float &down) {
+    uint32_t m = 0;
+    for (int k = first + lane; k < len; k += 32) m = max(m, __float_as_uint(x[k]) & 0x7FFFFFFFu);
+    m = __reduce_max_sync(0xffffffffu, m);
+    const uint32_t f = 253u - min(m >> 23, 252u);
+    up = __uint_as_float(f << 23);
+    down = __uint_as_float((254u - f) << 23);
+    return m != 0 && m < 0x7F800000u;
+}
+__device__ __forceinline__ bool scale_row(const double *x, int first, int len, int lane, double &up, double &down) {
+    uint32_t m = 0;  // by the high words
+    for (int k = first + lane; k < len; k += 32) m = max(m, uint32_t(__double2hiint(x[k])) & 0x7FFFFFFFu);
+    m = __reduce_max_sync(0xffffffffu, m);
+    const uint32_t f = 2045u - min(m >> 20, 2044u);
+    up = __hiloint2double(int(f << 20), 0);
+    down = __hiloint2double(int((2046u - f) << 20), 0);
+    return m != 0 && m < 0x7FF00000u;
+}
+
 // Factors the NB rows held in xs (`pitch` apart, len long; nr of them exist): row c's reflection
 // zeroes its elements beyond c.  vs receives the reflectors (zero before their
 // first element), Tm the triangular factor.  All 8 warps of the CTA, one per row.
@@ -112,20 +135,21 @@ __device__ void factor_panel(T *xs, int pitch, T *vs, T *Tm, T *gram, T *tau, in
         T *v = vs + c * len;
         if (warp == c) {
             T *x = xs + c * pitch;
-            T s = T(0);
-            const bool real = c < nr && c + 1 < len;
+            T s = T(0), up = T(1), down = T(1);
+            const bool real = c < nr && c + 1 < len && scale_row(x, c, len, lane, up, down);
             if (real)
-                for (int k = c + 1 + lane; k < len; k += 32) s = fma(x[k], x[k], s);
+                for (int k = c + 1 + lane; k < len; k += 32) s = fma(x[k] * up, x[k] * up, s);
             s = lsum(s);
             T t = T(0), scale = T(0), beta = T(0);
             if (real && s > T(0)) {
-                const T alpha = x[c];
+                const T alpha = x[c] * up;
                 beta = -copysign(sqrt(fma(alpha, alpha, s)), alpha);
                 t = (beta - alpha) / beta;
                 scale = T(1) / (alpha - beta);
+                beta *= down;
             }
             for (int k = lane; k < len; k += 32) {
-                const T y = t != T(0) && k > c ? x[k] * scale : (k == c && t != T(0) ? T(1) : T(0));
+                const T y = t != T(0) && k > c ? x[k] * up * scale : (k == c && t != T(0) ? T(1) : T(0));
                 v[k] = y;
                 if (t != T(0)) {
                     if (k == c) x[k] = beta;
