@@ -197,11 +197,11 @@ struct WarmDesc {
 };
 void launch_warm_apply(void *work, void *rot, void *tmp, const WarmDesc *wd, int nwarm, int ntiles, int f32);
 // LQ preconditioning (lq.cu): for each listed sector work (p x q, column-major at w_off) <- W Q and
-// rot (q x q at rot_off) <- Q, or rot Q with from_rot, Q orthogonal, W Q lower trapezoidal on its rows by falling norm.
+// rot (q x q at rot_off) <- Q, Q orthogonal, W Q lower trapezoidal on its rows by falling norm.
 // 2 <= q <= lq_max_q(f32, sectors) <= p.  The other offsets are the launcher's.
 struct LqSec {
     int64_t w_off, rot_off, x_off, v_off, o_off;
-    int32_t p, q, from_rot, pad;
+    int32_t p, q;
 };
 constexpr size_t LQ_SMEM_MAX = 200 * 1024;
 int lq_max_q(int f32, int nsec);

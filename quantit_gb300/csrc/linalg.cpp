@@ -251,16 +251,26 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     // always runs in FP64.
     // Sectors that are LQ-preconditioned (lq.cu).  Under a truncation, from 16 columns on: svd of a
     // graded theta at D = 60 1664 -> 907 us, at D = 100 2846 -> 1383, at D = 600 35.0 -> 12.7 ms.
-    // The plain svd also sees matrices that are not graded (bMPS.move_oc of a random state), where
-    // the sweeps saved do not pay for the factorisation of a small sector: D = 120 806 us without
-    // against 925 with.  With the deflation switched off the sweeps run from the identity as well: null
-    // columns that stay in keep a factored start sweeping as long.
-    const int lq_least = mode != 0 || trunc_hint().plain ? INT32_MAX : !trunc_hint().active ? 48 : svd_deflation() ? 16 : INT32_MAX;
+    // The untruncated svd in FP64 from 48 columns on.  It also sees matrices that are not graded (bMPS.move_oc of a
+    // random state), where the factorisation saves no sweep; without it and with it, us, sectors of q columns:
+    //            q x q, 0 / 4 / 12 decades            2q x q, 0 / 4 / 12 decades
+    //   q = 48   1466, 1490  1707, 1628  2512, 1149   1429, 1467  1403, 1418  1854, 1253
+    //   q = 96   3557, 3585  4542, 2939  6958, 2729   3288, 3681  3314, 3227  4732, 2921
+    //   q = 200  10.9, 9.8   13.7, 8.5   21.7, 7.4 ms 11.8, 12.0  11.9, 11.2  16.9, 9.9 ms
+    // In a split mode the untruncated svd has no factorisation: its FP32 sweeps are cheap, the FP64 sweeps after
+    // them number two from either start on ungraded sectors (random site, D = 400: 1811 us without, 1987 with) and at
+    // 12 decades 9 instead of 3 (2q x q, q = 300: 13.7 ms without, 18.1 with).
+    // With the deflation switched off the sweeps run from the identity as well: null columns that stay in keep a
+    // factored start sweeping as long.
+    const bool split_mode = gemm_mode() != GEMM_F64;
+    const int lq_least = mode != 0 || trunc_hint().plain ? INT32_MAX
+                         : trunc_hint().active           ? (svd_deflation() ? 16 : INT32_MAX)
+                                                         : (split_mode ? INT32_MAX : 48);
     auto lq_fits = [&](const SectorDesc &d, int prec32) { return d.q >= lq_least && d.q <= lq_max_q(prec32, nsec); };
     // A decomposition that is run again because its estimated truncation fell short is FP64
     // throughout, if the factorisation speeds its FP64 sweeps up.
     const bool redo = trunc_hint().active && !trunc_hint().allow_discard && max_q >= lq_least;
-    const int f32 = (mode == 0 && gemm_mode() != GEMM_F64 && !redo) ? 1 : 0;
+    const int f32 = (mode == 0 && split_mode && !redo) ? 1 : 0;
     const size_t es = f32 ? 4 : 8;
     D.work = dev_alloc(size_t(std::max<int64_t>(wtot, 1)) * es);
     D.rot = dev_alloc(size_t(std::max<int64_t>(rtot, 1)) * es);
@@ -294,13 +304,12 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             }
         }
     }
-    auto lq_of = [](const SectorDesc &d, bool from_rot) {
+    auto lq_of = [](const SectorDesc &d) {
         LqSec s{};
         s.w_off = d.w_off;
         s.rot_off = d.rot_off;
         s.p = d.p;
         s.q = d.q;
-        s.from_rot = from_rot ? 1 : 0;
         return s;
     };
     // warm starts: a sector whose key (orientation, batch element, q-side sections) matches
@@ -346,7 +355,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     if (mode == 0)
         for (SectorDesc &d : D.desc)
             if (lq_fits(d, f32)) {
-                lq.push_back(lq_of(d, false));
+                lq.push_back(lq_of(d));
                 d.warm = 1;
             }
     const int64_t packed = std::accumulate(lens.begin(), lens.end(), int64_t(0));
@@ -500,8 +509,10 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             std::vector<SectorDesc> d64 = D.desc;
             for (SectorDesc &d : d64) {
                 d.warm = resolve_anew ? 0 : 1;
-                if (discard.empty() && lq_fits(d, 0)) {
-                    lq64.push_back(lq_of(d, !resolve_anew));
+                // (never after the refinement: W1's columns are orthogonal to 1e-6 and need two sweeps, the columns
+                // of a triangular factor of W1 all eight again)
+                if (resolve_anew && lq_fits(d, 0)) {
+                    lq64.push_back(lq_of(d));
                     d.warm = 1;
                 }
             }

@@ -1,4 +1,4 @@
-// LQ preconditioning of the sector SVDs: W <- W Q, rot <- Q (or rot Q) with W Q lower trapezoidal on
+// LQ preconditioning of the sector SVDs: W <- W Q, rot <- Q with W Q lower trapezoidal on
 // its rows in order of falling norm, so that the one-sided Jacobi that follows runs on the
 // columns of a triangular factor whose rows are graded.
 //
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(LT) k_lq(LqParams<T> P) {
 
 // Transposed copies between the column-major work / rotation matrices and the vectors X, in 32 x 32
 // tiles through shared memory: rows of W (store == 0: X <- W, else W <- X) and the rotation's rows
-// (store == 0: X <- identity, or rot with from_rot; else rot <- X).
+// (store == 0: X <- identity; else rot <- X).
 template <class T>
 __global__ void __launch_bounds__(256) k_lq_move(T *__restrict__ work, T *__restrict__ rot, T *__restrict__ x,
                                                  const LqSec *__restrict__ secs, int store) {
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(256) k_lq_move(T *__restrict__ work, T *__rest
                 tile[i][tx] = r < rows && c < s.q ? v[int64_t(r) * s.q + c] : T(0);
             } else {
                 const int r = r0 + tx, c = c0 + i;
-                tile[tx][i] = r < rows && c < s.q ? (w || s.from_rot ? m[int64_t(c) * rows + r] : (r == c ? T(1) : T(0))) : T(0);
+                tile[tx][i] = r < rows && c < s.q ? (w ? m[int64_t(c) * rows + r] : (r == c ? T(1) : T(0))) : T(0);
             }
         }
         __syncthreads();
