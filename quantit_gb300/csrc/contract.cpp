@@ -680,6 +680,7 @@ void contract_f64(const ContractPlan &P, const BT &A, const BT &B, BT &out, cons
     g.Cadd = add ? static_cast<const double *>(add->data()) : nullptr;
     upload_many({table(pairs, g.pairs), table(outs, g.outs), table(tiles, g.tiles)});
     g.ntiles = int32_t(tiles.size());
+    g.b_strided = !pb && !P.freeB.empty() && P.freeB.back() != B.rank - 1 ? 1 : 0;
     g.alpha = alpha;
     g.beta = beta;
     StatScope sc(ST_GEMM, flops);

@@ -11,7 +11,7 @@
 //  * Operands are read where they lie, through L1, with no shared-memory staging: a
 //    2 x 2 register tile needs 4 loads for 64 clocks of FMA.  That leaves no CTA
 //    barrier in the loop, no padding of K, and any leg order whose free and contracted
-//    legs each fold to two strides needs no packed copy of the operand first.
+//    legs each fold to two strides needs no packed copy of the operand first (f64_square: warps of either shape).
 //  * The tile follows the block: 32 x 32, 16 x 16 where that leaves SMs idle or most of
 //    the tile outside the block, and 256 x 8 / 8 x 256 strips for the thin products of
 //    an MPO tensor (N or M of a few, K of a few), which are bound by memory.
@@ -44,11 +44,16 @@ __device__ __forceinline__ void store_out(const F64Args &g, const GemmOut &o, in
     g.C[o.c_off + idx] = v;
 }
 
-// A square tile: RT x RT outputs per thread, 16 x 16 threads.
+// A square tile: RT x RT outputs per thread, 16 x 16 threads.  A warp covers 2 rows x 16 columns, whose loads of B are one
+// line, or 8 x 4 where B's columns are strided (its last leg is contracted) and every one of them is a line of its own:
+// 12 instead of 18 lines a k where a warp's FMA takes 16 clocks.  M = N = K = 576 722 -> 366 us, 600 x 600 x 4000 5639 ->
+// 2670; with 8 x 4 for contiguous columns too the lines would be 9 instead of 3.
 template <int RT, int U>
 __device__ __forceinline__ void f64_square(const F64Args &g, const GemmTile &t, const GemmOut &o, F64Pair *sp) {
     constexpr int RM = RT, RN = RT, TX = 16, TY = 16;
-    const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+    const int tid = threadIdx.x;
+    const int tx = g.b_strided ? (tid & 3) | (tid >> 3 & 12) : tid % TX;
+    const int ty = g.b_strided ? (tid >> 2 & 7) | (tid >> 4 & 8) : tid / TX;
     // rows / columns of the register tile that the block reaches (the same for every thread)
     const int rm = min(RM, (o.M - t.m0 + TY - 1) / TY), rn = min(RN, (o.N - t.n0 + TX - 1) / TX);
     int m[RM], n[RN];

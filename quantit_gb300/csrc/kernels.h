@@ -65,6 +65,7 @@ struct F64Args {
     const GemmOut *outs;
     const GemmTile *tiles;
     int32_t ntiles;
+    int32_t b_strided;  // B's columns are not contiguous: square warps (f64_square)
     double alpha, beta;
 };
 enum : int32_t { F64_SQUARE = 0, F64_SMALL = 1, F64_TALL = 2, F64_WIDE = 3 };
