@@ -656,13 +656,13 @@ void contract_f64(const ContractPlan &P, const BT &A, const BT &B, BT &out, cons
             p.bk2 = int32_t(P.b_mode == 1 ? 1 : N);
         }
     }
-    // 32 x 32 tiles unless they would leave most SMs without one
-    auto square_tiles = [&]() {
-        int64_t n = 0;
-        for (const GemmOut &o : outs) n += ((int64_t(o.M) + 31) / 32) * ((int64_t(o.N) + 31) / 32);
-        return n;
-    };
-    const bool fine = square_tiles() < 4 * device_sm_count();
+    int64_t squares = 0;
+    double area = 0;
+    for (const GemmOut &o : outs) {
+        squares += ((int64_t(o.M) + 31) / 32) * ((int64_t(o.N) + 31) / 32);
+        area += double(o.M) * double(o.N);
+    }
+    const bool fine = gemm_f64_fine(squares, flops / (2.0 * std::max(area, 1.0)));
     std::vector<GemmTile> tiles;
     for (int32_t o : longest_first(outs, Ks)) {
         int64_t kmax = 0;

@@ -12,12 +12,12 @@
 //    2 x 2 register tile needs 4 loads for 64 clocks of FMA.  That leaves no CTA
 //    barrier in the loop, no padding of K, and any leg order whose free and contracted
 //    legs each fold to two strides needs no packed copy of the operand first (f64_square: warps of either shape).
-//  * The tile follows the block: 32 x 32, 16 x 16 where that leaves SMs idle or most of
+//  * The tile follows the block: 32 x 32, 16 x 16 where that leaves SMs idle (gemm_f64_fine) or most of
 //    the tile outside the block, and 256 x 8 / 8 x 256 strips for the thin products of
 //    an MPO tensor (N or M of a few, K of a few), which are bound by memory.
 // Against 64 x 64 x 16 tiles staged in shared memory (17 us of FP64 pipe for any tile,
 // however small the block), same sums to the last bit: theta pair contraction at D = 2048
-// 1787 -> 1303 us (0.98 TFLOP/s, 82% of what independent FMAs reach; mma.sync FP64 runs on the same pipe at
+// 1787 -> 1192 us (1.07 TFLOP/s, 89% of what independent FMAs reach; mma.sync FP64 runs on the same pipe at
 // 1.05 against their 1.20 TFLOP/s); the matvec of a Hubbard chain at D = 512 2584 -> 771 us, of which its kernels
 // take 124 and the host's planning the rest; an environment update of a spin chain at D = 777
 // 1271 -> 315 us; a 24-dimensional site pair 34 -> 15 us.
@@ -216,6 +216,16 @@ __global__ void __launch_bounds__(THREADS, 3) k_gemm_f64(F64Args g) {
     }
 }
 }  // namespace
+
+// 16 x 16 tiles take as long per FMA as 32 x 32 ones (the FP64 pipe is busy either way) and share out more evenly
+// over three CTAs an SM, until the lines that they load four times as often are what counts.  32 x 32 and 16 x 16,
+// us: M = N = K = 800 1045, 914; 1000 2298, 1781; 1700 8988, 8296; 2200 18244, 17714 (4761 tiles); 3000 44636,
+// 45546; 3500 71090, 74046; 3000 x 300 x 2000 4541, 3116; an environment of the cylinder at D = 1024 (4974 tiles, K
+// ~136) 2364, 2482.  Short sums store more than they load: 1400 x 1400 x 64 272, 282; the matvec of a cylinder at D = 512
+// 752, 784.
+bool gemm_f64_fine(int64_t square_tiles, double mean_k) {
+    return square_tiles < 4 * device_sm_count() || (square_tiles < 30 * device_sm_count() && mean_k >= 128.0);
+}
 
 int gemm_f64_class(int64_t M, int64_t N, int64_t K, int *tm, int *tn, bool fine) {
     // (a strip's short-side offsets are 32-bit)

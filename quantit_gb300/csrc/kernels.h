@@ -72,7 +72,8 @@ enum : int32_t { F64_SQUARE = 0, F64_SMALL = 1, F64_TALL = 2, F64_WIDE = 3 };
 constexpr int F64_STRIP = 8;  // rows or columns of the short side of a strip
 // The tile class of an M x N output block (K: the longest contracted length of its pairs)
 // and its tile extents; fine: 16 x 16 instead of 32 x 32 tiles (too few of the latter to
-// occupy the SMs).
+// occupy the SMs evenly: gemm_f64_fine, of the number of 32 x 32 tiles and the mean contracted length).
+bool gemm_f64_fine(int64_t square_tiles, double mean_k);
 int gemm_f64_class(int64_t M, int64_t N, int64_t K, int *tm, int *tn, bool fine);
 void launch_gemm_f64(const F64Args &a);
 

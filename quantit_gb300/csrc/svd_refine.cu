@@ -140,8 +140,13 @@ void products(const double *A, const double *B, double *C, const std::vector<Pro
     std::vector<GemmOut> outs;
     std::vector<GemmTile> tiles;
     int64_t square = 0;
-    for (const Product &t : tasks) square += ((int64_t(t.M) + 31) / 32) * ((int64_t(t.N) + 31) / 32);
-    const bool fine = square < 4 * device_sm_count();
+    double area = 0, volume = 0;
+    for (const Product &t : tasks) {
+        square += ((int64_t(t.M) + 31) / 32) * ((int64_t(t.N) + 31) / 32);
+        area += double(t.M) * t.N;
+        volume += double(t.M) * t.N * t.K;
+    }
+    const bool fine = gemm_f64_fine(square, volume / std::max(area, 1.0));
     for (const Product &t : tasks) {
         if (t.M <= 0 || t.N <= 0 || t.K <= 0) continue;
         F64Pair p{};
