@@ -678,7 +678,7 @@ void contract_f64(const ContractPlan &P, const BT &A, const BT &B, BT &out, cons
     g.B = Bp;
     g.C = static_cast<double *>(out.data());
     g.Cadd = add ? static_cast<const double *>(add->data()) : nullptr;
-    upload_many({table(pairs, g.pairs), table(outs, g.outs), table(tiles, g.tiles)});
+    const BufPtr tables = upload_many({table(pairs, g.pairs), table(outs, g.outs), table(tiles, g.tiles)});
     g.ntiles = int32_t(tiles.size());
     g.b_strided = !pb && !P.freeB.empty() && P.freeB.back() != B.rank - 1 ? 1 : 0;
     g.alpha = alpha;
@@ -789,11 +789,12 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
             g.amax_out = static_cast<unsigned long long *>(c_max->buf->p);
         }
     }
+    BufPtr tables;
     {
         StatScope sc(ST_PACK, (mode == GEMM_BF16X3 ? 14.0 : 16.0) * double(A.nnz + B.nnz));
         launch_amax(am);
-        upload_many({table(ents, sa.ents), table(stiles, sa.tiles), table(pairs, g.pairs), table(outs, g.outs),
-                     table(tiles, g.tiles)});
+        tables = upload_many({table(ents, sa.ents), table(stiles, sa.tiles), table(pairs, g.pairs), table(outs, g.outs),
+                              table(tiles, g.tiles)});
         bool flat = true;
         for (const SplitEntry &e : ents) flat = flat && e.folded && e.rd2 >= e.rows && e.kd2 >= e.K;
         launch_split(sa, int64_t(stiles.size()), mode, flat);

@@ -364,7 +364,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     const PackEntry *dpe = nullptr;
     const Chunk *dch = nullptr;
     const int *dslots = nullptr;
-    upload_many({table(D.desc, desc_table), table(pe, dpe), table(chunks, dch), table(slots, dslots)});
+    const BufPtr tables = upload_many({table(D.desc, desc_table), table(pe, dpe), table(chunks, dch), table(slots, dslots)});
     SectorDesc *dsec = const_cast<SectorDesc *>(desc_table);  // (eigh writes its shifts there)
     // FP32 sectors are packed at magnitude 1; what the host reads of them is scaled back
     BufPtr amax_buf;
@@ -704,7 +704,7 @@ struct Scatter {
             const std::vector<Chunk> part(chunks.begin() + first, chunks.begin() + std::min(chunks.size(), first + kChunks));
             const ScatterEntry *e = nullptr;
             const Chunk *c = nullptr;
-            upload_many({table(ents, e), table(part, c)});
+            const BufPtr tables = upload_many({table(ents, e), table(part, c)});
             launch_scatter(e, c, int64_t(part.size()));
         }
     }

@@ -356,12 +356,8 @@ int plan_join_device(ContractPlan &P, const BT &A, const BT &B, int *bad_dim, bo
         }
     a.nchk = int(ca.size());
     a.g = A.g;
-    a.abidx = upload_vec(ab);
-    a.bbidx = upload_vec(bb);
-    a.chkA = upload_vec(ca);
-    a.chkB = upload_vec(cb);
-    a.chkSzA = upload_vec(za);
-    a.chkSzB = upload_vec(zb);
+    const BufPtr tables = upload_many({table(ab, a.abidx), table(bb, a.bbidx), table(ca, a.chkA), table(cb, a.chkB),
+                                       table(za, a.chkSzA), table(zb, a.chkSzB)});
     const int64_t nmax = std::max(nA, nB);
     int64_t cap = std::max<int64_t>(4096, 4 * (nA + nB));
     Ctx &c = ctx();

@@ -181,6 +181,12 @@ struct Ctx {
     cudaEvent_t half_done[2] = {nullptr, nullptr};
     int cur_half = 0;
     bool half_used[2] = {false, false};
+    // pinned buffers through which larger tables go to device buffers of their own (upload_many; made when first needed)
+    struct Stage {
+        char *host = nullptr;
+        cudaEvent_t done = nullptr;
+    } stage[2];
+    int cur_stage = 0;
     // error word of this thread's tensor-core launches (bounded waits that expired)
     int *tc_err = nullptr;
     bool tc_used = false;
@@ -195,13 +201,16 @@ BufPtr dev_alloc(size_t bytes);
 // Copy a host table to device memory valid for work issued afterwards on the
 // current stream (ring-buffered; the region is reused after the stream passes it).
 void *upload(const void *host, size_t bytes);
-// Several tables in one copy; each device pointer lands in *dev (null for an empty table).
+// Several tables in one copy; each device pointer lands in *dev (null for an empty table).  Together they go to the
+// ring, or, above a sixteenth of it, to a buffer of their own, which is returned: keep it until the last launch that
+// reads the tables (it is freed in stream order).  So tables of any size fit, and no call takes so much of
+// the ring that the tables of an operation before its launch, or those it keeps over several launches, are overwritten.
 struct HostTable {
     const void *host;
     size_t bytes;
     const void **dev;
 };
-void upload_many(std::initializer_list<HostTable> tables);
+[[nodiscard]] BufPtr upload_many(std::initializer_list<HostTable> tables);
 template <class T>
 HostTable table(const std::vector<T> &v, const T *&dev) {
     return HostTable{v.data(), v.size() * sizeof(T), reinterpret_cast<const void **>(&dev)};

@@ -18,6 +18,7 @@ std::mutex g_ctx_mu;
 std::vector<Ctx *> g_ctxs;  // leaked on purpose: contexts live until process exit
 
 constexpr size_t RING_BYTES = size_t(64) << 20;
+constexpr size_t STAGE_BYTES = size_t(8) << 20;  // one of the two pinned buffers of the tables that have a buffer of their own
 
 void init_ring(Ctx &c) {
     if (c.host_ring) return;
@@ -77,9 +78,28 @@ BufPtr dev_alloc(size_t bytes) {
     return b;
 }
 
-void upload_many(std::initializer_list<HostTable> tables) {
+namespace {
+size_t padded(size_t n) { return (n + 255) & ~size_t(255); }
+
+// Offset of `need` bytes (at most half) in the ring, free to be written by the host.
+size_t ring_take(Ctx &c, size_t need) {
+    const size_t half = c.ring_bytes / 2;
+    if (c.ring_pos + need > (c.cur_half + 1) * half) {
+        // leave the current half: mark where the stream is, then enter the other half
+        cuda_check(cudaEventRecord(c.half_done[c.cur_half], c.stream), "cudaEventRecord");
+        c.half_used[c.cur_half] = true;
+        c.cur_half ^= 1;
+        if (c.half_used[c.cur_half]) cuda_check(cudaEventSynchronize(c.half_done[c.cur_half]), "cudaEventSync");
+        c.ring_pos = c.cur_half * half;
+    }
+    const size_t at = c.ring_pos;
+    c.ring_pos += need;
+    return at;
+}
+}  // namespace
+
+BufPtr upload_many(std::initializer_list<HostTable> tables) {
     Ctx &c = ctx();
-    auto padded = [](size_t n) { return (n + 255) & ~size_t(255); };
     size_t need = 0;
     for (const HostTable &t : tables) need += padded(t.bytes);
     char *d = nullptr, *h = nullptr;
@@ -94,24 +114,46 @@ void upload_many(std::initializer_list<HostTable> tables) {
         d = static_cast<char *>(p);
         staged.resize(need);
         h = staged.data();
+    } else if (need > c.ring_bytes / 16) {
+        // piece by piece through two pinned buffers of their own: the ring does not move on
+        BufPtr own = dev_alloc(need);
+        d = static_cast<char *>(own->p);
+        Ctx::Stage *s = nullptr;
+        size_t at = 0, sent = 0, fill = 0;  // this table, bytes copied to the device, bytes in the open buffer
+        auto send = [&] {
+            if (!fill) return;
+            cuda_check(cudaMemcpyAsync(d + sent, s->host, fill, cudaMemcpyHostToDevice, c.stream), "cudaMemcpyAsync(plan)");
+            cuda_check(cudaEventRecord(s->done, c.stream), "cudaEventRecord");
+            sent += fill;
+            fill = 0;
+        };
+        for (const HostTable &t : tables) {
+            *t.dev = t.bytes ? d + at : nullptr;
+            at += padded(t.bytes);
+            for (size_t done = 0; done < t.bytes;) {
+                if (!fill) {
+                    s = &c.stage[c.cur_stage ^= 1];
+                    if (!s->host) {
+                        cuda_check(cudaMallocHost(&s->host, STAGE_BYTES), "cudaMallocHost(table staging)");
+                        cuda_check(cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming), "cudaEventCreate");
+                    } else {
+                        cuda_check(cudaEventSynchronize(s->done), "cudaEventSync");
+                    }
+                }
+                const size_t n = std::min(t.bytes - done, STAGE_BYTES - fill);
+                std::memcpy(s->host + fill, static_cast<const char *>(t.host) + done, n);
+                done += n;
+                fill += n;
+                if (done == t.bytes) fill = at - sent;  // with the gap behind the table (both ends are multiples of 256)
+                if (fill == STAGE_BYTES) send();
+            }
+        }
+        send();
+        return own;
     } else {
-        if (need > c.ring_bytes / 2) {
-            if (tables.size() == 1) fail(ERR_RUNTIME, "planning table larger than the staging ring");
-            for (const HostTable &t : tables) upload_many({t});
-            return;
-        }
-        const size_t half = c.ring_bytes / 2;
-        if (c.ring_pos + need > (c.cur_half + 1) * half) {
-            // leave the current half: mark where the stream is, then enter the other half
-            cuda_check(cudaEventRecord(c.half_done[c.cur_half], c.stream), "cudaEventRecord");
-            c.half_used[c.cur_half] = true;
-            c.cur_half ^= 1;
-            if (c.half_used[c.cur_half]) cuda_check(cudaEventSynchronize(c.half_done[c.cur_half]), "cudaEventSync");
-            c.ring_pos = c.cur_half * half;
-        }
-        d = c.dev_ring + c.ring_pos;
-        h = c.host_ring + c.ring_pos;
-        c.ring_pos += need;
+        const size_t at = ring_take(c, need);
+        d = c.dev_ring + at;
+        h = c.host_ring + at;
     }
     size_t at = 0;
     for (const HostTable &t : tables) {
@@ -119,17 +161,28 @@ void upload_many(std::initializer_list<HostTable> tables) {
         if (t.bytes) std::memcpy(h + at, t.host, t.bytes);
         at += padded(t.bytes);
     }
-    if (need == 0) return;
+    if (need == 0) return nullptr;
     if (c.capturing)
         cuda_check(cudaMemcpy(d, h, need, cudaMemcpyHostToDevice), "cudaMemcpy(graph table)");
     else
         cuda_check(cudaMemcpyAsync(d, h, need, cudaMemcpyHostToDevice, c.stream), "cudaMemcpyAsync(plan)");
+    return nullptr;
 }
 
 void *upload(const void *host, size_t bytes) {
-    const void *d = nullptr;
-    upload_many({HostTable{host, bytes, &d}});
-    return const_cast<void *>(d);
+    Ctx &c = ctx();
+    if (c.capturing) {
+        const void *d = nullptr;
+        const BufPtr own = upload_many({HostTable{host, bytes, &d}});  // (null: a graph's tables are kept with it)
+        return const_cast<void *>(d);
+    }
+    const size_t need = padded(bytes);
+    if (need > c.ring_bytes / 2) fail(ERR_RUNTIME, "planning table larger than the staging ring");
+    const size_t at = ring_take(c, need);
+    std::memcpy(c.host_ring + at, host, bytes);
+    cuda_check(cudaMemcpyAsync(c.dev_ring + at, c.host_ring + at, bytes, cudaMemcpyHostToDevice, c.stream),
+               "cudaMemcpyAsync(plan)");
+    return c.dev_ring + at;
 }
 
 // ---------------------------------------------------------------- statistics

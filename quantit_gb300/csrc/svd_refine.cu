@@ -187,7 +187,7 @@ void products(const double *A, const double *B, double *C, const std::vector<Pro
     g.B = A;
     g.C = C;
     g.Cadd = nullptr;
-    upload_many({table(pairs, g.pairs), table(outs, g.outs), table(tiles, g.tiles)});
+    const BufPtr tables = upload_many({table(pairs, g.pairs), table(outs, g.outs), table(tiles, g.tiles)});
     g.ntiles = int32_t(tiles.size());
     g.b_strided = tasks.front().a_trans ? 1 : 0;
     g.alpha = 1.0;
