@@ -267,9 +267,13 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                          : trunc_hint().active           ? (svd_deflation() ? 16 : INT32_MAX)
                                                          : (split_mode ? INT32_MAX : 48);
     auto lq_fits = [&](const SectorDesc &d, int prec32) { return d.q >= lq_least && d.q <= lq_max_q(prec32, nsec); };
-    // A decomposition that is run again because its estimated truncation fell short is FP64
-    // throughout, if the factorisation speeds its FP64 sweeps up.
-    const bool redo = trunc_hint().active && !trunc_hint().allow_discard && max_q >= lq_least;
+    // Whether factored FP64 sweeps stand ready: not if a sector is too wide for the FP64 factorisation (about 1590
+    // columns).  Its FP64 sweeps start from the refined FP32 rotation as without factorisation, or they would
+    // start from the identity.
+    bool lq64_ready = max_q >= lq_least;
+    for (const SectorDesc &d : D.desc) lq64_ready = lq64_ready && (d.q < lq_least || lq_fits(d, 0));
+    // A decomposition that is run again because its estimated truncation fell short is FP64 throughout then.
+    const bool redo = trunc_hint().active && !trunc_hint().allow_discard && lq64_ready;
     const int f32 = (mode == 0 && split_mode && !redo) ? 1 : 0;
     const size_t es = f32 ? 4 : 8;
     D.work = dev_alloc(size_t(std::max<int64_t>(wtot, 1)) * es);
@@ -476,11 +480,11 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                 any = any || here;
                 clears = clears && here;
             }
-            if (lq.empty() ? any : clears)
+            if (lq64_ready ? clears : any)
                 th.discard_tau = std::max(th.discard_tau, tau);
             else
                 discard.clear();
-            resolve_anew = discard.empty() && !lq.empty();
+            resolve_anew = discard.empty() && lq64_ready;
         }
         if (f32) {
             StatScope sc64(ST_SVD64, 0.0);
