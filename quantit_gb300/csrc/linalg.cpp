@@ -457,18 +457,21 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             for (int i = 0; i < nsec; ++i)
                 for (int j = 0; j < D.desc[i].q; ++j) {
                     const size_t at = size_t(D.desc[i].s_off + j);
-                    vals[at] = std::ldexp(std::sqrt(std::max(n2[at], 0.0)), sector_exponent(top[i]));
+                    vals[at] = std::ldexp(std::sqrt(std::max(0.0, n2[at])), sector_exponent(top[i]));  // (NaN: 0)
                 }
-            std::sort(vals.begin(), vals.end(), std::greater<double>());
-            const double t_est = kept_threshold(vals, th.tol, th.pw, th.min_size, th.max_size);
+            std::vector<double> sorted = vals;
+            std::sort(sorted.begin(), sorted.end(), std::greater<double>());
+            const double t_est = kept_threshold(sorted, th.tol, th.pw, th.min_size, th.max_size);
             discard.assign(nsec, 0.0);
             null2.assign(nsec, 0.0);
-            // Where factored FP64 sweeps stand ready, the level has to clear FP32's resolution in every
-            // sector: the noise of one that it does not clear is among the values the threshold was
-            // estimated from (estimates from such noise had the decomposition run twice: D = 600, 14
-            // decades 31.8 ms, FP64 alone 12.8).  Otherwise each sector that it clears discards.
+            // Each sector whose FP32 resolution the level clears discards; the others resolve every column.  Where
+            // factored FP64 sweeps stand ready, though, a sector that is not cleared may have no column below its
+            // resolution: those are noise or deflated, the threshold was estimated from them (D = 600, 14 decades: the
+            // decomposition ran twice, 31.8 ms; FP64 alone 12.8), and the factored sweeps resolve them sooner (D = 2048,
+            // 10 decades: 162 ms against 431).  Without such columns the refined rotation is all but there: four sectors of
+            // 900 columns, 8 decades, beside a stronger one of condition 1e4 98 ms, all anew 282.
             const double tau = 0.5 * t_est;
-            bool clears = t_est > 0.0, any = false;
+            bool sound = t_est > 0.0, any = false;
             for (int i = 0; i < nsec; ++i) {
                 const SectorDesc &d = D.desc[i];
                 double f2 = 0.0;
@@ -478,9 +481,9 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                 const bool here = t_est > 0.0 && tau > 4.0 * kDeflateF32 * norm;
                 discard[i] = here ? tau : 0.0;
                 any = any || here;
-                clears = clears && here;
+                for (int j = 0; j < d.q && !here && sound; ++j) sound = vals[size_t(d.s_off + j)] > 4.0 * kDeflateF32 * norm;
             }
-            if (lq64_ready ? clears : any)
+            if (any && (sound || !lq64_ready))
                 th.discard_tau = std::max(th.discard_tau, tau);
             else
                 discard.clear();
