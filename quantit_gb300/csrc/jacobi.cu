@@ -59,11 +59,11 @@ __device__ __forceinline__ float ldcg(const float *p) { return __ldcg(p); }
 // For small angles c rounds to 1 while 1 - c = s tau does not, so the plain form
 // c x - s y would scale both columns by sqrt(1 + t^2) at every such rotation; in
 // FP32 that bias accumulates to ~1e-5 in the singular values over a few sweeps.
-// In FP64 the block kernel rotates columns of more than 128 rows by the same rotation as three shears, x -= tau y, y += s x,
-// x -= tau y: three instead of four instructions of GB300's narrow FP64 pipe per element pair.  A third
-// dependent rounding makes the values' error ~1.2 times that of the form above, which LQ's fewer sweeps more
-// than win back; shorter columns, which mostly run without LQ, keep the form above (eigh D = 300: 4 % more
-// time for the four instructions).
+// In FP64 the same rotation is also three shears, x -= tau y, y += s x, x -= tau y: three instead of four instructions of
+// GB300's narrow FP64 pipe per element pair.  A third dependent rounding makes the error of U d V^T about 1.15 times that
+// of the form above.  So the block kernel takes it only under a truncation, in sectors that its LQ factorisation spares more
+// sweeps than that (error 0.5 to 0.95 of the plain sweeps' with either form; svd D = 600 11.0 ms, with four instructions
+// 11.6), and only for columns of more than 128 rows.
 template <class T, bool FOUR = true>
 __device__ __forceinline__ void rot_apply(T &x, T &y, T s, T tau) {
     if constexpr (sizeof(T) == 8 && !FOUR) {
@@ -458,6 +458,7 @@ struct BJacobiParams {
     const T *defl; // per sector: squared-norm deflation threshold (null: no deflation)
     T *dnorm;      // per column (s_off + column): squared norm when deflated, 0 otherwise
     const T *skip; // per sector (null: none): squared discard level of pair_skipped
+    int shear_q;   // sectors of at least so many columns rotate by three shears (FP64, columns of more than 128 rows)
 };
 
 __device__ __forceinline__ int bj_items(int q, int B) {
@@ -723,7 +724,7 @@ __device__ __forceinline__ bool norm_kept(double a2, double al) {
 // EXACT: the plain formulas in FP64 too (launch_jacobi's `exact`).
 template <class T, int R, bool EXACT>
 __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], bool full, T &al, T &be, T tol, T thr, T &sn, T &tau, T &dx,
-                                          T &dy, T skip, float &rmax) {
+                                          T &dy, T skip, float &rmax, bool shears) {
     if (al == T(0) || be == T(0)) return false;
     if (pair_skipped(al, be, skip)) return false;
     T ga, t, a2, b2;
@@ -762,7 +763,12 @@ __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], bool full, T &al
     bool whole = true;
     if constexpr (sizeof(T) == 8 && !EXACT) whole = !unit_cosine(sn);
     if (whole) {
-        bj_each<T, R>(full, [&](int i) { rot_apply<T, EXACT || R <= 4>(x[i], y[i], sn, tau); });
+        bool four = true;
+        if constexpr (sizeof(T) == 8 && !EXACT && R > 4) four = !shears;
+        if (four)
+            bj_each<T, R>(full, [&](int i) { rot_apply<T, true>(x[i], y[i], sn, tau); });
+        else
+            bj_each<T, R>(full, [&](int i) { rot_apply<T, false>(x[i], y[i], sn, tau); });
     } else {
         bj_each<T, R>(full, [&](int i) {
             x[i] = fma(-sn, y[i], x[i]);
@@ -915,14 +921,23 @@ __device__ __forceinline__ void bj_apply_rots(T *V, int q, int bs, int a, int b,
     }
 }
 
+// (not inlined: the second form of a kernel that mostly runs the other)
+template <class T, int B, bool EVEN>
+__device__ __noinline__ void bj_apply_rots4(T *V, int q, int a, int b, int na, int nbc, bool intra, int roff, int r0, int r1,
+                                            int tid) {
+    bj_apply_rots<T, B, true, EVEN>(V, q, bj_width<B, EVEN>(q), a, b, na, nbc, intra, roff, r0, r1, tid);
+}
+
 // The V update of a block pair in whichever form Qs holds it.
 template <class T, int B, bool LIST, bool FOUR, bool EVEN>
 __device__ __forceinline__ void bj_update_v(T *V, int q, int a, int b, int na, int nbc, bool intra, const T *Qs, int roff,
-                                            int r0, int r1, int tid) {
-    if constexpr (LIST)
+                                            int r0, int r1, int tid, bool shears) {
+    if constexpr (!LIST)
+        bj_apply_v<T, B>(V, q, a, b, na, nbc, Qs, r0, r1, tid);
+    else if (FOUR || shears)
         bj_apply_rots<T, B, FOUR, EVEN>(V, q, bj_width<B, EVEN>(q), a, b, na, nbc, intra, roff, r0, r1, tid);
     else
-        bj_apply_v<T, B>(V, q, a, b, na, nbc, Qs, r0, r1, tid);
+        bj_apply_rots4<T, B, EVEN>(V, q, a, b, na, nbc, intra, roff, r0, r1, tid);
 }
 
 // The deferred V updates of step `st`: CTAs claim (job, row chunk) units from a
@@ -949,7 +964,7 @@ __device__ void bj_vwork(const BJacobiParams<T> &P, int64_t st, T *Qs, int roff,
         for (int e = tid; e < NP * NP; e += NT) Qs[e] = ldcg(qsrc + e);
         __syncthreads();
         bj_update_v<T, B, LIST, FOUR, EVEN>(P.rot + sd.rot_off, sd.q, a, b, nn & 0xFF, (nn >> 8) & 0xFF, nn >> 16, Qs, roff, r0,
-                                      min(sd.q, r0 + NT), tid);
+                                      min(sd.q, r0 + NT), tid, sd.q >= P.shear_q);
         __syncthreads();
     }
 }
@@ -1053,6 +1068,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
             const bool full = EXACT || p > 32 * bj_half<T, R>();
             const T thr = P.defl ? P.defl[s] : T(0);
             const T skp = P.skip ? P.skip[s] : T(0);
+            const bool shears = q >= P.shear_q;
             bool zeroed = false;
 
             for (int j = warp; j < NP; j += B) {
@@ -1107,7 +1123,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                         bj_load(x, cols + u * PP, lane, full);
                         bj_load(y, cols + v * PP, lane, full);
                         T al = nrm[u], be = nrm[v], dx = T(0), dy = T(0);
-                        if (bj_rotate<T, R, EXACT>(x, y, full, al, be, tol, thr, sn, tau, dx, dy, skp, rmax)) {
+                        if (bj_rotate<T, R, EXACT>(x, y, full, al, be, tol, thr, sn, tau, dx, dy, skp, rmax, shears)) {
                             if (lane == 0 && dx > T(0)) P.dnorm[sd.s_off + column(u)] = dx;
                             if (lane == 0 && dy > T(0)) P.dnorm[sd.s_off + column(v)] = dy;
                             bj_store(x, cols + u * PP, lane, full);
@@ -1150,7 +1166,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                     if (mine && valid(j)) {
                         bj_load(y, cols + j * PP, lane, full);
                         T be = nrm[j], dx = T(0), dy = T(0);
-                        if (bj_rotate<T, R, EXACT>(x, y, full, al, be, tol, thr, sn, tau, dx, dy, skp, rmax)) {
+                        if (bj_rotate<T, R, EXACT>(x, y, full, al, be, tol, thr, sn, tau, dx, dy, skp, rmax, shears)) {
                             if (lane == 0 && dx > T(0)) P.dnorm[sd.s_off + column(warp)] = dx;
                             if (lane == 0 && dy > T(0)) P.dnorm[sd.s_off + column(j)] = dy;
                             bj_store(y, cols + j * PP, lane, full);
@@ -1204,7 +1220,7 @@ __global__ void __launch_bounds__(B * 32) k_bjacobi(BJacobiParams<T> P) {
                         jr[3] = na | (nbc << 8) | ((k == 0) << 16);
                     }
                 } else {
-                    bj_update_v<T, B, LIST, FOUR, EVEN>(V, q, a, b, na, nbc, k == 0, Qs, roff, 0, q, tid);
+                    bj_update_v<T, B, LIST, FOUR, EVEN>(V, q, a, b, na, nbc, k == 0, Qs, roff, 0, q, tid, shears);
                 }
                 if (tid == 0) atomicMax(P.rotated + int64_t(s) * P.max_sweeps + sweep[s], s_rmax);
             }
@@ -1704,7 +1720,8 @@ void tune_save(const TuneKey &k, int w) {
 template <class T>
 void jacobi_impl(T *work, T *rot, const SectorDesc *sec, const int *slot_start, int nsec, int max_steps_per_sweep,
                  int max_sweeps, int *sweeps_out, int *flags, int max_p, int64_t sum_q, void *vwork, size_t vwork_bytes,
-                 const T *defl, T *dnorm, cudaStream_t stream, bool tune, const T *skip, bool exact) {
+                 const T *defl, T *dnorm, cudaStream_t stream, bool tune, const T *skip, bool exact,
+                 int shear_q) {
     if (nsec > 12 * 1024) fail(ERR_INVALID_ARGUMENT, "too many sectors for one decomposition launch");
     const size_t smem = size_t(2 * nsec) * sizeof(int);
     cuda_check(cudaMemsetAsync(flags, 0, size_t(nsec) * max_sweeps * sizeof(int), stream), "memset flags");
@@ -1721,6 +1738,7 @@ void jacobi_impl(T *work, T *rot, const SectorDesc *sec, const int *slot_start, 
         B.defl = defl;
         B.dnorm = dnorm;
         B.skip = skip;
+        B.shear_q = shear_q;
         B.max_q = max_steps_per_sweep + 1;  // the widest sector's even column count bounds q
         const bool f32 = sizeof(T) == 4;
         const int ex = exact && !f32 ? exact_r_class(max_p) : 0, R = ex ? ex : r_class(max_p, f32);
@@ -1856,27 +1874,27 @@ void launch_eigh_prepare(void *work, SectorDesc *sec, int nsec, int upper, int f
 void launch_jacobi_on(cudaStream_t stream, void *work, void *rot, const SectorDesc *sec, const int *slot_start,
                       int nsec, int max_steps_per_sweep, int max_sweeps, int *sweeps_out, int *flags, int f32,
                       int max_p, int64_t sum_q, void *vwork, size_t vwork_bytes, const void *defl, void *dnorm,
-                      bool tune, const void *skip, bool exact) {
+                      bool tune, const void *skip, bool exact, int shear_q) {
     if (nsec <= 0) return;
     if ((defl == nullptr) != (dnorm == nullptr)) fail(ERR_INVALID_ARGUMENT, "deflation needs thresholds and norms");
     if (f32)
         jacobi_impl(static_cast<float *>(work), static_cast<float *>(rot), sec, slot_start, nsec, max_steps_per_sweep,
                     max_sweeps, sweeps_out, flags, max_p, sum_q, vwork, vwork_bytes,
                     static_cast<const float *>(defl), static_cast<float *>(dnorm), stream, tune,
-                    static_cast<const float *>(skip), false);
+                    static_cast<const float *>(skip), false, INT32_MAX);
     else
         jacobi_impl(static_cast<double *>(work), static_cast<double *>(rot), sec, slot_start, nsec,
                     max_steps_per_sweep, max_sweeps, sweeps_out, flags, max_p, sum_q, vwork, vwork_bytes,
                     static_cast<const double *>(defl), static_cast<double *>(dnorm), stream, tune,
-                    static_cast<const double *>(skip), exact);
+                    static_cast<const double *>(skip), exact, shear_q);
 }
 
 void launch_jacobi(void *work, void *rot, const SectorDesc *sec, const int *slot_start, int nsec,
                    int max_steps_per_sweep, int max_sweeps, int *sweeps_out, int *flags, int f32, int max_p,
                    int64_t sum_q, void *vwork, size_t vwork_bytes, const void *defl, void *dnorm, const void *skip,
-                   bool exact) {
+                   bool exact, int shear_q) {
     launch_jacobi_on(ctx().stream, work, rot, sec, slot_start, nsec, max_steps_per_sweep, max_sweeps, sweeps_out, flags,
-                     f32, max_p, sum_q, vwork, vwork_bytes, defl, dnorm, true, skip, exact);
+                     f32, max_p, sum_q, vwork, vwork_bytes, defl, dnorm, true, skip, exact, shear_q);
 }
 
 void launch_warm_apply(void *work, void *rot, void *tmp, const WarmDesc *wd, int nwarm, int ntiles, int f32) {

@@ -267,10 +267,11 @@ void launch_eigh_prepare(void *work, SectorDesc *sec, int nsec, int upper, int f
 // the basis of equal singular values is that of the plain formulas; otherwise from FP32.
 // skip (optional, the work type): per sector, a pair whose squared column norms are both
 // below it is not rotated (columns the caller will discard).
+// shear_q: FP64 sectors of at least so many columns may rotate by three shears (see rot_apply).
 void launch_jacobi(void *work, void *rot, const SectorDesc *sec, const int *slot_start, int nsec,
                    int max_steps_per_sweep, int max_sweeps, int *sweeps_out, int *flags, int f32, int max_p,
                    int64_t sum_q, void *vwork = nullptr, size_t vwork_bytes = 0, const void *defl = nullptr,
-                   void *dnorm = nullptr, const void *skip = nullptr, bool exact = false);
+                   void *dnorm = nullptr, const void *skip = nullptr, bool exact = false, int shear_q = INT32_MAX);
 // thr[s] <- delta^2 ||W_s||_F^2 for every svd sector (0 for eigh), in the work type; norms: the
 // squared column norms (launch_col_norms).
 void launch_deflation_thresholds(const double *norms, const SectorDesc *sec, int nsec, double delta, void *thr, int f32);
@@ -297,7 +298,7 @@ void launch_jacobi_on(cudaStream_t stream, void *work, void *rot, const SectorDe
                       int nsec, int max_steps_per_sweep, int max_sweeps, int *sweeps_out, int *flags, int f32,
                       int max_p, int64_t sum_q, void *vwork = nullptr, size_t vwork_bytes = 0,
                       const void *defl = nullptr, void *dnorm = nullptr, bool tune = true,
-                      const void *skip = nullptr, bool exact = false);
+                      const void *skip = nullptr, bool exact = false, int shear_q = INT32_MAX);
 void launch_finish_on(cudaStream_t stream, const void *work, const void *rot, double *U, double *V, double *s,
                       const SectorDesc *sec, int nsec, int max_q, double *scratch, int f32, int complete_cap = -1,
                       const void *dnorm = nullptr, int *dpos = nullptr, int *perm_out = nullptr,

@@ -266,6 +266,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     const int lq_least = mode != 0 || trunc_hint().plain ? INT32_MAX
                          : trunc_hint().active           ? (svd_deflation() ? 16 : INT32_MAX)
                                                          : (split_mode ? INT32_MAX : 48);
+    const int shear_q = trunc_hint().active ? lq_least : INT32_MAX;
     auto lq_fits = [&](const SectorDesc &d, int prec32) { return d.q >= lq_least && d.q <= lq_max_q(prec32, nsec); };
     // Whether factored FP64 sweeps stand ready: not if a sector is too wide for the FP64 factorisation (about 1590
     // columns).  Its FP64 sweeps start from the refined FP32 rotation as without factorisation, or they would
@@ -429,7 +430,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
         launch_lq(W, D.rot->p, lq, f32);
         launch_jacobi(W, D.rot->p, dsec, dslots, nsec, max_steps, max_sweeps, sweeps, flags, f32, max_p, stot,
                       vwork->p, vb, deflate ? thr->p : nullptr, deflate ? dnorm->p : nullptr, nullptr,
-                      trunc_hint().plain);
+                      trunc_hint().plain, shear_q);
         const void *fw = W, *fr = D.rot->p;
         BufPtr w64, w1, va, vbuf, gbuf, ibuf64;
         // The FP32 sweeps resolved every value above FP32 resolution.  When the truncation
@@ -535,7 +536,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             auto fp64_sweeps = [&](int cap_sweeps, const void *thr, const void *skip) {
                 launch_jacobi(w1->p, vbuf->p, dsec64, dslots, nsec, max_steps, cap_sweeps, sw64, sw64 + nsec, 0,
                               max_p, stot, vwork64->p, vb64, deflate ? thr : nullptr, deflate ? dnorm->p : nullptr,
-                              skip, th.plain);
+                              skip, th.plain, shear_q);
             };
             if (discard.empty()) {
                 launch_lq(w1->p, vbuf->p, lq64, 0);
@@ -617,7 +618,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                                "cudaMemsetAsync(compact dnorm)");
                 }
                 launch_jacobi(wk->p, rk->p, ddk, dkslots, nsec, kmax_steps, max_sweeps, sw64, sw64 + nsec, 0, max_p, ks,
-                              vworkk->p, vbk, deflate ? thr64->p : nullptr, deflate ? dnk->p : nullptr, nullptr, th.plain);
+                              vworkk->p, vbk, deflate ? thr64->p : nullptr, deflate ? dnk->p : nullptr, nullptr, th.plain, shear_q);
                 launch_rot_product(static_cast<const double *>(vg->p), static_cast<const double *>(rk->p),
                                    static_cast<double *>(vn->p), rp);
                 launch_col_copy(static_cast<const double *>(wk->p), static_cast<double *>(w1->p), wscatter);
