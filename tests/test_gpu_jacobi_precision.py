@@ -29,3 +29,16 @@ def test_product_of_the_factors(p, n, plain):
         U, d, V = (t.blocks()[0][1] for t in q.linalg.svd(one_sector(a), 1))
         errors.append(np.linalg.norm((U * d) @ V.T - a) / np.linalg.norm(a))
     assert np.mean(errors) <= 1.06 * plain
+
+
+@pytest.mark.parametrize("n,plain", [(150, 2.73e-15), (300, 3.93e-15)])
+def test_eigenvalues(n, plain):
+    """Relative error of the eigenvalues of symmetric matrices, the mean over six (7 % apart from each other)."""
+    errors = []
+    for seed in range(6):
+        x = np.random.default_rng(seed).standard_normal((n, n))
+        a = (x + x.T) / np.sqrt(8 * n)
+        want = np.linalg.eigvalsh(a)
+        d, U = q.linalg.eigh(one_sector(a))
+        errors.append(np.linalg.norm(d.blocks()[0][1] - want) / np.linalg.norm(want))
+    assert np.mean(errors) <= 1.1 * plain
