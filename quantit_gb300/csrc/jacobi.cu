@@ -648,13 +648,14 @@ __device__ __forceinline__ void bj_params_fast(float al, float be, float ga, flo
 // instructions in all.
 //
 // Columns of norm ~ 2^ka, 2^kb (half the exponents of al, be); false: norms further apart, or closer to
-// the ends of the exponent range, than the conversions allow for (the caller takes the plain formulas).
+// the ends of the exponent range, than the conversions allow for (the caller takes the plain formulas): widen_f32
+// adds 896 + ka + kb to an FP32 exponent of 1 and more.
 __device__ __forceinline__ bool bj_exponents(double al, double be, int &ka, int &kb) {
     const int ea = int((uint32_t(__double2hiint(al)) >> 20) & 0x7FFu), eb = int((uint32_t(__double2hiint(be)) >> 20) & 0x7FFu);
     ka = (ea - 1023) >> 1;
     kb = (eb - 1023) >> 1;
     const int d = kb - ka;
-    return d <= 50 && d >= -50 && ea >= 64 && eb >= 64 && ea <= 1982 && eb <= 1982;
+    return d <= 50 && d >= -50 && ea >= 128 && eb >= 128 && ea <= 1982 && eb <= 1982;
 }
 // Newton's change of t = tan(theta / 2) towards the zero of ga (6 t^2 - 1 - t^4) + 2 (be - al) t (1 - t^2)
 // (the coupling after the rotation, times (1 + t^2)^2), ga = g + gl and be - al = d + dl.

@@ -42,3 +42,18 @@ def test_eigenvalues(n, plain):
         d, U = q.linalg.eigh(one_sector(a))
         errors.append(np.linalg.norm(d.blocks()[0][1] - want) / np.linalg.norm(want))
     assert np.mean(errors) <= 1.1 * plain
+
+
+@pytest.mark.parametrize("exponent", [-480, -470, -460, -440, 0, 440, 470])
+@pytest.mark.parametrize("p,n,decades", [(80, 60, 6), (60, 45, 0), (60, 30, 3)])
+def test_any_magnitude(exponent, p, n, decades):
+    """A power of two times a matrix has its factors, down to where squared norms come near the end of FP64's range."""
+    rng = np.random.default_rng(3)
+    a = rng.standard_normal((p, n)) * 10.0 ** (-decades * rng.permutation(n) / n)
+    U, d, V = (t.blocks()[0][1] for t in q.linalg.svd(one_sector(a * 2.0 ** exponent), 1))
+    d = d * 2.0 ** -exponent
+    want = np.linalg.svd(a, compute_uv=False)
+    np.testing.assert_allclose(d, want, atol=1e-13 * p * want[0], rtol=0)
+    assert np.linalg.norm((U * d) @ V.T - a, 2) <= 1e-13 * p * want[0]
+    for f in (U, V):
+        assert np.max(np.abs(f.T @ f - np.eye(n))) < 1e-12
