@@ -707,14 +707,16 @@ __device__ __forceinline__ int bj_params_fast64(double &al, double &be, double g
     return 1;
 }
 
-// Whether an updated squared norm kept more than 1/16 of the old one (FP64: by the high words,
-// without an FP64 instruction).
+// Whether an updated squared norm kept more than 1/16 of the old one; half of it in FP64, where its change is formed in
+// FP32: a cancelling update multiplies the norm's relative error by what the norm fell, and a column can fall at every
+// rotation of a step (at 1/16 a time the 1e-7 would be everything after six).  (FP64: by the high words, without an FP64
+// instruction.)
 template <bool EXACT>
 __device__ __forceinline__ bool norm_kept(float a2, float al) { return a2 > al * 0.0625f; }
 template <bool EXACT>
 __device__ __forceinline__ bool norm_kept(double a2, double al) {
     if constexpr (EXACT) return a2 > al * 0.0625;
-    return __double2hiint(a2) > __double2hiint(al) - (4 << 20);
+    return __double2hiint(a2) > __double2hiint(al) - (1 << 20);
 }
 
 // Hestenes rotation of two register-resident columns with tracked squared norms
@@ -779,7 +781,7 @@ __device__ __forceinline__ bool bj_rotate(T (&x)[R], T (&y)[R], bool full, T &al
             y[i] = fma(sn, x[i], y[i]);
         });
     }
-    // recomputed when the update cancelled (below about 1/16 of the norm)
+    // recomputed when the update cancelled
     al = norm_kept<EXACT>(a2, al) ? a2 : bj_dot(x, x, full);
     be = norm_kept<EXACT>(b2, be) ? b2 : bj_dot(y, y, full);
     if (thr > T(0)) {
