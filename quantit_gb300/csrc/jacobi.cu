@@ -1679,9 +1679,10 @@ bool bjacobi_dispatch(const BJacobiParams<T> &P, int max_steps_per_sweep, int ma
 // for the class from then on.  QTT_AUTOTUNE_FILE names a file the decisions are
 // read from at first use and appended to.
 struct TuneKey {
-    int f32, R, qcls, ncls;
+    int type;  // 1 FP32, 0 FP64, 2 FP64 with exactly computed angles (other kernels, of the same R)
+    int R, qcls, ncls;
     bool operator<(const TuneKey &o) const {
-        return std::tie(f32, R, qcls, ncls) < std::tie(o.f32, o.R, o.qcls, o.ncls);
+        return std::tie(type, R, qcls, ncls) < std::tie(o.type, o.R, o.qcls, o.ncls);
     }
 };
 struct TuneState {
@@ -1709,7 +1710,7 @@ void tune_load_locked() {
     if (FILE *f = std::fopen(path, "r")) {
         TuneKey k;
         int w;
-        while (std::fscanf(f, "%d %d %d %d %d", &k.f32, &k.R, &k.qcls, &k.ncls, &w) == 5) g_tune[k].winner = w;
+        while (std::fscanf(f, "%d %d %d %d %d", &k.type, &k.R, &k.qcls, &k.ncls, &w) == 5) g_tune[k].winner = w;
         std::fclose(f);
     }
 }
@@ -1718,7 +1719,7 @@ void tune_save(const TuneKey &k, int w) {
     const char *path = std::getenv("QTT_AUTOTUNE_FILE");
     if (!path) return;
     if (FILE *f = std::fopen(path, "a")) {
-        std::fprintf(f, "%d %d %d %d %d\n", k.f32, k.R, k.qcls, k.ncls, w);
+        std::fprintf(f, "%d %d %d %d %d\n", k.type, k.R, k.qcls, k.ncls, w);
         std::fclose(f);
     }
 }
@@ -1752,7 +1753,7 @@ void jacobi_impl(T *work, T *rot, const SectorDesc *sec, const int *slot_start, 
         if (!cands.empty()) {
             int ci = 0;
             bool timing = false;
-            const TuneKey key{f32 ? 1 : 0, R, ceil_log2(max_steps_per_sweep + 1), ceil_log2(nsec)};
+            const TuneKey key{f32 ? 1 : ex ? 2 : 0, R, ceil_log2(max_steps_per_sweep + 1), ceil_log2(nsec)};
             if (g_autotune.load() && cands.size() > 1) {
                 std::lock_guard<std::mutex> lk(g_tune_mu);
                 tune_load_locked();
@@ -1974,12 +1975,12 @@ std::string autotune_report() {
     for (auto &kv : g_tune) {
         const TuneKey &k = kv.first;
         const TuneState &st = kv.second;
-        const std::vector<int> c = block_widths(k.f32 != 0, k.R);
+        const std::vector<int> c = block_widths(k.type == 1, k.R);
         char t0[32] = "-", t1[32] = "-";
         if (st.tried[0]) std::snprintf(t0, sizeof(t0), "%.3f", st.best_ms[0]);
         if (st.tried[1]) std::snprintf(t1, sizeof(t1), "%.3f", st.best_ms[1]);
         std::snprintf(line, sizeof(line), "%s R=%d max_q<=2^%d nsec<=2^%d: B=%d (%s; B=%d %s ms, B=%d %s ms)\n",
-                      k.f32 ? "fp32" : "fp64", k.R, k.qcls, k.ncls,
+                      k.type == 1 ? "fp32" : k.type == 2 ? "fp64 exact" : "fp64", k.R, k.qcls, k.ncls,
                       st.winner >= 0 && st.winner < int(c.size()) ? c[st.winner] : (c.empty() ? 0 : c[0]),
                       st.winner >= 0 ? "tuned" : "tuning", c.size() > 0 ? c[0] : 0, t0, c.size() > 1 ? c[1] : 0, t1);
         out += line;
