@@ -552,9 +552,9 @@ bool f64_pairs_in_place(const ContractPlan &P, const BT &A, const BT &B, std::ve
 // The blocks of one operand (legs permuted by perm; the first nrow legs form the rows, the
 // rest K) as entries and tiles of the split kernel: offs receives the blocks' byte offsets
 // in the operand's split form, the return value is its size (a multiple of 128 bytes).
-int64_t split_tables(const BT &t, const std::vector<int64_t> &perm, int nrow, int operand, int mode,
+int64_t split_tables(const BT &t, const std::vector<int64_t> &perm, int nrow, int operand, int mode, int64_t ck,
                      std::vector<SplitEntry> &ents, std::vector<SplitTile> &tiles, std::vector<int64_t> &offs) {
-    const int64_t nb = t.nblocks(), ck = split_chunk_bytes(), es = split_elem_bytes(mode);
+    const int64_t nb = t.nblocks(), es = split_elem_bytes(mode);
     offs.assign(nb, 0);
     int64_t o = 0;
     for (int64_t b = 0; b < nb; ++b) {
@@ -718,11 +718,19 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
         contract_f64(P, A, B, out, add, beta, alpha, outs, Ks, flops);
         return;
     }
+    const int TM = gemm_tile_m();
+    auto tiles_of = [&](int tn) {
+        int64_t n = 0;
+        for (const GemmOut &o : outs) n += ((int64_t(o.M) + TM - 1) / TM) * ((int64_t(o.N) + tn - 1) / tn);
+        return n;
+    };
+    const int TN = gemm_tile_n(tiles_of(128));
+    const int chunk = split_chunk_bytes(tiles_of(TN));
     std::vector<SplitEntry> ents;
     std::vector<SplitTile> stiles;
     std::vector<int64_t> offa, offb;
-    const int64_t asz = split_tables(A, P.p1, int(P.freeA.size()), 0, mode, ents, stiles, offa);
-    const int64_t bsz = split_tables(B, P.p2p, int(P.freeB.size()), 1, mode, ents, stiles, offb);
+    const int64_t asz = split_tables(A, P.p1, int(P.freeA.size()), 0, mode, chunk, ents, stiles, offa);
+    const int64_t bsz = split_tables(B, P.p2p, int(P.freeB.size()), 1, mode, chunk, ents, stiles, offb);
     // one buffer: the two maxima, their per-CTA parts, then the split arrays.  The maxima of an operand that a
     // GEMM has just written come from its epilogue: reading the operand again for them is 8 of the 24 bytes an
     // element that the split moves otherwise.
@@ -752,10 +760,6 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
     sa.dst[0] = static_cast<char *>(split->p) + head;
     sa.dst[1] = sa.dst[0] + asz;
     sa.amax = amax;
-    const int TM = gemm_tile_m();
-    int64_t wide = 0;
-    for (const GemmOut &o : outs) wide += ((int64_t(o.M) + TM - 1) / TM) * ((int64_t(o.N) + 127) / 128);
-    const int TN = gemm_tile_n(wide);
     std::vector<GemmPair> pairs(P.pair_a.size());
     for (size_t k = 0; k < pairs.size(); ++k) {
         pairs[k].a_off = offa[P.pair_a[k]];
@@ -797,7 +801,7 @@ void run_contraction(const ContractPlan &P, const BT &A, const BT &B, BT &out, c
                               table(tiles, g.tiles)});
         bool flat = true;
         for (const SplitEntry &e : ents) flat = flat && e.folded && e.rd2 >= e.rows && e.kd2 >= e.K;
-        launch_split(sa, int64_t(stiles.size()), mode, flat);
+        launch_split(sa, int64_t(stiles.size()), mode, chunk, flat);
     }
     StatScope sc(ST_GEMM, flops);
     launch_gemm_tc(g, mode);

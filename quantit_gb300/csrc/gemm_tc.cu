@@ -37,7 +37,8 @@
 //    What bounds it is the one thread's issue (about 900 clocks a stage of six TF32 MMAs that
 //    take 450) and, for thin tiles, the epilogue; hence two CTAs per SM, each with half the
 //    ring: 88 against 121 us at the D = 4096 theta pair with one CTA and twice the stages,
-//    921 against 1518 us for the three contractions of the cylinder matvec at D = 2048.
+//    921 against 1518 us for the three contractions of the cylinder matvec at D = 2048.  Launches of no more
+//    tiles than SMs have one CTA an SM and stages of twice the K (split_chunk_bytes).
 //
 // Against row groups outermost (64 or 96 copies of 1 KB a stage), one pair per stage, one CTA
 // per SM, five launches and as many memsets: theta pair D = 4096, TF32X3 436 -> 162 us (gemm
@@ -64,8 +65,6 @@ namespace {
 using namespace tc;
 
 constexpr int TBM = 128, TBN = 128;
-constexpr int CKB = 64;                   // bytes of K per row and stage
-constexpr int COPY_BYTES = 128 * CKB;     // one operand copy of a stage
 constexpr int TTHREADS = 192;             // producer, MMA and four epilogue warps
 constexpr int CTAS_PER_SM = 2;
 constexpr int AMAX_THREADS = 512;
@@ -159,8 +158,9 @@ struct Bf16x3 {
     }
 };
 
-constexpr int stage_bytes(int nc) { return 2 * nc * COPY_BYTES; }
-constexpr int smem_bytes(int nc, int nstage) { return nstage * stage_bytes(nc) + EPI_BYTES; }
+// CKB: bytes of K per row and stage (split_chunk_bytes); one operand copy of a stage takes 128 rows of them
+constexpr int stage_bytes(int nc, int ckb) { return 2 * nc * 128 * ckb; }
+constexpr int smem_bytes(int nc, int nstage, int ckb) { return nstage * stage_bytes(nc, ckb) + EPI_BYTES; }
 
 // Maxima of |x| as bit patterns (bit order = value order for non-negative doubles), one
 // per CTA; operand b's CTAs follow operand a's.
@@ -217,7 +217,7 @@ __device__ __forceinline__ unsigned long long amax_of(const unsigned long long *
 
 // FLAT: every entry's rows have one stride and its K one (no index arithmetic but two
 // products); otherwise rows and K of two strides each, or any legs.
-template <class S, bool FLAT>
+template <class S, int CKB, bool FLAT>
 __global__ void __launch_bounds__(256) k_split(SplitArgs g) {
     constexpr int EV = 16 / S::ELEM;  // elements of a core matrix row
     __shared__ unsigned long long red[8];
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(256) k_split(SplitArgs g) {
     }
 }
 
-// What a stage holds, for the MMA thread: up to CKB / 32 units of k-steps (3 bits each from
+// What a stage holds, for the MMA thread: up to CKB / 32 <= 4 units of k-steps (3 bits each from
 // bit 0), flags, and the tile's N in units of 16.
 constexpr uint32_t ST_FIRST = 1u << 12, ST_LAST = 1u << 13, ST_END = 1u << 14;
 constexpr int ST_N16 = 16;
@@ -359,9 +359,9 @@ struct TileRegs {
     }
 };
 
-template <class S, int NSTAGE>
-__global__ void __launch_bounds__(TTHREADS, CTAS_PER_SM) k_gemm_tc(TcArgs g, int *err) {
-    constexpr int NC = S::NC, STAGE = stage_bytes(NC);
+template <class S, int CKB, int CTAS>
+__global__ void __launch_bounds__(TTHREADS, CTAS) k_gemm_tc(TcArgs g, int *err) {
+    constexpr int NC = S::NC, NSTAGE = S::NSTAGE, STAGE = stage_bytes(NC, CKB), COPY_BYTES = 128 * CKB;
     extern __shared__ __align__(128) char smem[];
     __shared__ uint64_t full[NSTAGE], empty[NSTAGE], acc_full[2], acc_empty[2], drained;
     __shared__ uint32_t stage_word[NSTAGE];
@@ -683,27 +683,24 @@ int *err_word() {
     return c.tc_err;
 }
 
-template <class S, int NSTAGE>
-void launch_ring(const TcArgs &a, int grid) {
+template <class S, int CKB, int CTAS>
+void launch_ring(const TcArgs &a) {
     static std::atomic<uint64_t> attr{0};
+    constexpr int smem = smem_bytes(S::NC, S::NSTAGE, CKB);
     once_per_device(attr, [] {
-        cuda_check(cudaFuncSetAttribute(k_gemm_tc<S, NSTAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        smem_bytes(S::NC, NSTAGE)),
+        cuda_check(cudaFuncSetAttribute(k_gemm_tc<S, CKB, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
                    "tcgen05 GEMM smem attribute");
     });
-    k_gemm_tc<S, NSTAGE><<<grid, TTHREADS, smem_bytes(S::NC, NSTAGE), ctx().stream>>>(a, err_word());
+    // CTAS persistent CTAs an SM; one CTA per tile with the persistent grid switched off
+    k_gemm_tc<S, CKB, CTAS><<<gemm_tc_grid(a.ntiles), TTHREADS, smem, ctx().stream>>>(a, err_word());
 }
 
 template <class S>
 void launch_gemm(const TcArgs &a) {
-    // CTAS_PER_SM persistent CTAs an SM; one CTA per tile with the persistent grid switched off.
-    // With no more tiles than SMs a CTA has its SM to itself and takes twice the stages.
-    const int sms = device_sm_count();
-    const int grid = gemm_tc_grid(a.ntiles);
-    if (a.ntiles <= sms)
-        launch_ring<S, 2 * S::NSTAGE>(a, grid);
+    if (split_chunk_bytes(a.ntiles) == 128)
+        launch_ring<S, 128, 1>(a);
     else
-        launch_ring<S, S::NSTAGE>(a, grid);
+        launch_ring<S, 64, CTAS_PER_SM>(a);
 }
 
 }  // namespace
@@ -713,7 +710,10 @@ int gemm_tile_m() { return TBM; }
 int gemm_tile_n(int64_t tiles) { return tiles <= device_sm_count() ? TBN / 2 : TBN; }
 int split_copies(int mode) { return mode == GEMM_BF16X3 ? Bf16x3::NC : Tf32x3::NC; }
 int split_elem_bytes(int mode) { return mode == GEMM_BF16X3 ? Bf16x3::ELEM : Tf32x3::ELEM; }
-int split_chunk_bytes() { return CKB; }
+// With no more tiles than SMs a CTA has its SM to itself and takes stages of twice the K: half as many
+// waits and commits in the chain of a tile.  1 x 1 results over K = 2^20 with 64 bytes and twice the stages 30.0 ms
+// (TF32X3), 20.0 with 128.
+int split_chunk_bytes(int64_t tiles) { return tiles <= device_sm_count() ? 128 : 64; }
 
 void launch_amax(const AmaxArgs &a) {
     const int n = a.parts[0] + a.parts[1];
@@ -723,21 +723,20 @@ void launch_amax(const AmaxArgs &a) {
     cuda_check(cudaGetLastError(), "amax kernel launch");
 }
 
-void launch_split(const SplitArgs &a, int64_t ntiles, int mode, bool flat) {
+template <class S, int CKB>
+static void split_with(const SplitArgs &a, unsigned grid, bool flat) {
+    if (flat)
+        k_split<S, CKB, true><<<grid, 256, 0, ctx().stream>>>(a);
+    else
+        k_split<S, CKB, false><<<grid, 256, 0, ctx().stream>>>(a);
+}
+void launch_split(const SplitArgs &a, int64_t ntiles, int mode, int chunk, bool flat) {
     if (ntiles <= 0) return;
     const unsigned grid = unsigned(ntiles);
-    const cudaStream_t st = ctx().stream;
-    if (mode == GEMM_BF16X3) {
-        if (flat)
-            k_split<Bf16x3, true><<<grid, 256, 0, st>>>(a);
-        else
-            k_split<Bf16x3, false><<<grid, 256, 0, st>>>(a);
-    } else {
-        if (flat)
-            k_split<Tf32x3, true><<<grid, 256, 0, st>>>(a);
-        else
-            k_split<Tf32x3, false><<<grid, 256, 0, st>>>(a);
-    }
+    if (mode == GEMM_BF16X3)
+        chunk == 128 ? split_with<Bf16x3, 128>(a, grid, flat) : split_with<Bf16x3, 64>(a, grid, flat);
+    else
+        chunk == 128 ? split_with<Tf32x3, 128>(a, grid, flat) : split_with<Tf32x3, 64>(a, grid, flat);
     count_launch();
     cuda_check(cudaGetLastError(), "split kernel launch");
 }

@@ -116,10 +116,11 @@ struct SplitArgs {
     unsigned long long *amax;  // receives the two operands' maxima
 };
 // flat: every entry is folded with rd2 >= rows and kd2 >= K (one stride each)
-void launch_split(const SplitArgs &a, int64_t ntiles, int mode, bool flat);
+// chunk: split_chunk_bytes of the GEMM's tiles
+void launch_split(const SplitArgs &a, int64_t ntiles, int mode, int chunk, bool flat);
 int split_copies(int mode);
 int split_elem_bytes(int mode);
-int split_chunk_bytes();
+int split_chunk_bytes(int64_t tiles);  // bytes of K per row and chunk, for a GEMM of so many tiles
 // A pair's a_off / b_off: byte offsets of its blocks in split form; A rows = M,
 // B rows = N.  A tile whose pairs all have K = 0 has cls 1, the others 0.
 struct TcArgs {
