@@ -568,7 +568,7 @@ int64_t split_tables(const BT &t, const std::vector<int64_t> &perm, int nrow, in
             (i < nrow ? rl[i] : kl[i - nrow]) = FoldLeg{e.dims[i], e.stride[i], 0};
             (i < nrow ? rows : K) *= e.dims[i];
         }
-        if (K * es > INT32_MAX - 64) fail(ERR_INVALID_ARGUMENT, "contracted dimension too large");
+        if (K > INT32_MAX - 64) fail(ERR_INVALID_ARGUMENT, "contracted dimension too large");
         if (rows > INT32_MAX - 64) fail(ERR_INVALID_ARGUMENT, "block too large");
         Fold fr, fk;
         e.folded = fold_legs(rl, nrow, fr) && fold_legs(kl, t.rank - nrow, fk) ? 1 : 0;
@@ -586,15 +586,15 @@ int64_t split_tables(const BT &t, const std::vector<int64_t> &perm, int nrow, in
         e.rank = t.rank;
         e.rows = int32_t(rows);
         e.K = int32_t(K);
-        e.kpb = int32_t((K * es + 31) & ~int64_t(31));
+        e.kpb = (K * es + 31) & ~int64_t(31);
         offs[b] = o;
-        o += ((rows + 7) / 8) * 8 * int64_t(e.kpb) * split_copies(mode);
+        o += ((rows + 7) / 8) * 8 * e.kpb * split_copies(mode);
         // 8192 elements a tile or so: few tiles to list, enough of them to spread
         for (int64_t k0 = 0; k0 < e.kpb; k0 += ck) {
             const int64_t kv = std::min<int64_t>(ck, e.kpb - k0);
             const int64_t step = 64 * std::max<int64_t>(1, 128 * es / kv / 2);
             for (int64_t r0 = 0; r0 < rows; r0 += step)
-                tiles.push_back(SplitTile{int32_t(ents.size()), int32_t(r0), int32_t(std::min(step, rows - r0)), int32_t(k0)});
+                tiles.push_back(SplitTile{int32_t(ents.size()), int32_t(r0), int32_t(std::min(step, rows - r0)), int32_t(k0 / ck)});
         }
         ents.push_back(e);
     }

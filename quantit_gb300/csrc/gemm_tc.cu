@@ -225,11 +225,11 @@ __global__ void __launch_bounds__(256) k_split(SplitArgs g) {
     const SplitEntry &e = g.ents[t.ent];
     const int op = e.operand;
     const double *__restrict__ src = g.src[op] + e.src_off;
-    const int kvb = min(CKB, e.kpb - t.k0b), nq = kvb / 16;
-    const int rows = e.rows, K = e.K, nrg = (rows + 7) >> 3, k00 = t.k0b / S::ELEM;
+    const int kvb = int(min(int64_t(CKB), e.kpb - int64_t(t.chunk) * CKB)), nq = kvb / 16;
+    const int rows = e.rows, K = e.K, nrg = (rows + 7) >> 3, k00 = t.chunk * (CKB / S::ELEM);
     const int total = ((t.rows + 7) >> 3) * nq * 8, inv = (65536 + nq - 1) / nq;
     const int64_t rs2 = e.rs2, ks2 = e.ks2;
-    char *dst0 = g.dst[op] + e.dst_off + int64_t(t.k0b / CKB) * nrg * (8 * S::NC * CKB);
+    char *dst0 = g.dst[op] + e.dst_off + int64_t(t.chunk) * nrg * (8 * S::NC * CKB);
     // row and 16-byte column of core matrix row i
     auto place = [&](int i, int &row, int &core) {
         const int u = i >> 3, rg = (u * inv) >> 16;  // u / nq, u < 2^14
@@ -362,6 +362,7 @@ struct TileRegs {
 template <class S, int CKB, int CTAS>
 __global__ void __launch_bounds__(TTHREADS, CTAS) k_gemm_tc(TcArgs g, int *err) {
     constexpr int NC = S::NC, NSTAGE = S::NSTAGE, STAGE = stage_bytes(NC, CKB), COPY_BYTES = 128 * CKB;
+    constexpr int KS = 32 / S::ELEM, CKU = CKB / 32;  // elements of a k-step, k-steps of a stage
     extern __shared__ __align__(128) char smem[];
     __shared__ uint64_t full[NSTAGE], empty[NSTAGE], acc_full[2], acc_empty[2], drained;
     __shared__ uint32_t stage_word[NSTAGE];
@@ -448,29 +449,29 @@ __global__ void __launch_bounds__(TTHREADS, CTAS) k_gemm_tc(TcArgs g, int *err) 
                 word &= 0xFu << ST_N16;
                 width = nu = 0;
             };
-            // the pair of each lane (a batch of 32): offset for this lane's operand and padded K
+            // the pair of each lane (a batch of 32): offset for this lane's operand and its k-steps
             for (int pb = 0; pb < np && !stop; pb += 32) {
                 int64_t a_off = 0, b_off = 0;
-                int kpb = 0;
+                int ksteps = 0;
                 if (pb + lane < np) {
                     const GemmPair pr = g.pairs[t.p0 + pb + lane];
                     a_off = pr.a_off;
                     b_off = pr.b_off;
-                    kpb = (pr.K * S::ELEM + 31) & ~31;
+                    ksteps = pr.K / KS + (pr.K % KS != 0);
                 }
-                for (uint32_t live = __ballot_sync(0xffffffffu, kpb > 0); live && !stop; live &= live - 1) {
+                for (uint32_t live = __ballot_sync(0xffffffffu, ksteps > 0); live && !stop; live &= live - 1) {
                     const int p = __ffs(int(live)) - 1;
-                    const int kp = __shfl_sync(0xffffffffu, kpb, p);
+                    const int kp = __shfl_sync(0xffffffffu, ksteps, p);
                     const int64_t ao = __shfl_sync(0xffffffffu, a_off, p), bo = __shfl_sync(0xffffffffu, b_off, p);
                     const char *src = base + (is_a ? ao : bo);
                     int k = 0;
-                    if (kp >= CKB) {
+                    if (kp >= CKU) {
                         if (width && !stop) close_stage(0);
-                        const bool ends = (live & (live - 1)) == 0 && pb + 32 >= np && kp % CKB == 0;
-                        for (; k + CKB <= kp; k += CKB) {
+                        const bool ends = (live & (live - 1)) == 0 && pb + 32 >= np && kp % CKU == 0;
+                        for (; k + CKU <= kp; k += CKU) {
                             if (!wait_slot()) break;
                             if (lane == 0) {
-                                stage_word[slot] = word | uint32_t(CKB / 32) | (ends && k + CKB == kp ? ST_LAST : 0u);
+                                stage_word[slot] = word | uint32_t(CKU) | (ends && k + CKU == kp ? ST_LAST : 0u);
                                 mbar_arrive_expect_tx(&full[slot], row_bytes * CKB);
                             }
                             __syncwarp();
@@ -482,8 +483,8 @@ __global__ void __launch_bounds__(TTHREADS, CTAS) k_gemm_tc(TcArgs g, int *err) 
                         if (stop) break;
                         ended = ends;
                     }
-                    const int kv = kp - k;
-                    if (kv > 0) {
+                    const int ku = kp - k, kv = ku * 32;
+                    if (ku > 0) {
                         if (width + kv > CKB) close_stage(0);
                         if (width == 0 && !wait_slot()) break;
                         if (lane == 0) mbar_expect_tx_only(&full[slot], row_bytes * uint32_t(kv));
@@ -491,7 +492,7 @@ __global__ void __launch_bounds__(TTHREADS, CTAS) k_gemm_tc(TcArgs g, int *err) 
                         if (copies)
                             bulk_g2s(stage0 + slot * STAGE + width * (128 * NC), src + my_first * kv, my_rows * uint32_t(kv),
                                      &full[slot]);
-                        word |= uint32_t(kv / 32) << (3 * nu++);
+                        word |= uint32_t(ku) << (3 * nu++);
                         width += kv;
                     }
                 }

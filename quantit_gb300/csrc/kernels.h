@@ -93,8 +93,8 @@ struct AmaxArgs {
 void launch_amax(const AmaxArgs &a);
 struct SplitEntry {
     int64_t src_off, dst_off;  // source elements; bytes within the operand's split form
-    int32_t operand, rows, K;
-    int32_t kpb;               // padded K in bytes
+    int64_t kpb;               // padded K in bytes
+    int32_t operand, rows, K, pad;
     // folded: element (row, k) is at (row / rd2) rs1 + (row % rd2) rs2 + (k / kd2) ks1 + (k % kd2) ks2;
     // otherwise at the row-major index row K + k over dims, with these strides
     int32_t folded, rd2, kd2, rank;
@@ -102,9 +102,9 @@ struct SplitEntry {
     int64_t dims[8];
     int64_t stride[8];
 };
-// One CTA: `rows` rows from row0 (a multiple of 8) of one chunk (k0b: its first byte of K).
+// One CTA: `rows` rows from row0 (a multiple of 8) of one chunk of K.
 struct SplitTile {
-    int32_t ent, row0, rows, k0b;
+    int32_t ent, row0, rows, chunk;
 };
 struct SplitArgs {
     const double *src[2];
