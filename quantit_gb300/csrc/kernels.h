@@ -218,13 +218,13 @@ void launch_svd_refine(const float *rot32, int64_t rot_size, const double *w64, 
 // out[s_off + j] = squared norm (FP64) of column j of every sector's work matrix (f32:
 // FP32 work matrices)
 void launch_col_norms(const void *W, const SectorDesc *secs, int nsec, int max_q, double *out, int f32);
-// Column copies dst[dst_off + r] = src[src_off + r], r < len (FP64), one task per column:
-// the gather and scatter of the kept columns around the restricted FP64 sweeps.
+// Copies dst[dst_off + r] = src[src_off + r], r < len (FP64, or FP32 with f32), one task each: the gather and scatter
+// of the kept columns around the restricted FP64 sweeps, and the rotations kept for warm starts.
 struct ColCopy {
     int64_t src_off, dst_off;
     int32_t len, pad;
 };
-void launch_col_copy(const double *src, double *dst, const std::vector<ColCopy> &cols);
+void launch_col_copy(const void *src, void *dst, const std::vector<ColCopy> &cols, int f32);
 // Vn = Vg R per sector (FP64): Vg (vrows x k at vg_off, column-major), R (k x k at r_off),
 // Vn (vrows x k at vn_off).
 struct RotProduct {

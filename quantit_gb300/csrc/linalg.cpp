@@ -331,14 +331,17 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             const Sector &s = D.secs[g];
             for (int64_t e = 0; e < s.batch; ++e) {
                 SectorDesc &d = D.desc[D.first_desc[g] + e];
-                std::vector<int64_t> key = {d.trans, d.q, e};
-                key.insert(key.end(), s.lead.begin(), s.lead.end());
-                for (const SecRow &sr : (d.trans ? s.rows : s.cols)) {
-                    key.push_back(sr.sec);
-                    key.push_back(sr.size);
+                std::vector<int64_t> key;  // (empty: not one that starts warm)
+                if (d.q >= 2 && !lq_fits(d, f32)) {
+                    key = {d.trans, d.q, e};
+                    key.insert(key.end(), s.lead.begin(), s.lead.end());
+                    for (const SecRow &sr : (d.trans ? s.rows : s.cols)) {
+                        key.push_back(sr.sec);
+                        key.push_back(sr.size);
+                    }
                 }
                 for (const WarmStart::Entry &en : ws->entries) {
-                    if (en.f32 != f32 || en.key != key || d.q < 2 || lq_fits(d, f32)) continue;
+                    if (key.empty() || en.f32 != f32 || en.key != key) continue;
                     d.warm = 1;
                     WarmDesc w{};
                     w.w_off = d.w_off;
@@ -603,8 +606,8 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                 BufPtr rk = dev_alloc(size_t(std::max<int64_t>(kr, 1)) * 8);
                 BufPtr vg = dev_alloc(size_t(std::max<int64_t>(kv, 1)) * 8);
                 BufPtr vn = dev_alloc(size_t(std::max<int64_t>(kv, 1)) * 8);
-                launch_col_copy(static_cast<const double *>(w1->p), static_cast<double *>(wk->p), wgather);
-                launch_col_copy(static_cast<const double *>(vbuf->p), static_cast<double *>(vg->p), vgather);
+                launch_col_copy(w1->p, wk->p, wgather, 0);
+                launch_col_copy(vbuf->p, vg->p, vgather, 0);
                 const SectorDesc *ddk = upload_vec(dk);
                 const int *dkslots = upload_vec(kslots);
                 const size_t vbk = jacobi_vwork_bytes(nsec, ks, kmax_steps, max_sweeps, 0);
@@ -621,9 +624,9 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                               vworkk->p, vbk, deflate ? thr64->p : nullptr, deflate ? dnk->p : nullptr, nullptr, th.plain, shear_q);
                 launch_rot_product(static_cast<const double *>(vg->p), static_cast<const double *>(rk->p),
                                    static_cast<double *>(vn->p), rp);
-                launch_col_copy(static_cast<const double *>(wk->p), static_cast<double *>(w1->p), wscatter);
-                launch_col_copy(static_cast<const double *>(vn->p), static_cast<double *>(vbuf->p), vscatter);
-                if (deflate) launch_col_copy(static_cast<const double *>(dnk->p), static_cast<double *>(dnorm->p), dscatter);
+                launch_col_copy(wk->p, w1->p, wscatter, 0);
+                launch_col_copy(vn->p, vbuf->p, vscatter, 0);
+                if (deflate) launch_col_copy(dnk->p, dnorm->p, dscatter, 0);
                 // the compact buffers are released in stream order after the copies above
             }
             fw = w1->p;
@@ -685,10 +688,26 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                       dnorm ? dnorm->p : nullptr, nullptr, permbuf ? static_cast<int *>(permbuf->p) : nullptr,
                       max_elems, norms);
         if (ws) {
-            // this decomposition's rotations (of the first stage) start the next one at the same bond
+            // this decomposition's rotations (of the first stage) start the next one at the same bond: those of the
+            // sectors that may start warm, in a buffer of their own unless they are most of all
             std::vector<WarmStart::Entry> next;
-            for (int i = 0; i < nsec; ++i)
-                next.push_back(WarmStart::Entry{std::move(keys[i]), D.rot, D.desc[i].rot_off, f32});
+            std::vector<ColCopy> kept;
+            int64_t elems = 0;
+            for (int i = 0; i < nsec; ++i) {
+                if (keys[i].empty()) continue;
+                const SectorDesc &d = D.desc[i];
+                next.push_back(WarmStart::Entry{std::move(keys[i]), D.rot, d.rot_off, f32});
+                kept.push_back({d.rot_off, elems, int32_t(d.q) * d.q, 0});
+                elems += int64_t(d.q) * d.q;
+            }
+            if (elems < rtot / 2 && !next.empty()) {
+                const BufPtr own = dev_alloc(size_t(elems) * es);
+                launch_col_copy(D.rot->p, own->p, kept, f32);
+                for (size_t i = 0; i < next.size(); ++i) {
+                    next[i].buf = own;
+                    next[i].off = kept[i].dst_off;
+                }
+            }
             ws->entries = std::move(next);
         }
         if (f32) {

@@ -210,7 +210,8 @@ __global__ void k_col_norms(const T *__restrict__ W, const SectorDesc *__restric
     if (lane == 0) out[sd.s_off + col] = acc;
 }
 
-__global__ void __launch_bounds__(256) k_col_copy(const double *__restrict__ src, double *__restrict__ dst,
+template <class T>
+__global__ void __launch_bounds__(256) k_col_copy(const T *__restrict__ src, T *__restrict__ dst,
                                                   const ColCopy *__restrict__ cc, int n) {
     for (int c = blockIdx.x; c < n; c += gridDim.x) {
         const ColCopy e = cc[c];
@@ -220,11 +221,16 @@ __global__ void __launch_bounds__(256) k_col_copy(const double *__restrict__ src
 
 }  // namespace
 
-void launch_col_copy(const double *src, double *dst, const std::vector<ColCopy> &cols) {
+void launch_col_copy(const void *src, void *dst, const std::vector<ColCopy> &cols, int f32) {
     if (cols.empty()) return;
     const ColCopy *d = upload_vec(cols);
     const int grid = int(std::min<size_t>(cols.size(), 8192));
-    k_col_copy<<<grid, 256, 0, ctx().stream>>>(src, dst, d, int(cols.size()));
+    if (f32)
+        k_col_copy<float><<<grid, 256, 0, ctx().stream>>>(static_cast<const float *>(src), static_cast<float *>(dst), d,
+                                                          int(cols.size()));
+    else
+        k_col_copy<double><<<grid, 256, 0, ctx().stream>>>(static_cast<const double *>(src), static_cast<double *>(dst), d,
+                                                           int(cols.size()));
     count_launch();
     cuda_check(cudaGetLastError(), "column copy launch");
 }
