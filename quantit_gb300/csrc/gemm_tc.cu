@@ -50,7 +50,7 @@
 // The order of the MMAs of a tile is that of its pairs and k-steps whatever the stages
 // hold, so results do not depend on the grid or the ring.
 //
-// Every mbarrier wait is bounded; on timeout the kernel records an error code in
+// Every mbarrier wait is bounded (the epilogue's by its tile's K); on timeout the kernel records an error code in
 // a device word that the host checks, drains (bounded) the copies and MMAs it
 // issued and frees its TMEM before returning.
 #include <cstdint>
@@ -595,7 +595,16 @@ __global__ void __launch_bounds__(TTHREADS, CTAS) k_gemm_tc(TcArgs g, int *err) 
             const int b = i & 1;
             if (have_acc) {
                 int ok = 1;
-                if (lane == 0) ok = mbar_wait(&acc_full[b], (i / 2) & 1) ? 1 : 0;
+                if (lane == 0) {
+                    ok = mbar_wait(&acc_full[b], (i / 2) & 1) ? 1 : 0;
+                    if (!ok) {
+                        // a tile of a long K takes longer than one bounded wait (2^23 k-steps, 1.3 s): as many more as
+                        // its k-steps can take
+                        int64_t steps = 0;
+                        for (int p = t.p0; p < t.p1; ++p) steps += (int64_t(g.pairs[p].K) * S::ELEM + 31) / 32;
+                        for (int64_t more = steps >> 20; more > 0 && !ok; --more) ok = mbar_wait(&acc_full[b], (i / 2) & 1) ? 1 : 0;
+                    }
+                }
                 ok = __shfl_sync(0xffffffffu, ok, 0);
                 if (!ok) {
                     if (lane == 0) atomicExch(err, S::ERR + 1);
