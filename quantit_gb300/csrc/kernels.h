@@ -217,7 +217,9 @@ void launch_svd_refine(const float *rot32, int64_t rot_size, const double *w64, 
                        double *g, const std::vector<SectorDesc> &secs, bool exact);
 // out[s_off + j] = squared norm (FP64) of column j of every sector's work matrix (f32:
 // FP32 work matrices)
-void launch_col_norms(const void *W, const SectorDesc *secs, int nsec, int max_q, double *out, int f32);
+// amax (optional): launch_pack's, by which the norms are scaled back.
+void launch_col_norms(const void *W, const SectorDesc *secs, int nsec, int max_q, double *out, int f32,
+                      const uint32_t *amax = nullptr);
 // Copies dst[dst_off + r] = src[src_off + r], r < len (FP64, or FP32 with f32), one task each: the gather and scatter
 // of the kept columns around the restricted FP64 sweeps, and the rotations kept for warm starts.
 struct ColCopy {

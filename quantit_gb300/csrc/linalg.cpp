@@ -372,20 +372,18 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     const PackEntry *dpe = nullptr;
     const Chunk *dch = nullptr;
     const int *dslots = nullptr;
-    const BufPtr tables = upload_many({table(D.desc, desc_table), table(pe, dpe), table(chunks, dch), table(slots, dslots)});
+    // FP32 sectors are packed at magnitude 1; the norms that the host reads of them are scaled back.  (Their maxima start
+    // as a table of zeros: a buffer and a memset of their own were 1 to 2 % of a small decomposition.)
+    const std::vector<uint32_t> zeros(f32 ? size_t(nsec) : 0, 0u);
+    const uint32_t *amax = nullptr;
+    const BufPtr tables = upload_many({table(D.desc, desc_table), table(pe, dpe), table(chunks, dch), table(slots, dslots),
+                                       table(zeros, amax)});
     SectorDesc *dsec = const_cast<SectorDesc *>(desc_table);  // (eigh writes its shifts there)
-    // FP32 sectors are packed at magnitude 1; what the host reads of them is scaled back
-    BufPtr amax_buf;
-    if (f32) {
-        amax_buf = dev_alloc(size_t(nsec) * sizeof(uint32_t));
-        cuda_check(cudaMemsetAsync(amax_buf->p, 0, size_t(nsec) * sizeof(uint32_t), ctx().stream), "cudaMemsetAsync(sector maxima)");
-    }
-    const uint32_t *amax = f32 ? static_cast<const uint32_t *>(amax_buf->p) : nullptr;
     {
         StatScope sc(ST_PACK, (f32 ? 2.5 : 2.0) * 8.0 * double(packed));
         if (f32)
             launch_sector_amax(static_cast<const double *>(t.data()), dpe, dch, int64_t(chunks.size()),
-                               static_cast<uint32_t *>(amax_buf->p));
+                               const_cast<uint32_t *>(amax));
         launch_pack(static_cast<const double *>(t.data()), W, dpe, dch, int64_t(chunks.size()), dsec, f32, amax);
     }
     if (mode == 1) launch_eigh_prepare(W, dsec, nsec, upper, f32);
@@ -449,20 +447,13 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
         TruncHint &th = trunc_hint();
         if (f32 && deflate && th.allow_discard && th.max_size > 0) {
             BufPtr cn = dev_alloc(size_t(std::max<int64_t>(stot, 1)) * 8);
-            launch_col_norms(W, dsec, nsec, max_q, static_cast<double *>(cn->p), 1);
+            launch_col_norms(W, dsec, nsec, max_q, static_cast<double *>(cn->p), 1, amax);
             std::vector<double> n2(size_t(std::max<int64_t>(stot, 1)));
             cuda_check(cudaMemcpyAsync(n2.data(), cn->p, size_t(stot) * 8, cudaMemcpyDeviceToHost, ctx().stream),
                        "cudaMemcpyAsync(column norms)");
-            std::vector<uint32_t> top(nsec);
-            cuda_check(cudaMemcpyAsync(top.data(), amax, size_t(nsec) * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx().stream),
-                       "cudaMemcpyAsync(sector maxima)");
             cuda_check(cudaStreamSynchronize(ctx().stream), "cudaStreamSynchronize");
-            std::vector<double> vals(static_cast<size_t>(stot));
-            for (int i = 0; i < nsec; ++i)
-                for (int j = 0; j < D.desc[i].q; ++j) {
-                    const size_t at = size_t(D.desc[i].s_off + j);
-                    vals[at] = std::ldexp(std::sqrt(std::max(0.0, n2[at])), sector_exponent(top[i]));  // (NaN: 0)
-                }
+            std::vector<double> vals(n2.begin(), n2.begin() + stot);
+            for (double &x : vals) x = std::sqrt(std::max(0.0, x));  // (NaN: 0)
             std::vector<double> sorted = vals;
             std::sort(sorted.begin(), sorted.end(), std::greater<double>());
             const double t_est = kept_threshold(sorted, th.tol, th.pw, th.min_size, th.max_size);
@@ -480,8 +471,8 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                 const SectorDesc &d = D.desc[i];
                 double f2 = 0.0;
                 for (int j = 0; j < d.q; ++j) f2 += n2[d.s_off + j];
-                const double norm = std::ldexp(std::sqrt(f2), sector_exponent(top[i]));
-                null2[i] = std::ldexp(kDeflateF64 * kDeflateF64 * f2, 2 * sector_exponent(top[i]));
+                const double norm = std::sqrt(f2);
+                null2[i] = kDeflateF64 * kDeflateF64 * f2;
                 const bool here = t_est > 0.0 && tau > 4.0 * kDeflateF32 * norm;
                 discard[i] = here ? tau : 0.0;
                 any = any || here;

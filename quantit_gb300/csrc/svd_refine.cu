@@ -195,10 +195,11 @@ void products(const double *A, const double *B, double *C, const std::vector<Pro
     launch_gemm_f64(g);
 }
 
-// Squared column norms of every sector matrix (one warp per column).
+// Squared column norms of every sector matrix (one warp per column); amax: of the sectors as they were before k_pack scaled
+// them.
 template <class T>
 __global__ void k_col_norms(const T *__restrict__ W, const SectorDesc *__restrict__ secs,
-                            double *__restrict__ out) {
+                            double *__restrict__ out, const uint32_t *__restrict__ amax) {
     const SectorDesc sd = secs[blockIdx.y];
     const int lane = threadIdx.x & 31;
     const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -207,7 +208,7 @@ __global__ void k_col_norms(const T *__restrict__ W, const SectorDesc *__restric
     double acc = 0.0;
     for (int r = lane; r < sd.p; r += 32) acc = fma(double(w[r]), double(w[r]), acc);
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) out[sd.s_off + col] = acc;
+    if (lane == 0) out[sd.s_off + col] = amax ? ldexp(acc, 2 * sector_exponent(amax[blockIdx.y])) : acc;
 }
 
 template <class T>
@@ -241,13 +242,13 @@ void launch_rot_product(const double *vg, const double *r, double *vn, const std
     products(vg, r, vn, g);
 }
 
-void launch_col_norms(const void *W, const SectorDesc *secs, int nsec, int max_q, double *out, int f32) {
+void launch_col_norms(const void *W, const SectorDesc *secs, int nsec, int max_q, double *out, int f32, const uint32_t *amax) {
     if (nsec <= 0 || max_q <= 0) return;
     const dim3 grid(unsigned((max_q + 7) / 8), unsigned(nsec));
     if (f32)
-        k_col_norms<float><<<grid, 256, 0, ctx().stream>>>(static_cast<const float *>(W), secs, out);
+        k_col_norms<float><<<grid, 256, 0, ctx().stream>>>(static_cast<const float *>(W), secs, out, amax);
     else
-        k_col_norms<double><<<grid, 256, 0, ctx().stream>>>(static_cast<const double *>(W), secs, out);
+        k_col_norms<double><<<grid, 256, 0, ctx().stream>>>(static_cast<const double *>(W), secs, out, amax);
     count_launch();
     cuda_check(cudaGetLastError(), "column norm launch");
 }
