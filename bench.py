@@ -348,8 +348,8 @@ def timed_kinds(kinds):
 
 def svd_stages(kinds, mode, peaks_cache):
     """The sector SVDs by precision stage: each stage's time and the FLOPs its Jacobi
-    sweeps performed (sweeps x (6 p q^2 + 3 q^3) per sector; the FP64 stage of the mixed
-    path adds its Newton-Schulz and W V products), against the SGEMM / DGEMM measured in
+    sweeps performed (sweeps x (4 p q^2 + 3 q^3) per sector: the inner product and the rotation of
+    every pair), its factorisations and, on the mixed path, the refinement's products, against the SGEMM / DGEMM measured in
     this run.  The algorithmic count of the roofline object does not depend on the method;
     these figures show how busy each stage keeps its pipe."""
     import torch

@@ -443,6 +443,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
         // truncation is checked against tau all the same (svd_truncated).
         std::vector<double> discard, null2;
         bool resolve_anew = false;  // the truncation was estimated to reach below FP32's resolution
+        std::vector<LqSec> lq64;     // sectors factored in the FP64 stage
         std::vector<int> kept_cols;  // discard path: columns of each sector's compact restricted sweeps
         TruncHint &th = trunc_hint();
         if (f32 && deflate && th.allow_discard && th.max_size > 0) {
@@ -495,7 +496,6 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             gbuf = dev_alloc(size_t(std::max<int64_t>(rtot, 1)) * 8);
             cuda_check(cudaMemsetAsync(w64->p, 0, size_t(wtot) * 8, ctx().stream), "cudaMemsetAsync(work64)");
             launch_pack(static_cast<const double *>(t.data()), w64->p, dpe, dch, int64_t(chunks.size()), dsec, 0);
-            std::vector<LqSec> lq64;
             if (resolve_anew) {
                 // The truncation reaches below FP32's resolution: the values there have to be resolved
                 // in FP64 from scratch, and the factored FP64 sweeps do that from the matrix itself as
@@ -636,35 +636,49 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             auto ev = std::shared_ptr<CUevent_st>(raw, [](cudaEvent_t e) { cudaEventDestroy(e); });
             std::vector<std::pair<double, double>> pq;
             for (const SectorDesc &d : D.desc) pq.push_back({double(d.p), double(d.q)});
-            // kc (discard path): the recorded sweeps ran on kc[i] kept columns after one
-            // decoupling sweep over the whole sector, and V's kept columns took one product
-            auto flops = [ev, pq, nsec](const BufPtr &b, bool refine, const std::vector<int> &kc) {
+            // A sweep as the inner product (2 p) and the rotation of W (6 p) and of V (6 q) of every pair, whether it was
+            // rotated or not and in however many instructions.  kc (discard path): the recorded sweeps ran on kc[i]
+            // kept columns after one decoupling sweep over the whole sector, and V's kept columns took one product.
+            // others: the stage's factorisation and refinement.
+            auto flops = [ev, pq, nsec](const BufPtr &b, double others, const std::vector<int> &kc) {
                 cudaEventSynchronize(ev.get());
                 std::vector<int> sw(size_t(std::max(nsec, 1)), 0);
                 cudaMemcpy(sw.data(), b->p, size_t(nsec) * sizeof(int), cudaMemcpyDeviceToHost);
-                double f = 0.0;
+                auto sweep = [](double P, double Q) { return 4.0 * P * Q * Q + 3.0 * Q * Q * Q; };
+                double f = others;
                 for (int i = 0; i < nsec; ++i) {
                     const double P = pq[i].first, Q = pq[i].second;
                     if (kc.empty()) {
-                        f += double(sw[i]) * (6.0 * P * Q * Q + 3.0 * Q * Q * Q);
+                        f += double(sw[i]) * sweep(P, Q);
                     } else {
                         const double K = kc[size_t(i)];
-                        f += 6.0 * P * Q * Q + 3.0 * Q * Q * Q;
-                        f += double(sw[i]) * (6.0 * P * K * K + 3.0 * K * K * K) + 2.0 * Q * K * K;
+                        f += sweep(P, Q) + double(sw[i]) * sweep(P, K) + 2.0 * Q * K * K;
                     }
-                    if (refine) f += 8.0 * Q * Q * Q + 2.0 * P * Q * Q;
                 }
+                return f;
+            };
+            auto lq_flops = [](const std::vector<LqSec> &secs) {
+                double f = 0.0;
+                for (const LqSec &s : secs) f += double(s.q) * s.q * (10.0 / 3.0 * s.q + 4.0 * (s.p - s.q));
                 return f;
             };
             if (f32) {
                 BufPtr b32 = ibuf, b64 = ibuf64;
                 const std::vector<int> none, kc = kept_cols;
-                stats_defer_work(ST_JAC32, [flops, b32, none] { return flops(b32, false, none); });
-                stats_defer_work(ST_JAC64, [flops, b64, kc] { return flops(b64, true, kc); });
+                double o32 = lq_flops(lq), o64 = lq_flops(lq64);
+                if (!resolve_anew)
+                    // two upper Gram halves and W V in FP64, two corrections V E in FP32 (`plain`: whole, in FP64)
+                    for (const auto &[P, Q] : pq) {
+                        o64 += 2.0 * Q * Q * Q + 2.0 * P * Q * Q;
+                        (th.plain ? o64 : o32) += 4.0 * Q * Q * Q;
+                    }
+                stats_defer_work(ST_JAC32, [flops, b32, o32, none] { return flops(b32, o32, none); });
+                stats_defer_work(ST_JAC64, [flops, b64, o64, kc] { return flops(b64, o64, kc); });
             } else {
                 BufPtr b = ibuf;
                 const std::vector<int> none;
-                stats_defer_work(ST_JAC64, [flops, b, none] { return flops(b, false, none); });
+                const double o64 = lq_flops(lq);
+                stats_defer_work(ST_JAC64, [flops, b, o64, none] { return flops(b, o64, none); });
             }
         }
         BufPtr permbuf;
