@@ -1620,9 +1620,13 @@ int r_class(int max_p, bool f32) {
     return 0;
 }
 
-// Register slice of the FP64 kernels with exactly computed angles (launch_jacobi's `exact`); 0: longer
-// columns than they are built for.
-int exact_r_class(int max_p) { return max_p <= 128 ? 4 : max_p <= 256 ? 8 : max_p <= 512 ? 16 : 0; }
+// Register slice of the FP64 block kernels with exactly computed angles (launch_jacobi's `exact`); 0: longer
+// columns than the block kernels are built for (the scalar kernel's angles are computed exactly).
+int exact_r_class(int max_p) {
+    for (int R : {4, 8, 16, 24, 32, 48})
+        if (max_p <= 32 * R) return R;
+    return 0;
+}
 
 // Block widths the block kernel is built with for (element type, R): FP32 16 (R <= 32)
 // and 8 (R <= 64); FP64 8 and 4 (R <= 48).  The first entry is the default.
@@ -1652,6 +1656,7 @@ bool bjacobi_dispatch(const BJacobiParams<T> &P, int max_steps_per_sweep, int ma
 #define QTT_BJX(BB, RR) \
     if (B == BB && E == RR) return bjacobi_launch<T, BB, RR, true>(P, steps(BB), sum_q, vwork, vwork_bytes, stream);
         QTT_BJX(8, 4) QTT_BJX(8, 8) QTT_BJX(8, 16) QTT_BJX(4, 4) QTT_BJX(4, 8) QTT_BJX(4, 16)
+        QTT_BJX(8, 24) QTT_BJX(8, 32) QTT_BJX(8, 48) QTT_BJX(4, 24) QTT_BJX(4, 32) QTT_BJX(4, 48)
 #undef QTT_BJX
     }
 #define QTT_BJ(BB, RR)                                                                                            \

@@ -266,7 +266,7 @@ void launch_eigh_prepare(void *work, SectorDesc *sec, int nsec, int upper, int f
 // defl (optional, launch_deflation_thresholds, the work type): per sector, a column
 // whose squared norm falls to the threshold or below is set to zero and leaves the
 // sweeps (a numerically zero column); null: no deflation.
-// exact: FP64 rotation angles from FP64 square roots and divisions (columns up to 512), so that
+// exact: FP64 rotation angles from FP64 square roots and divisions, so that
 // the basis of equal singular values is that of the plain formulas; otherwise from FP32.
 // skip (optional, the work type): per sector, a pair whose squared column norms are both
 // below it is not rotated (columns the caller will discard).
