@@ -306,8 +306,8 @@ void launch_finish_on(cudaStream_t stream, const void *work, const void *rot, do
                       const SectorDesc *sec, int nsec, int max_q, double *scratch, int f32, int complete_cap = -1,
                       const void *dnorm = nullptr, int *dpos = nullptr, int *perm_out = nullptr,
                       int64_t max_elems = 0, const double *norms = nullptr);
-// Segment = one output block (rows x k row-major at dst_off) from a column-major
-// (ld x *) sector matrix at src_off: dst[i*k + j] = src[src_off + (r0 + i) + j*ld].
+// Segment = one output block (rows x k, row-major) from a sector factor's rows, a block or a run of values:
+// dst[i k + j] = src[i rs + j cs].
 struct ScatterEntry {
     const double *src;  // element (row, column) of the block: src[row rs + column cs]
     double *dst;        // row-major, k columns

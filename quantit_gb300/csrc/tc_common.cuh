@@ -44,8 +44,7 @@ static __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity)
     return false;
 }
 
-// Arrive on an mbarrier and add `bytes` to its expected transaction count.
-// Arrival on an mbarrier that also adds to its pending transaction bytes.
+// Arrival on an mbarrier that also adds `bytes` to its pending transaction count.
 static __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
