@@ -1734,7 +1734,7 @@ void jacobi_impl(T *work, T *rot, const SectorDesc *sec, const int *slot_start, 
                  int max_sweeps, int *sweeps_out, int *flags, int max_p, int64_t sum_q, void *vwork, size_t vwork_bytes,
                  const T *defl, T *dnorm, cudaStream_t stream, bool tune, const T *skip, bool exact,
                  int shear_q) {
-    if (nsec > 12 * 1024) fail(ERR_INVALID_ARGUMENT, "too many sectors for one decomposition launch");
+    check_sector_count(nsec);
     const size_t smem = size_t(2 * nsec) * sizeof(int);
     cuda_check(cudaMemsetAsync(flags, 0, size_t(nsec) * max_sweeps * sizeof(int), stream), "memset flags");
     if (jacobi_variant() != 1) {
@@ -1860,6 +1860,11 @@ void launch_sector_amax(const double *src, const PackEntry *e, const Chunk *chun
     k_sector_amax<<<unsigned(nchunks), JT, 0, ctx().stream>>>(src, e, chunks, amax);
     count_launch();
     cuda_check(cudaGetLastError(), "sector maximum kernel launch");
+}
+
+// The sweeps' per-sector tables lie in shared memory, and other kernels take sectors as rows of their grid.
+void check_sector_count(int64_t nsec) {
+    if (nsec > 12 * 1024) fail(ERR_INVALID_ARGUMENT, "too many sectors for one decomposition launch");
 }
 
 void launch_pack(const double *src, void *work, const PackEntry *e, const Chunk *chunks, int64_t nchunks,

@@ -241,6 +241,7 @@ struct PackEntry {
     int32_t sector, rows, cols, r0, c0, pad;
 };
 void launch_zero(double *p, int64_t n);
+void check_sector_count(int64_t nsec);  // refuses more sectors than one decomposition takes
 // The work / rotation buffers hold float when f32 != 0 (mixed path), else double.
 // amax (optional): per sector its largest |x| (launch_sector_amax, zero on entry there), by whose power of two
 // (sector_exponent) the sector is scaled down.

@@ -246,6 +246,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     }
     D.total_k = stot;
     const int nsec = int(D.desc.size());
+    check_sector_count(nsec);
     // The mixed path (split-precision block GEMMs) runs its SVD sweeps in FP32 first and
     // finishes them in FP64 (svd_refine.cu): the result is an FP64 SVD either way.  eigh
     // always runs in FP64.
