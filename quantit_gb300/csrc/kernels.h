@@ -4,11 +4,13 @@
 #pragma once
 #include <atomic>
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 #include <cuda_runtime.h>
 
 namespace qtt {
+struct DevBuf;  // qtt_core.h
 
 // Work over many variable-length segments is cut into chunks of at most
 // CHUNK elements that never straddle a segment; one CTA handles one chunk.
@@ -208,7 +210,9 @@ struct LqSec {
 };
 constexpr size_t LQ_SMEM_MAX = 200 * 1024;
 int lq_max_q(int f32, int nsec);
-void launch_lq(void *work, void *rot, const std::vector<LqSec> &secs, int f32);
+// Tall sectors (p >= 1.5 q) whose largest squared row norm is at most `graded` times the smallest stay as they are, Q the
+// identity: their entry in the returned buffer (an int per sector) is 0.
+std::shared_ptr<DevBuf> launch_lq(void *work, void *rot, const std::vector<LqSec> &secs, int f32, double graded);
 // FP64 refinement of an FP32 sector decomposition (mixed path): from the FP32
 // rotations rot32 (at rot_off; rot_size elements in all), vb <- the FP64-orthogonalised rotation
 // (two Newton-Schulz steps through va, with g as q x q scratch; exact: wholly in FP64 products), w1 <- w64 vb (at w_off).

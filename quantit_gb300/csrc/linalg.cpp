@@ -252,8 +252,10 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     // always runs in FP64.
     // Sectors that are LQ-preconditioned (lq.cu).  Under a truncation, from 16 columns on: svd of a
     // graded theta at D = 60 1664 -> 907 us, at D = 100 2846 -> 1383, at D = 600 35.0 -> 12.7 ms.
-    // The untruncated svd in FP64 from 48 columns on.  It also sees matrices that are not graded (bMPS.move_oc of a
-    // random state), where the factorisation saves no sweep; without it and with it, us, sectors of q columns:
+    // The untruncated svd in FP64 from 48 columns on, but tall sectors only if their row norms span a factor of 4 and
+    // more: it also sees matrices that are not graded (bMPS.move_oc of a random state), where the factorisation saves no
+    // sweep unless they are as good as square (site svd of a random state, D = 220 1731 us with it, 1570 without; D = 300
+    // 2512, 2391).  Without and with it, us, sectors of q columns:
     //            q x q, 0 / 4 / 12 decades            2q x q, 0 / 4 / 12 decades
     //   q = 48   1466, 1490  1707, 1628  2512, 1149   1429, 1467  1403, 1418  1854, 1253
     //   q = 96   3557, 3585  4542, 2939  6958, 2729   3288, 3681  3314, 3227  4732, 2921
@@ -429,7 +431,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             BufPtr tmp = dev_alloc(size_t(std::max<int64_t>(wtot, 1)) * es);
             launch_warm_apply(W, D.rot->p, tmp->p, upload_vec(wdesc), int(wdesc.size()), ntiles, f32);
         }
-        launch_lq(W, D.rot->p, lq, f32);
+        const BufPtr lq_ran = launch_lq(W, D.rot->p, lq, f32, trunc_hint().active ? 0.0 : 16.0);
         launch_jacobi(W, D.rot->p, dsec, dslots, nsec, max_steps, max_sweeps, sweeps, flags, f32, max_p, stot,
                       vwork->p, vb, deflate ? thr->p : nullptr, deflate ? dnorm->p : nullptr, nullptr,
                       trunc_hint().plain, shear_q);
@@ -445,6 +447,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
         std::vector<double> discard, null2;
         bool resolve_anew = false;  // the truncation was estimated to reach below FP32's resolution
         std::vector<LqSec> lq64;     // sectors factored in the FP64 stage
+        BufPtr lq64_ran;
         std::vector<int> kept_cols;  // discard path: columns of each sector's compact restricted sweeps
         TruncHint &th = trunc_hint();
         if (f32 && deflate && th.allow_discard && th.max_size > 0) {
@@ -534,7 +537,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                               skip, th.plain, shear_q);
             };
             if (discard.empty()) {
-                launch_lq(w1->p, vbuf->p, lq64, 0);
+                lq64_ran = launch_lq(w1->p, vbuf->p, lq64, 0, 0.0);
                 fp64_sweeps(max_sweeps, thr64 ? thr64->p : nullptr, nullptr);
             } else {
                 // one sweep decouples the columns (pairs of two discarded columns stay as they
@@ -658,28 +661,34 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                 }
                 return f;
             };
-            auto lq_flops = [](const std::vector<LqSec> &secs) {
+            auto lq_flops = [ev](const std::vector<LqSec> &secs, const BufPtr &ran) {
+                if (secs.empty()) return 0.0;
+                cudaEventSynchronize(ev.get());
+                std::vector<int> panels(secs.size(), 0);
+                cudaMemcpy(panels.data(), ran->p, secs.size() * sizeof(int), cudaMemcpyDeviceToHost);
                 double f = 0.0;
-                for (const LqSec &s : secs) f += double(s.q) * s.q * (10.0 / 3.0 * s.q + 4.0 * (s.p - s.q));
+                for (size_t i = 0; i < secs.size(); ++i) {
+                    const double P = secs[i].p, Q = secs[i].q;
+                    if (panels[i] > 0) f += Q * Q * (10.0 / 3.0 * Q + 4.0 * (P - Q));
+                }
                 return f;
             };
             if (f32) {
                 BufPtr b32 = ibuf, b64 = ibuf64;
                 const std::vector<int> none, kc = kept_cols;
-                double o32 = lq_flops(lq), o64 = lq_flops(lq64);
+                double o32 = 0.0, o64 = 0.0;
                 if (!resolve_anew)
                     // two upper Gram halves and W V in FP64, two corrections V E in FP32 (`plain`: whole, in FP64)
                     for (const auto &[P, Q] : pq) {
                         o64 += 2.0 * Q * Q * Q + 2.0 * P * Q * Q;
                         (th.plain ? o64 : o32) += 4.0 * Q * Q * Q;
                     }
-                stats_defer_work(ST_JAC32, [flops, b32, o32, none] { return flops(b32, o32, none); });
-                stats_defer_work(ST_JAC64, [flops, b64, o64, kc] { return flops(b64, o64, kc); });
+                stats_defer_work(ST_JAC32, [=] { return flops(b32, o32 + lq_flops(lq, lq_ran), none); });
+                stats_defer_work(ST_JAC64, [=] { return flops(b64, o64 + lq_flops(lq64, lq64_ran), kc); });
             } else {
                 BufPtr b = ibuf;
                 const std::vector<int> none;
-                const double o64 = lq_flops(lq);
-                stats_defer_work(ST_JAC64, [flops, b, o64, none] { return flops(b, o64, none); });
+                stats_defer_work(ST_JAC64, [=] { return flops(b, lq_flops(lq, lq_ran), none); });
             }
         }
         BufPtr permbuf;

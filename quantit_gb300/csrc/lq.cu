@@ -36,7 +36,8 @@ struct LqParams {
     const LqSec *secs;
     const int *order;  // rows of W by falling norm
     int *next;         // per panel: update items claimed (zero on entry)
-    int nsec, panels, chunk, max_q;
+    const int *np;     // panels of each sector (0: left as it is), then the most of any
+    int nsec, chunk, max_q;
 };
 
 __device__ __forceinline__ double lsum(double v) {
@@ -215,7 +216,9 @@ __global__ void __launch_bounds__(LT) k_lq(LqParams<T> P) {
     __shared__ int item_sh;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // first sorted row beyond panel k's and, where there is one, panel k + 1's
+    // (of a sector that is factored)
     auto first_row = [&](const LqSec &s, int k) { return min(s.q, (k + 1 + (k + 1 < panels_of(s.q))) * NB); };
+    const int panels = P.np[P.nsec];
     auto vbuf = [&](const LqSec &s, int k) { return P.v + s.v_off + int64_t(k & 1) * (NB * (s.q + NB)); };
 
     // the panel k of sector s, its rows in xs; leaves reflectors and T in the panel's buffer
@@ -240,7 +243,7 @@ __global__ void __launch_bounds__(LT) k_lq(LqParams<T> P) {
 
     for (int i = blockIdx.x; i < P.nsec; i += gridDim.x) {
         const LqSec s = P.secs[i];
-        if (panels_of(s.q) < 1) continue;
+        if (P.np[i] < 1) continue;
         const int nr = min(NB, s.q);
         if (warp < nr) {
             const T *x = P.x + s.x_off + int64_t(P.order[s.o_off + warp]) * s.q;
@@ -250,12 +253,12 @@ __global__ void __launch_bounds__(LT) k_lq(LqParams<T> P) {
         factor(s, 0, buf, s.q);
     }
     grid.sync();
-    for (int k = 0; k < P.panels; ++k) {
+    for (int k = 0; k < panels; ++k) {
         const int j = k * NB;
         // owners: panel k on the rows of panel k + 1, then that panel's factorisation
         for (int i = blockIdx.x; i < P.nsec; i += gridDim.x) {
             const LqSec s = P.secs[i];
-            if (k + 1 >= panels_of(s.q)) continue;
+            if (k + 1 >= P.np[i]) continue;
             const int len = s.q - j, nr = min(NB, s.q - j - NB);
             load_v(s, k);
             T *x = buf + warp * len;
@@ -282,7 +285,7 @@ __global__ void __launch_bounds__(LT) k_lq(LqParams<T> P) {
                 int n = 0;
                 if (i < P.nsec) {
                     const LqSec &s = P.secs[i];
-                    if (k < panels_of(s.q)) n = (s.p - first_row(s, k) + s.q + P.chunk - 1) / P.chunk;
+                    if (k < P.np[i]) n = (s.p - first_row(s, k) + s.q + P.chunk - 1) / P.chunk;
                 }
                 int v = n;
                 for (int o = 1; o < 32; o <<= 1) {
@@ -393,26 +396,38 @@ __global__ void __launch_bounds__(256) k_lq_norms(const T *__restrict__ x, const
     if (lane == 0) norms[s.o_off + r] = d;
 }
 
-// order <- the rows by falling norm: ranks in bit order (a permutation also with NaN).
+// order <- the rows by falling norm: ranks in bit order (a permutation also with NaN).  np <- the sector's panels, none
+// if it is tall (p >= 1.5 q) and its largest squared row norm is at most `graded` times the smallest.
 __global__ void __launch_bounds__(256) k_lq_rank(const double *__restrict__ norms, const LqSec *__restrict__ secs,
-                                                 int *__restrict__ order) {
+                                                 int *__restrict__ order, int *__restrict__ np, double graded) {
     const LqSec s = secs[blockIdx.y];
     const int r = blockIdx.x * 256 + threadIdx.x;
     __shared__ long long keys[256];
     const long long mine = r < s.p ? __double_as_longlong(norms[s.o_off + r]) : 0;
     int rank = 0;
+    long long low = __double_as_longlong(norms[s.o_off]), high = low;
     for (int b = 0; b < s.p; b += 256) {
         __syncthreads();
         if (b + int(threadIdx.x) < s.p) keys[threadIdx.x] = __double_as_longlong(norms[s.o_off + b + threadIdx.x]);
         __syncthreads();
         const int n = min(256, s.p - b);
-        for (int i = 0; i < n; ++i) rank += keys[i] > mine || (keys[i] == mine && b + i < r);
+        for (int i = 0; i < n; ++i) {
+            rank += keys[i] > mine || (keys[i] == mine && b + i < r);
+            low = min(low, keys[i]);
+            high = max(high, keys[i]);
+        }
+    }
+    if (r == 0) {
+        const bool left = 2 * s.p >= 3 * s.q && !(__longlong_as_double(high) > graded * __longlong_as_double(low));
+        const int n = left ? 0 : panels_of(s.q);
+        np[blockIdx.y] = n;
+        atomicMax(np + gridDim.y, n);
     }
     if (r < s.p) order[s.o_off + rank] = r;
 }
 
 template <class T>
-void lq_impl(T *work, T *rot, const std::vector<LqSec> &host) {
+BufPtr lq_impl(T *work, T *rot, const std::vector<LqSec> &host, double graded) {
     std::vector<LqSec> secs = host;
     int64_t xs = 0, vs = 0, os = 0;
     int max_q = 0, max_p = 0;
@@ -428,22 +443,23 @@ void lq_impl(T *work, T *rot, const std::vector<LqSec> &host) {
     }
     const int nsec = int(secs.size()), panels = (max_q - 1 + NB - 1) / NB;
     const cudaStream_t st = ctx().stream;
-    // one buffer: vectors, reflectors, norms, order, counters
+    // one buffer for vectors, reflectors, norms and order, one for the panels and the counters
     const size_t xb = (size_t(xs) * sizeof(T) + 255) & ~size_t(255), vb = (size_t(vs) * sizeof(T) + 255) & ~size_t(255);
     const size_t nb = (size_t(os) * 8 + 255) & ~size_t(255), ob = (size_t(os) * 4 + 255) & ~size_t(255);
-    BufPtr buf = dev_alloc(xb + vb + nb + ob + size_t(panels + 1) * 4);
+    const size_t counters = size_t(panels + 1 + nsec + 1) * 4;
+    BufPtr buf = dev_alloc(xb + vb + nb + ob), ints = dev_alloc(counters);
     char *p = static_cast<char *>(buf->p);
     T *x = reinterpret_cast<T *>(p);
     double *norms = reinterpret_cast<double *>(p + xb + vb);
     int *order = reinterpret_cast<int *>(p + xb + vb + nb);
-    int *next = reinterpret_cast<int *>(p + xb + vb + nb + ob);
-    cuda_check(cudaMemsetAsync(next, 0, size_t(panels + 1) * 4, st), "cudaMemsetAsync(LQ counters)");
+    int *np = static_cast<int *>(ints->p), *next = np + nsec + 1;
+    cuda_check(cudaMemsetAsync(np, 0, counters, st), "cudaMemsetAsync(LQ counters)");
     const LqSec *dsecs = upload_vec(secs);
     const int tiles = ((max_p + 31) / 32 + (max_q + 31) / 32) * ((max_q + 31) / 32);
     const dim3 mv(unsigned(std::min(tiles, 4096)), unsigned(nsec));
     k_lq_move<T><<<mv, 256, 0, st>>>(work, rot, x, dsecs, 0);
     k_lq_norms<T><<<dim3(unsigned((max_p + 7) / 8), unsigned(nsec)), 256, 0, st>>>(x, dsecs, norms);
-    k_lq_rank<<<dim3(unsigned((max_p + 255) / 256), unsigned(nsec)), 256, 0, st>>>(norms, dsecs, order);
+    k_lq_rank<<<dim3(unsigned((max_p + 255) / 256), unsigned(nsec)), 256, 0, st>>>(norms, dsecs, order, np, graded);
     const size_t smem = (size_t(2) * NB * max_q + 2 * NB * NB + NB) * sizeof(T) + size_t(nsec + 1) * sizeof(int);
     static std::atomic<uint64_t> attr{0};
     once_per_device(attr, [] {
@@ -465,7 +481,7 @@ void lq_impl(T *work, T *rot, const std::vector<LqSec> &host) {
     P.order = order;
     P.next = next;
     P.nsec = nsec;
-    P.panels = panels;
+    P.np = np;
     P.chunk = int(std::max<int64_t>(8, (vectors + grid - 1) / grid / 8 * 8));
     P.max_q = max_q;
     void *args[] = {&P};
@@ -473,6 +489,7 @@ void lq_impl(T *work, T *rot, const std::vector<LqSec> &host) {
     k_lq_move<T><<<mv, 256, 0, st>>>(work, rot, x, dsecs, 1);
     count_launch(5);
     cuda_check(cudaGetLastError(), "LQ kernel launch");
+    return ints;
 }
 }  // namespace
 
@@ -482,12 +499,10 @@ int lq_max_q(int f32, int nsec) {
     return fixed >= LQ_SMEM_MAX ? 0 : int((LQ_SMEM_MAX - fixed) / (2 * NB * es));
 }
 
-void launch_lq(void *work, void *rot, const std::vector<LqSec> &secs, int f32) {
-    if (secs.empty()) return;
-    if (f32)
-        lq_impl(static_cast<float *>(work), static_cast<float *>(rot), secs);
-    else
-        lq_impl(static_cast<double *>(work), static_cast<double *>(rot), secs);
+BufPtr launch_lq(void *work, void *rot, const std::vector<LqSec> &secs, int f32, double graded) {
+    if (secs.empty()) return nullptr;
+    return f32 ? lq_impl(static_cast<float *>(work), static_cast<float *>(rot), secs, graded)
+               : lq_impl(static_cast<double *>(work), static_cast<double *>(rot), secs, graded);
 }
 
 }  // namespace qtt

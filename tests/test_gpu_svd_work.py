@@ -33,10 +33,11 @@ def factored(mats):
 
 
 def test_plain_fp64():
+    """Sectors of 48 columns and more are factored, tall ones (1.5 : 1 and more) if their rows are graded."""
     rng = np.random.default_rng(96)
-    small, wide = rng.standard_normal((30, 20)), rng.standard_normal((70, 90))
-    work, n = booked([small, wide], "f64")
-    assert work == [0.0, pytest.approx(sweeps([small, wide], n[1]) + factored([wide]))]
+    mats = [rng.standard_normal((30, 20)), rng.standard_normal((90, 60)), rng.standard_normal((60, 89)), graded(rng, 70, 120, 6)]
+    work, n = booked(mats, "f64")
+    assert work == [0.0, pytest.approx(sweeps(mats, n[1]) + factored(mats[2:]))]
 
 
 def test_plain_split():
