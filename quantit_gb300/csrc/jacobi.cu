@@ -119,34 +119,31 @@ __device__ __forceinline__ void rr_pair(int qp, int k, int slot, int &a, int &b)
     }
 }
 
-// Per sector the largest |x| of its blocks, as the high word of its bits (zero on entry).
-__global__ void __launch_bounds__(JT) k_sector_amax(const double *__restrict__ src, const PackEntry *__restrict__ ents,
-                                                    const Chunk *__restrict__ chunks, uint32_t *__restrict__ amax) {
-    const Chunk ch = chunks[blockIdx.x];
-    const PackEntry e = ents[ch.seg];
-    uint32_t m = 0;
-    for (int i = threadIdx.x; i < ch.len; i += blockDim.x)
-        m = max(m, uint32_t(__double2hiint(src[e.src_off + ch.start + i])) & 0x7FFFFFFFu);
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(amax + e.sector, m);
-}
-
-// amax (k_sector_amax's, or null): each sector is brought to magnitude 1 by a power of two on the way. FP32's
-// sweeps form squares: of a sector of 1e-20 those are subnormal or zero, and its columns would stay unresolved.
+// FP64 with amax: takes the largest |x| of each sector there (the high word of its bits, zero on entry).  FP32 with
+// such maxima: each sector is brought to magnitude 1 by a power of two on the way.  FP32's sweeps form squares: of
+// a sector of 1e-20 those are subnormal or zero, and its columns would stay unresolved.
 template <class T>
 __global__ void k_pack(const double *__restrict__ src, T *__restrict__ work, const PackEntry *__restrict__ ents,
                        const Chunk *__restrict__ chunks, const SectorDesc *__restrict__ secs,
-                       const uint32_t *__restrict__ amax) {
+                       uint32_t *__restrict__ amax) {
     const Chunk ch = chunks[blockIdx.x];
     const PackEntry e = ents[ch.seg];
     const SectorDesc sd = secs[e.sector];
-    const double scale = amax ? ldexp(1.0, -sector_exponent(amax[e.sector])) : 1.0;
+    const bool scaled = sizeof(T) == 4 && amax;
+    const double scale = scaled ? ldexp(1.0, -sector_exponent(amax[e.sector])) : 1.0;
+    uint32_t m = 0;
     for (int i = threadIdx.x; i < ch.len; i += blockDim.x) {
         int64_t k = ch.start + i;
         int r = int(k / e.cols), c = int(k - int64_t(r) * e.cols);
         int ar = e.r0 + r, ac = e.c0 + c;  // position in A (m x n)
         int64_t w = sd.trans ? (int64_t(ac) + int64_t(ar) * sd.p) : (int64_t(ar) + int64_t(ac) * sd.p);
-        work[sd.w_off + w] = T(amax ? src[e.src_off + k] * scale : src[e.src_off + k]);
+        const double x = src[e.src_off + k];
+        work[sd.w_off + w] = T(scaled ? x * scale : x);
+        m = max(m, uint32_t(__double2hiint(x)) & 0x7FFFFFFFu);
+    }
+    if (sizeof(T) == 8 && amax) {
+        m = __reduce_max_sync(0xffffffffu, m);
+        if ((threadIdx.x & 31) == 0 && m) atomicMax(amax + e.sector, m);
     }
 }
 
@@ -1855,20 +1852,13 @@ void finish_impl(const T *work, const T *rot, double *U, double *V, double *s, c
 }
 }  // namespace
 
-void launch_sector_amax(const double *src, const PackEntry *e, const Chunk *chunks, int64_t nchunks, uint32_t *amax) {
-    if (nchunks <= 0) return;
-    k_sector_amax<<<unsigned(nchunks), JT, 0, ctx().stream>>>(src, e, chunks, amax);
-    count_launch();
-    cuda_check(cudaGetLastError(), "sector maximum kernel launch");
-}
-
 // The sweeps' per-sector tables lie in shared memory, and other kernels take sectors as rows of their grid.
 void check_sector_count(int64_t nsec) {
     if (nsec > 12 * 1024) fail(ERR_INVALID_ARGUMENT, "too many sectors for one decomposition launch");
 }
 
 void launch_pack(const double *src, void *work, const PackEntry *e, const Chunk *chunks, int64_t nchunks,
-                 const SectorDesc *sec, int f32, const uint32_t *amax) {
+                 const SectorDesc *sec, int f32, uint32_t *amax) {
     if (nchunks <= 0) return;
     if (f32)
         k_pack<float><<<unsigned(nchunks), JT, 0, ctx().stream>>>(src, static_cast<float *>(work), e, chunks, sec, amax);

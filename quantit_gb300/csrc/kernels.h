@@ -247,15 +247,14 @@ struct PackEntry {
 void launch_zero(double *p, int64_t n);
 void check_sector_count(int64_t nsec);  // refuses more sectors than one decomposition takes
 // The work / rotation buffers hold float when f32 != 0 (mixed path), else double.
-// amax (optional): per sector its largest |x| (launch_sector_amax, zero on entry there), by whose power of two
-// (sector_exponent) the sector is scaled down.
-void launch_sector_amax(const double *src, const PackEntry *e, const Chunk *chunks, int64_t nchunks, uint32_t *amax);
+// amax (optional): packing to FP64 takes the largest |x| of each sector there (zero on entry); packing to FP32 scales each
+// sector down by the power of two of its own (sector_exponent).
 __host__ __device__ inline int sector_exponent(uint32_t high_word) {
     const int e = int(high_word >> 20);
     return e == 0 || e == 0x7FF ? 0 : e - 1023;
 }
 void launch_pack(const double *src, void *work, const PackEntry *e, const Chunk *chunks, int64_t nchunks,
-                 const SectorDesc *sec, int f32, const uint32_t *amax = nullptr);
+                 const SectorDesc *sec, int f32, uint32_t *amax = nullptr);
 // eigh: symmetrise W from one triangle, then shift the diagonal by the sector's
 // Frobenius norm (written back into sec[s].shift) so the matrix is positive definite.
 void launch_eigh_prepare(void *work, SectorDesc *sec, int nsec, int upper, int f32);

@@ -382,12 +382,16 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
     const BufPtr tables = upload_many({table(D.desc, desc_table), table(pe, dpe), table(chunks, dch), table(slots, dslots),
                                        table(zeros, amax)});
     SectorDesc *dsec = const_cast<SectorDesc *>(desc_table);  // (eigh writes its shifts there)
+    BufPtr w64;  // mixed path: the FP64 sector matrices
     {
-        StatScope sc(ST_PACK, (f32 ? 2.5 : 2.0) * 8.0 * double(packed));
-        if (f32)
-            launch_sector_amax(static_cast<const double *>(t.data()), dpe, dch, int64_t(chunks.size()),
-                               const_cast<uint32_t *>(amax));
-        launch_pack(static_cast<const double *>(t.data()), W, dpe, dch, int64_t(chunks.size()), dsec, f32, amax);
+        StatScope sc(ST_PACK, (f32 ? 3.5 : 2.0) * 8.0 * double(packed));
+        uint32_t *top = const_cast<uint32_t *>(amax);
+        if (f32) {
+            w64 = dev_alloc(size_t(std::max<int64_t>(wtot, 1)) * 8);
+            cuda_check(cudaMemsetAsync(w64->p, 0, size_t(wtot) * 8, ctx().stream), "cudaMemsetAsync(work64)");
+            launch_pack(static_cast<const double *>(t.data()), w64->p, dpe, dch, int64_t(chunks.size()), dsec, 0, top);
+        }
+        launch_pack(static_cast<const double *>(t.data()), W, dpe, dch, int64_t(chunks.size()), dsec, f32, top);
     }
     if (mode == 1) launch_eigh_prepare(W, dsec, nsec, upper, f32);
     const int max_sweeps = 80;
@@ -436,7 +440,7 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
                       vwork->p, vb, deflate ? thr->p : nullptr, deflate ? dnorm->p : nullptr, nullptr,
                       trunc_hint().plain, shear_q);
         const void *fw = W, *fr = D.rot->p;
-        BufPtr w64, w1, va, vbuf, gbuf, ibuf64;
+        BufPtr w1, va, vbuf, gbuf, ibuf64;
         // The FP32 sweeps resolved every value above FP32 resolution.  When the truncation
         // that follows keeps only values above 8 eps32 ||W_s|| (its threshold estimated from
         // the FP32 column norms with truncate's own rule), the FP64 sweeps may leave the
@@ -493,13 +497,10 @@ void run_decomp(const BT &t, Decomp &D, int mode, int upper) {
             StatScope sc64(ST_SVD64, 0.0);
             // FP64 stage: the FP64 sector matrices, the FP32 rotations made orthogonal in
             // FP64, W1 = W V, and FP64 Jacobi sweeps from that warm start
-            w64 = dev_alloc(size_t(std::max<int64_t>(wtot, 1)) * 8);
             w1 = dev_alloc(size_t(std::max<int64_t>(wtot, 1)) * 8);
             va = dev_alloc(size_t(std::max<int64_t>(rtot, 1)) * 8);
             vbuf = dev_alloc(size_t(std::max<int64_t>(rtot, 1)) * 8);
             gbuf = dev_alloc(size_t(std::max<int64_t>(rtot, 1)) * 8);
-            cuda_check(cudaMemsetAsync(w64->p, 0, size_t(wtot) * 8, ctx().stream), "cudaMemsetAsync(work64)");
-            launch_pack(static_cast<const double *>(t.data()), w64->p, dpe, dch, int64_t(chunks.size()), dsec, 0);
             if (resolve_anew) {
                 // The truncation reaches below FP32's resolution: the values there have to be resolved
                 // in FP64 from scratch, and the factored FP64 sweeps do that from the matrix itself as
